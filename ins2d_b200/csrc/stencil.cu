@@ -350,9 +350,9 @@ struct YRowsN {
 using YRows = YRowsN<RUN>;
 
 template <int NR>
-__device__ __forceinline__ void stage_yrows(const DevOps &P, int j0, YRowsN<NR> &Y) {
+__device__ __forceinline__ void stage_yrows(const DevOps &P, int j0, YRowsN<NR> &Y, int rows = NR) {
   const int t = threadIdx.x + blockDim.x * threadIdx.y;
-  if (t <= NR) {
+  if (t <= rows) {
     const int r = j0 + t;
     Y.auy0[t] = __ldg(P.rAUY.w0 + r);
     Y.auy1[t] = __ldg(P.rAUY.w1 + r);
@@ -365,7 +365,7 @@ __device__ __forceinline__ void stage_yrows(const DevOps &P, int j0, YRowsN<NR> 
     Y.svy0[t] = __ldg(P.rSVY.w0 + r);
     Y.svy1[t] = __ldg(P.rSVY.w1 + r);
   }
-  if (t < NR) {
+  if (t < rows) {
     const int j = j0 + t;
     Y.hy[t] = __ldg(P.hy + j);
     Y.rhy[t] = __ldg(P.rhy + j);
@@ -888,14 +888,16 @@ __global__ void __launch_bounds__(kTileThreads, INS2D_TILE_MINB)
     tile_v<S, MODE, TV, NP>(P, T, e, i, i0, j0, ja, jb, Y);
 }
 
-// one WX x RUN tile (bx, by): u walkers in warps with threadIdx.y == 0, v in 1
+// rows [z rows, (z + 1) rows) of one WX x RUN tile (bx, by): u walkers in
+// warps with threadIdx.y == 0, v in 1
 template <typename S, typename TV>
-__device__ __forceinline__ void tile_fast(const DevOps &P, const TV *__restrict__ V, const Epi &e, int bx, int by) {
+__device__ __forceinline__ void tile_fast(const DevOps &P, const TV *__restrict__ V, const Epi &e, int bx, int by,
+                                          int z, int rows) {
   __shared__ YRows Y;
   const int i = bx * WX + threadIdx.x;
-  const int j0 = by * RUN, j1 = j0 + RUN;
+  const int jt = by * RUN, j0 = jt + z * rows, j1 = min(j0 + rows, jt + RUN);
   const TV *u = V, *v = V + P.Nu;
-  stage_yrows(P, j0, Y);
+  stage_yrows(P, j0, Y, j1 - j0);
   __syncthreads();
   if (threadIdx.y == 0)
     fast_u<S, TV>(P, u, v, e, i, j0, j1, Y);
@@ -904,9 +906,9 @@ __device__ __forceinline__ void tile_fast(const DevOps &P, const TV *__restrict_
 }
 template <typename S, typename TV>
 __device__ __forceinline__ void tile_generic(const DevOps &P, const TV *__restrict__ V, const Epi &e, int bx,
-                                             int by) {
+                                             int by, int z, int rows) {
   const int i = bx * WX + threadIdx.x;
-  const int j0 = by * RUN, j1 = j0 + RUN;
+  const int j0 = by * RUN + z * rows, j1 = min(j0 + rows, (by + 1) * RUN);
   const TV *u = V, *v = V + P.Nu;
   if (threadIdx.y == 0)
     walk_u<S, TV>(P, u, v, e, i, j0, j1);
@@ -916,17 +918,17 @@ __device__ __forceinline__ void tile_generic(const DevOps &P, const TV *__restri
 
 template <typename S, typename TV>
 __global__ void __launch_bounds__(WX * 2, INS2D_WALK_MINB) k_walk_fast(const __grid_constant__ DevOps P, const TV *__restrict__ V,
-                                                      const __grid_constant__ Epi e) {
-  tile_fast<S, TV>(P, V, e, P.fbx0 + blockIdx.x, P.fby0 + blockIdx.y);
+                                                      const __grid_constant__ Epi e, int rows) {
+  tile_fast<S, TV>(P, V, e, P.fbx0 + blockIdx.x, P.fby0 + blockIdx.y, blockIdx.z, rows);
 }
 
 template <typename S, typename TV>
 __global__ void __launch_bounds__(WX * 2) k_walk(const __grid_constant__ DevOps P, const TV *__restrict__ V,
-                                                 const __grid_constant__ Epi e) {
+                                                 const __grid_constant__ Epi e, int rows) {
   if ((int)blockIdx.x >= P.fbx0 && (int)blockIdx.x < P.fbx1 && (int)blockIdx.y >= P.fby0 &&
       (int)blockIdx.y < P.fby1)
     return;  // interior tile: handled by k_walk_fast / k_walk_tile
-  tile_generic<S, TV>(P, V, e, blockIdx.x, blockIdx.y);
+  tile_generic<S, TV>(P, V, e, blockIdx.x, blockIdx.y, blockIdx.z, rows);
 }
 
 // --- ensembles: one launch over the tiles of all member grids ------------------
@@ -961,7 +963,7 @@ __device__ __forceinline__ const double *ens_epi(const EnsMemberD &M, const EnsW
 
 template <typename S, bool FAST>
 __device__ __forceinline__ void walk_ens_body(const EnsMemberD *__restrict__ mem, const int4 *__restrict__ work,
-                                              const EnsWalk &w) {
+                                              const EnsWalk &w, int rows) {
   __shared__ __align__(16) DevOps sP;
   __shared__ __align__(16) Epi sE;
   __shared__ const double *sV;
@@ -971,22 +973,23 @@ __device__ __forceinline__ void walk_ens_body(const EnsMemberD *__restrict__ mem
   if (threadIdx.x == 0 && threadIdx.y == 0) sV = ens_epi(M, w, sE);
   __syncthreads();
   if (FAST)
-    tile_fast<S, double>(sP, sV, sE, it.y, it.z);
+    tile_fast<S, double>(sP, sV, sE, it.y, it.z, blockIdx.y, rows);
   else
-    tile_generic<S, double>(sP, sV, sE, it.y, it.z);
+    tile_generic<S, double>(sP, sV, sE, it.y, it.z, blockIdx.y, rows);
 }
 
 template <typename S>
 __global__ void __launch_bounds__(WX * 2, INS2D_WALK_MINB) k_walk_ens_fast(const EnsMemberD *__restrict__ mem,
                                                                           const int4 *__restrict__ work,
-                                                                          const __grid_constant__ EnsWalk w) {
-  walk_ens_body<S, true>(mem, work, w);
+                                                                          const __grid_constant__ EnsWalk w,
+                                                                          int rows) {
+  walk_ens_body<S, true>(mem, work, w, rows);
 }
 template <typename S>
 __global__ void __launch_bounds__(WX * 2) k_walk_ens_gen(const EnsMemberD *__restrict__ mem,
                                                          const int4 *__restrict__ work,
-                                                         const __grid_constant__ EnsWalk w) {
-  walk_ens_body<S, false>(mem, work, w);
+                                                         const __grid_constant__ EnsWalk w, int rows) {
+  walk_ens_body<S, false>(mem, work, w, rows);
 }
 
 // MODE 0 and 2 with the count of earlier stages as a template argument (0..3
@@ -1007,6 +1010,30 @@ void launch_tile(const DevOps &P, const TV *V, const Epi &e, cudaStream_t s) {
   }
 }
 
+// Rows per thread of a table or global-memory walker launch of `tiles` tiles.
+// A walked row is a serial chain of dependent loads (table column, field
+// value; 1.7 us per row from cold caches), so a launch with few tiles is bound
+// by rows x that latency, not by bandwidth: the rows of a tile are split over
+// blocks (gridDim.z) until the launch has about five blocks of four warps per
+// SM (INS2D_WALK_FILL); a split costs one more face evaluation per run.
+// Measured on B200, whole RK44 steps, 32 rows against this rule: 64^2 cavity
+// 0.419 -> 0.284 ms, 40^2 periodic step on host arrays 0.379 -> 0.225 ms,
+// stretched 512^2 channel 1.90 -> 1.76 ms, 24-member ensemble 1.64 -> 1.52 ms.
+// Shortest run 1, 2, 4 rows: 0.278, 0.284, 0.294 ms (cavity), 1.768, 1.760,
+// 1.799 ms (channel); 2 kept.  Four times the fill: no gain (ensemble 1.54 ms).
+#ifndef INS2D_WALK_MINROWS
+#define INS2D_WALK_MINROWS 2
+#endif
+#ifndef INS2D_WALK_FILL
+#define INS2D_WALK_FILL 740
+#endif
+static_assert((RUN & (RUN - 1)) == 0, "tiles are split into equal runs");
+int walk_rows(long long tiles) {
+  int r = RUN;
+  while (r > INS2D_WALK_MINROWS && tiles * (RUN / r) < INS2D_WALK_FILL) r >>= 1;
+  return r;
+}
+
 template <typename S, typename TV>
 void launch_walk_t(const DevOps &P, const TV *V, const Epi &e, cudaStream_t s) {
   const int nx = P.Nux > P.Nvx ? P.Nux : P.Nvx;
@@ -1024,10 +1051,15 @@ void launch_walk_t(const DevOps &P, const TV *V, const Epi &e, cudaStream_t s) {
       else
         launch_tile<S, 1, TV>(P, V, e, s);  // residual and F
     } else {
-      k_walk_fast<S, TV><<<gf, dim3(WX, 2), 0, s>>>(P, V, e);
+      const int r = walk_rows((long long)gf.x * gf.y);
+      k_walk_fast<S, TV><<<dim3(gf.x, gf.y, RUN / r), dim3(WX, 2), 0, s>>>(P, V, e, r);
     }
   }
-  if (!P.all_fast) k_walk<S, TV><<<g, dim3(WX, 2), 0, s>>>(P, V, e);
+  if (!P.all_fast) {
+    const long long inner = has_fast ? (long long)(P.fbx1 - P.fbx0) * (P.fby1 - P.fby0) : 0;
+    const int r = walk_rows((long long)g.x * g.y - inner);
+    k_walk<S, TV><<<dim3(g.x, g.y, RUN / r), dim3(WX, 2), 0, s>>>(P, V, e, r);
+  }
 }
 
 // FP64 contexts: FP64 fields, FP64 arithmetic; FP32-stencil contexts: FP32
@@ -1102,17 +1134,18 @@ void walk_tiles(const DevOps &P, int member, std::vector<int4> &fast, std::vecto
 
 void launch_walk_ens(const EnsMemberD *mem, const int4 *fast, int nfast, const int4 *gen, int ngen, const EnsWalk &w,
                      bool fp32, cudaStream_t s) {
+  const int rf = walk_rows(nfast), rg = walk_rows(ngen);
   if (nfast > 0) {
     if (fp32)
-      k_walk_ens_fast<float><<<nfast, dim3(WX, 2), 0, s>>>(mem, fast, w);
+      k_walk_ens_fast<float><<<dim3(nfast, RUN / rf), dim3(WX, 2), 0, s>>>(mem, fast, w, rf);
     else
-      k_walk_ens_fast<double><<<nfast, dim3(WX, 2), 0, s>>>(mem, fast, w);
+      k_walk_ens_fast<double><<<dim3(nfast, RUN / rf), dim3(WX, 2), 0, s>>>(mem, fast, w, rf);
   }
   if (ngen > 0) {
     if (fp32)
-      k_walk_ens_gen<float><<<ngen, dim3(WX, 2), 0, s>>>(mem, gen, w);
+      k_walk_ens_gen<float><<<dim3(ngen, RUN / rg), dim3(WX, 2), 0, s>>>(mem, gen, w, rg);
     else
-      k_walk_ens_gen<double><<<ngen, dim3(WX, 2), 0, s>>>(mem, gen, w);
+      k_walk_ens_gen<double><<<dim3(ngen, RUN / rg), dim3(WX, 2), 0, s>>>(mem, gen, w, rg);
   }
 }
 
