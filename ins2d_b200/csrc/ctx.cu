@@ -157,6 +157,28 @@ const double *upload_vec(ins2d_ctx *c, const std::vector<double> &v) {
   return d;
 }
 
+// the separable inverse of c's pressure matrix (fdm_host.hpp) into D
+void upload_fdm(ins2d_ctx *c, FdmD &D) {
+  const FdmTri T = fdm_tri(c->H.TX, c->H.hx, c->H.TY, c->H.hy);
+  D.nx = c->H.Npx;
+  D.ny = c->H.Npy;
+  D.nsm = c->P.nsm;
+  D.nm = T.nm;
+  D.n = T.n;
+  D.xmodes = T.xmodes ? 1 : 0;
+  D.Q = upload_vec(c, T.Q);
+  D.piv = upload_vec(c, T.piv);
+  D.e = upload_vec(c, T.e);
+  D.h = upload_vec(c, T.h);
+  if (!T.g.empty()) {
+    D.g = upload_vec(c, T.g);
+    D.cr = upload_vec(c, T.cr);
+  }
+  D.null_mode = T.null_mode;
+  D.hsum = T.hsum;
+  D.t = dalloc<double>(c, (size_t)c->P.Np);
+}
+
 // Layout of the boundary-value blob: {name, length}.
 struct BcSlot {
   const double **dst;
@@ -334,7 +356,7 @@ int solve_pcg_graph(ins2d_ctx *c, const double *f, double *dp, bool accumulate, 
       [&](cudaStream_t bs, cudaGraphConditionalHandle h) {
         if (c->use_fdm) {
           pcg_iterations_fdm(c->P, c->fdm, c->pcg, chunk, bs);
-          c->launches[INS2D_PROF_POISSON] += (c->fdm.spectral ? 4LL + fft_kernels(c->fdm_fft) : 8LL) * chunk;
+          c->launches[INS2D_PROF_POISSON] += (c->fdm.spectral ? 4LL + fft_kernels(c->fdm_fft) : 6LL) * chunk;
         } else if (c->use_mg) {
           pcg_iterations_mg(c->P, c->mg, c->pcg, chunk, bs);
           c->launches[INS2D_PROF_POISSON] += (long long)(4 + 6 * mg_tail_level(c->mg) + 1) * chunk;
@@ -406,7 +428,7 @@ int solve_pcg(ins2d_ctx *c, const double *f, double *dp, bool accumulate, ins2d_
       return fail(c, INS2D_ETIMEOUT, "PCG: device convergence flag not set within the host's iteration limit");
     if (c->use_fdm) {
       pcg_iterations_fdm(c->P, c->fdm, c->pcg, chunk, c->stream);
-      c->launches[INS2D_PROF_POISSON] += (c->fdm.spectral ? 4LL + fft_kernels(c->fdm_fft) : 8LL) * chunk;
+      c->launches[INS2D_PROF_POISSON] += (c->fdm.spectral ? 4LL + fft_kernels(c->fdm_fft) : 6LL) * chunk;
     } else if (c->use_mg) {
       pcg_iterations_mg(c->P, c->mg, c->pcg, chunk, c->stream);
       c->launches[INS2D_PROF_POISSON] += (long long)(4 + 6 * mg_tail_level(c->mg) + 1) * chunk;
@@ -1045,14 +1067,8 @@ int ins2d_ctx_create(const ins2d_grid_desc *grid, const ins2d_bc_desc *bc, const
           if (std::max(H.Npx, H.Npy) > kFdmMaxN)
             throw std::invalid_argument("fast-diagonalization preconditioner: grid larger than " +
                                         std::to_string(kFdmMaxN) + " cells in a direction");
-          const FdmHost1D fx = fdm_1d(H.TX, H.hx), fy = fdm_1d(H.TY, H.hy);
-          D.Qx = upload_vec(c, fx.Q);
-          D.Qy = upload_vec(c, fy.Q);
-          D.lx = upload_vec(c, fx.lam);
-          D.ly = upload_vec(c, fy.lam);
-          D.thr = 1e-12 * (fx.lam.back() + fy.lam.back());
-          D.t1 = dalloc<double>(c, Np);
-          D.t2 = dalloc<double>(c, Np);
+          CK(fdm_prepare());
+          upload_fdm(c, D);
         }
         c->use_fdm = true;
       } else if (opts->precond != INS2D_PRECOND_JACOBI) {
@@ -1814,10 +1830,9 @@ struct ins2d_ens {
   bool dev_loop = false;
   cudaStream_t body_stream = nullptr;
   int *d_loops = nullptr;
-  EnsFdmD *d_fdm = nullptr;
+  std::vector<FdmD> h_fdm;
   std::vector<double *> fdm_z;
-  int4 *d_ftiles = nullptr;
-  int n_ftiles = 0;
+  EnsFdmPlan fdm_plan;
 };
 
 namespace {
@@ -1924,10 +1939,14 @@ void ens_build_batch(ins2d_ens *e, const std::vector<int> &order) {
   e->n_ctiles = (int)ct.size();
   if (e->use_fdm) {
     std::vector<int4> ft;
-    for (int m : order) fdm_tiles(m, e->mem[m]->P.Npx, e->mem[m]->P.Npy, ft);
-    e->d_ftiles = ens_alloc<int4>(e, ft.size());
-    CK(cudaMemcpy(e->d_ftiles, ft.data(), ft.size() * sizeof(int4), cudaMemcpyHostToDevice));
-    e->n_ftiles = (int)ft.size();
+    std::vector<int2> fr;
+    fdm_ens_lists(e->h_fdm, order, e->mem[0]->P.nsm, e->fdm_plan, ft, fr);
+    int4 *dt = ens_alloc<int4>(e, ft.size());
+    int2 *dr = ens_alloc<int2>(e, fr.size());
+    CK(cudaMemcpy(dt, ft.data(), ft.size() * sizeof(int4), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(dr, fr.data(), fr.size() * sizeof(int2), cudaMemcpyHostToDevice));
+    e->fdm_plan.tiles = dt;
+    e->fdm_plan.rows = dr;
   }
   std::vector<EnsCg> cg(n);
   for (int m = 0; m < n; ++m) {
@@ -1948,11 +1967,11 @@ void ens_solve_batched(ins2d_ens *e, int which) {
   const MgD &M0 = e->mem[0]->mg;
   const double om = M0.omega, al = M0.alpha;
   cudaStream_t s = e->stream;
-  // the preconditioner: fast diagonalization (four products over all
-  // members' tiles) or the members' V-cycles
+  // the preconditioner: fast diagonalization over all members' tiles, or the
+  // members' V-cycles
   auto precond_on = [&](cudaStream_t st) {
     if (e->use_fdm)
-      fdm_apply_ens(e->d_fdm, e->d_ftiles, e->n_ftiles, e->d_cg, st);
+      fdm_apply_ens(e->fdm_plan, e->d_cg, st);
     else
       ens_vcycle(e->d_mem, e->mgd, e->d_cg, e->plan, om, al, st);
   };
@@ -2245,28 +2264,20 @@ int ins2d_ens_create(int32_t n, const ins2d_grid_desc *grids, const ins2d_bc_des
               std::max(c->H.Npx, c->H.Npy) <= kFdmMaxN;
       }
       if (fdm) {
-        std::vector<EnsFdmD> hf(n);
+        CK(fdm_prepare());
+        std::vector<FdmD> &hf = e->h_fdm;
+        hf.resize(n);
         for (int m = 0; m < n; ++m) {
           ins2d_ctx *c = e->mem[m];
-          const HostOps &H = c->H;
-          const FdmHost1D fx = fdm_1d(H.TX, H.hx), fy = fdm_1d(H.TY, H.hy);
-          EnsFdmD &D = hf[m];
-          D.nx = H.Npx;
-          D.ny = H.Npy;
-          D.Qx = upload_vec(c, fx.Q);
-          D.Qy = upload_vec(c, fy.Q);
-          D.lx = upload_vec(c, fx.lam);
-          D.ly = upload_vec(c, fy.lam);
-          D.thr = 1e-12 * (fx.lam.back() + fy.lam.back());
+          FdmD &D = hf[m];
+          upload_fdm(c, D);
           D.r = c->pcg.r;
-          const size_t Np = (size_t)c->P.Np;
-          D.t1 = dalloc<double>(c, Np);
-          D.t2 = dalloc<double>(c, Np);
-          D.z = dalloc<double>(c, Np);
+          D.z = dalloc<double>(c, (size_t)c->P.Np);
           e->fdm_z.push_back(D.z);
         }
-        e->d_fdm = ens_alloc<EnsFdmD>(e, n);
-        CK(cudaMemcpy(e->d_fdm, hf.data(), n * sizeof(EnsFdmD), cudaMemcpyHostToDevice));
+        FdmD *df = ens_alloc<FdmD>(e, n);
+        CK(cudaMemcpy(df, hf.data(), n * sizeof(FdmD), cudaMemcpyHostToDevice));
+        e->fdm_plan.F = df;
         e->use_fdm = true;
       }
       CK(cudaStreamCreateWithFlags(&e->own_stream, cudaStreamNonBlocking));

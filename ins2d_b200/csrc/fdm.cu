@@ -1,293 +1,392 @@
 // Fast-diagonalization preconditioner of the device PCG.
 //
 // The pressure matrix is separable, A = M Om^-1 G = -(diag(hy) (x) TX + TY (x)
-// diag(hx)) (operator_divergence.m:208 with the 1D factors of setup.cpp), so
-// with the generalized eigen-decompositions TX Qx = diag(hx) Qx Lx,
-// TY Qy = diag(hy) Qy Ly (Q' diag(h) Q = I, fdm_host.cpp)
-//   A^+ r = -Qy . [ (Qy' R Qx) ./ (lx_a + ly_b) ] . Qx'
-// where R is r as an Npy x Npx matrix (rows j, x fastest) and the null mode of
-// a singular A (closed or periodic domains) is left out.  Applied exactly this
-// is the inverse on the range of A, so the PCG -- which keeps cg.F's control
-// flow and stopping rule -- converges in one or two iterations.  Four dense
-// products per application, run by a tiled FP64 GEMM on the FP64 tensor cores
-// (mma.sync m8n8k4 .f64; a CUDA-core form of the same tile stays available
-// with INS2D_FDM_DMMA=0).
+// diag(hx)) (operator_divergence.m:208 with the 1D factors of setup.cpp).
+// With the generalized eigenbasis of ONE direction, T_m Q = diag(h_m) Q Lam
+// (Q' diag(h_m) Q = I, fdm_host.cpp), an application is
+//   w = Q' r,   (T_s + lam_b diag(h_s)) zh_b = -w_b for every mode b,   z = Q zh
+// (the null mode of a singular A left out): two dense FP64 products and a
+// batch of tridiagonal solves.  Applied exactly this is the inverse on the
+// range of A, so the PCG -- which keeps cg.F's control flow and stopping rule
+// -- converges in one or two iterations.  Diagonalizing both directions
+// instead costs four products.
+//
+// What bounds it: the FP64 tensor-core rate (mma.sync m8n8k4 .f64; FP64 has
+// no tcgen05 kind) on grids of 512 cells per direction and more, and on
+// smaller ones the number of output tiles (fewer than SMs) and their serial
+// K loop.  So the tile shape follows the grid (tile_config), and operand
+// slabs are copied to shared memory by cp.async, kStages - 1 slabs ahead.
+#include <algorithm>
+
+#include "fdm_tri.cuh"
+#include "ins2d.h"
 #include "kernels.cuh"
+#include "reduce.cuh"
 
 namespace ins2d {
 
 namespace {
 
-#ifndef INS2D_FDM_BM
-#define INS2D_FDM_BM 64
-#endif
-constexpr int kBM = INS2D_FDM_BM, kBN = 64, kBK = 16, kCoreThreads = 256;
+constexpr int kBK = 16;       // depth of an operand slab
+constexpr int kThreads = 128;  // 2 x 2 warps per output tile
 
-// C (M x N, row-major, ldc) = op(A) op(B), op(A) M x K, op(B) K x N.
-// TA: A stored K x M (element (m,k) at A[k*lda + m]); else A[m*lda + k].
-// TB: B stored N x K (element (k,n) at B[n*ldb + k]); else B[k*ldb + n].
-// SCALE: C(b, a) *= -1/(lx[a] + ly[b]), 0 where lx[a] + ly[b] <= thr.
-// one kBM x kBN tile (rows m0.., columns n0..) of C by a block of kCoreThreads.
-// Thread (ty, tx) of 16 x 16 owns rows {2ty, 2ty+1, 32+2ty, 33+2ty} and the
-// same columns with tx, so its operands of one k are two 16-byte shared
-// loads each (conflict-free); the next k-slab's global loads are issued into
-// registers before the current slab's products (INS2D_FDM_PREFETCH).
-#ifndef INS2D_FDM_PREFETCH
-#define INS2D_FDM_PREFETCH 1
-#endif
-template <bool TA, bool TB, bool SCALE>
-__device__ __forceinline__ void gemm_tile(int M, int N, int K, const double *__restrict__ A, int lda,
-                                          const double *__restrict__ B, int ldb, double *__restrict__ C, int ldc,
-                                          const double *__restrict__ lx, const double *__restrict__ ly, double thr,
-                                          int m0, int n0) {
-  __shared__ __align__(16) double As[kBK][kBM];
-  __shared__ __align__(16) double Bs[kBK][kBN];
-  constexpr int QA = (kBM * kBK) / kCoreThreads, QB = (kBN * kBK) / kCoreThreads;
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  // global -> registers of the k-slab starting at k0
-  auto load = [&](int k0, double (&ra)[QA], double (&rb)[QB]) {
-#pragma unroll
-    for (int q = 0; q < QA; ++q) {
-      const int e = tid + kCoreThreads * q;
-      const int m = TA ? e % kBM : e / kBK, k = TA ? e / kBM : e % kBK;
-      const int gm = m0 + m, gk = k0 + k;
-      ra[q] = (gm < M && gk < K) ? (TA ? __ldg(A + (size_t)gk * lda + gm) : __ldg(A + (size_t)gm * lda + gk)) : 0.0;
-    }
-#pragma unroll
-    for (int q = 0; q < QB; ++q) {
-      const int e = tid + kCoreThreads * q;
-      const int n = TB ? e / kBK : e % kBN, k = TB ? e % kBK : e / kBN;
-      const int gn = n0 + n, gk = k0 + k;
-      rb[q] = (gn < N && gk < K) ? (TB ? __ldg(B + (size_t)gn * ldb + gk) : __ldg(B + (size_t)gk * ldb + gn)) : 0.0;
-    }
-  };
-  auto store = [&](const double (&ra)[QA], const double (&rb)[QB]) {
-#pragma unroll
-    for (int q = 0; q < QA; ++q) {
-      const int e = tid + kCoreThreads * q;
-      As[TA ? e / kBM : e % kBK][TA ? e % kBM : e / kBK] = ra[q];
-    }
-#pragma unroll
-    for (int q = 0; q < QB; ++q) {
-      const int e = tid + kCoreThreads * q;
-      Bs[TB ? e % kBK : e / kBN][TB ? e / kBK : e % kBN] = rb[q];
-    }
-  };
-  double acc[4][4] = {};
-  double ra[QA], rb[QB];
-  load(0, ra, rb);
-  for (int k0 = 0; k0 < K; k0 += kBK) {
-    store(ra, rb);
-    __syncthreads();
-#if INS2D_FDM_PREFETCH
-    if (k0 + kBK < K) load(k0 + kBK, ra, rb);
-#endif
-#pragma unroll
-    for (int k = 0; k < kBK; ++k) {
-      const double2 a0 = *reinterpret_cast<const double2 *>(&As[k][2 * ty]);
-      const double2 a1 = *reinterpret_cast<const double2 *>(&As[k][32 + 2 * ty]);
-      const double2 b0 = *reinterpret_cast<const double2 *>(&Bs[k][2 * tx]);
-      const double2 b1 = *reinterpret_cast<const double2 *>(&Bs[k][32 + 2 * tx]);
-      const double a[4] = {a0.x, a0.y, a1.x, a1.y}, b[4] = {b0.x, b0.y, b1.x, b1.y};
-#pragma unroll
-      for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) acc[r][c] = fma(a[r], b[c], acc[r][c]);
-    }
-    __syncthreads();
-#if !INS2D_FDM_PREFETCH
-    if (k0 + kBK < K) load(k0 + kBK, ra, rb);
-#endif
-  }
-#pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    const int gm = m0 + (r >> 1) * 32 + 2 * ty + (r & 1);
-    if (gm >= M) continue;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const int gn = n0 + (c >> 1) * 32 + 2 * tx + (c & 1);
-      if (gn >= N) continue;
-      double v = acc[r][c];
-      if (SCALE) {
-        const double lam = __ldg(lx + gn) + __ldg(ly + gm);
-        v = lam > thr ? -v / lam : 0.0;
-      }
-      C[(size_t)gm * ldc + gn] = v;
-    }
-  }
+// tile shapes; their shared memory: kStages slabs of both operands, each
+// padded to rows of 4 mod 16 doubles, so that a warp's fragment loads (four
+// consecutive rows by four consecutive columns per half warp) hit distinct banks
+template <int CFG>
+struct Tile;
+template <>
+struct Tile<0> {
+  static constexpr int BM = 64, BN = 64, STAGES = 3;
+};
+template <>
+struct Tile<1> {
+  static constexpr int BM = 64, BN = 32, STAGES = 4;
+};
+template <>
+struct Tile<2> {
+  static constexpr int BM = 32, BN = 32, STAGES = 4;
+};
+__host__ __device__ constexpr int slab(int bmn) {
+  const int kmajor = kBK * (bmn + 4), mmajor = bmn * (kBK + 4);
+  return kmajor > mmajor ? kmajor : mmajor;
+}
+template <int CFG>
+constexpr int tile_smem() {
+  return Tile<CFG>::STAGES * (slab(Tile<CFG>::BM) + slab(Tile<CFG>::BN)) * (int)sizeof(double);
 }
 
-// The same tile on the FP64 tensor cores (INS2D_FDM_DMMA): mma.sync
-// m8n8k4 .f64, each warp a 32 x kTcWarpN block of C (4 x kTcWarpN/8
-// fragments of 8 x 8; INS2D_FDM_WARP_N 32: four warps per tile, 16: eight).
-// Fragment layout of m8n8k4 .f64 (group g = lane / 4, t = lane % 4): A holds
-// (row g, col t), B (row t, col g), C/D (row g, cols 2t, 2t+1).  The operand
-// slabs are staged with padded rows (kBM + 4) so a warp's fragment loads hit
-// distinct banks.
-#ifndef INS2D_FDM_DMMA
-#define INS2D_FDM_DMMA 1
-#endif
-#ifndef INS2D_FDM_WARP_N
-#define INS2D_FDM_WARP_N 32
-#endif
-constexpr int kTcWarpN = INS2D_FDM_WARP_N, kTcThreads = 32 * (kBM / 32) * (kBN / kTcWarpN);
-static_assert(INS2D_FDM_DMMA || (kBM == 64 && kBN == 64), "the CUDA-core tile is 64 x 64");
-constexpr int kGemmThreads = INS2D_FDM_DMMA ? kTcThreads : kCoreThreads;
 __device__ __forceinline__ void dmma_884(double &d0, double &d1, double a, double b) {
   asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
                : "+d"(d0), "+d"(d1)
                : "d"(a), "d"(b));
 }
-template <bool TA, bool TB, bool SCALE>
-__device__ __forceinline__ void gemm_tile_tc(int M, int N, int K, const double *__restrict__ A, int lda,
-                                             const double *__restrict__ B, int ldb, double *__restrict__ C, int ldc,
-                                             const double *__restrict__ lx, const double *__restrict__ ly,
-                                             double thr, int m0, int n0) {
-  constexpr int PA = kBM + 4, PB = kBN + 4;
-  __shared__ __align__(16) double As[kBK][PA];
-  __shared__ __align__(16) double Bs[kBK][PB];
-  constexpr int QA = (kBM * kBK) / kTcThreads, QB = (kBN * kBK) / kTcThreads;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+// asynchronous copy of BYTES (8 or 16); the last BYTES - valid are zero-filled
+template <int BYTES>
+__device__ __forceinline__ void cp_async_fill(double *dst, const double *src, int valid) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  if constexpr (BYTES == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(valid) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src), "r"(valid) : "memory");
+}
+
+// Copies one operand slab: rows of `len` contiguous elements.  The operand is
+// stored R x L row-major (ld); the slab takes R0.. (NR of them) by L0.. (NL),
+// to S with pitch NL + 4.  V elements per copy.
+template <int NR, int NL, int V>
+__device__ __forceinline__ void load_slab(double *S, const double *__restrict__ A, int ld, int r0, int R, int l0,
+                                          int L) {
+  constexpr int PER = NL / V;
+#pragma unroll
+  for (int q = 0; q < (NR * PER) / kThreads; ++q) {
+    const int e = threadIdx.x + kThreads * q;
+    const int r = e / PER, l = (e % PER) * V;
+    const int gr = r0 + r, gl = l0 + l;
+    const int left = gr < R ? L - gl : 0;
+    const int valid = left >= V ? V : (left > 0 ? left : 0);
+    const double *src = valid > 0 ? A + (size_t)gr * ld + gl : A;
+    cp_async_fill<8 * V>(S + r * (NL + 4) + l, src, 8 * valid);
+  }
+}
+template <int NR, int NL>
+__device__ __forceinline__ void load_slab(double *S, const double *__restrict__ A, int ld, int r0, int R, int l0,
+                                          int L, bool v16) {
+  if (v16)
+    load_slab<NR, NL, 2>(S, A, ld, r0, R, l0, L);
+  else
+    load_slab<NR, NL, 1>(S, A, ld, r0, R, l0, L);
+}
+
+// One BM x BN tile (rows m0.., columns n0..) of C = op(A) op(B), op(A) M x K,
+// op(B) K x N.  TA: A stored K x M (element (m,k) at A[k*lda + m]); else
+// A[m*lda + k].  TB: B stored N x K; else K x N.  epi(row, column, value) for
+// every element of C in range.  Fragment layout of m8n8k4 .f64 (group
+// g = lane / 4, t = lane % 4): A holds (row g, col t), B (row t, col g), C/D
+// (row g, cols 2t, 2t+1).
+template <int CFG, bool TA, bool TB, class Epi>
+__device__ __forceinline__ void gemm_tile(int M, int N, int K, const double *__restrict__ A, int lda,
+                                          const double *__restrict__ B, int ldb, int m0, int n0, Epi epi) {
+  constexpr int BM = Tile<CFG>::BM, BN = Tile<CFG>::BN, ST = Tile<CFG>::STAGES;
+  constexpr int SA = slab(BM), SB = slab(BN);
+  extern __shared__ __align__(16) double smem[];
+  double *As = smem, *Bs = smem + ST * SA;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, t = lane & 3;
-  constexpr int NJ = kTcWarpN / 8;  // fragments per warp along n
-  constexpr int WM = kBM / 32;  // warps along m
-  const int wm = (warp % WM) * 32, wn = (warp / WM) * kTcWarpN;
-  double ra[QA], rb[QB];
-  auto load = [&](int k0) {
-#pragma unroll
-    for (int q = 0; q < QA; ++q) {
-      const int e = tid + kTcThreads * q;
-      const int m = TA ? e % kBM : e / kBK, k = TA ? e / kBM : e % kBK;
-      const int gm = m0 + m, gk = k0 + k;
-      ra[q] = (gm < M && gk < K) ? (TA ? __ldg(A + (size_t)gk * lda + gm) : __ldg(A + (size_t)gm * lda + gk)) : 0.0;
-    }
-#pragma unroll
-    for (int q = 0; q < QB; ++q) {
-      const int e = tid + kTcThreads * q;
-      const int n = TB ? e / kBK : e % kBN, k = TB ? e % kBK : e / kBN;
-      const int gn = n0 + n, gk = k0 + k;
-      rb[q] = (gn < N && gk < K) ? (TB ? __ldg(B + (size_t)gn * ldb + gk) : __ldg(B + (size_t)gk * ldb + gn)) : 0.0;
-    }
+  constexpr int WM = BM / 2, WN = BN / 2, NI = WM / 8, NJ = WN / 8;
+  const int wm = (warp & 1) * WM, wn = (warp >> 1) * WN;
+  // 16-byte copies where every row starts on a 16-byte boundary
+  const bool va = (lda & 1) == 0 && ((uintptr_t)A & 15) == 0, vb = (ldb & 1) == 0 && ((uintptr_t)B & 15) == 0;
+  const int nk = (K + kBK - 1) / kBK;
+  auto load = [&](int kt) {
+    double *as = As + (kt % ST) * SA, *bs = Bs + (kt % ST) * SB;
+    if (TA)
+      load_slab<kBK, BM>(as, A, lda, kt * kBK, K, m0, M, va);
+    else
+      load_slab<BM, kBK>(as, A, lda, m0, M, kt * kBK, K, va);
+    if (TB)
+      load_slab<BN, kBK>(bs, B, ldb, n0, N, kt * kBK, K, vb);
+    else
+      load_slab<kBK, BN>(bs, B, ldb, kt * kBK, K, n0, N, vb);
   };
-  double acc[4][NJ][2] = {};
-  load(0);
-  for (int k0 = 0; k0 < K; k0 += kBK) {
+  double acc[NI][NJ][2] = {};
 #pragma unroll
-    for (int q = 0; q < QA; ++q) {
-      const int e = tid + kTcThreads * q;
-      As[TA ? e / kBM : e % kBK][TA ? e % kBM : e / kBK] = ra[q];
-    }
-#pragma unroll
-    for (int q = 0; q < QB; ++q) {
-      const int e = tid + kTcThreads * q;
-      Bs[TB ? e % kBK : e / kBN][TB ? e / kBK : e % kBN] = rb[q];
-    }
-    __syncthreads();
-    if (k0 + kBK < K) load(k0 + kBK);
+  for (int q = 0; q < ST - 1; ++q) {
+    if (q < nk) load(q);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  }
+  for (int kt = 0; kt < nk; ++kt) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(ST - 2) : "memory");
+    __syncthreads();  // slab kt complete for every thread; slab kt - 1 read by every thread
+    if (kt + ST - 1 < nk) load(kt + ST - 1);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    const double *as = As + (kt % ST) * SA, *bs = Bs + (kt % ST) * SB;
 #pragma unroll
     for (int kk = 0; kk < kBK; kk += 4) {
-      double a[4], b[NJ];
+      double a[NI], b[NJ];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[kk + t][wm + 8 * i + g];
+      for (int i = 0; i < NI; ++i) {
+        const int m = wm + 8 * i + g;
+        a[i] = TA ? as[(kk + t) * (BM + 4) + m] : as[m * (kBK + 4) + kk + t];
+      }
 #pragma unroll
-      for (int j = 0; j < NJ; ++j) b[j] = Bs[kk + t][wn + 8 * j + g];
+      for (int j = 0; j < NJ; ++j) {
+        const int n = wn + 8 * j + g;
+        b[j] = TB ? bs[n * (kBK + 4) + kk + t] : bs[(kk + t) * (BN + 4) + n];
+      }
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < NI; ++i)
 #pragma unroll
         for (int j = 0; j < NJ; ++j) dmma_884(acc[i][j][0], acc[i][j][1], a[i], b[j]);
     }
-    __syncthreads();
   }
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int gm = m0 + wm + 8 * i + g;
-    if (gm >= M) continue;
+  for (int i = 0; i < NI; ++i)
 #pragma unroll
     for (int j = 0; j < NJ; ++j)
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        const int gn = n0 + wn + 8 * j + 2 * t + h;
-        if (gn >= N) continue;
-        double v = acc[i][j][h];
-        if (SCALE) {
-          const double lam = __ldg(lx + gn) + __ldg(ly + gm);
-          v = lam > thr ? -v / lam : 0.0;
-        }
-        C[(size_t)gm * ldc + gn] = v;
+        const int gm = m0 + wm + 8 * i + g, gn = n0 + wn + 8 * j + 2 * t + h;
+        if (gm < M && gn < N) epi(gm, gn, acc[i][j][h]);
       }
+}
+
+// w = Q' r: rows = modes, columns = the unknowns of the systems
+template <int CFG>
+__device__ __forceinline__ void fdm_forward(const FdmD &F, const double *__restrict__ r, int m0, int n0) {
+  const int nm = F.nm, n = F.n;
+  auto store = [&](int b, int i, double v) { F.t[(size_t)b * n + i] = v; };
+  if (F.xmodes)  // r is n x nm (rows j = unknowns)
+    gemm_tile<CFG, true, true>(nm, n, nm, F.Q, nm, r, nm, m0, n0, store);
+  else  // r is nm x n
+    gemm_tile<CFG, true, false>(nm, n, nm, F.Q, nm, r, n, m0, n0, store);
+}
+// z = Q zh, element (j, i) handed to epi(index, value)
+template <int CFG, class Epi>
+__device__ __forceinline__ void fdm_backward(const FdmD &F, int m0, int n0, Epi epi) {
+  const int nm = F.nm, n = F.n, nx = F.nx;
+  auto out = [&](int j, int i, double v) { epi((size_t)j * nx + i, v); };
+  if (F.xmodes)
+    gemm_tile<CFG, true, true>(n, nm, nm, F.t, n, F.Q, nm, m0, n0, out);
+  else
+    gemm_tile<CFG, false, false>(nm, n, nm, F.Q, nm, F.t, n, m0, n0, out);
+}
+
+template <int CFG>
+__global__ void __launch_bounds__(kThreads) k_fdm_fwd(const __grid_constant__ FdmD F, const double *__restrict__ r,
+                                                      const int *__restrict__ done) {
+  if (*(volatile const int *)done) return;
+  fdm_forward<CFG>(F, r, blockIdx.y * Tile<CFG>::BM, blockIdx.x * Tile<CFG>::BN);
+}
+
+// z = Q zh with r'z reduced in the same pass (deterministic, reduce.cuh):
+// init: rz, and p = z; otherwise beta = rz / rz_old
+template <int CFG>
+__global__ void __launch_bounds__(kThreads) k_fdm_bwd(const __grid_constant__ FdmD F, const PcgWork W,
+                                                      const double *__restrict__ r, int init) {
+  if (*(volatile int *)&W.sc->done) return;
+  double q[1] = {0.0};
+  const int ops[1] = {R_SUM};
+  fdm_backward<CFG>(F, blockIdx.y * Tile<CFG>::BM, blockIdx.x * Tile<CFG>::BN, [&](size_t k, double v) {
+    F.z[k] = v;
+    if (init) W.p[k] = v;
+    q[0] += __ldg(r + k) * v;
+  });
+  RedScratch red;
+  red.partials = W.partials;
+  red.counter = &W.sc->counter;
+  red.result = W.partials + (size_t)W.blocks * 8;
+  red.max_blocks = W.blocks;
+  double out[1];
+  if (grid_reduce<1>(q, ops, red, out)) {
+    PcgScalars *s = W.sc;
+    if (!isfinite(out[0])) {
+      s->status = INS2D_ENONFINITE;
+      s->done = 1;
+    } else if (init) {
+      s->rz = out[0];
+    } else {
+      s->beta = out[0] / s->rz;
+      s->rz = out[0];
+    }
   }
 }
 
-template <bool TA, bool TB, bool SCALE>
-__global__ void __launch_bounds__(kGemmThreads) k_gemm(int M, int N, int K, const double *__restrict__ A, int lda,
-                                                       const double *__restrict__ B, int ldb, double *__restrict__ C,
-                                                       int ldc, const double *__restrict__ lx,
-                                                       const double *__restrict__ ly, double thr,
-                                                       const int *__restrict__ done) {
-  if (done && *(volatile const int *)done) return;
-#if INS2D_FDM_DMMA
-  gemm_tile_tc<TA, TB, SCALE>(M, N, K, A, lda, B, ldb, C, ldc, lx, ly, thr, blockIdx.y * kBM, blockIdx.x * kBN);
-#else
-  gemm_tile<TA, TB, SCALE>(M, N, K, A, lda, B, ldb, C, ldc, lx, ly, thr, blockIdx.y * kBM, blockIdx.x * kBN);
-#endif
+template <int W>
+__global__ void __launch_bounds__(128) k_fdm_tri(const __grid_constant__ FdmD F, const int *__restrict__ done) {
+  __shared__ double sh[4][4];
+  if (*(volatile const int *)done) return;
+  const int warp = threadIdx.x >> 5;
+  tri_row<W>(F, blockIdx.x * (4 / W) + warp / W, warp % W, sh);
 }
 
-// The four products of fdm_apply for many members in one launch per product:
-// work items {member, tile row, tile column}; members whose CG has converged
-// (cg[m].done) skip their tiles.  OP 0: T1 = R Qx; 1: T2 = -(Qy' T1) ./ lam;
-// 2: T1 = Qy T2; 3: Z = T1 Qx'.
-#if INS2D_FDM_DMMA
-#define GEMM_TILE gemm_tile_tc
-#else
-#define GEMM_TILE gemm_tile
-#endif
-template <int OP>
-__global__ void __launch_bounds__(kGemmThreads) k_gemm_ens(const EnsFdmD *__restrict__ F,
-                                                           const int4 *__restrict__ tiles,
-                                                           const EnsCg *__restrict__ cg) {
+// the same for the members of an ensemble that still iterate
+template <int CFG>
+__global__ void __launch_bounds__(kThreads) k_fdm_fwd_ens(const FdmD *__restrict__ Fs, const int4 *__restrict__ tiles,
+                                                          const EnsCg *__restrict__ cg) {
   const int4 t = tiles[blockIdx.x];
-  const int m = t.x;
-  if (*(volatile const int *)&cg[m].done) return;
-  const EnsFdmD &D = F[m];
-  const int nx = D.nx, ny = D.ny, m0 = t.y * kBM, n0 = t.z * kBN;
-  if (OP == 0)
-    GEMM_TILE<false, false, false>(ny, nx, nx, D.r, nx, D.Qx, nx, D.t1, nx, D.lx, D.ly, D.thr, m0, n0);
-  else if (OP == 1)
-    GEMM_TILE<true, false, true>(ny, nx, ny, D.Qy, ny, D.t1, nx, D.t2, nx, D.lx, D.ly, D.thr, m0, n0);
-  else if (OP == 2)
-    GEMM_TILE<false, false, false>(ny, nx, ny, D.Qy, ny, D.t2, nx, D.t1, nx, D.lx, D.ly, D.thr, m0, n0);
-  else
-    GEMM_TILE<false, true, false>(ny, nx, nx, D.t1, nx, D.Qx, nx, D.z, nx, D.lx, D.ly, D.thr, m0, n0);
+  if (*(volatile const int *)&cg[t.x].done) return;
+  const FdmD &F = Fs[t.x];
+  const int m0 = t.y * Tile<CFG>::BM, n0 = t.z * Tile<CFG>::BN;
+  if (m0 < F.nm && n0 < F.n) fdm_forward<CFG>(F, F.r, m0, n0);
+}
+template <int CFG>
+__global__ void __launch_bounds__(kThreads) k_fdm_bwd_ens(const FdmD *__restrict__ Fs, const int4 *__restrict__ tiles,
+                                                          const EnsCg *__restrict__ cg) {
+  const int4 t = tiles[blockIdx.x];
+  if (*(volatile const int *)&cg[t.x].done) return;
+  const FdmD &F = Fs[t.x];
+  const int m0 = t.y * Tile<CFG>::BM, n0 = t.z * Tile<CFG>::BN;
+  if (m0 < F.ny && n0 < F.nx) fdm_backward<CFG>(F, m0, n0, [&](size_t k, double v) { F.z[k] = v; });
+}
+template <int W>
+__global__ void __launch_bounds__(128) k_fdm_tri_ens(const FdmD *__restrict__ Fs, const int2 *__restrict__ rows,
+                                                     const EnsCg *__restrict__ cg) {
+  __shared__ double sh[4][4];
+  const int2 t = rows[blockIdx.x];
+  if (*(volatile const int *)&cg[t.x].done) return;
+  const int warp = threadIdx.x >> 5;
+  tri_row<W>(Fs[t.x], t.y + warp / W, warp % W, sh);
 }
 
-template <bool TA, bool TB, bool SCALE>
-void gemm(int M, int N, int K, const double *A, int lda, const double *B, int ldb, double *C, int ldc,
-          const FdmD &F, const int *done, cudaStream_t s) {
-  const dim3 g((N + kBN - 1) / kBN, (M + kBM - 1) / kBM);
-  k_gemm<TA, TB, SCALE><<<g, kGemmThreads, 0, s>>>(M, N, K, A, lda, B, ldb, C, ldc, F.lx, F.ly, F.thr, done);
+// Tile shape: the one with the least work on the busiest SM, tiles of one
+// launch spread evenly; the larger one on a tie (it reads its operands fewer
+// times).
+int tile_config(long long t64, long long t6432, long long t32, int nsm) {
+  const long long w0 = ((t64 + nsm - 1) / nsm) * 4, w1 = ((t6432 + nsm - 1) / nsm) * 2, w2 = (t32 + nsm - 1) / nsm;
+  return w0 <= w1 && w0 <= w2 ? 0 : (w1 <= w2 ? 1 : 2);
+}
+long long tiles_of(long long M, long long N, int bm, int bn) { return ((M + bm - 1) / bm) * ((N + bn - 1) / bn); }
+int row_warps(int n) { return n <= 32 * kTriChunk ? 1 : (n <= 64 * kTriChunk ? 2 : 4); }
+static_assert(4 * 32 * kTriChunk >= 1024, "four warps hold the longest row (kFdmMaxN)");
+
+template <int CFG>
+void launch_fwd(const FdmD &F, const double *r, const int *done, cudaStream_t s) {
+  const dim3 g((F.n + Tile<CFG>::BN - 1) / Tile<CFG>::BN, (F.nm + Tile<CFG>::BM - 1) / Tile<CFG>::BM);
+  k_fdm_fwd<CFG><<<g, kThreads, tile_smem<CFG>(), s>>>(F, r, done);
+}
+template <int CFG>
+void launch_bwd(const FdmD &F, const PcgWork &W, const double *r, bool init, cudaStream_t s) {
+  const dim3 g((F.nx + Tile<CFG>::BN - 1) / Tile<CFG>::BN, (F.ny + Tile<CFG>::BM - 1) / Tile<CFG>::BM);
+  k_fdm_bwd<CFG><<<g, kThreads, tile_smem<CFG>(), s>>>(F, W, r, init ? 1 : 0);
+}
+template <int W>
+void launch_tri(const FdmD &F, const int *done, cudaStream_t s) {
+  k_fdm_tri<W><<<(F.nm + 4 / W - 1) / (4 / W), 128, 0, s>>>(F, done);
 }
 
 }  // namespace
 
-void fdm_tiles(int member, int nx, int ny, std::vector<int4> &out) {
-  for (int bm = 0; bm < (ny + kBM - 1) / kBM; ++bm)
-    for (int bn = 0; bn < (nx + kBN - 1) / kBN; ++bn) out.push_back(make_int4(member, bm, bn, 0));
+cudaError_t fdm_prepare() {
+  cudaError_t first = cudaSuccess;
+  auto opt_in = [&](const void *k, int bytes) {
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (first == cudaSuccess) first = e;
+  };
+#define INS2D_FDM_OPT_IN(C)                                   \
+  opt_in((const void *)k_fdm_fwd<C>, tile_smem<C>());         \
+  opt_in((const void *)k_fdm_bwd<C>, tile_smem<C>());         \
+  opt_in((const void *)k_fdm_fwd_ens<C>, tile_smem<C>());     \
+  opt_in((const void *)k_fdm_bwd_ens<C>, tile_smem<C>());
+  INS2D_FDM_OPT_IN(0)
+  INS2D_FDM_OPT_IN(1)
+  INS2D_FDM_OPT_IN(2)
+#undef INS2D_FDM_OPT_IN
+  return first;
 }
 
-void fdm_apply_ens(const EnsFdmD *F, const int4 *tiles, int ntiles, const EnsCg *cg, cudaStream_t s) {
-  if (ntiles <= 0) return;
-  k_gemm_ens<0><<<ntiles, kGemmThreads, 0, s>>>(F, tiles, cg);
-  k_gemm_ens<1><<<ntiles, kGemmThreads, 0, s>>>(F, tiles, cg);
-  k_gemm_ens<2><<<ntiles, kGemmThreads, 0, s>>>(F, tiles, cg);
-  k_gemm_ens<3><<<ntiles, kGemmThreads, 0, s>>>(F, tiles, cg);
+void fdm_apply(const FdmD &F, const PcgWork &W, const double *r, bool init, cudaStream_t s) {
+  const int *done = &W.sc->done;
+  const int cfg = tile_config(tiles_of(F.ny, F.nx, 64, 64),
+                              std::min(tiles_of(F.ny, F.nx, 64, 32), tiles_of(F.nx, F.ny, 64, 32)),
+                              tiles_of(F.ny, F.nx, 32, 32), F.nsm);
+  if (cfg == 0)
+    launch_fwd<0>(F, r, done, s);
+  else if (cfg == 1)
+    launch_fwd<1>(F, r, done, s);
+  else
+    launch_fwd<2>(F, r, done, s);
+  const int w = row_warps(F.n);
+  if (w == 1)
+    launch_tri<1>(F, done, s);
+  else if (w == 2)
+    launch_tri<2>(F, done, s);
+  else
+    launch_tri<4>(F, done, s);
+  if (cfg == 0)
+    launch_bwd<0>(F, W, r, init, s);
+  else if (cfg == 1)
+    launch_bwd<1>(F, W, r, init, s);
+  else
+    launch_bwd<2>(F, W, r, init, s);
 }
 
-void fdm_apply(const FdmD &F, const double *r, double *z, const int *done, cudaStream_t s) {
-  const int nx = F.nx, ny = F.ny;
-  gemm<false, false, false>(ny, nx, nx, r, nx, F.Qx, nx, F.t1, nx, F, done, s);        // T1 = R Qx
-  gemm<true, false, true>(ny, nx, ny, F.Qy, ny, F.t1, nx, F.t2, nx, F, done, s);       // T2 = -(Qy' T1) ./ lam
-  gemm<false, false, false>(ny, nx, ny, F.Qy, ny, F.t2, nx, F.t1, nx, F, done, s);     // T1 = Qy T2
-  gemm<false, true, false>(ny, nx, nx, F.t1, nx, F.Qx, nx, z, nx, F, done, s);         // Z = T1 Qx'
+void fdm_ens_lists(const std::vector<FdmD> &F, const std::vector<int> &order, int nsm, EnsFdmPlan &pl,
+                   std::vector<int4> &tiles, std::vector<int2> &rows) {
+  long long t0 = 0, t1 = 0, t2 = 0;
+  int nmax = 0;
+  for (const FdmD &f : F) {
+    t0 += tiles_of(f.nm, f.n, 64, 64);
+    t1 += tiles_of(f.nm, f.n, 64, 32);
+    t2 += tiles_of(f.nm, f.n, 32, 32);
+    nmax = std::max(nmax, f.n);
+  }
+  pl.cfg = tile_config(t0, t1, t2, nsm);
+  pl.warps = row_warps(nmax);
+  const int bm = pl.cfg == 2 ? 32 : 64, bn = pl.cfg == 0 ? 64 : 32;
+  // one list for both products: the forward one's nm x n and the backward
+  // one's ny x nx tiles (a tile outside a product's range returns)
+  for (int m : order) {
+    const int M = std::max(F[m].nm, F[m].ny), N = std::max(F[m].n, F[m].nx);
+    for (int bi = 0; bi < (M + bm - 1) / bm; ++bi)
+      for (int bj = 0; bj < (N + bn - 1) / bn; ++bj) tiles.push_back(make_int4(m, bi, bj, 0));
+    for (int b = 0; b < F[m].nm; b += 4 / pl.warps) rows.push_back(make_int2(m, b));
+  }
+  pl.ntiles = (int)tiles.size();
+  pl.nrows = (int)rows.size();
+}
+
+void fdm_apply_ens(const EnsFdmPlan &pl, const EnsCg *cg, cudaStream_t s) {
+  if (pl.ntiles <= 0) return;
+  if (pl.cfg == 0)
+    k_fdm_fwd_ens<0><<<pl.ntiles, kThreads, tile_smem<0>(), s>>>(pl.F, pl.tiles, cg);
+  else if (pl.cfg == 1)
+    k_fdm_fwd_ens<1><<<pl.ntiles, kThreads, tile_smem<1>(), s>>>(pl.F, pl.tiles, cg);
+  else
+    k_fdm_fwd_ens<2><<<pl.ntiles, kThreads, tile_smem<2>(), s>>>(pl.F, pl.tiles, cg);
+  if (pl.warps == 1)
+    k_fdm_tri_ens<1><<<pl.nrows, 128, 0, s>>>(pl.F, pl.rows, cg);
+  else if (pl.warps == 2)
+    k_fdm_tri_ens<2><<<pl.nrows, 128, 0, s>>>(pl.F, pl.rows, cg);
+  else
+    k_fdm_tri_ens<4><<<pl.nrows, 128, 0, s>>>(pl.F, pl.rows, cg);
+  if (pl.cfg == 0)
+    k_fdm_bwd_ens<0><<<pl.ntiles, kThreads, tile_smem<0>(), s>>>(pl.F, pl.tiles, cg);
+  else if (pl.cfg == 1)
+    k_fdm_bwd_ens<1><<<pl.ntiles, kThreads, tile_smem<1>(), s>>>(pl.F, pl.tiles, cg);
+  else
+    k_fdm_bwd_ens<2><<<pl.ntiles, kThreads, tile_smem<2>(), s>>>(pl.F, pl.tiles, cg);
 }
 
 }  // namespace ins2d

@@ -6,6 +6,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <limits>
 #include <numeric>
 #include <stdexcept>
@@ -167,6 +168,74 @@ FdmHost1D fdm_1d(const Table &T, const std::vector<double> &h) {
   const double top = n ? std::fabs(F.lam[n - 1]) : 0.0;
   for (double &l : F.lam)
     if (l < 0.0 && l > -1e-12 * top) l = 0.0;
+  return F;
+}
+
+FdmTri fdm_tri(const Table &TX, const std::vector<double> &hx, const Table &TY, const std::vector<double> &hy) {
+  FdmTri F;
+  F.xmodes = TX.nrows < TY.nrows;
+  const Table &Tm = F.xmodes ? TX : TY, &Ts = F.xmodes ? TY : TX;
+  const FdmHost1D m = fdm_1d(Tm, F.xmodes ? hx : hy);
+  const int nm = F.nm = m.n, n = F.n = Ts.nrows;
+  F.Q = m.Q;
+  F.lam = m.lam;
+  F.h = F.xmodes ? hy : hx;
+  for (double h : F.h) F.hsum += h;
+  auto at = [&](int i, int k) {
+    auto it = Ts.T.rows[i].find(k);
+    return it == Ts.T.rows[i].end() ? 0.0 : it->second;
+  };
+  std::vector<double> d(n);
+  F.e.assign((size_t)((n + 7) / 8) * 8, 0.0);
+  for (int i = 0; i < n; ++i) d[i] = at(i, i);
+  for (int i = 0; i + 1 < n; ++i) F.e[i] = 0.5 * (at(i, i + 1) + at(i + 1, i));
+  const double c = n > 2 ? 0.5 * (at(0, n - 1) + at(n - 1, 0)) : 0.0;  // cyclic corner
+  for (int i = 0; i < n; ++i)
+    for (const auto &kv : Ts.T.rows[i])
+      if (kv.second != 0.0 && std::abs(kv.first - i) > 1 && !(n > 2 && std::abs(kv.first - i) == n - 1))
+        throw std::runtime_error("fdm: the 1D pressure factor is not tridiagonal");
+  // singular for the zero mode: every row of T_s sums to zero (no pressure
+  // boundary), and so does T_m's (its smallest eigenvalue, clipped, is zero)
+  double smax = 0.0, dmax = 0.0;
+  for (int i = 0; i < n; ++i) {
+    double s = 0.0;
+    for (const auto &kv : Ts.T.rows[i]) s += kv.second;
+    smax = std::max(smax, std::fabs(s));
+    dmax = std::max(dmax, std::fabs(d[i]));
+  }
+  if (smax <= 1e-10 * dmax && m.lam[0] <= 1e-12 * std::max(m.lam[nm - 1], dmax / F.h[0])) F.null_mode = 0;
+  F.piv.assign((size_t)nm * n, 0.0);
+  if (c != 0.0) {
+    F.g.assign((size_t)nm * n, 0.0);
+    F.cr.assign(nm, 0.0);
+  }
+  std::vector<double> db(n);
+  for (int b = 0; b < nm; ++b) {
+    double *p = &F.piv[(size_t)b * n];
+    for (int i = 0; i < n; ++i) db[i] = d[i] + F.lam[b] * F.h[i];
+    const bool null = b == F.null_mode;
+    double gam = 0.0;
+    if (c != 0.0 && !null) {
+      gam = -db[0];
+      db[0] -= gam;
+      db[n - 1] -= c * c / gam;
+    }
+    p[0] = 1.0 / db[0];
+    for (int i = 1; i < n; ++i) p[i] = 1.0 / (db[i] - F.e[i - 1] * F.e[i - 1] * p[i - 1]);
+    if (null) p[n - 1] = 0.0;  // zh_{n-1} = 0; also drops the cyclic corner, which only couples to it
+    if (c != 0.0 && !null) {
+      // q solves the modified system for u = (gam, 0, .., 0, c); g = q / (1 + v'q)
+      double *q = &F.g[(size_t)b * n];
+      for (int i = 0; i < n; ++i) {
+        const double u = i == 0 ? gam : (i == n - 1 ? c : 0.0);
+        q[i] = (u - (i ? F.e[i - 1] * q[i - 1] : 0.0)) * p[i];
+      }
+      for (int i = n - 2; i >= 0; --i) q[i] -= F.e[i] * p[i] * q[i + 1];
+      F.cr[b] = c / gam;
+      const double den = 1.0 + q[0] + F.cr[b] * q[n - 1];
+      for (int i = 0; i < n; ++i) q[i] /= den;
+    }
+  }
   return F;
 }
 

@@ -1,0 +1,187 @@
+// The tridiagonal systems of the fast-diagonalization preconditioner
+// (fdm_host.hpp, FdmTri): for every mode b of the diagonalized direction
+//   (T_s + lam_b diag(h_s)) zh_b = -w_b,
+// solved in place on the rows of the nm x n array w.  With the reciprocal
+// pivots tabulated, elimination and back substitution are first-order linear
+// recurrences y_k = a_k y_{k-1} + b_k with |a_k| < 1; W warps share a row,
+// each lane holds kTriChunk consecutive unknowns, composes their affine maps,
+// and the maps' prefix is scanned over the lanes (and the warps).  So a row
+// takes two serial chains of kTriChunk steps and five shuffle rounds each
+// instead of two chains of n steps.
+#pragma once
+
+#include "kernels.cuh"
+
+namespace ins2d {
+
+constexpr int kTriChunk = 8;
+
+__device__ __forceinline__ double tri_warp_sum(double v) {
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+  return v;
+}
+
+// Row b (systems b of F; b >= F.nm: no row, the threads only take part in the
+// barriers) by W warps of a block of 4; wr: this warp's place in the row.
+// sh: 4 x 4 doubles per block, unused (may be null) for W == 1, which has no
+// block-level synchronisation.
+template <int W>
+__device__ __forceinline__ void tri_row(const FdmD &F, int b, int wr, double (*sh)[4]) {
+  constexpr int C = kTriChunk;
+  constexpr unsigned ALL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, w0 = warp - wr;  // w0: the row's first warp
+  const int n = F.n, s0 = (wr * 32 + lane) * C;
+  const bool row = b < F.nm;
+  double *__restrict__ w = F.t + (size_t)(row ? b : 0) * n;
+  const double *__restrict__ pv = F.piv + (size_t)(row ? b : 0) * n;
+  const bool null = row && b == F.null_mode;
+  double y[C], m[C], e[C];
+  const double ep = (row && s0 > 0 && s0 <= n) ? __ldg(F.e + s0 - 1) : 0.0;
+#pragma unroll
+  for (int k = 0; k < C; ++k) {
+    const bool in = row && s0 + k < n;
+    y[k] = in ? w[s0 + k] : 0.0;
+    m[k] = in ? __ldg(pv + s0 + k) : 0.0;
+    e[k] = in ? __ldg(F.e + s0 + k) : 0.0;
+  }
+  // the null mode: a right-hand side without its component along diag(h) 1
+  double sum = 0.0;
+  if (null) {
+#pragma unroll
+    for (int k = 0; k < C; ++k) sum += y[k];
+    sum = tri_warp_sum(sum);
+  }
+  if constexpr (W > 1) {
+    if (lane == 0) sh[warp][0] = sum;
+    __syncthreads();
+    if (null) {
+      sum = 0.0;
+#pragma unroll
+      for (int v = 0; v < W; ++v) sum += sh[w0 + v][0];
+    }
+  }
+  if (null) {
+    const double c = sum / F.hsum;
+#pragma unroll
+    for (int k = 0; k < C; ++k)
+      if (s0 + k < n) y[k] -= __ldg(F.h + s0 + k) * c;
+  }
+  // elimination: y_k = -(w_k + e_{k-1} y_{k-1}) m_k
+  double A = 1.0, B = 0.0;
+#pragma unroll
+  for (int k = 0; k < C; ++k) {
+    const double a = -(k ? e[k - 1] : ep) * m[k];
+    y[k] = -y[k] * m[k];
+    B = fma(a, B, y[k]);
+    A *= a;
+  }
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const double a2 = __shfl_up_sync(ALL, A, d), b2 = __shfl_up_sync(ALL, B, d);
+    if (lane >= d) {
+      B = fma(A, b2, B);
+      A *= a2;
+    }
+  }
+  double y0 = 0.0;  // value just before this warp's part
+  if constexpr (W > 1) {
+    if (lane == 31) {
+      sh[warp][1] = A;
+      sh[warp][2] = B;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int v = 0; v < W - 1; ++v)
+      if (v < wr) y0 = fma(sh[w0 + v][1], y0, sh[w0 + v][2]);
+  }
+  double yi;
+  {
+    const double a2 = __shfl_up_sync(ALL, A, 1), b2 = __shfl_up_sync(ALL, B, 1);
+    yi = lane ? fma(a2, y0, b2) : y0;
+  }
+#pragma unroll
+  for (int k = 0; k < C; ++k) {
+    y[k] = fma(-(k ? e[k - 1] : ep) * m[k], yi, y[k]);
+    yi = y[k];
+  }
+  // back substitution: z_k = y_k - e_k m_k z_{k+1}
+  A = 1.0;
+  B = 0.0;
+#pragma unroll
+  for (int k = C - 1; k >= 0; --k) {
+    const double a = -e[k] * m[k];
+    B = fma(a, B, y[k]);
+    A *= a;
+  }
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const double a2 = __shfl_down_sync(ALL, A, d), b2 = __shfl_down_sync(ALL, B, d);
+    if (lane + d < 32) {
+      B = fma(A, b2, B);
+      A *= a2;
+    }
+  }
+  y0 = 0.0;
+  if constexpr (W > 1) {
+    __syncthreads();
+    if (lane == 0) {
+      sh[warp][1] = A;
+      sh[warp][2] = B;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int v = W - 1; v > 0; --v)
+      if (v > wr) y0 = fma(sh[w0 + v][1], y0, sh[w0 + v][2]);
+  }
+  {
+    const double a2 = __shfl_down_sync(ALL, A, 1), b2 = __shfl_down_sync(ALL, B, 1);
+    yi = lane < 31 ? fma(a2, y0, b2) : y0;
+  }
+#pragma unroll
+  for (int k = C - 1; k >= 0; --k) {
+    y[k] = fma(-e[k] * m[k], yi, y[k]);
+    yi = y[k];
+  }
+  // cyclic systems: zh = y - (y_0 + cr y_{n-1}) g; null mode: the h-weighted
+  // mean removed.  Both need one value of the whole row.
+  double part = 0.0;
+  const bool cyc = row && F.g && !null;
+  if (cyc) {
+    const double cr = __ldg(F.cr + b);
+#pragma unroll
+    for (int k = 0; k < C; ++k) {
+      if (s0 + k == 0) part += y[k];
+      if (s0 + k == n - 1) part += cr * y[k];
+    }
+  } else if (null) {
+#pragma unroll
+    for (int k = 0; k < C; ++k)
+      if (s0 + k < n) part += __ldg(F.h + s0 + k) * y[k];
+  }
+  if (cyc || null) part = tri_warp_sum(part);
+  if constexpr (W > 1) {
+    if (lane == 0) sh[warp][3] = part;
+    __syncthreads();
+    if (cyc || null) {
+      part = 0.0;
+#pragma unroll
+      for (int v = 0; v < W; ++v) part += sh[w0 + v][3];
+    }
+  }
+  if (cyc) {
+    const double *__restrict__ g = F.g + (size_t)b * n;
+#pragma unroll
+    for (int k = 0; k < C; ++k)
+      if (s0 + k < n) y[k] -= part * __ldg(g + s0 + k);
+  } else if (null) {
+    const double c = part / F.hsum;
+#pragma unroll
+    for (int k = 0; k < C; ++k) y[k] -= c;
+  }
+#pragma unroll
+  for (int k = 0; k < C; ++k)
+    if (row && s0 + k < n) w[s0 + k] = y[k];
+}
+
+}  // namespace ins2d

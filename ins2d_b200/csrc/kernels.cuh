@@ -210,38 +210,47 @@ cudaError_t launch_fft_poisson_div_split(const DevOps &P, const FftPlan &plan, c
 // device; returns the first failure.
 cudaError_t fft_prepare();
 
-// --- fast-diagonalization preconditioner (fdm.cu) -----------------------------------
-// Generalized eigenbases of the pressure matrix's 1D factors (fdm_host.cpp)
-// and the work arrays of one application.
+// --- fast-diagonalization preconditioner (fdm.cu, fdm_tri.cuh) ----------------------
+// The separable inverse with one diagonalized direction (fdm_host.hpp,
+// FdmTri) and the work arrays of one application.
 struct FdmD {
   int nx = 0, ny = 0;
-  const double *Qx = nullptr, *Qy = nullptr;  // nx x nx, ny x ny row-major (Q[i*n + a])
-  const double *lx = nullptr, *ly = nullptr;  // eigenvalues
-  double thr = 0.0;                           // lx + ly <= thr: the null mode (left out)
-  double *t1 = nullptr, *t2 = nullptr;        // nx*ny each
-  double *z = nullptr;                        // the preconditioned residual
+  int nsm = 148;                  // multiprocessors (tile shape of the products)
+  int nm = 0, n = 0, xmodes = 0;  // modes, unknowns per system, modes along x
+  const double *Q = nullptr;      // nm x nm row-major (Q[i*nm + b])
+  const double *piv = nullptr, *e = nullptr, *h = nullptr;  // nm x n, n, n
+  const double *g = nullptr, *cr = nullptr;                 // cyclic systems: nm x n, nm
+  int null_mode = -1;
+  double hsum = 0.0;
+  const double *r = nullptr;  // ensembles: the member's CG residual
+  double *t = nullptr;        // nm x n: transformed residual, then the systems' solutions
+  double *z = nullptr;        // the preconditioned residual
   // periodic uniform grids: the Fourier basis, applied by the FFT solve
   bool spectral = false;
   const FftPlan *fft = nullptr;
   const unsigned long long *gate = nullptr;  // device word holding 1.0 (no early return)
 };
-// z = A^+ r (four dense products); no work once *done is set (done may be null)
-void fdm_apply(const FdmD &F, const double *r, double *z, const int *done, cudaStream_t s);
-// one ensemble member's fast-diagonalization data (device copy): z = A^+ r
-struct EnsFdmD {
-  int nx, ny;
-  const double *Qx, *Qy, *lx, *ly;
-  double thr;
-  const double *r;  // the member's CG residual
-  double *t1, *t2, *z;
-};
+struct PcgWork;
+// opts the product kernels in to their dynamic shared memory on the current device
+cudaError_t fdm_prepare();
+// z = A^+ r (product, tridiagonal systems, product) and the PCG's r'z: on the
+// first application (init) also p = z.  No work once W.sc->done is set.
+void fdm_apply(const FdmD &F, const PcgWork &W, const double *r, bool init, cudaStream_t s);
 struct EnsCg;
-// Host: the 64x64 output tiles {member, tile row, tile column, 0} of a member
-// with an ny x nx pressure grid
-void fdm_tiles(int member, int nx, int ny, std::vector<int4> &out);
-// z = A^+ r for every member not yet converged (cg[m].done == 0): the four
-// products, one launch each over all members' tiles
-void fdm_apply_ens(const EnsFdmD *F, const int4 *tiles, int ntiles, const EnsCg *cg, cudaStream_t s);
+// Work lists of an ensemble's applications: output tiles {member, tile row,
+// tile column, 0} of the products and groups of rows {member, first row} of
+// the tridiagonal systems
+struct EnsFdmPlan {
+  const FdmD *F = nullptr;
+  const int4 *tiles = nullptr;
+  const int2 *rows = nullptr;
+  int ntiles = 0, nrows = 0, cfg = 0, warps = 1;
+};
+// Host: the tile shape for the members' sizes, and the lists
+void fdm_ens_lists(const std::vector<FdmD> &F, const std::vector<int> &order, int nsm, EnsFdmPlan &pl,
+                   std::vector<int4> &tiles, std::vector<int2> &rows);
+// z = A^+ r for every member not yet converged (cg[m].done == 0)
+void fdm_apply_ens(const EnsFdmPlan &pl, const EnsCg *cg, cudaStream_t s);
 
 // --- PCG (pcg.cu) ---------------------------------------------------------------
 struct PcgScalars {

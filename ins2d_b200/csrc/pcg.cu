@@ -43,14 +43,13 @@ __device__ __forceinline__ RedScratch red_of(const PcgWork &W) {
 }
 
 // q = A p and p'q (alpha), walking columns: a thread takes one column i and
-// kSpmvRows rows, so the x-row of TX at i (columns and weights) is read once,
+// `rows` rows, so the x-row of TX at i (columns and weights) is read once,
 // the TY row of each j is a warp-uniform read, and the p values of a column
 // reach the thread through L1.  Same arithmetic per cell as lap().
-constexpr int kSpmvRows = 16;
-__global__ void __launch_bounds__(256) k_spmv_cols(const __grid_constant__ DevOps P, const PcgWork W) {
+__global__ void __launch_bounds__(256) k_spmv_cols(const __grid_constant__ DevOps P, const PcgWork W, int rows) {
   if (*(volatile int *)&W.sc->done) return;
   const int i = blockIdx.x * BX + threadIdx.x;
-  const int j0 = (blockIdx.y * BY + threadIdx.y) * kSpmvRows;
+  const int j0 = (blockIdx.y * BY + threadIdx.y) * rows;
   double q1[1] = {0.0};
   const int ops[1] = {R_SUM};
   if (i < P.Npx && j0 < P.Npy) {
@@ -59,7 +58,7 @@ __global__ void __launch_bounds__(256) k_spmv_cols(const __grid_constant__ DevOp
     const int cx0 = __ldg(cx), cx1 = __ldg(cx + 1), cx2 = __ldg(cx + 2);
     const double wx0 = __ldg(wx), wx1 = __ldg(wx + 1), wx2 = __ldg(wx + 2);
     const double hxi = __ldg(P.hx + i);
-    const int j1 = min(j0 + kSpmvRows, P.Npy);
+    const int j1 = min(j0 + rows, P.Npy);
     const double *__restrict__ p = W.p;
 #pragma unroll 4
     for (int j = j0; j < j1; ++j) {
@@ -90,8 +89,13 @@ __global__ void __launch_bounds__(256) k_spmv_cols(const __grid_constant__ DevOp
     }
   }
 }
-inline dim3 spmv_grid(const DevOps &P) {
-  return dim3((P.Npx + BX - 1) / BX, (P.Npy + BY * kSpmvRows - 1) / (BY * kSpmvRows));
+// rows per thread: 16 (the column's table row is read once for all of them),
+// fewer while the launch has less than two blocks per SM
+void launch_spmv(const DevOps &P, const PcgWork &W, cudaStream_t s) {
+  int rows = 16;
+  auto grid = [&](int r) { return dim3((P.Npx + BX - 1) / BX, (P.Npy + BY * r - 1) / (BY * r)); };
+  while (rows > 1 && (long long)grid(rows).x * grid(rows).y < 2LL * P.nsm) rows >>= 1;
+  k_spmv_cols<<<grid(rows), dim3(BX, BY), 0, s>>>(P, W, rows);
 }
 
 __global__ void __launch_bounds__(256) k_update(const __grid_constant__ DevOps P, const PcgWork W) {
@@ -610,7 +614,7 @@ void pcg_init(const DevOps &P, const PcgWork &W, const double *f, double tol, lo
 void pcg_iterations(const DevOps &P, const PcgWork &W, int n, cudaStream_t s) {
   const dim3 g = pgrid(P), b(BX, BY);
   for (int it = 0; it < n; ++it) {
-    k_spmv_cols<<<spmv_grid(P), b, 0, s>>>(P, W);
+    launch_spmv(P, W, s);
     k_update<<<g, b, 0, s>>>(P, W);
     k_pupdate<<<g, b, 0, s>>>(P, W);
   }
@@ -636,29 +640,28 @@ void pcg_iterations_mg(const DevOps &P, const MgD &M, const PcgWork &W, int n, c
   }
 }
 
-namespace {
-void precond_fdm(const DevOps &P, const FdmD &F, const PcgWork &W, cudaStream_t s) {
-  if (F.spectral)
-    launch_fft_precond(P, *F.fft, W.r, F.z, F.gate, &W.sc->done, s);
-  else
-    fdm_apply(F, W.r, F.z, &W.sc->done, s);
-}
-}  // namespace
-
 void pcg_init_fdm(const DevOps &P, const FdmD &F, const PcgWork &W, const double *f, double tol, long long maxit,
                   cudaStream_t s) {
   k_init_g<<<vec_blocks(P, W), kVecThreads, 0, s>>>(P, W, f, tol * tol, maxit);
-  precond_fdm(P, F, W, s);
-  k_rz_g<<<vec_blocks(P, W), kVecThreads, 0, s>>>(W, F.z, P.Np, 1);
+  if (F.spectral) {
+    launch_fft_precond(P, *F.fft, W.r, F.z, F.gate, &W.sc->done, s);
+    k_rz_g<<<vec_blocks(P, W), kVecThreads, 0, s>>>(W, F.z, P.Np, 1);
+  } else {
+    fdm_apply(F, W, W.r, true, s);
+  }
 }
 
 void pcg_iterations_fdm(const DevOps &P, const FdmD &F, const PcgWork &W, int n, cudaStream_t s) {
   const unsigned g = vec_blocks(P, W);
   for (int it = 0; it < n; ++it) {
-    k_spmv_cols<<<spmv_grid(P), dim3(BX, BY), 0, s>>>(P, W);
+    launch_spmv(P, W, s);
     k_update_g<<<g, kVecThreads, 0, s>>>(W, P.Np);
-    precond_fdm(P, F, W, s);
-    k_rz_g<<<g, kVecThreads, 0, s>>>(W, F.z, P.Np, 0);
+    if (F.spectral) {
+      launch_fft_precond(P, *F.fft, W.r, F.z, F.gate, &W.sc->done, s);
+      k_rz_g<<<g, kVecThreads, 0, s>>>(W, F.z, P.Np, 0);
+    } else {
+      fdm_apply(F, W, W.r, false, s);
+    }
     k_pupdate_g<<<g, kVecThreads, 0, s>>>(W, F.z, P.Np);
   }
 }
