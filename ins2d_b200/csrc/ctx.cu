@@ -316,6 +316,9 @@ void capture_while(cudaStream_t s, cudaStream_t body_stream, Pre pre, Body body)
   CK(ee);
 }
 
+// kernels of one pass of the fast-diagonalization PCG
+long long fdm_pass_kernels(const ins2d_ctx *c) { return c->fdm.spectral ? 3LL + fft_kernels(c->fdm_fft) : 5LL; }
+
 // The PCG solve inside a step being captured as a CUDA graph (c->dev_loop):
 // no host round trip.  The iterations are the body of a conditional WHILE
 // node, captured on the context's second stream into the node's body graph;
@@ -340,24 +343,34 @@ int solve_pcg_graph(ins2d_ctx *c, const double *f, double *dp, bool accumulate, 
     CK(cudaGetLastError());
     return INS2D_OK;
   }
-  if (c->use_fdm)
-    pcg_init_fdm(c->P, c->fdm, c->pcg, f, tol, c->opts.CG_maxit, c->stream);
-  else if (c->use_mg)
+  const int chunk = (c->use_fdm || c->use_mg) ? 1 : 4;
+  const long long lim = c->poll_limit >= 0 ? c->poll_limit : (long long)c->opts.CG_maxit / chunk + 4;
+  const int limit = (int)std::min<long long>(lim, 1 << 30);
+  if (c->use_fdm) {
+    // the kernels that know the state of the solve set the condition themselves
+    capture_while(
+        c->stream, c->body_stream,
+        [&](cudaGraphConditionalHandle h) {
+          pcg_init_fdm(c->P, c->fdm, c->pcg, f, tol, c->opts.CG_maxit, h, limit, c->stream);
+        },
+        [&](cudaStream_t bs, cudaGraphConditionalHandle h) {
+          CK(pcg_pass_fdm(c->P, c->fdm, c->pcg, f, h, limit, bs));
+          c->launches[INS2D_PROF_POISSON] += fdm_pass_kernels(c);
+        });
+    pcg_finish_fdm(c->P, c->pcg, dp, accumulate, c->accum, c->stream);
+    CK(cudaGetLastError());
+    return INS2D_OK;
+  }
+  if (c->use_mg)
     pcg_init_mg(c->P, c->mg, c->pcg, f, tol, c->opts.CG_maxit, c->stream);
   else
     pcg_init(c->P, c->pcg, f, tol, c->opts.CG_maxit, c->stream);
   CK(cudaGetLastError());
-  const int chunk = (c->use_fdm || c->use_mg) ? 1 : 4;
-  const long long lim = c->poll_limit >= 0 ? c->poll_limit : (long long)c->opts.CG_maxit / chunk + 4;
-  const int limit = (int)std::min<long long>(lim, 1 << 30);
   capture_while(
       c->stream, c->body_stream,
       [&](cudaGraphConditionalHandle h) { launch_pcg_cond(c->pcg.sc, h, limit, 0, c->stream); },
       [&](cudaStream_t bs, cudaGraphConditionalHandle h) {
-        if (c->use_fdm) {
-          pcg_iterations_fdm(c->P, c->fdm, c->pcg, chunk, bs);
-          c->launches[INS2D_PROF_POISSON] += (c->fdm.spectral ? 4LL + fft_kernels(c->fdm_fft) : 6LL) * chunk;
-        } else if (c->use_mg) {
+        if (c->use_mg) {
           pcg_iterations_mg(c->P, c->mg, c->pcg, chunk, bs);
           c->launches[INS2D_PROF_POISSON] += (long long)(4 + 6 * mg_tail_level(c->mg) + 1) * chunk;
         } else {
@@ -409,26 +422,29 @@ int solve_pcg(ins2d_ctx *c, const double *f, double *dp, bool accumulate, ins2d_
     return INS2D_OK;
   }
   if (c->use_fdm)
-    pcg_init_fdm(c->P, c->fdm, c->pcg, f, tol, c->opts.CG_maxit, c->stream);
+    pcg_init_fdm(c->P, c->fdm, c->pcg, f, tol, c->opts.CG_maxit, 0, -1, c->stream);
   else if (c->use_mg)
     pcg_init_mg(c->P, c->mg, c->pcg, f, tol, c->opts.CG_maxit, c->stream);
   else
     pcg_init(c->P, c->pcg, f, tol, c->opts.CG_maxit, c->stream);
   CK(cudaGetLastError());
   // the fast-diagonalization preconditioner is exact up to rounding: one
-  // iteration at a time between the polls
+  // iteration at a time between the polls, the first one before any poll
+  // (its kernels return at once when there is nothing to solve)
+  const long long limit = c->poll_limit >= 0 ? c->poll_limit : (long long)c->opts.CG_maxit + 1024;
   int chunk = c->use_fdm ? 1 : (c->use_mg ? 2 : 4);
   long long launched = 0;
   for (;;) {
-    CK(cudaMemcpyAsync(c->h_sc, c->pcg.sc, sizeof(PcgScalars), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
-    if (c->h_sc->done) break;
-    const long long limit = c->poll_limit >= 0 ? c->poll_limit : (long long)c->opts.CG_maxit + 1024;
-    if (launched >= limit)
-      return fail(c, INS2D_ETIMEOUT, "PCG: device convergence flag not set within the host's iteration limit");
+    if (!(c->use_fdm && launched == 0 && limit > 0)) {
+      CK(cudaMemcpyAsync(c->h_sc, c->pcg.sc, sizeof(PcgScalars), cudaMemcpyDeviceToHost, c->stream));
+      CK(cudaStreamSynchronize(c->stream));
+      if (c->h_sc->done) break;
+      if (launched >= limit)
+        return fail(c, INS2D_ETIMEOUT, "PCG: device convergence flag not set within the host's iteration limit");
+    }
     if (c->use_fdm) {
-      pcg_iterations_fdm(c->P, c->fdm, c->pcg, chunk, c->stream);
-      c->launches[INS2D_PROF_POISSON] += (c->fdm.spectral ? 4LL + fft_kernels(c->fdm_fft) : 6LL) * chunk;
+      CK(pcg_pass_fdm(c->P, c->fdm, c->pcg, f, 0, -1, c->stream));
+      c->launches[INS2D_PROF_POISSON] += fdm_pass_kernels(c);
     } else if (c->use_mg) {
       pcg_iterations_mg(c->P, c->mg, c->pcg, chunk, c->stream);
       c->launches[INS2D_PROF_POISSON] += (long long)(4 + 6 * mg_tail_level(c->mg) + 1) * chunk;
@@ -454,7 +470,10 @@ int solve_pcg(ins2d_ctx *c, const double *f, double *dp, bool accumulate, ins2d_
   }
   if (h.status == INS2D_EBREAKDOWN) return fail(c, INS2D_EBREAKDOWN, "PCG breakdown: p'Ap = 0");
   if (h.status == INS2D_ENONFINITE) return fail(c, INS2D_ENONFINITE, "PCG: non-finite residual");
-  pcg_finish(c->P, c->pcg, dp, accumulate, c->stream);
+  if (c->use_fdm)
+    pcg_finish_fdm(c->P, c->pcg, dp, accumulate, nullptr, c->stream);
+  else
+    pcg_finish(c->P, c->pcg, dp, accumulate, c->stream);
   c->launches[INS2D_PROF_POISSON] += 1;
   CK(cudaGetLastError());
   return INS2D_OK;
@@ -1029,6 +1048,7 @@ int ins2d_ctx_create(const ins2d_grid_desc *grid, const ins2d_bc_desc *bc, const
       W.r = dalloc<double>(c, Np);
       W.p = dalloc<double>(c, Np);
       W.q = dalloc<double>(c, Np);
+      W.p2 = dalloc<double>(c, Np);
       W.sc = dalloc<PcgScalars>(c, 1);
       W.blocks = pcg_blocks(P);
       W.partials = dalloc<double>(c, (size_t)W.blocks * 8 + 16);

@@ -194,23 +194,22 @@ __device__ __forceinline__ void fdm_backward(const FdmD &F, int m0, int n0, Epi 
 }
 
 template <int CFG>
-__global__ void __launch_bounds__(kThreads) k_fdm_fwd(const __grid_constant__ FdmD F, const double *__restrict__ r,
-                                                      const int *__restrict__ done) {
-  if (*(volatile const int *)done) return;
-  fdm_forward<CFG>(F, r, blockIdx.y * Tile<CFG>::BM, blockIdx.x * Tile<CFG>::BN);
+__global__ void __launch_bounds__(kThreads) k_fdm_fwd(const __grid_constant__ FdmD F, const PcgWork W,
+                                                      const double *__restrict__ f) {
+  if (*(volatile const int *)&W.sc->done) return;
+  fdm_forward<CFG>(F, W.sc->it == 0 ? f : W.r, blockIdx.y * Tile<CFG>::BM, blockIdx.x * Tile<CFG>::BN);
 }
 
-// z = Q zh with r'z reduced in the same pass (deterministic, reduce.cuh):
-// init: rz, and p = z; otherwise beta = rz / rz_old
+// z = Q zh with r'z reduced in the same pass (deterministic, reduce.cuh)
 template <int CFG>
 __global__ void __launch_bounds__(kThreads) k_fdm_bwd(const __grid_constant__ FdmD F, const PcgWork W,
-                                                      const double *__restrict__ r, int init) {
+                                                      const double *__restrict__ f) {
   if (*(volatile int *)&W.sc->done) return;
+  const double *__restrict__ r = W.sc->it == 0 ? f : W.r;
   double q[1] = {0.0};
   const int ops[1] = {R_SUM};
   fdm_backward<CFG>(F, blockIdx.y * Tile<CFG>::BM, blockIdx.x * Tile<CFG>::BN, [&](size_t k, double v) {
     F.z[k] = v;
-    if (init) W.p[k] = v;
     q[0] += __ldg(r + k) * v;
   });
   RedScratch red;
@@ -219,18 +218,7 @@ __global__ void __launch_bounds__(kThreads) k_fdm_bwd(const __grid_constant__ Fd
   red.result = W.partials + (size_t)W.blocks * 8;
   red.max_blocks = W.blocks;
   double out[1];
-  if (grid_reduce<1>(q, ops, red, out)) {
-    PcgScalars *s = W.sc;
-    if (!isfinite(out[0])) {
-      s->status = INS2D_ENONFINITE;
-      s->done = 1;
-    } else if (init) {
-      s->rz = out[0];
-    } else {
-      s->beta = out[0] / s->rz;
-      s->rz = out[0];
-    }
-  }
+  if (grid_reduce<1>(q, ops, red, out)) pcg_new_rz(W.sc, out[0]);
 }
 
 template <int W>
@@ -282,14 +270,14 @@ int row_warps(int n) { return n <= 32 * kTriChunk ? 1 : (n <= 64 * kTriChunk ? 2
 static_assert(4 * 32 * kTriChunk >= 1024, "four warps hold the longest row (kFdmMaxN)");
 
 template <int CFG>
-void launch_fwd(const FdmD &F, const double *r, const int *done, cudaStream_t s) {
+void launch_fwd(const FdmD &F, const PcgWork &W, const double *f, cudaStream_t s) {
   const dim3 g((F.n + Tile<CFG>::BN - 1) / Tile<CFG>::BN, (F.nm + Tile<CFG>::BM - 1) / Tile<CFG>::BM);
-  k_fdm_fwd<CFG><<<g, kThreads, tile_smem<CFG>(), s>>>(F, r, done);
+  k_fdm_fwd<CFG><<<g, kThreads, tile_smem<CFG>(), s>>>(F, W, f);
 }
 template <int CFG>
-void launch_bwd(const FdmD &F, const PcgWork &W, const double *r, bool init, cudaStream_t s) {
+void launch_bwd(const FdmD &F, const PcgWork &W, const double *f, cudaStream_t s) {
   const dim3 g((F.nx + Tile<CFG>::BN - 1) / Tile<CFG>::BN, (F.ny + Tile<CFG>::BM - 1) / Tile<CFG>::BM);
-  k_fdm_bwd<CFG><<<g, kThreads, tile_smem<CFG>(), s>>>(F, W, r, init ? 1 : 0);
+  k_fdm_bwd<CFG><<<g, kThreads, tile_smem<CFG>(), s>>>(F, W, f);
 }
 template <int W>
 void launch_tri(const FdmD &F, const int *done, cudaStream_t s) {
@@ -316,17 +304,17 @@ cudaError_t fdm_prepare() {
   return first;
 }
 
-void fdm_apply(const FdmD &F, const PcgWork &W, const double *r, bool init, cudaStream_t s) {
+void fdm_apply(const FdmD &F, const PcgWork &W, const double *f, cudaStream_t s) {
   const int *done = &W.sc->done;
   const int cfg = tile_config(tiles_of(F.ny, F.nx, 64, 64),
                               std::min(tiles_of(F.ny, F.nx, 64, 32), tiles_of(F.nx, F.ny, 64, 32)),
                               tiles_of(F.ny, F.nx, 32, 32), F.nsm);
   if (cfg == 0)
-    launch_fwd<0>(F, r, done, s);
+    launch_fwd<0>(F, W, f, s);
   else if (cfg == 1)
-    launch_fwd<1>(F, r, done, s);
+    launch_fwd<1>(F, W, f, s);
   else
-    launch_fwd<2>(F, r, done, s);
+    launch_fwd<2>(F, W, f, s);
   const int w = row_warps(F.n);
   if (w == 1)
     launch_tri<1>(F, done, s);
@@ -335,11 +323,11 @@ void fdm_apply(const FdmD &F, const PcgWork &W, const double *r, bool init, cuda
   else
     launch_tri<4>(F, done, s);
   if (cfg == 0)
-    launch_bwd<0>(F, W, r, init, s);
+    launch_bwd<0>(F, W, f, s);
   else if (cfg == 1)
-    launch_bwd<1>(F, W, r, init, s);
+    launch_bwd<1>(F, W, f, s);
   else
-    launch_bwd<2>(F, W, r, init, s);
+    launch_bwd<2>(F, W, f, s);
 }
 
 void fdm_ens_lists(const std::vector<FdmD> &F, const std::vector<int> &order, int nsm, EnsFdmPlan &pl,

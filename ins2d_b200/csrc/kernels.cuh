@@ -11,6 +11,7 @@
 namespace ins2d {
 
 constexpr int kMaxStages = 8;
+constexpr int kStatusNonFinite = 4;  // INS2D_ENONFINITE
 
 // Programmatic dependent launch of the explicit step's kernels (the stage and
 // residual walkers, the FFT passes, the projections): off unless INS2D_PDL=1
@@ -233,9 +234,9 @@ struct FdmD {
 struct PcgWork;
 // opts the product kernels in to their dynamic shared memory on the current device
 cudaError_t fdm_prepare();
-// z = A^+ r (product, tridiagonal systems, product) and the PCG's r'z: on the
-// first application (init) also p = z.  No work once W.sc->done is set.
-void fdm_apply(const FdmD &F, const PcgWork &W, const double *r, bool init, cudaStream_t s);
+// z = A^+ r (product, tridiagonal systems, product) and the PCG's r'z, beta;
+// r = f on the first pass, W.r later.  No work once W.sc->done is set.
+void fdm_apply(const FdmD &F, const PcgWork &W, const double *f, cudaStream_t s);
 struct EnsCg;
 // Work lists of an ensemble's applications: output tiles {member, tile row,
 // tile column, 0} of the products and groups of rows {member, first row} of
@@ -278,6 +279,7 @@ void launch_pcg_cond(PcgScalars *sc, cudaGraphConditionalHandle h, int limit, in
 void launch_solve_accum(const PcgScalars *sc, SolveAccum *acc, cudaStream_t s);
 struct PcgWork {
   double *x, *r, *p, *q;
+  double *p2;          // fast diagonalization: directions alternate between p and p2
   PcgScalars *sc;      // device
   double *partials;    // >= blocks * 4
   int blocks;
@@ -291,10 +293,26 @@ int pcg_blocks(const DevOps &P);
 void pcg_init_mg(const DevOps &P, const MgD &M, const PcgWork &W, const double *f, double tol, long long maxit,
                  cudaStream_t s);
 void pcg_iterations_mg(const DevOps &P, const MgD &M, const PcgWork &W, int n, cudaStream_t s);
-// The same with the fast-diagonalization preconditioner
+// The same with the fast-diagonalization preconditioner: the solve's scalars;
+// one pass (application, direction and product, update); dp from the solution
+// (acc: its statistics, or null).  h: the condition of the WHILE node around
+// the passes, set while the solve needs another one and fewer than `limit`
+// ran (limit < 0: none).  f must stay unchanged until the passes are done.
 void pcg_init_fdm(const DevOps &P, const FdmD &F, const PcgWork &W, const double *f, double tol, long long maxit,
-                  cudaStream_t s);
-void pcg_iterations_fdm(const DevOps &P, const FdmD &F, const PcgWork &W, int n, cudaStream_t s);
+                  cudaGraphConditionalHandle h, int limit, cudaStream_t s);
+cudaError_t pcg_pass_fdm(const DevOps &P, const FdmD &F, const PcgWork &W, const double *f,
+                         cudaGraphConditionalHandle h, int limit, cudaStream_t s);
+void pcg_finish_fdm(const DevOps &P, const PcgWork &W, double *dp, bool accumulate, SolveAccum *acc, cudaStream_t s);
+// r'z of a new application (one thread): the first one's, or beta
+__device__ __forceinline__ void pcg_new_rz(PcgScalars *s, double rz) {
+  if (!isfinite(rz)) {
+    s->status = kStatusNonFinite;
+    s->done = 1;
+  } else {
+    s->beta = s->it == 0 ? 0.0 : rz / s->rz;
+    s->rz = rz;
+  }
+}
 // small grids (at most 128 cells per direction, not the spectral form): the
 // whole fast-diagonalization PCG solve in one thread block
 bool pcg_use_block_fdm(const FdmD &F);
