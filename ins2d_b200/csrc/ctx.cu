@@ -162,7 +162,6 @@ void upload_fdm(ins2d_ctx *c, FdmD &D) {
   const FdmTri T = fdm_tri(c->H.TX, c->H.hx, c->H.TY, c->H.hy);
   D.nx = c->H.Npx;
   D.ny = c->H.Npy;
-  D.nsm = c->P.nsm;
   D.nm = T.nm;
   D.n = T.n;
   D.xmodes = T.xmodes ? 1 : 0;
@@ -328,13 +327,10 @@ long long fdm_pass_kernels(const ins2d_ctx *c) { return c->fdm.spectral ? 3LL + 
 // added to c->accum, which the host reads after the graph launches (cg.F's
 // errors are reported then).
 int solve_pcg_graph(ins2d_ctx *c, const double *f, double *dp, bool accumulate, double tol) {
-  const bool block = c->use_fdm ? pcg_use_block_fdm(c->fdm)
-                                : (c->use_mg ? (c->P.Np <= kPcgBlockMgMaxCells) : pcg_use_block(c->P));
+  const bool block = !c->use_fdm && (c->use_mg ? (c->P.Np <= kPcgBlockMgMaxCells) : pcg_use_block(c->P));
   Prof pr(c, INS2D_PROF_POISSON, block ? 1 : 2);
   if (block) {
-    if (c->use_fdm)
-      pcg_solve_block_fdm(c->P, c->fdm, c->pcg, f, dp, tol, c->opts.CG_maxit, accumulate, c->stream);
-    else if (c->use_mg)
+    if (c->use_mg)
       pcg_solve_block_mg(c->P, c->mg, c->pcg, f, dp, tol, c->opts.CG_maxit, accumulate, c->stream);
     else
       pcg_solve_block(c->P, c->pcg, f, dp, tol, c->opts.CG_maxit, accumulate, c->stream);
@@ -386,40 +382,66 @@ int solve_pcg_graph(ins2d_ctx *c, const double *f, double *dp, bool accumulate, 
   return INS2D_OK;
 }
 
+// statistics and status of the finished solve in c->h_sc
+int solve_outcome(ins2d_ctx *c, ins2d_solve_stats *st) {
+  const PcgScalars &h = *c->h_sc;
+  if (st) {
+    st->iters = (int32_t)h.it;
+    st->norm1 = std::sqrt(h.rr);
+    st->norm2 = (h.maxx - h.minx) != 0.0 ? h.maxres / (h.maxx - h.minx) : 0.0;
+  }
+  if (h.status == INS2D_ENOTCONV) {
+    char buf[160];
+    snprintf(buf, sizeof buf, "CG didn't converge in %d iterations; residual= %g", c->opts.CG_maxit, std::sqrt(h.rr));
+    return fail(c, INS2D_ENOTCONV, buf);
+  }
+  if (h.status == INS2D_EBREAKDOWN) return fail(c, INS2D_EBREAKDOWN, "PCG breakdown: p'Ap = 0");
+  if (h.status == INS2D_ENONFINITE) return fail(c, INS2D_ENONFINITE, "PCG: non-finite residual");
+  return INS2D_OK;
+}
+
+// the same for a single-launch solve, read back from the device
+int read_solve(ins2d_ctx *c, ins2d_solve_stats *st) {
+  CK(cudaMemcpyAsync(c->h_sc, c->pcg.sc, sizeof(PcgScalars), cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaStreamSynchronize(c->stream));
+  return solve_outcome(c, st);
+}
+
+bool cluster_solver(const ins2d_ctx *c) { return c->use_fdm && pcg_use_cluster(c->fdm); }
+
+// a small grid's whole solve in one launch (inside a step graph its statistics
+// go to c->accum)
+int solve_cluster(ins2d_ctx *c, const SolveSrc &src, double *dp, bool accumulate, ins2d_solve_stats *st, double tol) {
+  if (st) *st = ins2d_solve_stats{0, 0.0, 0.0};
+  {
+    Prof pr(c, INS2D_PROF_POISSON, 1);
+    pcg_solve_cluster(c->P, c->fdm, c->pcg, src, dp, tol, c->opts.CG_maxit, accumulate,
+                      c->dev_loop ? c->accum : nullptr, c->stream);
+    CK(cudaGetLastError());
+  }
+  return c->dev_loop ? INS2D_OK : read_solve(c, st);
+}
+
 // PCG to the relative residual tol (cg.F's rule ||r|| <= tol ||f||)
 int solve_pcg(ins2d_ctx *c, const double *f, double *dp, bool accumulate, ins2d_solve_stats *st, double tol) {
+  if (cluster_solver(c)) {
+    SolveSrc src;
+    src.f = f;
+    return solve_cluster(c, src, dp, accumulate, st, tol);
+  }
   if (c->dev_loop) {
     if (st) *st = ins2d_solve_stats{0, 0.0, 0.0};
     return solve_pcg_graph(c, f, dp, accumulate, tol);
   }
-  const bool block = c->use_fdm ? pcg_use_block_fdm(c->fdm)
-                                : (c->use_mg ? (c->P.Np <= kPcgBlockMgMaxCells) : pcg_use_block(c->P));
+  const bool block = !c->use_fdm && (c->use_mg ? (c->P.Np <= kPcgBlockMgMaxCells) : pcg_use_block(c->P));
   Prof pr(c, INS2D_PROF_POISSON, block ? 1 : 2);
   if (block) {
-    if (c->use_fdm)
-      pcg_solve_block_fdm(c->P, c->fdm, c->pcg, f, dp, tol, c->opts.CG_maxit, accumulate, c->stream);
-    else if (c->use_mg)
+    if (c->use_mg)
       pcg_solve_block_mg(c->P, c->mg, c->pcg, f, dp, tol, c->opts.CG_maxit, accumulate, c->stream);
     else
       pcg_solve_block(c->P, c->pcg, f, dp, tol, c->opts.CG_maxit, accumulate, c->stream);
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(c->h_sc, c->pcg.sc, sizeof(PcgScalars), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
-    const PcgScalars &h = *c->h_sc;
-    if (st) {
-      st->iters = (int32_t)h.it;
-      st->norm1 = std::sqrt(h.rr);
-      st->norm2 = (h.maxx - h.minx) != 0.0 ? h.maxres / (h.maxx - h.minx) : 0.0;
-    }
-    if (h.status == INS2D_ENOTCONV) {
-      char buf[160];
-      snprintf(buf, sizeof buf, "CG didn't converge in %d iterations; residual= %g", c->opts.CG_maxit,
-               std::sqrt(h.rr));
-      return fail(c, INS2D_ENOTCONV, buf);
-    }
-    if (h.status == INS2D_EBREAKDOWN) return fail(c, INS2D_EBREAKDOWN, "PCG breakdown: p'Ap = 0");
-    if (h.status == INS2D_ENONFINITE) return fail(c, INS2D_ENONFINITE, "PCG: non-finite residual");
-    return INS2D_OK;
+    return read_solve(c, st);
   }
   if (c->use_fdm)
     pcg_init_fdm(c->P, c->fdm, c->pcg, f, tol, c->opts.CG_maxit, 0, -1, c->stream);
@@ -456,20 +478,8 @@ int solve_pcg(ins2d_ctx *c, const double *f, double *dp, bool accumulate, ins2d_
     launched += chunk;
     chunk = c->use_fdm ? 1 : (c->use_mg ? 4 : std::min(chunk * 2, 128));
   }
-  const PcgScalars &h = *c->h_sc;
-  if (st) {
-    st->iters = (int32_t)h.it;
-    st->norm1 = std::sqrt(h.rr);
-    st->norm2 = (h.maxx - h.minx) != 0.0 ? h.maxres / (h.maxx - h.minx) : 0.0;
-  }
-  if (h.status == INS2D_ENOTCONV) {
-    char buf[160];
-    snprintf(buf, sizeof buf, "CG didn't converge in %d iterations; residual= %g", c->opts.CG_maxit,
-             std::sqrt(h.rr));
-    return fail(c, INS2D_ENOTCONV, buf);
-  }
-  if (h.status == INS2D_EBREAKDOWN) return fail(c, INS2D_EBREAKDOWN, "PCG breakdown: p'Ap = 0");
-  if (h.status == INS2D_ENONFINITE) return fail(c, INS2D_ENONFINITE, "PCG: non-finite residual");
+  const int rc = solve_outcome(c, st);
+  if (rc) return rc;
   if (c->use_fdm)
     pcg_finish_fdm(c->P, c->pcg, dp, accumulate, nullptr, c->stream);
   else
@@ -608,8 +618,9 @@ int solve(ins2d_ctx *c, const double *f, double *dp, bool accumulate, ins2d_solv
 }
 
 // dp = pressure_poisson(f) with f = (M W + alpha yM + beta ydM) gamma: on the
-// FFT path the divergence is computed inside the first transform pass;
-// otherwise by its own kernel before the solve.
+// FFT path the divergence is computed inside the first transform pass, on
+// small grids inside the cluster solve (unless the network or a recording
+// needs f); otherwise by its own kernel before the solve.
 int solve_div(ins2d_ctx *c, const double *W, double alpha, double beta, double gamma, double *dp, bool accumulate,
               ins2d_solve_stats *st) {
   if (c->poisson == INS2D_POISSON_FFT && fft_fuses_div(c->fft)) {
@@ -618,6 +629,15 @@ int solve_div(ins2d_ctx *c, const double *W, double alpha, double beta, double g
     CK(launch_fft_poisson_div(c->P, c->fft, W, alpha, beta, gamma, dp, accumulate, c->stream));
     CK(cudaGetLastError());
     return INS2D_OK;
+  }
+  if (cluster_solver(c) && !c->cnn && c->rec_n >= c->rec_cap) {
+    SolveSrc src;
+    src.mode = 1;
+    src.f = W;
+    src.alpha = alpha;
+    src.beta = beta;
+    src.gamma = gamma;
+    return solve_cluster(c, src, dp, accumulate, st, c->opts.CG_acc);
   }
   {
     Prof pr(c, INS2D_PROF_DIV, 1);
@@ -636,6 +656,15 @@ int solve_div_split(ins2d_ctx *c, const double *Vn, const float *T, double sv, d
     CK(launch_fft_poisson_div_split(c->P, c->fft, Vn, T, sv, sa, alpha, beta, gamma, dp, accumulate, c->stream));
     CK(cudaGetLastError());
     return INS2D_OK;
+  }
+  if (cluster_solver(c) && !c->cnn && c->rec_n >= c->rec_cap) {
+    SolveSrc src;
+    src.mode = 2;
+    src.ws = WSplit{Vn, T, sv, sa};
+    src.alpha = alpha;
+    src.beta = beta;
+    src.gamma = gamma;
+    return solve_cluster(c, src, dp, accumulate, st, c->opts.CG_acc);
   }
   {
     Prof pr(c, INS2D_PROF_DIV, 1);
@@ -1087,8 +1116,8 @@ int ins2d_ctx_create(const ins2d_grid_desc *grid, const ins2d_bc_desc *bc, const
           if (std::max(H.Npx, H.Npy) > kFdmMaxN)
             throw std::invalid_argument("fast-diagonalization preconditioner: grid larger than " +
                                         std::to_string(kFdmMaxN) + " cells in a direction");
-          CK(fdm_prepare());
           upload_fdm(c, D);
+          if (pcg_use_cluster(D)) CK(pcg_cluster_prepare());
         }
         c->use_fdm = true;
       } else if (opts->precond != INS2D_PRECOND_JACOBI) {
@@ -1960,7 +1989,7 @@ void ens_build_batch(ins2d_ens *e, const std::vector<int> &order) {
   if (e->use_fdm) {
     std::vector<int4> ft;
     std::vector<int2> fr;
-    fdm_ens_lists(e->h_fdm, order, e->mem[0]->P.nsm, e->fdm_plan, ft, fr);
+    fdm_ens_lists(e->h_fdm, order, e->fdm_plan, ft, fr);
     int4 *dt = ens_alloc<int4>(e, ft.size());
     int2 *dr = ens_alloc<int2>(e, fr.size());
     CK(cudaMemcpy(dt, ft.data(), ft.size() * sizeof(int4), cudaMemcpyHostToDevice));
@@ -2284,7 +2313,6 @@ int ins2d_ens_create(int32_t n, const ins2d_grid_desc *grids, const ins2d_bc_des
               std::max(c->H.Npx, c->H.Npy) <= kFdmMaxN;
       }
       if (fdm) {
-        CK(fdm_prepare());
         std::vector<FdmD> &hf = e->h_fdm;
         hf.resize(n);
         for (int m = 0; m < n; ++m) {

@@ -12,10 +12,14 @@
 // instead costs four products.
 //
 // What bounds it: the FP64 tensor-core rate (mma.sync m8n8k4 .f64; FP64 has
-// no tcgen05 kind) on grids of 512 cells per direction and more, and on
-// smaller ones the number of output tiles (fewer than SMs) and their serial
-// K loop.  So the tile shape follows the grid (tile_config), and operand
-// slabs are copied to shared memory by cp.async, kStages - 1 slabs ahead.
+// no tcgen05 kind) on grids of more than 512 cells per direction, and on
+// smaller ones the number of output tiles and their serial K loop.  Hence
+// 32 x 32 output tiles (257 x 301 cells: 90 tiles, 512^2: 256, for 148 SMs)
+// and operand slabs copied to shared memory by cp.async, kStages - 1 ahead.
+// One solve of one pass on B200, tiles of 64 x 64 / 64 x 32 / 32 x 32 with
+// four warps / 32 x 32 with eight: 301 x 257 cells 128 / 114 / 99.0 / 98.6 us,
+// 512^2 150 / 127 / 120 / 118 us, 1024^2 276 / 334 / 281 / 285 us; 2 slabs
+// instead of 4: 512^2 129 us; slabs of depth 32: 121 us.
 #include <algorithm>
 
 #include "fdm_tri.cuh"
@@ -27,34 +31,13 @@ namespace ins2d {
 
 namespace {
 
-constexpr int kBK = 16;       // depth of an operand slab
-constexpr int kThreads = 128;  // 2 x 2 warps per output tile
-
-// tile shapes; their shared memory: kStages slabs of both operands, each
-// padded to rows of 4 mod 16 doubles, so that a warp's fragment loads (four
-// consecutive rows by four consecutive columns per half warp) hit distinct banks
-template <int CFG>
-struct Tile;
-template <>
-struct Tile<0> {
-  static constexpr int BM = 64, BN = 64, STAGES = 3;
-};
-template <>
-struct Tile<1> {
-  static constexpr int BM = 64, BN = 32, STAGES = 4;
-};
-template <>
-struct Tile<2> {
-  static constexpr int BM = 32, BN = 32, STAGES = 4;
-};
-__host__ __device__ constexpr int slab(int bmn) {
-  const int kmajor = kBK * (bmn + 4), mmajor = bmn * (kBK + 4);
-  return kmajor > mmajor ? kmajor : mmajor;
-}
-template <int CFG>
-constexpr int tile_smem() {
-  return Tile<CFG>::STAGES * (slab(Tile<CFG>::BM) + slab(Tile<CFG>::BN)) * (int)sizeof(double);
-}
+constexpr int kBM = 32, kBN = 32, kBK = 16, kStages = 4;  // output tile, depth and number of operand slabs
+constexpr int kWarpsM = 2, kWarpsN = 4, kThreads = 32 * kWarpsM * kWarpsN;
+// a slab in shared memory is padded to rows of 4 mod 16 doubles, so that a
+// warp's fragment loads (four consecutive rows by four consecutive columns
+// per half warp) hit distinct banks, whichever of its two indices is the row
+constexpr int kSlab = kBM * (kBK + 4) > kBK * (kBM + 4) ? kBM * (kBK + 4) : kBK * (kBM + 4);
+static_assert(kBM == kBN, "one slab size for both operands");
 
 __device__ __forceinline__ void dmma_884(double &d0, double &d1, double a, double b) {
   asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
@@ -71,9 +54,9 @@ __device__ __forceinline__ void cp_async_fill(double *dst, const double *src, in
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src), "r"(valid) : "memory");
 }
 
-// Copies one operand slab: rows of `len` contiguous elements.  The operand is
-// stored R x L row-major (ld); the slab takes R0.. (NR of them) by L0.. (NL),
-// to S with pitch NL + 4.  V elements per copy.
+// Copies one operand slab, V elements per copy: rows r0.. (NR) and columns
+// l0.. (NL) of the R x L row-major operand A (ld), to S with pitch NL + 4;
+// zero outside A.
 template <int NR, int NL, int V>
 __device__ __forceinline__ void load_slab(double *S, const double *__restrict__ A, int ld, int r0, int R, int l0,
                                           int L) {
@@ -98,61 +81,58 @@ __device__ __forceinline__ void load_slab(double *S, const double *__restrict__ 
     load_slab<NR, NL, 1>(S, A, ld, r0, R, l0, L);
 }
 
-// One BM x BN tile (rows m0.., columns n0..) of C = op(A) op(B), op(A) M x K,
+// One kBM x kBN tile (rows m0.., columns n0..) of C = op(A) op(B), op(A) M x K,
 // op(B) K x N.  TA: A stored K x M (element (m,k) at A[k*lda + m]); else
 // A[m*lda + k].  TB: B stored N x K; else K x N.  epi(row, column, value) for
-// every element of C in range.  Fragment layout of m8n8k4 .f64 (group
+// every element of C in range; sm: both operands' slabs.  Fragment layout of m8n8k4 .f64 (group
 // g = lane / 4, t = lane % 4): A holds (row g, col t), B (row t, col g), C/D
 // (row g, cols 2t, 2t+1).
-template <int CFG, bool TA, bool TB, class Epi>
+template <bool TA, bool TB, class Epi>
 __device__ __forceinline__ void gemm_tile(int M, int N, int K, const double *__restrict__ A, int lda,
-                                          const double *__restrict__ B, int ldb, int m0, int n0, Epi epi) {
-  constexpr int BM = Tile<CFG>::BM, BN = Tile<CFG>::BN, ST = Tile<CFG>::STAGES;
-  constexpr int SA = slab(BM), SB = slab(BN);
-  extern __shared__ __align__(16) double smem[];
-  double *As = smem, *Bs = smem + ST * SA;
+                                          const double *__restrict__ B, int ldb, int m0, int n0, double *sm, Epi epi) {
+  double *As = sm, *Bs = sm + kStages * kSlab;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, t = lane & 3;
-  constexpr int WM = BM / 2, WN = BN / 2, NI = WM / 8, NJ = WN / 8;
-  const int wm = (warp & 1) * WM, wn = (warp >> 1) * WN;
+  constexpr int WM = kBM / kWarpsM, WN = kBN / kWarpsN, NI = WM / 8, NJ = WN / 8;
+  const int wm = (warp % kWarpsM) * WM, wn = (warp / kWarpsM) * WN;
   // 16-byte copies where every row starts on a 16-byte boundary
   const bool va = (lda & 1) == 0 && ((uintptr_t)A & 15) == 0, vb = (ldb & 1) == 0 && ((uintptr_t)B & 15) == 0;
   const int nk = (K + kBK - 1) / kBK;
   auto load = [&](int kt) {
-    double *as = As + (kt % ST) * SA, *bs = Bs + (kt % ST) * SB;
+    double *as = As + (kt % kStages) * kSlab, *bs = Bs + (kt % kStages) * kSlab;
     if (TA)
-      load_slab<kBK, BM>(as, A, lda, kt * kBK, K, m0, M, va);
+      load_slab<kBK, kBM>(as, A, lda, kt * kBK, K, m0, M, va);
     else
-      load_slab<BM, kBK>(as, A, lda, m0, M, kt * kBK, K, va);
+      load_slab<kBM, kBK>(as, A, lda, m0, M, kt * kBK, K, va);
     if (TB)
-      load_slab<BN, kBK>(bs, B, ldb, n0, N, kt * kBK, K, vb);
+      load_slab<kBN, kBK>(bs, B, ldb, n0, N, kt * kBK, K, vb);
     else
-      load_slab<kBK, BN>(bs, B, ldb, kt * kBK, K, n0, N, vb);
+      load_slab<kBK, kBN>(bs, B, ldb, kt * kBK, K, n0, N, vb);
   };
   double acc[NI][NJ][2] = {};
 #pragma unroll
-  for (int q = 0; q < ST - 1; ++q) {
+  for (int q = 0; q < kStages - 1; ++q) {
     if (q < nk) load(q);
     asm volatile("cp.async.commit_group;\n" ::: "memory");
   }
   for (int kt = 0; kt < nk; ++kt) {
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(ST - 2) : "memory");
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(kStages - 2) : "memory");
     __syncthreads();  // slab kt complete for every thread; slab kt - 1 read by every thread
-    if (kt + ST - 1 < nk) load(kt + ST - 1);
+    if (kt + kStages - 1 < nk) load(kt + kStages - 1);
     asm volatile("cp.async.commit_group;\n" ::: "memory");
-    const double *as = As + (kt % ST) * SA, *bs = Bs + (kt % ST) * SB;
+    const double *as = As + (kt % kStages) * kSlab, *bs = Bs + (kt % kStages) * kSlab;
 #pragma unroll
     for (int kk = 0; kk < kBK; kk += 4) {
       double a[NI], b[NJ];
 #pragma unroll
       for (int i = 0; i < NI; ++i) {
         const int m = wm + 8 * i + g;
-        a[i] = TA ? as[(kk + t) * (BM + 4) + m] : as[m * (kBK + 4) + kk + t];
+        a[i] = TA ? as[(kk + t) * (kBM + 4) + m] : as[m * (kBK + 4) + kk + t];
       }
 #pragma unroll
       for (int j = 0; j < NJ; ++j) {
         const int n = wn + 8 * j + g;
-        b[j] = TB ? bs[n * (kBK + 4) + kk + t] : bs[(kk + t) * (BN + 4) + n];
+        b[j] = TB ? bs[n * (kBK + 4) + kk + t] : bs[(kk + t) * (kBN + 4) + n];
       }
 #pragma unroll
       for (int i = 0; i < NI; ++i)
@@ -173,42 +153,41 @@ __device__ __forceinline__ void gemm_tile(int M, int N, int K, const double *__r
 }
 
 // w = Q' r: rows = modes, columns = the unknowns of the systems
-template <int CFG>
-__device__ __forceinline__ void fdm_forward(const FdmD &F, const double *__restrict__ r, int m0, int n0) {
+__device__ __forceinline__ void fdm_forward(const FdmD &F, const double *__restrict__ r, int m0, int n0, double *sm) {
   const int nm = F.nm, n = F.n;
   auto store = [&](int b, int i, double v) { F.t[(size_t)b * n + i] = v; };
   if (F.xmodes)  // r is n x nm (rows j = unknowns)
-    gemm_tile<CFG, true, true>(nm, n, nm, F.Q, nm, r, nm, m0, n0, store);
+    gemm_tile<true, true>(nm, n, nm, F.Q, nm, r, nm, m0, n0, sm, store);
   else  // r is nm x n
-    gemm_tile<CFG, true, false>(nm, n, nm, F.Q, nm, r, n, m0, n0, store);
+    gemm_tile<true, false>(nm, n, nm, F.Q, nm, r, n, m0, n0, sm, store);
 }
 // z = Q zh, element (j, i) handed to epi(index, value)
-template <int CFG, class Epi>
-__device__ __forceinline__ void fdm_backward(const FdmD &F, int m0, int n0, Epi epi) {
+template <class Epi>
+__device__ __forceinline__ void fdm_backward(const FdmD &F, int m0, int n0, double *sm, Epi epi) {
   const int nm = F.nm, n = F.n, nx = F.nx;
   auto out = [&](int j, int i, double v) { epi((size_t)j * nx + i, v); };
   if (F.xmodes)
-    gemm_tile<CFG, true, true>(n, nm, nm, F.t, n, F.Q, nm, m0, n0, out);
+    gemm_tile<true, true>(n, nm, nm, F.t, n, F.Q, nm, m0, n0, sm, out);
   else
-    gemm_tile<CFG, false, false>(nm, n, nm, F.Q, nm, F.t, n, m0, n0, out);
+    gemm_tile<false, false>(nm, n, nm, F.Q, nm, F.t, n, m0, n0, sm, out);
 }
 
-template <int CFG>
 __global__ void __launch_bounds__(kThreads) k_fdm_fwd(const __grid_constant__ FdmD F, const PcgWork W,
                                                       const double *__restrict__ f) {
+  __shared__ __align__(16) double sm[2 * kStages * kSlab];
   if (*(volatile const int *)&W.sc->done) return;
-  fdm_forward<CFG>(F, W.sc->it == 0 ? f : W.r, blockIdx.y * Tile<CFG>::BM, blockIdx.x * Tile<CFG>::BN);
+  fdm_forward(F, W.sc->it == 0 ? f : W.r, blockIdx.y * kBM, blockIdx.x * kBN, sm);
 }
 
 // z = Q zh with r'z reduced in the same pass (deterministic, reduce.cuh)
-template <int CFG>
 __global__ void __launch_bounds__(kThreads) k_fdm_bwd(const __grid_constant__ FdmD F, const PcgWork W,
                                                       const double *__restrict__ f) {
+  __shared__ __align__(16) double sm[2 * kStages * kSlab];
   if (*(volatile int *)&W.sc->done) return;
   const double *__restrict__ r = W.sc->it == 0 ? f : W.r;
   double q[1] = {0.0};
   const int ops[1] = {R_SUM};
-  fdm_backward<CFG>(F, blockIdx.y * Tile<CFG>::BM, blockIdx.x * Tile<CFG>::BN, [&](size_t k, double v) {
+  fdm_backward(F, blockIdx.y * kBM, blockIdx.x * kBN, sm, [&](size_t k, double v) {
     F.z[k] = v;
     q[0] += __ldg(r + k) * v;
   });
@@ -230,23 +209,23 @@ __global__ void __launch_bounds__(128) k_fdm_tri(const __grid_constant__ FdmD F,
 }
 
 // the same for the members of an ensemble that still iterate
-template <int CFG>
 __global__ void __launch_bounds__(kThreads) k_fdm_fwd_ens(const FdmD *__restrict__ Fs, const int4 *__restrict__ tiles,
                                                           const EnsCg *__restrict__ cg) {
+  __shared__ __align__(16) double sm[2 * kStages * kSlab];
   const int4 t = tiles[blockIdx.x];
   if (*(volatile const int *)&cg[t.x].done) return;
   const FdmD &F = Fs[t.x];
-  const int m0 = t.y * Tile<CFG>::BM, n0 = t.z * Tile<CFG>::BN;
-  if (m0 < F.nm && n0 < F.n) fdm_forward<CFG>(F, F.r, m0, n0);
+  const int m0 = t.y * kBM, n0 = t.z * kBN;
+  if (m0 < F.nm && n0 < F.n) fdm_forward(F, F.r, m0, n0, sm);
 }
-template <int CFG>
 __global__ void __launch_bounds__(kThreads) k_fdm_bwd_ens(const FdmD *__restrict__ Fs, const int4 *__restrict__ tiles,
                                                           const EnsCg *__restrict__ cg) {
+  __shared__ __align__(16) double sm[2 * kStages * kSlab];
   const int4 t = tiles[blockIdx.x];
   if (*(volatile const int *)&cg[t.x].done) return;
   const FdmD &F = Fs[t.x];
-  const int m0 = t.y * Tile<CFG>::BM, n0 = t.z * Tile<CFG>::BN;
-  if (m0 < F.ny && n0 < F.nx) fdm_backward<CFG>(F, m0, n0, [&](size_t k, double v) { F.z[k] = v; });
+  const int m0 = t.y * kBM, n0 = t.z * kBN;
+  if (m0 < F.ny && n0 < F.nx) fdm_backward(F, m0, n0, sm, [&](size_t k, double v) { F.z[k] = v; });
 }
 template <int W>
 __global__ void __launch_bounds__(128) k_fdm_tri_ens(const FdmD *__restrict__ Fs, const int2 *__restrict__ rows,
@@ -258,27 +237,9 @@ __global__ void __launch_bounds__(128) k_fdm_tri_ens(const FdmD *__restrict__ Fs
   tri_row<W>(Fs[t.x], t.y + warp / W, warp % W, sh);
 }
 
-// Tile shape: the one with the least work on the busiest SM, tiles of one
-// launch spread evenly; the larger one on a tie (it reads its operands fewer
-// times).
-int tile_config(long long t64, long long t6432, long long t32, int nsm) {
-  const long long w0 = ((t64 + nsm - 1) / nsm) * 4, w1 = ((t6432 + nsm - 1) / nsm) * 2, w2 = (t32 + nsm - 1) / nsm;
-  return w0 <= w1 && w0 <= w2 ? 0 : (w1 <= w2 ? 1 : 2);
-}
-long long tiles_of(long long M, long long N, int bm, int bn) { return ((M + bm - 1) / bm) * ((N + bn - 1) / bn); }
 int row_warps(int n) { return n <= 32 * kTriChunk ? 1 : (n <= 64 * kTriChunk ? 2 : 4); }
 static_assert(4 * 32 * kTriChunk >= 1024, "four warps hold the longest row (kFdmMaxN)");
 
-template <int CFG>
-void launch_fwd(const FdmD &F, const PcgWork &W, const double *f, cudaStream_t s) {
-  const dim3 g((F.n + Tile<CFG>::BN - 1) / Tile<CFG>::BN, (F.nm + Tile<CFG>::BM - 1) / Tile<CFG>::BM);
-  k_fdm_fwd<CFG><<<g, kThreads, tile_smem<CFG>(), s>>>(F, W, f);
-}
-template <int CFG>
-void launch_bwd(const FdmD &F, const PcgWork &W, const double *f, cudaStream_t s) {
-  const dim3 g((F.nx + Tile<CFG>::BN - 1) / Tile<CFG>::BN, (F.ny + Tile<CFG>::BM - 1) / Tile<CFG>::BM);
-  k_fdm_bwd<CFG><<<g, kThreads, tile_smem<CFG>(), s>>>(F, W, f);
-}
 template <int W>
 void launch_tri(const FdmD &F, const int *done, cudaStream_t s) {
   k_fdm_tri<W><<<(F.nm + 4 / W - 1) / (4 / W), 128, 0, s>>>(F, done);
@@ -286,35 +247,9 @@ void launch_tri(const FdmD &F, const int *done, cudaStream_t s) {
 
 }  // namespace
 
-cudaError_t fdm_prepare() {
-  cudaError_t first = cudaSuccess;
-  auto opt_in = [&](const void *k, int bytes) {
-    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (first == cudaSuccess) first = e;
-  };
-#define INS2D_FDM_OPT_IN(C)                                   \
-  opt_in((const void *)k_fdm_fwd<C>, tile_smem<C>());         \
-  opt_in((const void *)k_fdm_bwd<C>, tile_smem<C>());         \
-  opt_in((const void *)k_fdm_fwd_ens<C>, tile_smem<C>());     \
-  opt_in((const void *)k_fdm_bwd_ens<C>, tile_smem<C>());
-  INS2D_FDM_OPT_IN(0)
-  INS2D_FDM_OPT_IN(1)
-  INS2D_FDM_OPT_IN(2)
-#undef INS2D_FDM_OPT_IN
-  return first;
-}
-
 void fdm_apply(const FdmD &F, const PcgWork &W, const double *f, cudaStream_t s) {
   const int *done = &W.sc->done;
-  const int cfg = tile_config(tiles_of(F.ny, F.nx, 64, 64),
-                              std::min(tiles_of(F.ny, F.nx, 64, 32), tiles_of(F.nx, F.ny, 64, 32)),
-                              tiles_of(F.ny, F.nx, 32, 32), F.nsm);
-  if (cfg == 0)
-    launch_fwd<0>(F, W, f, s);
-  else if (cfg == 1)
-    launch_fwd<1>(F, W, f, s);
-  else
-    launch_fwd<2>(F, W, f, s);
+  k_fdm_fwd<<<dim3((F.n + kBN - 1) / kBN, (F.nm + kBM - 1) / kBM), kThreads, 0, s>>>(F, W, f);
   const int w = row_warps(F.n);
   if (w == 1)
     launch_tri<1>(F, done, s);
@@ -322,33 +257,20 @@ void fdm_apply(const FdmD &F, const PcgWork &W, const double *f, cudaStream_t s)
     launch_tri<2>(F, done, s);
   else
     launch_tri<4>(F, done, s);
-  if (cfg == 0)
-    launch_bwd<0>(F, W, f, s);
-  else if (cfg == 1)
-    launch_bwd<1>(F, W, f, s);
-  else
-    launch_bwd<2>(F, W, f, s);
+  k_fdm_bwd<<<dim3((F.nx + kBN - 1) / kBN, (F.ny + kBM - 1) / kBM), kThreads, 0, s>>>(F, W, f);
 }
 
-void fdm_ens_lists(const std::vector<FdmD> &F, const std::vector<int> &order, int nsm, EnsFdmPlan &pl,
-                   std::vector<int4> &tiles, std::vector<int2> &rows) {
-  long long t0 = 0, t1 = 0, t2 = 0;
+void fdm_ens_lists(const std::vector<FdmD> &F, const std::vector<int> &order, EnsFdmPlan &pl, std::vector<int4> &tiles,
+                   std::vector<int2> &rows) {
   int nmax = 0;
-  for (const FdmD &f : F) {
-    t0 += tiles_of(f.nm, f.n, 64, 64);
-    t1 += tiles_of(f.nm, f.n, 64, 32);
-    t2 += tiles_of(f.nm, f.n, 32, 32);
-    nmax = std::max(nmax, f.n);
-  }
-  pl.cfg = tile_config(t0, t1, t2, nsm);
+  for (const FdmD &f : F) nmax = std::max(nmax, f.n);
   pl.warps = row_warps(nmax);
-  const int bm = pl.cfg == 2 ? 32 : 64, bn = pl.cfg == 0 ? 64 : 32;
   // one list for both products: the forward one's nm x n and the backward
   // one's ny x nx tiles (a tile outside a product's range returns)
   for (int m : order) {
     const int M = std::max(F[m].nm, F[m].ny), N = std::max(F[m].n, F[m].nx);
-    for (int bi = 0; bi < (M + bm - 1) / bm; ++bi)
-      for (int bj = 0; bj < (N + bn - 1) / bn; ++bj) tiles.push_back(make_int4(m, bi, bj, 0));
+    for (int bi = 0; bi < (M + kBM - 1) / kBM; ++bi)
+      for (int bj = 0; bj < (N + kBN - 1) / kBN; ++bj) tiles.push_back(make_int4(m, bi, bj, 0));
     for (int b = 0; b < F[m].nm; b += 4 / pl.warps) rows.push_back(make_int2(m, b));
   }
   pl.ntiles = (int)tiles.size();
@@ -357,24 +279,14 @@ void fdm_ens_lists(const std::vector<FdmD> &F, const std::vector<int> &order, in
 
 void fdm_apply_ens(const EnsFdmPlan &pl, const EnsCg *cg, cudaStream_t s) {
   if (pl.ntiles <= 0) return;
-  if (pl.cfg == 0)
-    k_fdm_fwd_ens<0><<<pl.ntiles, kThreads, tile_smem<0>(), s>>>(pl.F, pl.tiles, cg);
-  else if (pl.cfg == 1)
-    k_fdm_fwd_ens<1><<<pl.ntiles, kThreads, tile_smem<1>(), s>>>(pl.F, pl.tiles, cg);
-  else
-    k_fdm_fwd_ens<2><<<pl.ntiles, kThreads, tile_smem<2>(), s>>>(pl.F, pl.tiles, cg);
+  k_fdm_fwd_ens<<<pl.ntiles, kThreads, 0, s>>>(pl.F, pl.tiles, cg);
   if (pl.warps == 1)
     k_fdm_tri_ens<1><<<pl.nrows, 128, 0, s>>>(pl.F, pl.rows, cg);
   else if (pl.warps == 2)
     k_fdm_tri_ens<2><<<pl.nrows, 128, 0, s>>>(pl.F, pl.rows, cg);
   else
     k_fdm_tri_ens<4><<<pl.nrows, 128, 0, s>>>(pl.F, pl.rows, cg);
-  if (pl.cfg == 0)
-    k_fdm_bwd_ens<0><<<pl.ntiles, kThreads, tile_smem<0>(), s>>>(pl.F, pl.tiles, cg);
-  else if (pl.cfg == 1)
-    k_fdm_bwd_ens<1><<<pl.ntiles, kThreads, tile_smem<1>(), s>>>(pl.F, pl.tiles, cg);
-  else
-    k_fdm_bwd_ens<2><<<pl.ntiles, kThreads, tile_smem<2>(), s>>>(pl.F, pl.tiles, cg);
+  k_fdm_bwd_ens<<<pl.ntiles, kThreads, 0, s>>>(pl.F, pl.tiles, cg);
 }
 
 }  // namespace ins2d

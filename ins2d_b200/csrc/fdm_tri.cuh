@@ -4,9 +4,9 @@
 // solved in place on the rows of the nm x n array w.  With the reciprocal
 // pivots tabulated, elimination and back substitution are first-order linear
 // recurrences y_k = a_k y_{k-1} + b_k with |a_k| < 1; W warps share a row,
-// each lane holds kTriChunk consecutive unknowns, composes their affine maps,
+// each lane holds C consecutive unknowns, composes their affine maps,
 // and the maps' prefix is scanned over the lanes (and the warps).  So a row
-// takes two serial chains of kTriChunk steps and five shuffle rounds each
+// takes two serial chains of C steps and five shuffle rounds each
 // instead of two chains of n steps.
 #pragma once
 
@@ -22,29 +22,40 @@ __device__ __forceinline__ double tri_warp_sum(double v) {
   return v;
 }
 
-// Row b (systems b of F; b >= F.nm: no row, the threads only take part in the
-// barriers) by W warps of a block of 4; wr: this warp's place in the row.
-// sh: 4 x 4 doubles per block, unused (may be null) for W == 1, which has no
-// block-level synchronisation.
-template <int W>
-__device__ __forceinline__ void tri_row(const FdmD &F, int b, int wr, double (*sh)[4]) {
-  constexpr int C = kTriChunk;
+// one lane's part of a system's tables: C unknowns from s0 (zero outside)
+template <int C>
+struct TriTab {
+  double m[C], e[C], ep;  // reciprocal pivots, off-diagonals, the one before s0
+};
+template <int C>
+__device__ __forceinline__ void tri_tables(const FdmD &F, int b, int s0, TriTab<C> &T) {
+  const bool row = b < F.nm;
+  const double *__restrict__ pv = F.piv + (size_t)(row ? b : 0) * F.n;
+  T.ep = (row && s0 > 0 && s0 <= F.n) ? __ldg(F.e + s0 - 1) : 0.0;
+#pragma unroll
+  for (int k = 0; k < C; ++k) {
+    const bool in = row && s0 + k < F.n;
+    T.m[k] = in ? __ldg(pv + s0 + k) : 0.0;
+    T.e[k] = in ? __ldg(F.e + s0 + k) : 0.0;
+  }
+}
+
+// Solves system b (b >= F.nm: none, the threads only take part in the
+// barriers) by W warps; wr: this warp's place among them.  y: the lane's C
+// values of w_b from unknown s0 = (32 wr + lane) C (zero outside), replaced by
+// those of zh_b.  sh: 4 doubles per warp of the block, unused (may be null)
+// for W == 1, which has no block-level synchronisation.
+template <int W, int C>
+__device__ __forceinline__ void tri_solve(const FdmD &F, int b, int wr, const TriTab<C> &T, double (&y)[C],
+                                          double (*sh)[4]) {
   constexpr unsigned ALL = 0xffffffffu;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, w0 = warp - wr;  // w0: the row's first warp
   const int n = F.n, s0 = (wr * 32 + lane) * C;
   const bool row = b < F.nm;
-  double *__restrict__ w = F.t + (size_t)(row ? b : 0) * n;
-  const double *__restrict__ pv = F.piv + (size_t)(row ? b : 0) * n;
   const bool null = row && b == F.null_mode;
-  double y[C], m[C], e[C];
-  const double ep = (row && s0 > 0 && s0 <= n) ? __ldg(F.e + s0 - 1) : 0.0;
-#pragma unroll
-  for (int k = 0; k < C; ++k) {
-    const bool in = row && s0 + k < n;
-    y[k] = in ? w[s0 + k] : 0.0;
-    m[k] = in ? __ldg(pv + s0 + k) : 0.0;
-    e[k] = in ? __ldg(F.e + s0 + k) : 0.0;
-  }
+  const double ep = T.ep;
+  const double(&m)[C] = T.m;
+  const double(&e)[C] = T.e;
   // the null mode: a right-hand side without its component along diag(h) 1
   double sum = 0.0;
   if (null) {
@@ -179,6 +190,21 @@ __device__ __forceinline__ void tri_row(const FdmD &F, int b, int wr, double (*s
 #pragma unroll
     for (int k = 0; k < C; ++k) y[k] -= c;
   }
+}
+
+// Row b of the nm x n array F.t in place, by W warps of a block of 4
+template <int W>
+__device__ __forceinline__ void tri_row(const FdmD &F, int b, int wr, double (*sh)[4]) {
+  constexpr int C = kTriChunk;
+  const int n = F.n, s0 = (wr * 32 + (threadIdx.x & 31)) * C;
+  const bool row = b < F.nm;
+  double *__restrict__ w = F.t + (size_t)(row ? b : 0) * n;
+  TriTab<C> T;
+  double y[C];
+#pragma unroll
+  for (int k = 0; k < C; ++k) y[k] = (row && s0 + k < n) ? w[s0 + k] : 0.0;
+  tri_tables<C>(F, b, s0, T);
+  tri_solve<W, C>(F, b, wr, T, y, sh);
 #pragma unroll
   for (int k = 0; k < C; ++k)
     if (row && s0 + k < n) w[s0 + k] = y[k];

@@ -11,7 +11,7 @@
 namespace ins2d {
 
 constexpr int kMaxStages = 8;
-constexpr int kStatusNonFinite = 4;  // INS2D_ENONFINITE
+constexpr int kStatusNonFinite = 4, kStatusTimeout = 5;  // INS2D_ENONFINITE, INS2D_ETIMEOUT
 
 // Programmatic dependent launch of the explicit step's kernels (the stage and
 // residual walkers, the FFT passes, the projections): off unless INS2D_PDL=1
@@ -216,7 +216,6 @@ cudaError_t fft_prepare();
 // FdmTri) and the work arrays of one application.
 struct FdmD {
   int nx = 0, ny = 0;
-  int nsm = 148;                  // multiprocessors (tile shape of the products)
   int nm = 0, n = 0, xmodes = 0;  // modes, unknowns per system, modes along x
   const double *Q = nullptr;      // nm x nm row-major (Q[i*nm + b])
   const double *piv = nullptr, *e = nullptr, *h = nullptr;  // nm x n, n, n
@@ -232,8 +231,6 @@ struct FdmD {
   const unsigned long long *gate = nullptr;  // device word holding 1.0 (no early return)
 };
 struct PcgWork;
-// opts the product kernels in to their dynamic shared memory on the current device
-cudaError_t fdm_prepare();
 // z = A^+ r (product, tridiagonal systems, product) and the PCG's r'z, beta;
 // r = f on the first pass, W.r later.  No work once W.sc->done is set.
 void fdm_apply(const FdmD &F, const PcgWork &W, const double *f, cudaStream_t s);
@@ -245,11 +242,10 @@ struct EnsFdmPlan {
   const FdmD *F = nullptr;
   const int4 *tiles = nullptr;
   const int2 *rows = nullptr;
-  int ntiles = 0, nrows = 0, cfg = 0, warps = 1;
+  int ntiles = 0, nrows = 0, warps = 1;
 };
-// Host: the tile shape for the members' sizes, and the lists
-void fdm_ens_lists(const std::vector<FdmD> &F, const std::vector<int> &order, int nsm, EnsFdmPlan &pl,
-                   std::vector<int4> &tiles, std::vector<int2> &rows);
+void fdm_ens_lists(const std::vector<FdmD> &F, const std::vector<int> &order, EnsFdmPlan &pl, std::vector<int4> &tiles,
+                   std::vector<int2> &rows);
 // z = A^+ r for every member not yet converged (cg[m].done == 0)
 void fdm_apply_ens(const EnsFdmPlan &pl, const EnsCg *cg, cudaStream_t s);
 
@@ -313,11 +309,39 @@ __device__ __forceinline__ void pcg_new_rz(PcgScalars *s, double rz) {
     s->rz = rz;
   }
 }
-// small grids (at most 128 cells per direction, not the spectral form): the
-// whole fast-diagonalization PCG solve in one thread block
-bool pcg_use_block_fdm(const FdmD &F);
-void pcg_solve_block_fdm(const DevOps &P, const FdmD &F, const PcgWork &W, const double *f, double *dp, double tol,
-                         long long maxit, bool accumulate, cudaStream_t s);
+// a finished solve's statistics added to *a (one thread; a loop that stopped at
+// its pass limit before convergence counts as INS2D_ETIMEOUT)
+__device__ __forceinline__ void solve_accum(const PcgScalars *sc, SolveAccum *a) {
+  const long long it = sc->it;
+  a->n_solves += 1;
+  a->iters_total += it;
+  if (it > a->iters_max) a->iters_max = it;
+  const double n1 = sqrt(sc->rr);
+  if (n1 > a->norm1_max) a->norm1_max = n1;
+  const int st = sc->done ? sc->status : kStatusTimeout;
+  if (st != 0 && a->status == 0) {
+    a->status = st;
+    a->fail_rr = sc->rr;
+    a->fail_maxit = sc->maxit;
+  }
+}
+// Small grids (at most kFdmClusterMaxN cells per direction, not the spectral
+// form): the whole fast-diagonalization PCG solve in one thread-block cluster
+// (pcg_cluster.cu); dp written or accumulated when converged, status and
+// iterations in W.sc, statistics added to *acc (may be null)
+constexpr int kFdmClusterMaxN = 128;
+// right-hand side of a solve: mode 0: f; 1: (M f + alpha yM + beta ydM) gamma
+// of the velocity-sized f; 2: the same of ws
+struct SolveSrc {
+  int mode = 0;
+  const double *f = nullptr;
+  WSplit ws{};
+  double alpha = 0.0, beta = 0.0, gamma = 0.0;
+};
+bool pcg_use_cluster(const FdmD &F);
+cudaError_t pcg_cluster_prepare();  // opts the kernels in to their shared memory on the current device
+void pcg_solve_cluster(const DevOps &P, const FdmD &F, const PcgWork &W, const SolveSrc &src, double *dp, double tol,
+                       long long maxit, bool accumulate, SolveAccum *acc, cudaStream_t s);
 
 struct EnsMemberD {
   DevOps P;

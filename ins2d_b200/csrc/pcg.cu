@@ -24,7 +24,6 @@
 #include "ins2d.h"
 #include "kernels.cuh"
 #include "mg.cuh"
-#include "fdm_block.cuh"
 #include "reduce.cuh"
 
 namespace ins2d {
@@ -181,11 +180,10 @@ __device__ void block_reduce(double (&v)[NQ], const int (&ops)[NQ], double (*sh)
 }
 
 // The whole solve by one thread block.  PK 0: Jacobi preconditioner
-// (z = r / diag A); 1: one multigrid V-cycle per application (mg.cuh);
-// 2: fast diagonalization (fdm_block.cuh).  Results go to out (the
-// PcgScalars of this solve).
+// (z = r / diag A); 1: one multigrid V-cycle per application (mg.cuh).
+// Results go to out (the PcgScalars of this solve).
 template <int PK>
-__device__ void pcg_block_body(const DevOps &P, const MgD *M, const FdmD *F, const PcgWork &W,
+__device__ void pcg_block_body(const DevOps &P, const MgD *M, const PcgWork &W,
                                const double *__restrict__ f, double *__restrict__ dp, double tol2, long long maxit,
                                int accumulate, PcgScalars *out, double (*sh)[5], double *ysh) {
   constexpr bool MG = PK != 0;  // a preconditioner with its own z buffer
@@ -193,13 +191,9 @@ __device__ void pcg_block_body(const DevOps &P, const MgD *M, const FdmD *F, con
   const long long Np = P.Np;
   const int tid = threadIdx.x, nt = blockDim.x;
   double *__restrict__ x = W.x, *__restrict__ r = W.r, *__restrict__ p = W.p, *__restrict__ q = W.q;
-  double *zw = PK == 1 ? mg_result(*M, 0) : (PK == 2 ? F->z : nullptr);
-  const double *z = zw;
+  const double *z = PK == 1 ? mg_result(*M, 0) : nullptr;
   auto precond = [&]() {
-    if constexpr (PK == 1)
-      mg_vcycle_block(*M, r, 0, ysh);
-    else if constexpr (PK == 2)
-      fdm_apply_block(*F, r, zw);
+    if constexpr (PK == 1) mg_vcycle_block(*M, r, 0, ysh);
   };
   // init (cg.F:207-229 with x_in = 0)
   double a3[3] = {0.0, 0.0, 0.0};
@@ -340,7 +334,7 @@ __global__ void __launch_bounds__(kBlockThreads, 1) k_pcg_block(const __grid_con
                                                                const double *__restrict__ f, double *__restrict__ dp,
                                                                double tol2, long long maxit, int accumulate) {
   __shared__ double sh[kBlockThreads / 32][5];
-  pcg_block_body<0>(P, nullptr, nullptr, W, f, dp, tol2, maxit, accumulate, W.sc, sh, nullptr);
+  pcg_block_body<0>(P, nullptr, W, f, dp, tol2, maxit, accumulate, W.sc, sh, nullptr);
 }
 
 // multigrid variant: 512 threads (the chunked line solves need ~128 registers)
@@ -355,18 +349,7 @@ __global__ void __launch_bounds__(kBlockThreadsMg, 1) k_pcg_block_mg(const __gri
                                                                   long long maxit, int accumulate) {
   __shared__ double sh[kBlockThreads / 32][5];
   __shared__ double ysh[2 * kBlockThreadsMg];
-  pcg_block_body<1>(P, &M, nullptr, W, f, dp, tol2, maxit, accumulate, W.sc, sh, ysh);
-}
-
-// fast-diagonalization variant for grids up to kFdmBlockMaxN cells per direction
-constexpr int kBlockThreadsFdm = 512;
-__global__ void __launch_bounds__(kBlockThreadsFdm, 1) k_pcg_block_fdm(const __grid_constant__ DevOps P,
-                                                                    const __grid_constant__ FdmD F, const PcgWork W,
-                                                                    const double *__restrict__ f,
-                                                                    double *__restrict__ dp, double tol2,
-                                                                    long long maxit, int accumulate) {
-  __shared__ double sh[kBlockThreads / 32][5];
-  pcg_block_body<2>(P, nullptr, &F, W, f, dp, tol2, maxit, accumulate, W.sc, sh, nullptr);
+  pcg_block_body<1>(P, &M, W, f, dp, tol2, maxit, accumulate, W.sc, sh, ysh);
 }
 
 // Grid-stride CG kernels of the multigrid path for large grids: the SpMV uses
@@ -687,21 +670,6 @@ __global__ void __launch_bounds__(kVecThreads) k_update_f(const PcgWork W, const
   }
 }
 
-__device__ __forceinline__ void solve_accum(const PcgScalars *sc, SolveAccum *a) {
-  const long long it = sc->it;
-  a->n_solves += 1;
-  a->iters_total += it;
-  if (it > a->iters_max) a->iters_max = it;
-  const double n1 = sqrt(sc->rr);
-  if (n1 > a->norm1_max) a->norm1_max = n1;
-  const int st = sc->done ? sc->status : INS2D_ETIMEOUT;
-  if (st != 0 && a->status == 0) {
-    a->status = st;
-    a->fail_rr = sc->rr;
-    a->fail_maxit = sc->maxit;
-  }
-}
-
 // dp = x or dp += x (x = 0 when no pass ran); acc (may be null): the solve's
 // statistics
 __global__ void __launch_bounds__(kVecThreads) k_finish_f(const PcgWork W, double *__restrict__ dp, long long n,
@@ -743,9 +711,9 @@ __global__ void __launch_bounds__(kBlockThreadsMg, 1) k_pcg_members(const EnsMem
     __syncthreads();
     double *dst = which ? E.p : E.dp;
     if (mg)
-      pcg_block_body<1>(sP, &sM, nullptr, E.W, E.f, dst, tol2, maxit, which, E.W.sc, sh, ysh);
+      pcg_block_body<1>(sP, &sM, E.W, E.f, dst, tol2, maxit, which, E.W.sc, sh, ysh);
     else
-      pcg_block_body<0>(sP, nullptr, nullptr, E.W, E.f, dst, tol2, maxit, which, E.W.sc, sh, ysh);
+      pcg_block_body<0>(sP, nullptr, E.W, E.f, dst, tol2, maxit, which, E.W.sc, sh, ysh);
     __syncthreads();
     if (tid == 0) {
       const PcgScalars &o = *E.W.sc;
@@ -793,13 +761,6 @@ extern "C" int ins2d_debug_mg_clocks(unsigned long long out[128], int reset) {
 void pcg_solve_block_mg(const DevOps &P, const MgD &M, const PcgWork &W, const double *f, double *dp, double tol,
                         long long maxit, bool accumulate, cudaStream_t s) {
   k_pcg_block_mg<<<1, kBlockThreadsMg, 0, s>>>(P, M, W, f, dp, tol * tol, maxit, accumulate ? 1 : 0);
-}
-
-bool pcg_use_block_fdm(const FdmD &F) { return !F.spectral && F.nx <= kFdmBlockMaxN && F.ny <= kFdmBlockMaxN; }
-
-void pcg_solve_block_fdm(const DevOps &P, const FdmD &F, const PcgWork &W, const double *f, double *dp, double tol,
-                         long long maxit, bool accumulate, cudaStream_t s) {
-  k_pcg_block_fdm<<<1, kBlockThreadsFdm, 0, s>>>(P, F, W, f, dp, tol * tol, maxit, accumulate ? 1 : 0);
 }
 
 int pcg_blocks(const DevOps &P) {

@@ -30,3 +30,31 @@ def test_walker_runs(shape, bc):
     mr_ref, F_ref = R.F(V, V, p, 0.0, o)
     assert _rel(F, F_ref) < 1e-12 and abs(mr - mr_ref) < 1e-12 * mr_ref
     m.close()
+
+
+# one-cluster solves: slices of 1 .. 16 columns, empty blocks, both mode
+# directions, cyclic systems, the basis in shared memory (up to about 112
+# modes) and read through L1; 129: the multi-launch path.  The bound is the
+# stopping rule's, 1e-12 relative, with a factor 2 for the residual's rounding.
+@pytest.mark.parametrize("combo", ["cavity", "channel", "per_x_walls", "per_y_open", "periodic"])
+@pytest.mark.parametrize("shape", [(4, 3), (9, 16), (16, 9), (64, 64), (65, 40), (112, 112), (113, 120), (128, 128),
+                                   (128, 7), (7, 128), (129, 128)])
+def test_small_grid_solve(shape, combo):
+    bc = BC_COMBOS[combo]
+    x, y = grid_stretched(shape[0], 0.0, 1.7), grid_stretched(shape[1], -0.5, 0.5, beta=1.2)
+    m = api.Options(x, y, bc, poisson=4, CG_acc=1e-12, CG_maxit=50, precond="fdm")
+    o = R.make_options(x, y, bc, poisson=1)
+    M, A = o.discretization.M, o.discretization.A
+    f = M @ np.random.default_rng(5).standard_normal(o.grid.NV)
+    dp, st = m.pressure_poisson(f, return_stats=True)
+    assert np.linalg.norm(A @ dp - f) <= 2e-12 * np.linalg.norm(f) and st["iters"] <= 4
+    assert np.all(m.pressure_poisson(np.zeros(m.Np)) == 0.0)
+    # the divergence formed inside the solve: one host-driven step and the
+    # same step in a captured run against the oracle's
+    V = R.initial_projection(0.3 * np.random.default_rng(6).standard_normal(o.grid.NV), 0.0, o)
+    ref, pref = R.time_ERK(V, np.zeros(m.Np), 0.0, 1e-3, o)
+    V1, p1 = m.time_ERK(V, np.zeros(m.Np), 0.0, 1e-3)
+    assert _rel(V1, ref) < 1e-10
+    ref, pref = R.time_ERK(ref, pref, 1e-3, 1e-3, o)
+    assert _rel(m.time_ERK(V, np.zeros(m.Np), 0.0, 1e-3, nsteps=2)[0], ref) < 1e-10
+    m.close()
