@@ -623,7 +623,7 @@ int solve(ins2d_ctx *c, const double *f, double *dp, bool accumulate, ins2d_solv
 // needs f); otherwise by its own kernel before the solve.
 int solve_div(ins2d_ctx *c, const double *W, double alpha, double beta, double gamma, double *dp, bool accumulate,
               ins2d_solve_stats *st) {
-  if (c->poisson == INS2D_POISSON_FFT && fft_fuses_div(c->fft)) {
+  if (c->poisson == INS2D_POISSON_FFT) {
     if (st) *st = ins2d_solve_stats{0, 0.0, 0.0};
     Prof pr(c, INS2D_PROF_POISSON, fft_kernels(c->fft));
     CK(launch_fft_poisson_div(c->P, c->fft, W, alpha, beta, gamma, dp, accumulate, c->stream));
@@ -650,7 +650,7 @@ int solve_div(ins2d_ctx *c, const double *W, double alpha, double beta, double g
 // the same with W = Vn sv + sa T, T in FP32 (FP32-storage stages)
 int solve_div_split(ins2d_ctx *c, const double *Vn, const float *T, double sv, double sa, double alpha, double beta,
                     double gamma, double *dp, bool accumulate, ins2d_solve_stats *st) {
-  if (c->poisson == INS2D_POISSON_FFT && fft_fuses_div(c->fft)) {
+  if (c->poisson == INS2D_POISSON_FFT) {
     if (st) *st = ins2d_solve_stats{0, 0.0, 0.0};
     Prof pr(c, INS2D_PROF_POISSON, fft_kernels(c->fft));
     CK(launch_fft_poisson_div_split(c->P, c->fft, Vn, T, sv, sa, alpha, beta, gamma, dp, accumulate, c->stream));
@@ -1065,8 +1065,8 @@ int ins2d_ctx_create(const ins2d_grid_desc *grid, const ins2d_bc_desc *bc, const
       F.logx = is_pow2(H.Nx) ? (int)std::lround(std::log2((double)H.Nx)) : -1;
       F.logy = is_pow2(H.Ny) ? (int)std::lround(std::log2((double)H.Ny)) : -1;
       const std::vector<double> tx = fft_twiddle_table(H.Nx), ty = fft_twiddle_table(H.Ny);
-      F.twx = dalloc<double2>(c, 2 * (size_t)H.Nx);
-      F.twy = dalloc<double2>(c, 2 * (size_t)H.Ny);
+      F.twx = dalloc<double2>(c, tx.size() / 2);
+      F.twy = dalloc<double2>(c, ty.size() / 2);
       CK(cudaMemcpy(F.twx, tx.data(), tx.size() * sizeof(double), cudaMemcpyHostToDevice));
       CK(cudaMemcpy(F.twy, ty.data(), ty.size() * sizeof(double), cudaMemcpyHostToDevice));
       F.spec = dalloc<double2>(c, (size_t)(H.Nx / 2 + 1) * H.Ny);
@@ -1100,8 +1100,8 @@ int ins2d_ctx_create(const ins2d_grid_desc *grid, const ins2d_bc_desc *bc, const
           F.logx = is_pow2(H.Nx) ? (int)std::lround(std::log2((double)H.Nx)) : -1;
           F.logy = is_pow2(H.Ny) ? (int)std::lround(std::log2((double)H.Ny)) : -1;
           const std::vector<double> tx = fft_twiddle_table(H.Nx), ty = fft_twiddle_table(H.Ny);
-          F.twx = dalloc<double2>(c, 2 * (size_t)H.Nx);
-          F.twy = dalloc<double2>(c, 2 * (size_t)H.Ny);
+          F.twx = dalloc<double2>(c, tx.size() / 2);
+          F.twy = dalloc<double2>(c, ty.size() / 2);
           CK(cudaMemcpy(F.twx, tx.data(), tx.size() * sizeof(double), cudaMemcpyHostToDevice));
           CK(cudaMemcpy(F.twy, ty.data(), ty.size() * sizeof(double), cudaMemcpyHostToDevice));
           F.spec = dalloc<double2>(c, (size_t)(H.Nx / 2 + 1) * H.Ny);

@@ -11,12 +11,14 @@
 //     FFT (scaled 1/Ny), and the max |fhat| reduction;
 //  3. rows, complex half spectrum -> real: two rows packed as one complex
 //     inverse FFT (scaled 1/Nx).
-// Power-of-two lengths use radix-2 DIT/DIF with a twiddle table; other
-// lengths use a shared-memory DFT (O(N^2), small grids).
+// Power-of-two lengths of 64 and more use kernels with compile-time shapes;
+// other lengths the mixed-radix or Bluestein line transforms of fft_line.cuh.
+#include <algorithm>
 #include <cmath>
 #include <type_traits>
 #include <vector>
 
+#include "fft_line.cuh"
 #include "kernels.cuh"
 
 namespace ins2d {
@@ -45,198 +47,80 @@ constexpr int kMaxGeneric = 2048;
 __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
   return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
-__device__ __forceinline__ double2 twid(const double2 *tw, int k, bool inv) {
-  double2 w = __ldg(tw + k);
-  if (inv) w.y = -w.y;
-  return w;
-}
 __device__ __forceinline__ int brev(int k, int logn) { return (int)(__brev((unsigned)k) >> (32 - logn)); }
 
-// Shared-memory layout: complex value i sits at i + i/8 + i/64 + i/512 +
-// i/4096.  A 16-byte access is served eight lanes at a time, so the eight
-// lanes must fall on distinct 16-byte bank groups (slot mod 8): the i/8 term
-// does that for the strided butterfly accesses, the others for the
-// bit-reversed readouts (eight lanes 2^(L-3) apart).  Line strides are 4 mod 8,
-// so two lines interleaved in one warp (column blocks) use disjoint groups.
-__host__ __device__ __forceinline__ int pd(int i) { return i + (i >> 3) + (i >> 6) + (i >> 9) + (i >> 12); }
-__host__ __device__ __forceinline__ int padded(int n) {
-  const int p = pd(n - 1) + 1;
-  return p + ((4 - p) & 7);
-}
-
-// In-place radix-2 decimation in time on G lines of length n (input in
-// bit-reversed order, output natural), three stages per pass: each thread
-// loads 8 values spaced by the first stage's half size, applies the stages in
-// registers and writes them back.  tw has n entries e^{-2 pi i k/n}.
-__device__ void dit(double2 *a, int G, int n, int logn, const double2 *tw, bool inv) {
-  const int t = threadIdx.x, nt = blockDim.x, ld = padded(n);
-  for (int s0 = 0; s0 < logn; s0 += 3) {
-    const int ns = min(3, logn - s0), R = 1 << ns, h = 1 << s0, per = n >> ns;
-    for (int g = t; g < G * per; g += nt) {
-      const int line = g / per, gg = g - line * per;
-      const int k = gg & (h - 1), blk = gg >> s0;
-      const int base = blk * R * h + k;
-      double2 *L = a + (size_t)line * ld;
-      double2 x[8];
-#pragma unroll
-      for (int m = 0; m < 8; ++m)
-        if (m < R) x[m] = L[pd(base + m * h)];
-#pragma unroll
-      for (int st = 0; st < 3; ++st) {
-        if (st >= ns) break;
-        const int hh = 1 << st, sh = logn - (s0 + st + 1);
-#pragma unroll
-        for (int m = 0; m < 8; ++m) {
-          if (m >= R || (m & (2 * hh - 1)) >= hh) continue;
-          const int off = k + (m & (hh - 1)) * h;
-          const double2 y = cmul(twid(tw, off << sh, inv), x[m + hh]);
-          x[m + hh] = make_double2(x[m].x - y.x, x[m].y - y.y);
-          x[m] = make_double2(x[m].x + y.x, x[m].y + y.y);
-        }
-      }
-#pragma unroll
-      for (int m = 0; m < 8; ++m)
-        if (m < R) L[pd(base + m * h)] = x[m];
-    }
-    __syncthreads();
-  }
-}
-
-// In-place radix-2 decimation in frequency (input natural, output
-// bit-reversed), three stages per pass from the largest half size down.
-__device__ void dif(double2 *a, int G, int n, int logn, const double2 *tw, bool inv) {
-  const int t = threadIdx.x, nt = blockDim.x, ld = padded(n);
-  for (int s_hi = logn; s_hi >= 1; s_hi -= 3) {
-    const int ns = min(3, s_hi), s_lo = s_hi - ns + 1;
-    const int R = 1 << ns, h = 1 << (s_lo - 1), per = n >> ns;
-    for (int g = t; g < G * per; g += nt) {
-      const int line = g / per, gg = g - line * per;
-      const int k = gg & (h - 1), blk = gg >> (s_lo - 1);
-      const int base = blk * R * h + k;
-      double2 *L = a + (size_t)line * ld;
-      double2 x[8];
-#pragma unroll
-      for (int m = 0; m < 8; ++m)
-        if (m < R) x[m] = L[pd(base + m * h)];
-#pragma unroll
-      for (int st = 2; st >= 0; --st) {
-        if (st >= ns) continue;
-        const int hh = 1 << st, sh = logn - (s_lo + st);
-#pragma unroll
-        for (int m = 0; m < 8; ++m) {
-          if (m >= R || (m & (2 * hh - 1)) >= hh) continue;
-          const int off = k + (m & (hh - 1)) * h;
-          const double2 x0 = x[m], x1 = x[m + hh];
-          x[m] = make_double2(x0.x + x1.x, x0.y + x1.y);
-          x[m + hh] = cmul(make_double2(x0.x - x1.x, x0.y - x1.y), twid(tw, off << sh, inv));
-        }
-      }
-#pragma unroll
-      for (int m = 0; m < 8; ++m)
-        if (m < R) L[pd(base + m * h)] = x[m];
-    }
-    __syncthreads();
-  }
-}
-
-// Plain DFT of G lines from a into b (natural order, padded layout), any n.
-__device__ void dft(const double2 *a, double2 *b, int G, int n, const double2 *tw, bool inv) {
-  const int ld = padded(n);
-  for (int o = threadIdx.x; o < G * n; o += blockDim.x) {
-    const int line = o / n, k = o - line * n;
-    const double2 *L = a + (size_t)line * ld;
-    double2 s = make_double2(0.0, 0.0);
-    int idx = 0;
-    for (int m = 0; m < n; ++m) {
-      const double2 p = cmul(L[pd(m)], twid(tw, idx, inv));
-      s.x += p.x;
-      s.y += p.y;
-      idx += k;
-      if (idx >= n) idx -= n;
-    }
-    b[(size_t)line * ld + pd(k)] = s;
-  }
-  __syncthreads();
-}
-
-// Pass 1: rows j0=2*blockIdx.x, j1=j0+1 -> half spectra.
-__global__ void __launch_bounds__(kThreads) k_rows_r2c(int Nx, int Ny, int logx, const double2 *__restrict__ tw,
-                                                       const double *__restrict__ f, double2 *__restrict__ spec) {
+// --- lengths without a compile-time shape (fft_line.cuh) ---------------------------
+// Rows 2 blockIdx.x and the next one, packed as one complex line -> half
+// spectra.  SRC as k_rows_r2c_t: 0: the rows of f; 1, 2: the divergence.
+template <int SRC>
+__global__ void __launch_bounds__(kThreads) k_rows_r2c(const __grid_constant__ FftLine Lx, int Ny,
+                                                       const double2 *__restrict__ tab, const double *__restrict__ f,
+                                                       const WSplit ws, double2 *__restrict__ spec,
+                                                       const __grid_constant__ DevOps P, double alpha, double beta,
+                                                       double gamma, const int *__restrict__ skip,
+                                                       unsigned long long *__restrict__ zero_max) {
   extern __shared__ double2 sm[];
+  const int N = Lx.n, H = N / 2 + 1, ld = line_ld(Lx.m);
+  if (zero_max && blockIdx.x == 0 && threadIdx.x == 0) *zero_max = 0ull;  // the column pass's max |fhat|
+  if (skip && *(volatile const int *)skip) return;
   const int j0 = 2 * blockIdx.x, j1 = j0 + 1;
   const bool has1 = j1 < Ny;
-  const int H = Nx / 2 + 1;
-  for (int k = threadIdx.x; k < Nx; k += blockDim.x) {
-    const double a = f[(size_t)j0 * Nx + k];
-    const double b = has1 ? f[(size_t)j1 * Nx + k] : 0.0;
-    sm[pd(logx >= 0 ? brev(k, logx) : k)] = make_double2(a, b);
+  for (int k = threadIdx.x; k < N; k += blockDim.x) {
+    double2 v;
+    if constexpr (SRC == 0)
+      v = make_double2(__ldg(f + (size_t)j0 * N + k), has1 ? __ldg(f + (size_t)j1 * N + k) : 0.0);
+    else if constexpr (SRC == 1)
+      v = make_double2(div_cell(P, f, alpha, beta, gamma, k, j0), has1 ? div_cell(P, f, alpha, beta, gamma, k, j1) : 0.0);
+    else
+      v = make_double2(div_cell_f(P, ws, alpha, beta, gamma, k, j0),
+                       has1 ? div_cell_f(P, ws, alpha, beta, gamma, k, j1) : 0.0);
+    sm[line_slot(k)] = v;
   }
   __syncthreads();
-  const double2 *Z = sm;
-  if (logx >= 0) {
-    dit(sm, 1, Nx, logx, tw, false);
-  } else {
-    dft(sm, sm + padded(Nx), 1, Nx, tw, false);
-    Z = sm + padded(Nx);
-  }
+  const double2 *Z = line_transform(Lx, sm, sm + ld, 1, ld, tab);
   for (int I = threadIdx.x; I < H; I += blockDim.x) {
-    const double2 z = Z[pd(I)], m = Z[pd((Nx - I) % Nx)];
+    const double2 z = Z[line_slot(I)], m = Z[line_slot(I ? N - I : 0)];
     spec[(size_t)j0 * H + I] = make_double2(0.5 * (z.x + m.x), 0.5 * (z.y - m.y));
     if (has1) spec[(size_t)j1 * H + I] = make_double2(0.5 * (z.y + m.y), 0.5 * (m.x - z.x));
   }
 }
 
-// Pass 2: G consecutive spectrum columns per block.
-__global__ void __launch_bounds__(kThreads) k_cols(int Nx, int Ny, int logy, int G, const double2 *__restrict__ tw,
-                                                   const double *__restrict__ ax, const double *__restrict__ ay,
-                                                   double dxdy, double2 *__restrict__ spec,
-                                                   unsigned long long *__restrict__ maxbits) {
+// G consecutive spectrum columns per block: forward, -1/Ahat, inverse; max |fhat|
+__global__ void __launch_bounds__(kThreads) k_cols(const __grid_constant__ FftLine Ly, int H, int G,
+                                                   const double2 *__restrict__ tab, const double *__restrict__ ax,
+                                                   const double *__restrict__ ay, double dxdy,
+                                                   double2 *__restrict__ spec,
+                                                   unsigned long long *__restrict__ maxbits,
+                                                   const int *__restrict__ skip) {
   extern __shared__ double2 sm[];
   __shared__ double wmax[kThreads / 32];
-  const int H = Nx / 2 + 1;
-  const int c0 = blockIdx.x * G;
-  const int g_here = min(G, H - c0);
-  // power-of-two columns: forward decimation in frequency (natural order in,
-  // bit-reversed out), scaling in bit-reversed order, inverse decimation in
-  // time (bit-reversed in, natural out) -- no permutation pass is needed
-  const int ldy = padded(Ny);
-  for (int o = threadIdx.x; o < g_here * Ny; o += blockDim.x) {
+  if (skip && *(volatile const int *)skip) return;
+  const int N = Ly.n, ld = line_ld(Ly.m);
+  const int c0 = blockIdx.x * G, g_here = min(G, H - c0);
+  double2 *a = sm, *b = sm + G * ld;
+  for (int o = threadIdx.x; o < g_here * N; o += blockDim.x) {
     const int j = o / g_here, g = o - j * g_here;
-    sm[(size_t)g * ldy + pd(j)] = spec[(size_t)j * H + c0 + g];
+    a[g * ld + line_slot(j)] = spec[(size_t)j * H + c0 + g];
   }
   __syncthreads();
-  double2 *A = sm;
-  if (logy >= 0) {
-    dif(sm, g_here, Ny, logy, tw, false);
-  } else {
-    dft(sm, sm + (size_t)G * ldy, g_here, Ny, tw, false);
-    A = sm + (size_t)G * ldy;
-  }
+  double2 *F = line_transform(Ly, a, b, g_here, ld, tab);
   double lmax = 0.0;
-  for (int o = threadIdx.x; o < g_here * Ny; o += blockDim.x) {
-    const int g = o / Ny, pos = o - g * Ny;
-    const int J = logy >= 0 ? brev(pos, logy) : pos;
-    const int I = c0 + g;
-    double2 *slot = A + (size_t)g * ldy + pd(pos);
-    const double2 F = *slot;
-    lmax = fmax(lmax, sqrt(F.x * F.x + F.y * F.y));
+  for (int o = threadIdx.x; o < g_here * N; o += blockDim.x) {
+    const int g = o / N, J = o - g * N, I = c0 + g;
+    double2 *slot = F + g * ld + line_slot(J);
+    const double2 v = *slot;
+    lmax = fmax(lmax, v.x * v.x + v.y * v.y);  // squared; one square root per block
     const double lam = (I == 0 && J == 0) ? 1.0 : (dxdy * 4.0) * (__ldg(ax + I) + __ldg(ay + J));
     const double r = -1.0 / lam;
-    *slot = make_double2(F.x * r, F.y * r);
+    *slot = make_double2(v.y * r, v.x * r);  // exchanged: the next transform is the inverse
   }
   __syncthreads();
-  double2 *Bout = A;
-  if (logy >= 0) {
-    dit(A, g_here, Ny, logy, tw, true);
-  } else {
-    dft(A, sm, g_here, Ny, tw, true);
-    Bout = sm;
-  }
-  const double sc = 1.0 / Ny;
-  for (int o = threadIdx.x; o < g_here * Ny; o += blockDim.x) {
+  const double2 *B = line_transform(Ly, F, F == a ? b : a, g_here, ld, tab);
+  const double sc = 1.0 / N;
+  for (int o = threadIdx.x; o < g_here * N; o += blockDim.x) {
     const int j = o / g_here, g = o - j * g_here;
-    const double2 v = Bout[(size_t)g * ldy + pd(j)];
-    spec[(size_t)j * H + c0 + g] = make_double2(v.x * sc, v.y * sc);
+    const double2 v = B[g * ld + line_slot(j)];
+    spec[(size_t)j * H + c0 + g] = make_double2(v.y * sc, v.x * sc);
   }
   for (int off = 16; off > 0; off >>= 1) lmax = fmax(lmax, __shfl_down_sync(0xffffffffu, lmax, off));
   if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = lmax;
@@ -244,61 +128,57 @@ __global__ void __launch_bounds__(kThreads) k_cols(int Nx, int Ny, int logy, int
   if (threadIdx.x == 0) {
     double m = wmax[0];
     for (int w = 1; w < (int)(blockDim.x >> 5); ++w) m = fmax(m, wmax[w]);
-    atomicMax(maxbits, (unsigned long long)__double_as_longlong(m));  // m >= 0: bit order = value order
+    atomicMax(maxbits, (unsigned long long)__double_as_longlong(sqrt(m)));  // m >= 0: bit order = value order
   }
 }
 
-// Pass 3: half spectra of rows j0, j1 -> real rows (scaled 1/Nx).
-__global__ void __launch_bounds__(kThreads) k_rows_c2r(int Nx, int Ny, int logx, const double2 *__restrict__ tw,
+// half spectra of two rows -> real rows (scaled 1/Nx)
+__global__ void __launch_bounds__(kThreads) k_rows_c2r(const __grid_constant__ FftLine Lx, int Ny,
+                                                       const double2 *__restrict__ tab,
                                                        const double2 *__restrict__ spec, double *__restrict__ out,
-                                                       int accumulate, const unsigned long long *__restrict__ maxbits) {
+                                                       int accumulate, const unsigned long long *__restrict__ maxbits,
+                                                       const int *__restrict__ skip) {
   extern __shared__ double2 sm[];
+  if (skip && *(volatile const int *)skip) return;
+  const int N = Lx.n, H = N / 2 + 1, ld = line_ld(Lx.m);
   const int j0 = 2 * blockIdx.x, j1 = j0 + 1;
   const bool has1 = j1 < Ny;
-  const int H = Nx / 2 + 1;
   const double mx = __longlong_as_double((long long)*maxbits);
   if (mx < 1e-14) {  // pressure_poisson.m:21-32: dp stays zero
     if (!accumulate)
-      for (int k = threadIdx.x; k < Nx; k += blockDim.x) {
-        out[(size_t)j0 * Nx + k] = 0.0;
-        if (has1) out[(size_t)j1 * Nx + k] = 0.0;
+      for (int k = threadIdx.x; k < N; k += blockDim.x) {
+        out[(size_t)j0 * N + k] = 0.0;
+        if (has1) out[(size_t)j1 * N + k] = 0.0;
       }
     return;
   }
-  for (int k = threadIdx.x; k < Nx; k += blockDim.x) {
+  for (int k = threadIdx.x; k < N; k += blockDim.x) {
     double2 g0, g1;
     if (k < H) {
       g0 = spec[(size_t)j0 * H + k];
       g1 = has1 ? spec[(size_t)j1 * H + k] : make_double2(0.0, 0.0);
     } else {
-      const double2 a = spec[(size_t)j0 * H + (Nx - k)];
-      const double2 b = has1 ? spec[(size_t)j1 * H + (Nx - k)] : make_double2(0.0, 0.0);
+      const double2 a = spec[(size_t)j0 * H + (N - k)];
+      const double2 b = has1 ? spec[(size_t)j1 * H + (N - k)] : make_double2(0.0, 0.0);
       g0 = make_double2(a.x, -a.y);
       g1 = make_double2(b.x, -b.y);
     }
-    sm[pd(logx >= 0 ? brev(k, logx) : k)] = make_double2(g0.x - g1.y, g0.y + g1.x);
+    sm[line_slot(k)] = make_double2(g0.y + g1.x, g0.x - g1.y);  // exchanged: inverse transform
   }
   __syncthreads();
-  const double2 *W = sm;
-  if (logx >= 0) {
-    dit(sm, 1, Nx, logx, tw, true);
-  } else {
-    dft(sm, sm + padded(Nx), 1, Nx, tw, true);
-    W = sm + padded(Nx);
-  }
-  const double sc = 1.0 / Nx;
-  for (int k = threadIdx.x; k < Nx; k += blockDim.x) {
-    const double2 w = W[pd(k)];
+  const double2 *Z = line_transform(Lx, sm, sm + ld, 1, ld, tab);
+  const double sc = 1.0 / N;
+  for (int k = threadIdx.x; k < N; k += blockDim.x) {
+    const double2 w = Z[line_slot(k)];
     if (accumulate) {
-      out[(size_t)j0 * Nx + k] += w.x * sc;
-      if (has1) out[(size_t)j1 * Nx + k] += w.y * sc;
+      out[(size_t)j0 * N + k] += w.y * sc;
+      if (has1) out[(size_t)j1 * N + k] += w.x * sc;
     } else {
-      out[(size_t)j0 * Nx + k] = w.x * sc;
-      if (has1) out[(size_t)j1 * Nx + k] = w.y * sc;
+      out[(size_t)j0 * N + k] = w.y * sc;
+      if (has1) out[(size_t)j1 * N + k] = w.x * sc;
     }
   }
 }
-
 
 // ---------------------------------------------------------------------------
 // Register groups of up to three radix-2 stages on 8 values x[m] at positions
@@ -474,10 +354,12 @@ __device__ __forceinline__ void group_dit16(double2 (&x)[16], int k, int h, cons
 // stores, no permutation passes; tw is the table of fft_twiddle_table (the
 // pyramid at tw + 2^L) ---------------------------------------------------------
 
-// Slot of complex value i in a line of length 2^L: the general layout above,
-// or for L >= 9 the cheaper i + i/8 + i/2^(L-3), conflict-free for the same
-// accesses at those lengths (the last term spreads the bit-reversed readouts,
-// whose eight lanes lie 2^(L-3) apart).
+// Slot of complex value i in a line of length 2^L.  A 16-byte access is served
+// eight lanes at a time, so the eight lanes must fall on distinct 16-byte bank
+// groups (slot mod 8): the i/8 term does that for the strided butterfly
+// accesses, the others for the bit-reversed readouts (eight lanes 2^(L-3)
+// apart; for L >= 9 one term is enough).  Line strides are 4 mod 8, so two
+// lines interleaved in one warp (column blocks) use disjoint groups.
 template <int L>
 __host__ __device__ constexpr int pdl(int i) {
   return L >= 9 ? i + (i >> 3) + (i >> (L - 3)) : i + (i >> 3) + (i >> 6) + (i >> 9) + (i >> 12);
@@ -905,32 +787,130 @@ int ilog2_exact(int n) {
   return ((1 << l) == n) ? l : -1;
 }
 
-int cols_group(int Ny, bool pow2) {
-  // two columns (32-byte row segments) per block; more for short columns
-  const size_t per = (size_t)padded(Ny) * sizeof(double2) * (pow2 ? 1 : 2);
-  int G = (int)((INS2D_FFT_COLS_BUDGET * 1024) / per);
-  if (G > 8) G = 8;
-  if (G < 1) G = 1;
-  if (Ny >= 1024 && G > INS2D_FFT_COLS_G) G = INS2D_FFT_COLS_G;
-  return G;
+// columns per block of k_cols: up to 64-byte row segments within the
+// shared-memory budget (two buffers per line)
+int cols_group(const FftLine &L) {
+  const size_t per = 2 * (size_t)line_ld(L.m) * sizeof(double2);
+  return (int)std::max<size_t>(1, std::min<size_t>(4, (INS2D_FFT_COLS_BUDGET * 1024) / per));
+}
+// threads per block for `lines` lines: about one butterfly of radix 4 each
+int line_threads(const FftLine &L, int lines) {
+  int t = 32;
+  while (t < kThreads && t * 4 < lines * L.m) t *= 2;
+  return t;
+}
+// in-place transform of length 2^l values in extended precision (tables only)
+void host_fft(std::vector<long double> &re, std::vector<long double> &im) {
+  const size_t n = re.size();
+  for (size_t i = 1, j = 0; i < n; ++i) {
+    size_t bit = n >> 1;
+    for (; j & bit; bit >>= 1) j ^= bit;
+    j |= bit;
+    if (i < j) {
+      std::swap(re[i], re[j]);
+      std::swap(im[i], im[j]);
+    }
+  }
+  const long double pi = std::acos(-1.0L);
+  for (size_t len = 2; len <= n; len <<= 1)
+    for (size_t k = 0; k < len / 2; ++k) {
+      const long double a = -2.0L * pi * (long double)k / (long double)len, c = std::cos(a), s = std::sin(a);
+      for (size_t i = k; i < n; i += len) {
+        const size_t j = i + len / 2;
+        const long double xr = re[j] * c - im[j] * s, xi = re[j] * s + im[j] * c;
+        re[j] = re[i] - xr;
+        im[j] = im[i] - xi;
+        re[i] += xr;
+        im[i] += xi;
+      }
+    }
 }
 
 }  // namespace
 
-std::vector<double> fft_twiddle_table(int n) {
-  std::vector<double> v(4 * (size_t)n, 0.0);
-  for (int k = 0; k < n; ++k) {
-    const double ang = 2.0 * M_PI * (double)k / (double)n;
-    v[2 * k] = std::cos(ang);
-    v[2 * k + 1] = -std::sin(ang);
+FftLine fft_line(int n) {
+  FftLine L;
+  L.n = L.m = n;
+  int rest = n, twos = 0;
+  std::vector<int> odd;
+  while (rest % 2 == 0) {
+    rest /= 2;
+    ++twos;
   }
-  if (ilog2_exact(n) >= 0)
+  for (int p = 3; rest > 1; p += 2)
+    while (rest % p == 0) {
+      rest /= p;
+      odd.push_back(p);
+    }
+  if (!odd.empty() && odd.back() > kMaxFactor) {  // Bluestein: a power of two
+    odd.clear();
+    twos = 0;
+    while ((1 << twos) < 2 * n - 1) ++twos;
+    L.m = 1 << twos;
+  }
+  std::vector<int> f;
+  while (twos >= 3 && twos != 4) {
+    f.push_back(8);
+    twos -= 3;
+  }
+  for (; twos >= 2; twos -= 2) f.push_back(4);
+  if (twos) f.push_back(2);
+  f.insert(f.end(), odd.rbegin(), odd.rend());
+  int s = 1;
+  for (int r : f) {
+    auto inv = [](unsigned d) { return (unsigned)(((1ull << 32) + d - 1) / d); };
+    L.r[L.np] = r;
+    L.s[L.np] = s;
+    L.inv_s[L.np] = inv((unsigned)s);
+    L.inv_b[L.np] = inv((unsigned)(L.m / r));
+    ++L.np;
+    s *= r;
+  }
+  return L;
+}
+
+std::vector<double> fft_twiddle_table(int n) {
+  std::vector<double> v;
+  auto root = [&](size_t at, long long k, long long len) {  // e^{-2 pi i k / len}
+    const double ang = 2.0 * M_PI * (double)k / (double)len;
+    v[2 * at] = std::cos(ang);
+    v[2 * at + 1] = -std::sin(ang);
+  };
+  const int l = ilog2_exact(n);
+  if (l >= kFusedMinLog) {
+    v.assign(4 * (size_t)n, 0.0);
+    for (int k = 0; k < n; ++k) root(k, k, n);
     for (int Lt = 2; Lt <= n; Lt *= 2)
-      for (int k = 0; k < Lt / 2; ++k) {
-        const double ang = 2.0 * M_PI * (double)k / (double)Lt;
-        v[2 * ((size_t)n + Lt / 2 + k)] = std::cos(ang);
-        v[2 * ((size_t)n + Lt / 2 + k) + 1] = -std::sin(ang);
+      for (int k = 0; k < Lt / 2; ++k) root((size_t)n + Lt / 2 + k, k, Lt);
+    return v;
+  }
+  const FftLine L = fft_line(n);
+  const size_t m = (size_t)L.m;
+  v.assign(2 * (m == (size_t)n ? m : m + n + m / 2 + 1), 0.0);
+  for (size_t k = 0; k < m; ++k) root(k, (long long)k, (long long)m);
+  if (m != (size_t)n) {
+    // chirp c_k = e^{-i pi k^2/n} (k^2 taken mod 2n: exact arguments) and the
+    // transform of the filter 1/c_|k| over the cyclic length m
+    std::vector<long double> re(m, 0.0L), im(m, 0.0L);
+    const long double pi = std::acos(-1.0L);
+    for (long long k = 0; k < n; ++k) {
+      const long double a = pi * (long double)((k * k) % (2LL * n)) / (long double)n;
+      const long double c = std::cos(a), s = std::sin(a);
+      v[2 * (m + k)] = (double)c;
+      v[2 * (m + k) + 1] = (double)-s;
+      re[k] = c;
+      im[k] = s;
+      if (k) {
+        re[m - k] = c;
+        im[m - k] = s;
       }
+    }
+    host_fft(re, im);
+    for (size_t k = 0; k <= m / 2; ++k) {
+      v[2 * (m + n + k)] = (double)re[k];
+      v[2 * (m + n + k) + 1] = (double)im[k];
+    }
+  }
   return v;
 }
 
@@ -956,7 +936,9 @@ cudaError_t fft_prepare() {
       opt_in((const void *)k_cols_t<L, cols_per_block<L>(), cols_radix<L>()>);
       opt_in((const void *)k_rows_c2r_t<L>);
     });
-  opt_in((const void *)k_rows_r2c);
+  opt_in((const void *)k_rows_r2c<0>);
+  opt_in((const void *)k_rows_r2c<1>);
+  opt_in((const void *)k_rows_r2c<2>);
   opt_in((const void *)k_cols);
   opt_in((const void *)k_rows_c2r);
   return first;
@@ -972,13 +954,8 @@ cudaError_t fft_passes(const DevOps &P, const FftPlan &plan, const double *src, 
   const int pairs = (Ny + 1) / 2;
   const int H = Nx / 2 + 1;
   unsigned long long *maxbits = (unsigned long long *)plan.maxabs;
-  // the fused row pass zeroes max |fhat| itself (no memset node between the
-  // passes, so the step's kernels chain by programmatic launch)
-  if (!(plan.logx >= kFusedMinLog && plan.logx <= 13)) {
-    const cudaError_t ms = cudaMemsetAsync(plan.maxabs, 0, sizeof(double), s);
-    if (ms != cudaSuccess) return ms;
-  }
-  // rows, real -> half spectrum
+  // rows, real -> half spectrum (the first pass also zeroes max |fhat|: no
+  // memset node between the passes)
   const int fastdiv = P.rMX.lo <= 0 && P.rMX.hi >= Nx && P.rMY.lo <= 0 && P.rMY.hi >= Ny && P.rMX.two && P.rMY.two;
   const bool fx = with_log2<kFusedMinLog>(plan.logx, [&](auto c) {
     constexpr int L = decltype(c)::value;
@@ -995,8 +972,19 @@ cudaError_t fft_passes(const DevOps &P, const FftPlan &plan, const double *src, 
       launch_k(k_rows_r2c_t<L, 0>, dim3(pairs), dim3(kThreads), sm, s, Ny, plan.twx, src, w0, plan.spec, P, 0.0,
                0.0, 0.0, 0, skip, maxbits);
   });
-  const size_t smx = (size_t)padded(Nx) * sizeof(double2) * (plan.logx >= 0 ? 1 : 2);
-  if (!fx) k_rows_r2c<<<pairs, kThreads, smx, s>>>(Nx, Ny, plan.logx, plan.twx, src, plan.spec);
+  const FftLine Lx = fx ? FftLine{} : fft_line(Nx);
+  const size_t smx = fx ? 0 : 2 * (size_t)line_ld(Lx.m) * sizeof(double2);
+  if (!fx) {
+    const int t = line_threads(Lx, 1);
+    if (ws)
+      k_rows_r2c<2><<<pairs, t, smx, s>>>(Lx, Ny, plan.twx, nullptr, *ws, plan.spec, P, alpha, beta, gamma, skip,
+                                         maxbits);
+    else if (div)
+      k_rows_r2c<1><<<pairs, t, smx, s>>>(Lx, Ny, plan.twx, src, WSplit{}, plan.spec, P, alpha, beta, gamma, skip,
+                                         maxbits);
+    else
+      k_rows_r2c<0><<<pairs, t, smx, s>>>(Lx, Ny, plan.twx, src, WSplit{}, plan.spec, P, 0.0, 0.0, 0.0, skip, maxbits);
+  }
   // columns: forward, scaling, inverse
   const bool fy = with_log2<kFusedMinLog>(plan.logy, [&](auto c) {
     constexpr int L = decltype(c)::value, G = cols_per_block<L>();
@@ -1005,10 +993,11 @@ cudaError_t fft_passes(const DevOps &P, const FftPlan &plan, const double *src, 
              P.fft_ax, P.fft_ay, P.fft_dxdy, plan.spec, maxbits, skip);
   });
   if (!fy) {
-    const int G = cols_group(Ny, plan.logy >= 0);
-    const size_t smy = (size_t)G * padded(Ny) * sizeof(double2) * (plan.logy >= 0 ? 1 : 2);
-    k_cols<<<(H + G - 1) / G, kThreads, smy, s>>>(Nx, Ny, plan.logy, G, plan.twy, P.fft_ax, P.fft_ay, P.fft_dxdy,
-                                                  plan.spec, maxbits);
+    const FftLine Ly = fft_line(Ny);
+    const int G = cols_group(Ly);
+    const size_t smy = 2 * (size_t)G * line_ld(Ly.m) * sizeof(double2);
+    k_cols<<<(H + G - 1) / G, line_threads(Ly, G), smy, s>>>(Ly, H, G, plan.twy, P.fft_ax, P.fft_ay, P.fft_dxdy,
+                                                            plan.spec, maxbits, skip);
   }
   // rows, half spectrum -> real
   const bool fx2 = with_log2<kFusedMinLog>(plan.logx, [&](auto c) {
@@ -1019,8 +1008,8 @@ cudaError_t fft_passes(const DevOps &P, const FftPlan &plan, const double *src, 
              skip);
   });
   if (!fx2)
-    k_rows_c2r<<<pairs, kThreads, smx, s>>>(Nx, Ny, plan.logx, plan.twx, plan.spec, dp, accumulate ? 1 : 0,
-                                            gate ? gate : maxbits);
+    k_rows_c2r<<<pairs, line_threads(Lx, 1), smx, s>>>(Lx, Ny, plan.twx, plan.spec, dp, accumulate ? 1 : 0,
+                                                       gate ? gate : maxbits, skip);
   return cudaSuccess;
 }
 }  // namespace
@@ -1029,8 +1018,6 @@ cudaError_t launch_fft_poisson(const DevOps &P, const FftPlan &plan, const doubl
                                cudaStream_t s) {
   return fft_passes(P, plan, f, nullptr, false, 0.0, 0.0, 0.0, dp, accumulate, s);
 }
-
-bool fft_fuses_div(const FftPlan &plan) { return plan.logx >= kFusedMinLog && plan.logx <= 13; }
 
 int fft_kernels(const FftPlan &) { return 3; }
 

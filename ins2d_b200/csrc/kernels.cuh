@@ -175,14 +175,16 @@ void launch_stage_cached_ens(const EnsMemberD *mem, const int4 *tiles, int n, do
 // --- FFT Poisson (fft.cu) -------------------------------------------------------
 struct FftPlan {
   int Nx = 0, Ny = 0, logx = -1, logy = -1;  // log2 when a power of two, else -1
-  double2 *twx = nullptr, *twy = nullptr;    // 2N entries each: fft_twiddle_table(N)
+  double2 *twx = nullptr, *twy = nullptr;    // fft_twiddle_table of Nx and Ny
   double2 *spec = nullptr;                   // (Nx/2+1) x Ny complex spectrum
   double *maxabs = nullptr;                  // max |fhat| of the last solve
 };
 bool fft_supported(int Nx, int Ny);
-// Twiddles of a length-n transform as 2n complex values (4n doubles): entries
-// [0, n) hold e^{-2 pi i k/n}; for power-of-two n, entry n + Lt/2 + k holds
-// e^{-2 pi i k/Lt} for every power of two 2 <= Lt <= n and k < Lt/2.
+// Tables of a length-n transform as complex values (pairs of doubles).
+// Powers of two from 64: 2n values, e^{-2 pi i k/n} at k and e^{-2 pi i k/Lt}
+// at n + Lt/2 + k for every power of two 2 <= Lt <= n, k < Lt/2.  Other
+// lengths: those of fft_line.cuh, n values, or m + n + m/2 + 1 where the
+// transform runs over m > n (Bluestein; at most 8192 values up to n = 2048).
 std::vector<double> fft_twiddle_table(int n);
 // dp = real(ifft2(-fft2(f)./Ahat)) (pressure_poisson.m:92-104); dp += result when
 // accumulate.  Returns 0 (dp untouched / zero) when max|fhat| < 1e-14 (:21-32).
@@ -191,8 +193,7 @@ std::vector<double> fft_twiddle_table(int n);
 cudaError_t launch_fft_poisson(const DevOps &P, const FftPlan &plan, const double *f, double *dp, bool accumulate,
                                cudaStream_t s);
 // Same with the right-hand side f = (M W + alpha yM + beta ydM) gamma computed
-// inside the first pass (only when fft_fuses_div(plan): power-of-two rows >= 64).
-bool fft_fuses_div(const FftPlan &plan);
+// inside the first pass.
 // kernel launches of one solve (the column transform takes one or three)
 int fft_kernels(const FftPlan &plan);
 cudaError_t launch_fft_poisson_div(const DevOps &P, const FftPlan &plan, const double *W, double alpha,

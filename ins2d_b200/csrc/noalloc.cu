@@ -24,7 +24,7 @@ namespace {
 constexpr int kMaxN = INS2D_NOALLOC_MAX_N;
 constexpr long long kMaxCells = INS2D_NOALLOC_MAX_CELLS;
 // layout in double2 units: spectrum ((Nx/2+1)*Ny <= kMaxCells/2 + kMaxN),
-// twiddle tables x and y (2N <= 2 kMaxN each), symbol factors x and y
+// transform tables x and y (fft_twiddle_table: at most 2 kMaxN values each), symbol factors x and y
 // (<= kMaxN doubles each = kMaxN/2 double2), max|fhat| (one double, padded to
 // a double2)
 constexpr size_t kSpec = (size_t)(kMaxCells / 2 + kMaxN);

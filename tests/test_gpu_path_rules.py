@@ -58,3 +58,36 @@ def test_small_grid_solve(shape, combo):
     ref, pref = R.time_ERK(ref, pref, 1e-3, 1e-3, o)
     assert _rel(m.time_ERK(V, np.zeros(m.Np), 0.0, 1e-3, nsteps=2)[0], ref) < 1e-10
     m.close()
+
+
+# line transforms: every radix and leftover, primes by direct sums (up to 31)
+# and by Bluestein's algorithm (37 and more, up to the longest length), odd
+# lengths, one side a compile-time power of two; right-hand sides given, and
+# formed from a velocity inside the first pass (FP64 and FP32 stages)
+@pytest.mark.parametrize("shape", [(2, 3), (6, 2), (12, 10), (40, 32), (31, 29), (49, 37), (125, 343), (74, 961), (64, 1009),
+                                   (2039, 64), (2047, 17), (24, 2039), (1000, 600), (1536, 640), (375, 2000)])
+def test_line_transforms(shape):
+    nx, ny = shape
+    x, y = np.arange(nx + 1) / nx * 1.5, np.arange(ny + 1) / ny
+    bc = BC_COMBOS["periodic"]
+    m = api.Options(x, y, bc, poisson=6)
+    rng = np.random.default_rng(nx)
+    f = rng.standard_normal((ny, nx))
+    f -= f.mean()
+    J, I = np.arange(ny)[:, None], np.arange(nx)[None, :]
+    dx, dy = x[1], y[1]
+    a = 4 * dx * dy * (np.sin(np.pi * I / nx) ** 2 / dx ** 2 + np.sin(np.pi * J / ny) ** 2 / dy ** 2)
+    a[0, 0] = 1.0
+    ref = np.real(np.fft.ifft2(-np.fft.fft2(f) / a)).ravel()
+    assert _rel(m.pressure_poisson(f.ravel()), ref) < 1e-12
+    assert np.all(m.pressure_poisson(np.zeros(nx * ny)) == 0.0)
+    if min(shape) < 12 or max(shape) > 1000:
+        return
+    o = R.make_options(x, y, bc, poisson=6, Re=100.0)
+    V = R.initial_projection(rng.standard_normal(o.grid.NV), 0.0, o)
+    ref, pref = R.time_ERK(V, np.zeros(m.Np), 0.0, 1e-4, o)
+    m = api.Options(x, y, bc, poisson=6, Re=100.0)
+    V1, p1 = m.time_ERK(V, np.zeros(m.Np), 0.0, 1e-4)
+    assert _rel(V1, ref) < 1e-11 and _rel(p1, pref) < 1e-9
+    m = api.Options(x, y, bc, poisson=6, Re=100.0, precision="fp32")
+    assert _rel(m.time_ERK(V, np.zeros(m.Np), 0.0, 1e-4)[0], ref) < 1e-5
