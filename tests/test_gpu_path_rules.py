@@ -91,3 +91,22 @@ def test_line_transforms(shape):
     assert _rel(V1, ref) < 1e-11 and _rel(p1, pref) < 1e-9
     m = api.Options(x, y, bc, poisson=6, Re=100.0, precision="fp32")
     assert _rel(m.time_ERK(V, np.zeros(m.Np), 0.0, 1e-4)[0], ref) < 1e-5
+
+
+# the network's edge layers and weight gradients: tile edges of 62, 64 and 16,
+# one column or row left over, several fields; the learned tests' bounds
+@pytest.mark.parametrize("path", ["tcgen05", "mma_sync"])
+@pytest.mark.parametrize("shape", [(1, 1, 62), (1, 16, 63), (2, 17, 64), (1, 15, 65), (3, 33, 124), (1, 129, 130)])
+def test_network_tiles(shape, path):
+    from oracle import cnn_ref as N
+    from tests import test_gpu_learned as L
+    net, w, scale = L._net(seed=11, scale=0.8, path=path)
+    inp, tgt, ti, tt = L._inputs(9, *shape)
+    acts = L._check_layers(net, w, scale, inp, net.forward(ti).cpu().numpy())
+    loss, g = net.loss_grad(ti, tt)
+    loss_ref, g_ref = N.loss_grad(w, scale, inp, tgt, bf16_mode=True, acts=acts)
+    assert abs(loss - loss_ref) / loss_ref < 1e-5
+    bounds = [0, N.OFF_WM] + [N.OFF_WM + (k + 1) * N.SZ_WM for k in range(N.NMID)] + [N.NPARAM]
+    for a, b in zip(bounds[:-1], bounds[1:]):
+        assert L._rel(g[a:b], g_ref[a:b]) < 1e-2, (a, b)
+    assert L._rel(g[N.OFF_W6:], g_ref[N.OFF_W6:]) < 1e-5
