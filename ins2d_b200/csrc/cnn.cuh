@@ -67,6 +67,7 @@ struct CudaError : std::runtime_error {
   using std::runtime_error::runtime_error;
 };
 // doubles of reduction scratch the helpers below need
+cudaError_t prepare_kernels();
 size_t red_doubles();
 
 // network inputs (and targets) from a Poisson right-hand side f (and its
