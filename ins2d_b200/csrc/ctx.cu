@@ -168,13 +168,15 @@ void upload_fdm(ins2d_ctx *c, FdmD &D) {
   D.Q = upload_vec(c, T.Q);
   D.piv = upload_vec(c, T.piv);
   D.e = upload_vec(c, T.e);
-  D.h = upload_vec(c, T.h);
   if (!T.g.empty()) {
     D.g = upload_vec(c, T.g);
     D.cr = upload_vec(c, T.cr);
   }
   D.null_mode = T.null_mode;
-  D.hsum = T.hsum;
+  if (T.null_mode >= 0) {
+    D.ng = upload_vec(c, T.ng);
+    D.nmu = upload_vec(c, T.nmu);
+  }
   D.t = dalloc<double>(c, (size_t)c->P.Np);
 }
 
@@ -415,9 +417,8 @@ int solve_cluster(ins2d_ctx *c, const SolveSrc &src, double *dp, bool accumulate
   if (st) *st = ins2d_solve_stats{0, 0.0, 0.0};
   {
     Prof pr(c, INS2D_PROF_POISSON, 1);
-    pcg_solve_cluster(c->P, c->fdm, c->pcg, src, dp, tol, c->opts.CG_maxit, accumulate,
-                      c->dev_loop ? c->accum : nullptr, c->stream);
-    CK(cudaGetLastError());
+    CK(pcg_solve_cluster(c->P, c->fdm, c->pcg, src, dp, tol, c->opts.CG_maxit, accumulate,
+                         c->dev_loop ? c->accum : nullptr, c->stream));
   }
   return c->dev_loop ? INS2D_OK : read_solve(c, st);
 }
@@ -1117,7 +1118,10 @@ int ins2d_ctx_create(const ins2d_grid_desc *grid, const ins2d_bc_desc *bc, const
             throw std::invalid_argument("fast-diagonalization preconditioner: grid larger than " +
                                         std::to_string(kFdmMaxN) + " cells in a direction");
           upload_fdm(c, D);
-          if (pcg_use_cluster(D)) CK(pcg_cluster_prepare());
+          if (pcg_use_cluster(D)) {
+            CK(pcg_cluster_prepare());
+            P.pdl = 1;
+          }
         }
         c->use_fdm = true;
       } else if (opts->precond != INS2D_PRECOND_JACOBI) {

@@ -76,6 +76,7 @@ struct DevOps {
   int tile_ok32;  // ... on FP32 fields
   int all_fast;   // the rectangle holds every tile of the grid (no table-walker tiles)
   int nsm;        // multiprocessors of the device (persistent launches)
+  int pdl;        // programmatic dependent launch of this grid's step kernels
 };
 
 // --- 1D table application ---------------------------------------------------

@@ -180,7 +180,6 @@ FdmTri fdm_tri(const Table &TX, const std::vector<double> &hx, const Table &TY, 
   F.Q = m.Q;
   F.lam = m.lam;
   F.h = F.xmodes ? hy : hx;
-  for (double h : F.h) F.hsum += h;
   auto at = [&](int i, int k) {
     auto it = Ts.T.rows[i].find(k);
     return it == Ts.T.rows[i].end() ? 0.0 : it->second;
@@ -222,7 +221,25 @@ FdmTri fdm_tri(const Table &TX, const std::vector<double> &hx, const Table &TY, 
     }
     p[0] = 1.0 / db[0];
     for (int i = 1; i < n; ++i) p[i] = 1.0 / (db[i] - F.e[i - 1] * F.e[i - 1] * p[i - 1]);
-    if (null) p[n - 1] = 0.0;  // zh_{n-1} = 0; also drops the cyclic corner, which only couples to it
+    if (null) {
+      p[n - 1] = 0.0;  // y_{n-1} = 0; also drops the cyclic corner, which only couples to it
+      // g = y(h), the elimination being symmetric: with H = sum(h),
+      // zh = P y(w - h sum(w)/H), P v = v - (h'v)/H
+      std::vector<double> g(n);
+      double hsum = 0.0, hg = 0.0;
+      for (int i = 0; i < n; ++i) {
+        g[i] = -(F.h[i] + (i ? F.e[i - 1] * g[i - 1] : 0.0)) * p[i];
+        hsum += F.h[i];
+      }
+      for (int i = n - 2; i >= 0; --i) g[i] -= F.e[i] * p[i] * g[i + 1];
+      for (int i = 0; i < n; ++i) hg += F.h[i] * g[i];
+      F.ng.resize(n);
+      F.nmu.resize(n);
+      for (int i = 0; i < n; ++i) {
+        F.ng[i] = g[i] / hsum - hg / (hsum * hsum);
+        F.nmu[i] = g[i] / hsum;
+      }
+    }
     if (c != 0.0 && !null) {
       // q solves the modified system for u = (gam, 0, .., 0, c); g = q / (1 + v'q)
       double *q = &F.g[(size_t)b * n];

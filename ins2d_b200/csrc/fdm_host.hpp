@@ -33,10 +33,12 @@ struct FdmTri {
   // cyclic systems (Sherman-Morrison): zh = y - (y_0 + cr_b y_{n-1}) g_b
   std::vector<double> g, cr;   // nm x n and nm, empty when not cyclic
   // mode whose system is singular (closed and periodic domains; -1: none):
-  // its right-hand side is made consistent, its last unknown set to zero and
-  // the h-weighted mean removed, i.e. the null mode is left out
+  // its right-hand side is made consistent and the h-weighted mean of its
+  // solution removed, i.e. the null mode is left out.  With y the elimination
+  // that sets the last unknown to zero, both are rank-one corrections:
+  //   zh = y - sum(w) ng - (nmu' w),  ng, nmu of n values
   int null_mode = -1;
-  double hsum = 0.0;
+  std::vector<double> ng, nmu;
 };
 // the mode direction is the one with fewer cells (fewer operations)
 FdmTri fdm_tri(const Table &TX, const std::vector<double> &hx, const Table &TY, const std::vector<double> &hy);

@@ -56,27 +56,23 @@ __device__ __forceinline__ void tri_solve(const FdmD &F, int b, int wr, const Tr
   const double ep = T.ep;
   const double(&m)[C] = T.m;
   const double(&e)[C] = T.e;
-  // the null mode: a right-hand side without its component along diag(h) 1
-  double sum = 0.0;
+  // the null mode's two sums over w (fdm_host.hpp): independent of the scans
+  // below, so their shuffles overlap
+  double sum = 0.0, part = 0.0;
   if (null) {
 #pragma unroll
-    for (int k = 0; k < C; ++k) sum += y[k];
+    for (int k = 0; k < C; ++k) {
+      sum += y[k];
+      if (s0 + k < n) part += __ldg(F.nmu + s0 + k) * y[k];
+    }
     sum = tri_warp_sum(sum);
+    part = tri_warp_sum(part);
   }
   if constexpr (W > 1) {
-    if (lane == 0) sh[warp][0] = sum;
-    __syncthreads();
-    if (null) {
-      sum = 0.0;
-#pragma unroll
-      for (int v = 0; v < W; ++v) sum += sh[w0 + v][0];
+    if (lane == 0) {
+      sh[warp][0] = sum;
+      sh[warp][3] = part;
     }
-  }
-  if (null) {
-    const double c = sum / F.hsum;
-#pragma unroll
-    for (int k = 0; k < C; ++k)
-      if (s0 + k < n) y[k] -= __ldg(F.h + s0 + k) * c;
   }
   // elimination: y_k = -(w_k + e_{k-1} y_{k-1}) m_k
   double A = 1.0, B = 0.0;
@@ -154,41 +150,44 @@ __device__ __forceinline__ void tri_solve(const FdmD &F, int b, int wr, const Tr
     y[k] = fma(-e[k] * m[k], yi, y[k]);
     yi = y[k];
   }
-  // cyclic systems: zh = y - (y_0 + cr y_{n-1}) g; null mode: the h-weighted
-  // mean removed.  Both need one value of the whole row.
-  double part = 0.0;
-  const bool cyc = row && F.g && !null;
-  if (cyc) {
-    const double cr = __ldg(F.cr + b);
+  if (null) {
+    if constexpr (W > 1) {  // written before the scans' barriers
+      sum = part = 0.0;
+#pragma unroll
+      for (int v = 0; v < W; ++v) {
+        sum += sh[w0 + v][0];
+        part += sh[w0 + v][3];
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < C; ++k)
+      if (s0 + k < n) y[k] -= fma(sum, __ldg(F.ng + s0 + k), part);
+  }
+  // cyclic systems: zh = y - (y_0 + cr y_{n-1}) g
+  if (F.g) {
+    double first = __shfl_sync(ALL, y[0], 0), last = 0.0;
 #pragma unroll
     for (int k = 0; k < C; ++k) {
-      if (s0 + k == 0) part += y[k];
-      if (s0 + k == n - 1) part += cr * y[k];
+      const double v = __shfl_sync(ALL, y[k], ((n - 1) / C) & 31);
+      if (k == (n - 1) % C) last = v;
     }
-  } else if (null) {
-#pragma unroll
-    for (int k = 0; k < C; ++k)
-      if (s0 + k < n) part += __ldg(F.h + s0 + k) * y[k];
-  }
-  if (cyc || null) part = tri_warp_sum(part);
-  if constexpr (W > 1) {
-    if (lane == 0) sh[warp][3] = part;
-    __syncthreads();
-    if (cyc || null) {
-      part = 0.0;
-#pragma unroll
-      for (int v = 0; v < W; ++v) part += sh[w0 + v][3];
+    if constexpr (W > 1) {
+      __syncthreads();  // the null row's sums were read
+      if (lane == 0) {
+        sh[warp][0] = first;
+        sh[warp][3] = last;
+      }
+      __syncthreads();
+      first = sh[w0][0];
+      last = sh[w0 + (n - 1) / (32 * C)][3];
     }
-  }
-  if (cyc) {
-    const double *__restrict__ g = F.g + (size_t)b * n;
+    if (row && !null) {
+      const double *__restrict__ g = F.g + (size_t)b * n;
+      const double c = first + __ldg(F.cr + b) * last;
 #pragma unroll
-    for (int k = 0; k < C; ++k)
-      if (s0 + k < n) y[k] -= part * __ldg(g + s0 + k);
-  } else if (null) {
-    const double c = part / F.hsum;
-#pragma unroll
-    for (int k = 0; k < C; ++k) y[k] -= c;
+      for (int k = 0; k < C; ++k)
+        if (s0 + k < n) y[k] -= c * __ldg(g + s0 + k);
+    }
   }
 }
 

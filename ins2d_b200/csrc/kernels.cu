@@ -140,6 +140,8 @@ template <typename TO>
 __global__ void __launch_bounds__(256) k_project32(const __grid_constant__ DevOps P, const double *Vn,
                                                   const float *__restrict__ T, double a, const double *__restrict__ dp,
                                                   double dt, double c, TO *Vo) {
+  pdl_wait();
+  pdl_trigger();
   const int i = blockIdx.x * BX + threadIdx.x;
   const int j0 = blockIdx.y * (BY * kProjRows) + threadIdx.y;
 #pragma unroll
@@ -329,7 +331,7 @@ void launch_project(const DevOps &P, const double *Wt, const double *dp, double 
                     cudaStream_t s) {
   const int nx = P.Nux > P.Nvx ? P.Nux : P.Nvx, ny = P.Nuy > P.Nvy ? P.Nuy : P.Nvy;
   const dim3 g((nx + BX - 1) / BX, (ny + BY * kProjRows - 1) / (BY * kProjRows));
-  launch_k(k_project, g, dim3(BX, BY), 0, s, P, Wt, dp, dt, c, V_out);
+  launch_kp(P.pdl, k_project, g, dim3(BX, BY), 0, s, P, Wt, dp, dt, c, V_out);
 }
 
 template <typename TO>
@@ -337,7 +339,7 @@ void launch_project32_t(const DevOps &P, const double *Vn, const float *T, doubl
                         double c, TO *V_out, cudaStream_t s) {
   const int nx = P.Nux > P.Nvx ? P.Nux : P.Nvx, ny = P.Nuy > P.Nvy ? P.Nuy : P.Nvy;
   const dim3 g((nx + BX - 1) / BX, (ny + BY * kProjRows - 1) / (BY * kProjRows));
-  k_project32<TO><<<g, dim3(BX, BY), 0, s>>>(P, Vn, T, a, dp, dt, c, V_out);
+  launch_kp(P.pdl, k_project32<TO>, g, dim3(BX, BY), 0, s, P, Vn, T, a, dp, dt, c, V_out);
 }
 void launch_project32(const DevOps &P, const double *Vn, const float *T, double a, const double *dp, double dt,
                       double c, float *V_out, cudaStream_t s) {
@@ -352,7 +354,7 @@ void launch_project_cached(const DevOps &P, const double *Vn, const double *kV0,
                            const double *dp, double dt, double c, double *V_out, cudaStream_t s) {
   const int nx = P.Nux > P.Nvx ? P.Nux : P.Nvx, ny = P.Nuy > P.Nvy ? P.Nuy : P.Nvy;
   const dim3 g((nx + BX - 1) / BX, (ny + BY * kProjRows - 1) / (BY * kProjRows));
-  launch_k(k_project_cached, g, dim3(BX, BY), 0, s, P, Vn, kV0, aii, inv_dt, dp, dt, c, V_out);
+  launch_kp(P.pdl, k_project_cached, g, dim3(BX, BY), 0, s, P, Vn, kV0, aii, inv_dt, dp, dt, c, V_out);
 }
 
 void launch_correct(const DevOps &P, const double *V_in, const double *dp, double *V_out, cudaStream_t s) {

@@ -14,18 +14,21 @@ constexpr int kMaxStages = 8;
 constexpr int kStatusNonFinite = 4, kStatusTimeout = 5;  // INS2D_ENONFINITE, INS2D_ETIMEOUT
 
 // Programmatic dependent launch of the explicit step's kernels (the stage and
-// residual walkers, the FFT passes, the projections): off unless INS2D_PDL=1
-// in the environment of the process.  Measured on B200 in the step graphs it
-// did not pay: 0.863 against 0.859 ms per RK4 step at 2048^2, 0.164 against
-// 0.140 ms at 512^2.
+// residual walkers, the FFT passes, the projections): on for grids whose
+// solves are one cluster (DevOps::pdl; their kernels are short and leave most
+// SMs idle, so a kernel's start-up hides behind its predecessor: RK44 step of
+// the 64^2 cavity 0.104 -> 0.096 ms); else off unless INS2D_PDL=1 in the environment of the process.  Measured on B200
+// in the step graphs of larger grids it did not pay: 0.863 against 0.859 ms
+// per RK4 step at 2048^2, 0.164 against 0.140 ms at 512^2.
 bool pdl_enabled();
 
-// k<<<g, b, sm, s>>>(args...) for a kernel that begins with pdl_wait(); with
-// programmatic serialisation allowed when pdl_enabled().  Launch errors are
-// left for cudaGetLastError, as with <<< >>>.
+// k<<<g, b, sm, s>>>(args...) for a kernel that calls pdl_wait() before it
+// reads what earlier kernels wrote; with programmatic serialisation allowed
+// when pdl or pdl_enabled().  Launch errors are left for cudaGetLastError, as
+// with <<< >>>.
 template <typename... KArgs, typename... Args>
-inline void launch_k(void (*k)(KArgs...), dim3 g, dim3 b, size_t sm, cudaStream_t s, Args &&...args) {
-  if (!pdl_enabled()) {
+inline void launch_kp(bool pdl, void (*k)(KArgs...), dim3 g, dim3 b, size_t sm, cudaStream_t s, Args &&...args) {
+  if (!pdl && !pdl_enabled()) {
     k<<<g, b, sm, s>>>(static_cast<KArgs>(args)...);
     return;
   }
@@ -40,6 +43,11 @@ inline void launch_k(void (*k)(KArgs...), dim3 g, dim3 b, size_t sm, cudaStream_
   cfg.attrs = at;
   cfg.numAttrs = 1;
   cudaLaunchKernelEx(&cfg, k, static_cast<KArgs>(args)...);
+}
+
+template <typename... KArgs, typename... Args>
+inline void launch_k(void (*k)(KArgs...), dim3 g, dim3 b, size_t sm, cudaStream_t s, Args &&...args) {
+  launch_kp(false, k, g, b, sm, s, static_cast<Args &&>(args)...);
 }
 
 // Makes `dev` the calling thread's current device for the lifetime of the
@@ -219,10 +227,10 @@ struct FdmD {
   int nx = 0, ny = 0;
   int nm = 0, n = 0, xmodes = 0;  // modes, unknowns per system, modes along x
   const double *Q = nullptr;      // nm x nm row-major (Q[i*nm + b])
-  const double *piv = nullptr, *e = nullptr, *h = nullptr;  // nm x n, n, n
+  const double *piv = nullptr, *e = nullptr;                // nm x n, n
   const double *g = nullptr, *cr = nullptr;                 // cyclic systems: nm x n, nm
   int null_mode = -1;
-  double hsum = 0.0;
+  const double *ng = nullptr, *nmu = nullptr;               // its corrections: n
   const double *r = nullptr;  // ensembles: the member's CG residual
   double *t = nullptr;        // nm x n: transformed residual, then the systems' solutions
   double *z = nullptr;        // the preconditioned residual
@@ -341,8 +349,8 @@ struct SolveSrc {
 };
 bool pcg_use_cluster(const FdmD &F);
 cudaError_t pcg_cluster_prepare();  // opts the kernels in to their shared memory on the current device
-void pcg_solve_cluster(const DevOps &P, const FdmD &F, const PcgWork &W, const SolveSrc &src, double *dp, double tol,
-                       long long maxit, bool accumulate, SolveAccum *acc, cudaStream_t s);
+cudaError_t pcg_solve_cluster(const DevOps &P, const FdmD &F, const PcgWork &W, const SolveSrc &src, double *dp,
+                              double tol, long long maxit, bool accumulate, SolveAccum *acc, cudaStream_t s);
 
 struct EnsMemberD {
   DevOps P;

@@ -11,9 +11,15 @@
 // systems run along s, so the blocks exchange the transformed residual and
 // the solution through distributed shared memory (block c solves its slice of
 // the modes b, a warp per system).  A pass takes five cluster barriers.
-// Measured on B200 against one thread block working from L1/L2 and a separate
-// divergence launch: RK44 step of the 64^2 cavity (four solves) 0.228 ->
-// 0.117 ms.
+// Beside the barriers (about 1000 cycles each) a launch pays for the first
+// touch of its parameters, tables and instructions; what depends on the
+// context alone is loaded before the wait for the previous kernel
+// (programmatic dependent launch, DevOps::pdl).  Measured on B200, RK44 step
+// of the 64^2 cavity (four solves): one thread block working from L1/L2 and a
+// separate divergence launch 0.228 ms; eight blocks of 256 threads with
+// scattered 8-byte exchanges 0.117 ms; 512 threads, 16-byte exchanges and
+// staged operator rows 0.104 ms (two or four blocks: 0.131, 0.112 ms); with
+// programmatic launches 0.096 ms.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -30,36 +36,41 @@ namespace ins2d {
 
 namespace {
 
-constexpr int kC = 8;             // blocks of the cluster
-constexpr int kThreads = 256;
+constexpr int kThreads = 512;
 constexpr int kWarps = kThreads / 32;
-constexpr int kTriC = kFdmClusterMaxN / 32;  // unknowns per lane of a system
-constexpr int kSmemMax = 226 * 1024;  // dynamic; the reductions' slots are static
+constexpr int kN = kFdmClusterMaxN;
+constexpr int kTriC = kN / 32;        // unknowns per lane of a system
+constexpr int kSmemMax = 197 * 1024;  // dynamic; 29.5 KB of tables are static
+constexpr int kC = 8;                // blocks of the cluster
 
 // sizes of one solve
 struct Geo {
   int nm, n;      // modes, unknowns per system
-  int ns, nb;     // systems' unknowns and modes per block (the last blocks may hold fewer or none)
+  int ns, nb;     // systems' unknowns (even) and modes per block (the last blocks may hold fewer or none)
   int ld;         // pitch of the cell arrays: ns rounded up to 8, plus 4 (4 or 12 mod 16: conflict-free fragments)
   int ldt;        // pitch of the rows of systems
   int mp;         // modes rounded up to 8
   int qp;         // pitch of the basis (4 mod 16), 0: not in shared memory
+  int lg;         // cells of a slice are numbered with a power-of-two pitch 2^lg of the fast index
 };
 __host__ __device__ inline size_t cells(const Geo &g) { return (size_t)g.mp * g.ld; }
 __host__ __device__ inline size_t smem_doubles(const Geo &g) {
-  return 6 * cells(g) + (size_t)g.nb * g.ldt + 2 * (size_t)g.mp + (size_t)g.mp * g.qp;
+  return 6 * cells(g) + (size_t)g.nb * g.ldt + 4 * (size_t)g.mp + (size_t)g.mp * g.qp;
 }
 Geo make_geo(const FdmD &F) {
   Geo g;
   g.nm = F.nm;
   g.n = F.n;
-  g.ns = (F.n + kC - 1) / kC;
+  g.ns = 2 * ((F.n + 2 * kC - 1) / (2 * kC));
   g.nb = (F.nm + kC - 1) / kC;
   g.ld = ((g.ns + 7) / 8) * 8 + 4;
-  g.ldt = F.n + 1;
+  g.ldt = (F.n + 3) & ~1;
   g.mp = ((F.nm + 7) / 8) * 8;
   g.qp = ((F.nm + 15) / 16) * 16 + 4;
   if (smem_doubles(g) * sizeof(double) > kSmemMax) g.qp = 0;
+  const int fast = F.xmodes ? F.nm : g.ns;
+  g.lg = 0;
+  while ((1 << g.lg) < fast) ++g.lg;
   return g;
 }
 
@@ -71,15 +82,20 @@ __device__ __forceinline__ void mma884(double &d0, double &d1, double a, double 
 
 // C = op(Q) B on 8 x 8 fragments taken by the block's warps in turn; B: cell
 // array (rows k, pitch ld), zero-padded rows and columns; TRANS: op(Q)(i, k) =
-// Q(k, i), else Q(i, k); epi(row, column, value) for every fragment element.
-// Two accumulator pairs halve the chain of dependent MMAs.
+// Q(k, i), else Q(i, k); epi(row, column, value, next column's value), columns
+// even.  Two accumulator pairs halve the chain of dependent MMAs.
 template <bool TRANS, class QF, class Epi>
 __device__ __forceinline__ void product(const Geo &g, const QF &q, const double *B, Epi epi) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int gr = lane >> 2, t = lane & 3;
-  const int tn = g.ld >> 3, tiles = (g.mp >> 3) * tn;  // ld = 8 tn + 4
+  const int tm = g.mp >> 3, tiles = tm * (g.ld >> 3);  // ld = 8 x column tiles + 4
   for (int f = warp; f < tiles; f += kWarps) {
-    const int bm = (f / tn) * 8, bn = (f % tn) * 8;
+    int bn = 0, bm = f;
+    while (bm >= tm) {
+      bm -= tm;
+      bn += 8;
+    }
+    bm *= 8;
     double c0 = 0.0, c1 = 0.0, d0 = 0.0, d1 = 0.0;
     const double *b = B + (size_t)t * g.ld + bn + gr;
 #pragma unroll 4
@@ -89,34 +105,42 @@ __device__ __forceinline__ void product(const Geo &g, const QF &q, const double 
       mma884(c0, c1, a0, b[(size_t)k * g.ld]);
       mma884(d0, d1, a1, b[(size_t)(k + 4) * g.ld]);
     }
-    epi(bm + gr, bn + 2 * t, c0 + d0);
-    epi(bm + gr, bn + 2 * t + 1, c1 + d1);
+    epi(bm + gr, bn + 2 * t, c0 + d0, c1 + d1);
   }
 }
 
-// Sum / max / min of NQ values over the cluster: every block's partial to
-// every block, a cluster barrier, and the same ordered combination in every
-// thread.  slot alternates between two buffers.
+__device__ __forceinline__ double combine(double a, double b, int op) {
+  return op == R_SUM ? a + b : (op == R_MAX ? (a > b ? a : b) : (a < b ? a : b));
+}
+// Sum / max / min of NQ values over the cluster: the block's value (warp
+// shuffles, then warp 0), one packet to every block, a cluster barrier, and
+// the same ordered combination in every thread.  slot alternates between two
+// buffers.  Remote stores are few and wide throughout this kernel: an SM
+// sends one packet in several cycles (a packet per warp instead of per block
+// made the four-value reduction 4300 cycles, against about 1700).
 template <int NQ>
 __device__ __forceinline__ void cluster_reduce(cg::cluster_group &cl, double (&v)[NQ], const int (&ops)[NQ],
-                                               double (*warp_part)[4], double (*part)[kC][4], int &slot) {
+                                               double (*warp_part)[kWarps], double (*part)[kC][4], int &slot) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-  for (int q = 0; q < NQ; ++q)
+  for (int off = 16; off > 0; off >>= 1)
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) v[q] = red_combine(v[q], __shfl_xor_sync(0xffffffffu, v[q], off), ops[q]);
+    for (int q = 0; q < NQ; ++q) v[q] = combine(v[q], __shfl_xor_sync(0xffffffffu, v[q], off), ops[q]);
   if (lane == 0)
 #pragma unroll
-    for (int q = 0; q < NQ; ++q) warp_part[warp][q] = v[q];
+    for (int q = 0; q < NQ; ++q) warp_part[q][warp] = v[q];
   __syncthreads();
-  if (threadIdx.x < kC) {
-    double *dst = cl.map_shared_rank(&part[slot][cl.block_rank()][0], threadIdx.x);
+  if (warp == 0) {
 #pragma unroll
-    for (int q = 0; q < NQ; ++q) {
-      double a = warp_part[0][q];
+    for (int q = 0; q < NQ; ++q) v[q] = warp_part[q][lane & (kWarps - 1)];
 #pragma unroll
-      for (int w = 1; w < kWarps; ++w) a = red_combine(a, warp_part[w][q], ops[q]);
-      dst[q] = a;
+    for (int off = kWarps / 2; off > 0; off >>= 1)
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) v[q] = combine(v[q], __shfl_xor_sync(0xffffffffu, v[q], off), ops[q]);
+    if (lane < kC) {
+      double2 *dst = reinterpret_cast<double2 *>(cl.map_shared_rank(&part[slot][cl.block_rank()][0], lane));
+      dst[0] = make_double2(v[0], NQ > 1 ? v[NQ > 1 ? 1 : 0] : 0.0);
+      if (NQ > 2) dst[1] = make_double2(v[NQ > 2 ? 2 : 0], v[NQ > 3 ? 3 : 0]);
     }
   }
   cl.sync();
@@ -124,81 +148,151 @@ __device__ __forceinline__ void cluster_reduce(cg::cluster_group &cl, double (&v
   for (int q = 0; q < NQ; ++q) {
     double a = part[slot][0][q];
 #pragma unroll
-    for (int c = 1; c < kC; ++c) a = red_combine(a, part[slot][c][q], ops[q]);
+    for (int c = 1; c < kC; ++c) a = combine(a, part[slot][c][q], ops[q]);
     v[q] = a;
   }
   slot ^= 1;
 }
+static_assert(kWarps == 16, "two lanes per warp partial");
+
+// one direction's rows of the operators in shared memory: the factor of A, the
+// divergence (W is read at their columns), boundary coefficients and values
+struct DirRows {
+  int ac[kT][kN], mc[kT][kN];
+  double aw[kT][kN], mw[kT][kN], h[kN], b1[kN], b2[kN], v1[kN], v2[kN];
+};
+__device__ __forceinline__ void load_dir(DirRows &D, int k, const Tab &A, const Tab &M, const double *h, int r,
+                                         bool div, const double *v1, const double *v2) {
+  D.h[k] = __ldg(h + r);
+#pragma unroll
+  for (int q = 0; q < kT; ++q) {
+    const double w = __ldg(A.w + kT * r + q);
+    const int c = __ldg(A.c + kT * r + q);
+    D.aw[q][k] = w;
+    D.ac[q][k] = w != 0.0 ? c : r;
+  }
+  if (!div) return;
+#pragma unroll
+  for (int q = 0; q < kT; ++q) {
+    D.mw[q][k] = __ldg(M.w + kT * r + q);
+    D.mc[q][k] = __ldg(M.c + kT * r + q);
+  }
+  D.b1[k] = __ldg(M.b1 + r);
+  D.b2[k] = __ldg(M.b2 + r);
+  D.v1[k] = __ldg(v1 + r);
+  D.v2[k] = __ldg(v2 + r);
+}
 
 // QS: the basis in shared memory
 template <bool QS>
-__global__ void __cluster_dims__(kC, 1, 1) __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kThreads, 1)
     k_pcg_cluster(const __grid_constant__ DevOps P, const __grid_constant__ FdmD F, const PcgWork W, const Geo g,
                   const __grid_constant__ SolveSrc src, double *__restrict__ dp, double tol2, long long maxit,
                   int accumulate, SolveAccum *acc) {
   extern __shared__ __align__(16) double sm[];
-  __shared__ double warp_part[kWarps][4];
-  __shared__ double part[2][kC][4];
+  __shared__ double warp_part[4][kWarps];
+  __shared__ __align__(16) double part2[2][kC][4], part4[2][kC][4];
+  __shared__ DirRows dm, ds;  // along the modes' and the systems' direction
   cg::cluster_group cl = cg::this_cluster();
+  cl.barrier_arrive();  // every block runs before any other writes to its shared memory (waited for below)
   const int c = (int)cl.block_rank(), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nm = g.nm, n = g.n, ld = g.ld;
   const int s0 = c * g.ns, s1 = min(s0 + g.ns, n), nl = max(s1 - s0, 0);  // this block's slice
   const size_t nc = cells(g);
   double *r = sm, *p = r + nc, *x = p + nc, *q = x + nc, *z = q + nc, *zh = z + nc;
-  double *rows = zh + nc, *pl = rows + (size_t)g.nb * g.ldt, *pr = pl + g.mp, *Qs = pr + g.mp;
-  int slot = 0;
-  cl.sync();  // every block runs before any other writes to its shared memory
-  // zero padding of the products' right operands
-  for (size_t k = tid; k < nc; k += kThreads) {
-    r[k] = 0.0;
-    zh[k] = 0.0;
+  // halo columns of p on the left and right, of z as the neighbours send them
+  double *rows = zh + nc, *ph = rows + (size_t)g.nb * g.ldt, *zhalo = ph + 2 * g.mp, *Qs = zhalo + 2 * g.mp;
+  int slot2 = 0, slot4 = 0;
+  if (QS) {  // asynchronous: complete before the first product
+    for (int i = warp; i < g.mp; i += kWarps)
+      for (int b = lane; b < g.mp; b += 32) {
+        const bool in = i < nm && b < nm;
+        const unsigned d = (unsigned)__cvta_generic_to_shared(Qs + (size_t)i * g.qp + b);
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d),
+                     "l"(F.Q + (in ? (size_t)i * nm + b : 0)), "r"(in ? 8 : 0)
+                     : "memory");
+      }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
   }
-  if (QS)
-    for (int k = tid; k < g.mp * g.mp; k += kThreads) {
-      const int i = k / g.mp, b = k - i * g.mp;
-      Qs[(size_t)i * g.qp + b] = (i < nm && b < nm) ? __ldg(F.Q + (size_t)i * nm + b) : 0.0;
-    }
   auto basis = [&](int i, int b) -> double {
     if constexpr (QS)
       return Qs[(size_t)i * g.qp + b];
     else
       return (i < nm && b < nm) ? __ldg(F.Q + (size_t)i * nm + b) : 0.0;
   };
-  // this warp's systems: rows warp, warp + 8 of the block's slice of modes
-  constexpr int RW = (kFdmClusterMaxN / kC + kWarps - 1) / kWarps;
-  TriTab<kTriC> tab[RW];
-#pragma unroll
-  for (int u = 0; u < RW; ++u) {
-    const int lb = warp + u * kWarps, b = c * g.nb + lb;
-    tri_tables<kTriC>(F, lb < g.nb ? b : F.nm, lane * kTriC, tab[u]);
+  // the operators' rows
+  const bool xm = F.xmodes;
+  const bool div = src.mode != 0 && src.beta == 0.0;
+  if (tid < nm)
+    load_dir(dm, tid, xm ? P.TX : P.TY, xm ? P.MX : P.MY, xm ? P.hx : P.hy, tid, div, xm ? P.bc.vLo_i : P.bc.uLe_i,
+             xm ? P.bc.vUp_i : P.bc.uRi_i);
+  else if (tid >= kThreads / 2 && tid - kThreads / 2 < nl)
+    load_dir(ds, tid - kThreads / 2, xm ? P.TY : P.TX, xm ? P.MY : P.MX, xm ? P.hy : P.hx, s0 + tid - kThreads / 2,
+             div, xm ? P.bc.uLe_i : P.bc.vLo_i, xm ? P.bc.uRi_i : P.bc.vUp_i);
+  // zero padding of the products' right operands
+  for (int k = tid; k < (int)nc; k += kThreads) {
+    r[k] = 0.0;
+    zh[k] = 0.0;
   }
   __syncthreads();
-  // cell l of the slice: (m, s), x fastest in memory
+  // cell l of the slice: (m, sl), the index of x fastest; false: padding
+  const int nslots = (xm ? nl : nm) << g.lg;
   auto cell = [&](int l, int &m, int &sl) {
-    if (F.xmodes) {
-      sl = l / nm;
-      m = l - sl * nm;
-    } else {
-      m = l / nl;
-      sl = l - m * nl;
-    }
+    const int a = l & ((1 << g.lg) - 1), b = l >> g.lg;
+    m = xm ? a : b;
+    sl = xm ? b : a;
+    return m < nm && sl < nl;
   };
-  const int ncell = nm * nl;
+  // f = (M W + alpha yM) gamma from the rows above
+  auto div_at = [&](const auto &Wf, int m, int sl, int i, int j) {
+    const DirRows &dx = xm ? dm : ds, &dy = xm ? ds : dm;
+    const int a = xm ? m : sl, b = xm ? sl : m;
+    double u = 0.0, v = 0.0;
+#pragma unroll
+    for (int k = 0; k < kT; ++k) {
+      u += dx.mw[k][a] * Wf((long long)j * P.Nux + dx.mc[k][a]);
+      v += dy.mw[k][b] * Wf(P.Nu + (long long)dy.mc[k][b] * P.Nvx + i);
+    }
+    double d = dy.h[b] * u + dx.h[a] * v;
+    if (src.alpha != 0.0)
+      d += src.alpha * (dy.h[b] * (dx.b1[a] * dy.v1[b] + dx.b2[a] * dy.v2[b]) +
+                        dx.h[a] * (dy.b1[b] * dx.v1[a] + dy.b2[b] * dx.v2[a]));
+    return d * src.gamma;
+  };
+  // this warp's first system (tables of the others are read when they are solved)
+  const int b0 = c * g.nb, b1 = min(b0 + g.nb, nm);
+  TriTab<kTriC> tab;
+  tri_tables<kTriC>(F, b0 + warp < b1 ? b0 + warp : nm, lane * kTriC, tab);
+  // everything above depends on the context alone; the right-hand side on the
+  // kernels before this one
+  pdl_wait();
+  pdl_trigger();
   // right-hand side (cg.F:207-229 with x_in = 0)
   double a2[2] = {0.0, 0.0};
   const int op2[2] = {R_SUM, R_MAX};
-  for (int l = tid; l < ncell; l += kThreads) {
+#pragma unroll 2
+  for (int l = tid; l < nslots; l += kThreads) {
     int m, sl;
-    cell(l, m, sl);
-    const int i = F.xmodes ? m : s0 + sl, j = F.xmodes ? s0 + sl : m;
-    const double f = src.mode == 0   ? src.f[(size_t)j * P.Npx + i]
-                     : src.mode == 1 ? div_cell_f(P, WPlain{src.f}, src.alpha, src.beta, src.gamma, i, j)
-                                     : div_cell_f(P, src.ws, src.alpha, src.beta, src.gamma, i, j);
+    if (!cell(l, m, sl)) continue;
+    const int s = s0 + sl, i = xm ? m : s, j = xm ? s : m;
+    double f;
+    if (src.mode == 0)
+      f = src.f[(size_t)j * P.Npx + i];
+    else if (src.mode == 1)
+      f = div ? div_at(WPlain{src.f}, m, sl, i, j)
+              : div_cell_f(P, WPlain{src.f}, src.alpha, src.beta, src.gamma, i, j);
+    else
+      f = div ? div_at(src.ws, m, sl, i, j) : div_cell_f(P, src.ws, src.alpha, src.beta, src.gamma, i, j);
     r[m * ld + sl] = f;
     a2[0] += f * f;
-    a2[1] = fmax(a2[1], fabs(f));
+    a2[1] = fabs(f) > a2[1] ? fabs(f) : a2[1];
   }
-  cluster_reduce<2>(cl, a2, op2, warp_part, part, slot);
+  // the halo columns (wrapped ones serve cyclic rows only) and the blocks whose
+  // left / right halo column is this block's last / first one
+  const int sL = s0 > 0 ? s0 - 1 : n - 1, sR = s1 < n ? s1 : 0;
+  const int bl = sR / g.ns, br = sL / g.ns;
+  cl.barrier_wait();
+  cluster_reduce<2>(cl, a2, op2, warp_part, part2, slot2);
   const double rr0 = a2[0];
   double rz = 0.0, rr = 0.0, maxx = 0.0, minx = 0.0, maxres = 0.0;
   long long it = 0;
@@ -208,47 +302,66 @@ __global__ void __cluster_dims__(kC, 1, 1) __launch_bounds__(kThreads, 1)
     status = INS2D_ENONFINITE;
     done = true;
   }
-  const Tab &Tm = F.xmodes ? P.TX : P.TY, &Ts = F.xmodes ? P.TY : P.TX;
-  const double *hm = F.xmodes ? P.hx : P.hy, *hs = F.xmodes ? P.hy : P.hx;
   const int op1[1] = {R_SUM};
+  if (QS) {
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();
+  }
   // the loop's exits are taken by all blocks alike: every condition comes
   // from a cluster-wide reduction
   while (!done) {
     // w = Q' r, each row to the block that solves it
-    product<true>(g, basis, r, [&](int b, int sl, double v) {
+    product<true>(g, basis, r, [&](int b, int sl, double v0, double v1) {
       if (b < nm && sl < nl) {
         const int o = b / g.nb;
-        cl.map_shared_rank(rows, o)[(size_t)(b - o * g.nb) * g.ldt + s0 + sl] = v;
+        double *d = cl.map_shared_rank(rows, o) + (size_t)(b - o * g.nb) * g.ldt + s0 + sl;
+        *reinterpret_cast<double2 *>(d) = make_double2(v0, v1);  // rows hold n + 1 values or more
       }
     });
     cl.sync();
-#pragma unroll
-    for (int u = 0; u < RW; ++u) {
-      const int lb = warp + u * kWarps, b = lb < g.nb ? c * g.nb + lb : F.nm;
-      if (b >= nm) continue;
-      const double *w = rows + (size_t)lb * g.ldt;
+    for (int b = b0 + warp; b < b1; b += kWarps) {
+      double *w = rows + (size_t)(b - b0) * g.ldt;
       double y[kTriC];
 #pragma unroll
       for (int k = 0; k < kTriC; ++k) y[k] = lane * kTriC + k < n ? w[lane * kTriC + k] : 0.0;
-      tri_solve<1, kTriC>(F, b, 0, tab[u], y, nullptr);
+      if (b != b0 + warp) {
+        TriTab<kTriC> t2;
+        tri_tables<kTriC>(F, b, lane * kTriC, t2);
+        tri_solve<1, kTriC>(F, b, 0, t2, y, nullptr);
+      } else {
+        tri_solve<1, kTriC>(F, b, 0, tab, y, nullptr);
+      }
+      // back through the row, so that consecutive lanes send consecutive values
 #pragma unroll
-      for (int k = 0; k < kTriC; ++k) {
-        const int s = lane * kTriC + k;
+      for (int k = 0; k < kTriC; ++k)
+        if (lane * kTriC + k < n) w[lane * kTriC + k] = y[k];
+      __syncwarp();
+#pragma unroll
+      for (int k = 0; k < kN / 64; ++k) {
+        const int s = 2 * (lane + 32 * k);
         if (s < n) {
           const int o = s / g.ns;
-          cl.map_shared_rank(zh, o)[(size_t)b * ld + s - o * g.ns] = y[k];
+          double *d = cl.map_shared_rank(zh, o) + (size_t)b * ld + s - o * g.ns;
+          *reinterpret_cast<double2 *>(d) =
+              make_double2(w[s], s + 1 < n ? w[s + 1] : 0.0);  // a padding column stays zero
         }
       }
     }
     cl.sync();
     double a1[1] = {0.0};
-    product<false>(g, basis, zh, [&](int m, int sl, double v) {
-      if (m < nm && sl < nl) {
-        z[m * ld + sl] = v;
-        a1[0] += r[m * ld + sl] * v;
+    product<false>(g, basis, zh, [&](int m, int sl, double v0, double v1) {
+      if (m >= nm || sl >= nl) return;
+      const int k = m * ld + sl;
+      z[k] = v0;
+      a1[0] += r[k] * v0;
+      if (sl == 0) cl.map_shared_rank(zhalo, br)[g.mp + m] = v0;
+      if (sl + 1 < nl) {
+        z[k + 1] = v1;
+        a1[0] += r[k + 1] * v1;
       }
+      if (sl + 2 >= nl) cl.map_shared_rank(zhalo, bl)[m] = sl + 1 < nl ? v1 : v0;
     });
-    cluster_reduce<1>(cl, a1, op1, warp_part, part, slot);
+    cluster_reduce<1>(cl, a1, op1, warp_part, part2, slot2);
     if (!isfinite(a1[0])) {
       status = INS2D_ENONFINITE;
       break;
@@ -256,45 +369,29 @@ __global__ void __cluster_dims__(kC, 1, 1) __launch_bounds__(kThreads, 1)
     const bool first = it == 0;
     const double beta = first ? 0.0 : a1[0] / rz;
     rz = a1[0];
-    // p = z + beta p, with the neighbouring columns' (kept in pl, pr)
-    for (int l = tid; l < ncell; l += kThreads) {
-      int m, sl;
-      cell(l, m, sl);
-      const int k = m * ld + sl;
-      p[k] = first ? z[k] : z[k] + beta * p[k];
-    }
-    const int sL = s0 > 0 ? s0 - 1 : n - 1, sR = s1 < n ? s1 : 0;  // wrapped: used by cyclic rows only
-    for (int l = tid; l < 2 * nm && nl > 0; l += kThreads) {
-      const int m = l % nm;
-      const bool left = l < nm;
-      const int s = left ? sL : sR, o = s / g.ns;
-      const double zv = cl.map_shared_rank(z, o)[(size_t)m * ld + s - o * g.ns];
-      double &h = (left ? pl : pr)[m];
-      h = first ? zv : zv + beta * h;
-    }
+    // p = z + beta p, with the neighbouring columns'
+    for (int k = tid; k < (int)nc; k += kThreads) p[k] = first ? z[k] : z[k] + beta * p[k];
+    for (int k = tid; k < 2 * g.mp; k += kThreads) ph[k] = first ? zhalo[k] : zhalo[k] + beta * ph[k];
     __syncthreads();
     // q = A p, p'q
     a1[0] = 0.0;
-    for (int l = tid; l < ncell; l += kThreads) {
+#pragma unroll 2
+    for (int l = tid; l < nslots; l += kThreads) {
       int m, sl;
-      cell(l, m, sl);
-      const int s = s0 + sl;
-      const int32_t *cm = Tm.c + kT * m, *cs = Ts.c + kT * s;
-      const double *wm = Tm.w + kT * m, *ws = Ts.w + kT * s;
+      if (!cell(l, m, sl)) continue;
       double tm = 0.0, ts = 0.0;
 #pragma unroll
       for (int k = 0; k < kT; ++k) {
-        tm += __ldg(wm + k) * p[__ldg(cm + k) * ld + sl];
-        const int sc = __ldg(cs + k);
-        const double wv = __ldg(ws + k);
-        const double pv = sc >= s0 && sc < s1 ? p[m * ld + sc - s0] : (sc == sL ? pl[m] : pr[m]);
-        if (wv != 0.0) ts += wv * pv;
+        tm += dm.aw[k][m] * p[dm.ac[k][m] * ld + sl];
+        const int sc = ds.ac[k][sl];
+        const double *at = sc >= s0 && sc < s1 ? p + m * ld + sc - s0 : (sc == sL ? ph + m : ph + g.mp + m);
+        ts += ds.aw[k][sl] * *at;
       }
-      const double aq = -(__ldg(hs + s) * tm + __ldg(hm + m) * ts);
+      const double aq = -(ds.h[sl] * tm + dm.h[m] * ts);
       q[m * ld + sl] = aq;
       a1[0] += p[m * ld + sl] * aq;
     }
-    cluster_reduce<1>(cl, a1, op1, warp_part, part, slot);
+    cluster_reduce<1>(cl, a1, op1, warp_part, part2, slot2);
     const double pq = a1[0];
     if (!isfinite(pq)) {
       status = INS2D_ENONFINITE;
@@ -307,20 +404,21 @@ __global__ void __cluster_dims__(kC, 1, 1) __launch_bounds__(kThreads, 1)
     const double alpha = rz / pq;
     double a4[4] = {0.0, -DBL_MAX, DBL_MAX, 0.0};
     const int op4[4] = {R_SUM, R_MAX, R_MIN, R_MAX};
-    for (int l = tid; l < ncell; l += kThreads) {
+#pragma unroll 2
+    for (int l = tid; l < nslots; l += kThreads) {
       int m, sl;
-      cell(l, m, sl);
+      if (!cell(l, m, sl)) continue;
       const int k = m * ld + sl;
       const double xv = (first ? 0.0 : x[k]) + alpha * p[k];
       const double rv = r[k] - alpha * q[k];
       x[k] = xv;
       r[k] = rv;
       a4[0] += rv * rv;
-      a4[1] = fmax(a4[1], xv);
-      a4[2] = fmin(a4[2], xv);
-      a4[3] = fmax(a4[3], fabs(rv));
+      a4[1] = combine(a4[1], xv, R_MAX);
+      a4[2] = combine(a4[2], xv, R_MIN);
+      a4[3] = combine(a4[3], fabs(rv), R_MAX);
     }
-    cluster_reduce<4>(cl, a4, op4, warp_part, part, slot);
+    cluster_reduce<4>(cl, a4, op4, warp_part, part4, slot4);
     ++it;
     rr = a4[0] / rr0;
     maxx = a4[1];
@@ -337,10 +435,11 @@ __global__ void __cluster_dims__(kC, 1, 1) __launch_bounds__(kThreads, 1)
     }
   }
   if (status == 0)
-    for (int l = tid; l < ncell; l += kThreads) {
+#pragma unroll 2
+    for (int l = tid; l < nslots; l += kThreads) {
       int m, sl;
-      cell(l, m, sl);
-      const int i = F.xmodes ? m : s0 + sl, j = F.xmodes ? s0 + sl : m;
+      if (!cell(l, m, sl)) continue;
+      const int s = s0 + sl, i = xm ? m : s, j = xm ? s : m;
       const size_t k = (size_t)j * P.Npx + i;
       const double xv = it ? x[m * ld + sl] : 0.0;
       W.x[k] = xv;  // the recorded solution (ins2d_record_pairs)
@@ -363,26 +462,46 @@ __global__ void __cluster_dims__(kC, 1, 1) __launch_bounds__(kThreads, 1)
   cl.sync();  // no block leaves while another may still write to its shared memory
 }
 
+template <bool QS>
+cudaError_t launch_cluster(const DevOps &P, const FdmD &F, const PcgWork &W, const Geo &g, const SolveSrc &src,
+                           double *dp, double tol2, long long maxit, int accumulate, SolveAccum *acc, cudaStream_t s) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(kC);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem_doubles(g) * sizeof(double);
+  cfg.stream = s;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = kC;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = P.pdl ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, k_pcg_cluster<QS>, P, F, W, g, src, dp, tol2, maxit, accumulate, acc);
+}
+
 }  // namespace
 
 bool pcg_use_cluster(const FdmD &F) { return !F.spectral && std::max(F.nm, F.n) <= kFdmClusterMaxN; }
 
 cudaError_t pcg_cluster_prepare() {
-  const cudaError_t e = cudaFuncSetAttribute((const void *)k_pcg_cluster<true>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
-  if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute((const void *)k_pcg_cluster<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              kSmemMax);
+  cudaError_t first = cudaSuccess;
+  auto opt_in = [&](const void *k) {
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
+    if (first == cudaSuccess) first = e;
+  };
+  opt_in((const void *)k_pcg_cluster<true>);
+  opt_in((const void *)k_pcg_cluster<false>);
+  return first;
 }
 
-void pcg_solve_cluster(const DevOps &P, const FdmD &F, const PcgWork &W, const SolveSrc &src, double *dp, double tol,
-                       long long maxit, bool accumulate, SolveAccum *acc, cudaStream_t s) {
+cudaError_t pcg_solve_cluster(const DevOps &P, const FdmD &F, const PcgWork &W, const SolveSrc &src, double *dp,
+                              double tol, long long maxit, bool accumulate, SolveAccum *acc, cudaStream_t s) {
   const Geo g = make_geo(F);
-  const size_t bytes = smem_doubles(g) * sizeof(double);
-  if (g.qp)
-    k_pcg_cluster<true><<<kC, kThreads, bytes, s>>>(P, F, W, g, src, dp, tol * tol, maxit, accumulate ? 1 : 0, acc);
-  else
-    k_pcg_cluster<false><<<kC, kThreads, bytes, s>>>(P, F, W, g, src, dp, tol * tol, maxit, accumulate ? 1 : 0, acc);
+  const int ac = accumulate ? 1 : 0;
+  return g.qp ? launch_cluster<true>(P, F, W, g, src, dp, tol * tol, maxit, ac, acc, s)
+              : launch_cluster<false>(P, F, W, g, src, dp, tol * tol, maxit, ac, acc, s);
 }
 
 }  // namespace ins2d

@@ -919,12 +919,16 @@ __device__ __forceinline__ void tile_generic(const DevOps &P, const TV *__restri
 template <typename S, typename TV>
 __global__ void __launch_bounds__(WX * 2, INS2D_WALK_MINB) k_walk_fast(const __grid_constant__ DevOps P, const TV *__restrict__ V,
                                                       const __grid_constant__ Epi e, int rows) {
+  pdl_wait();
+  pdl_trigger();
   tile_fast<S, TV>(P, V, e, P.fbx0 + blockIdx.x, P.fby0 + blockIdx.y, blockIdx.z, rows);
 }
 
 template <typename S, typename TV>
 __global__ void __launch_bounds__(WX * 2) k_walk(const __grid_constant__ DevOps P, const TV *__restrict__ V,
                                                  const __grid_constant__ Epi e, int rows) {
+  pdl_wait();
+  pdl_trigger();
   if ((int)blockIdx.x >= P.fbx0 && (int)blockIdx.x < P.fbx1 && (int)blockIdx.y >= P.fby0 &&
       (int)blockIdx.y < P.fby1)
     return;  // interior tile: handled by k_walk_fast / k_walk_tile
@@ -999,14 +1003,14 @@ void launch_tile(const DevOps &P, const TV *V, const Epi &e, cudaStream_t s) {
   const dim3 gf(P.fbx1 - P.fbx0, P.fby1 - P.fby0), tb(WX, kTileThreads / WX);
   if constexpr (MODE == 0 || MODE == 2) {
     switch (e.nprev) {
-      case 0: launch_k(k_walk_tile<S, MODE, TV, 0>, gf, tb, 0, s, P, V, e); break;
-      case 1: launch_k(k_walk_tile<S, MODE, TV, 1>, gf, tb, 0, s, P, V, e); break;
-      case 2: launch_k(k_walk_tile<S, MODE, TV, 2>, gf, tb, 0, s, P, V, e); break;
-      case 3: launch_k(k_walk_tile<S, MODE, TV, 3>, gf, tb, 0, s, P, V, e); break;
-      default: launch_k(k_walk_tile<S, MODE, TV, -1>, gf, tb, 0, s, P, V, e); break;
+      case 0: launch_kp(P.pdl, k_walk_tile<S, MODE, TV, 0>, gf, tb, 0, s, P, V, e); break;
+      case 1: launch_kp(P.pdl, k_walk_tile<S, MODE, TV, 1>, gf, tb, 0, s, P, V, e); break;
+      case 2: launch_kp(P.pdl, k_walk_tile<S, MODE, TV, 2>, gf, tb, 0, s, P, V, e); break;
+      case 3: launch_kp(P.pdl, k_walk_tile<S, MODE, TV, 3>, gf, tb, 0, s, P, V, e); break;
+      default: launch_kp(P.pdl, k_walk_tile<S, MODE, TV, -1>, gf, tb, 0, s, P, V, e); break;
     }
   } else {
-    launch_k(k_walk_tile<S, MODE, TV, -1>, gf, tb, 0, s, P, V, e);
+    launch_kp(P.pdl, k_walk_tile<S, MODE, TV, -1>, gf, tb, 0, s, P, V, e);
   }
 }
 
@@ -1052,13 +1056,13 @@ void launch_walk_t(const DevOps &P, const TV *V, const Epi &e, cudaStream_t s) {
         launch_tile<S, 1, TV>(P, V, e, s);  // residual and F
     } else {
       const int r = walk_rows((long long)gf.x * gf.y);
-      k_walk_fast<S, TV><<<dim3(gf.x, gf.y, RUN / r), dim3(WX, 2), 0, s>>>(P, V, e, r);
+      launch_kp(P.pdl, k_walk_fast<S, TV>, dim3(gf.x, gf.y, RUN / r), dim3(WX, 2), 0, s, P, V, e, r);
     }
   }
   if (!P.all_fast) {
     const long long inner = has_fast ? (long long)(P.fbx1 - P.fbx0) * (P.fby1 - P.fby0) : 0;
     const int r = walk_rows((long long)g.x * g.y - inner);
-    k_walk<S, TV><<<dim3(g.x, g.y, RUN / r), dim3(WX, 2), 0, s>>>(P, V, e, r);
+    launch_kp(P.pdl, k_walk<S, TV>, dim3(g.x, g.y, RUN / r), dim3(WX, 2), 0, s, P, V, e, r);
   }
 }
 

@@ -19,25 +19,20 @@ extern "C" void probe_fdm_tri_apply(void *h, const double *r, double *z, int *ou
   std::vector<double> y(n), Z((size_t)nm * n);
   for (int b = 0; b < nm; ++b) {
     const double *p = &F.piv[(size_t)b * n];
-    double sum = 0.0;
+    double sum = 0.0, part = 0.0;
     for (int s = 0; s < n; ++s) {
       double w = 0.0;
       for (int m = 0; m < nm; ++m) w += F.Q[(size_t)m * nm + b] * r[at(m, s)];
       y[s] = w;
       sum += w;
+      if (b == F.null_mode) part += F.nmu[s] * w;
     }
     const bool null = b == F.null_mode;
-    if (null)
-      for (int s = 0; s < n; ++s) y[s] -= F.h[s] * sum / F.hsum;
     for (int s = 0; s < n; ++s) y[s] = -(y[s] + (s ? F.e[s - 1] * y[s - 1] : 0.0)) * p[s];
     for (int s = n - 2; s >= 0; --s) y[s] -= F.e[s] * p[s] * y[s + 1];
-    double part = 0.0;
-    if (null)
-      for (int s = 0; s < n; ++s) part += F.h[s] * y[s] / F.hsum;
-    else if (!F.g.empty())
-      part = y[0] + F.cr[b] * y[n - 1];
+    if (!null && !F.g.empty()) part = y[0] + F.cr[b] * y[n - 1];
     for (int s = 0; s < n; ++s)
-      Z[(size_t)b * n + s] = y[s] - (null ? part : (F.g.empty() ? 0.0 : part * F.g[(size_t)b * n + s]));
+      Z[(size_t)b * n + s] = y[s] - (null ? part + sum * F.ng[s] : (F.g.empty() ? 0.0 : part * F.g[(size_t)b * n + s]));
   }
   for (int m = 0; m < nm; ++m)
     for (int s = 0; s < n; ++s) {
