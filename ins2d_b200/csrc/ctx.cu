@@ -1853,8 +1853,8 @@ struct ins2d_ens {
   // device tables
   EnsMemberD *d_mem = nullptr;
   std::vector<MgD *> d_mg;
-  int4 *d_fast = nullptr, *d_gen = nullptr, *d_cells = nullptr;
-  int n_fast = 0, n_gen = 0, n_cells = 0;
+  int4 *d_walk = nullptr, *d_cells = nullptr;
+  int n_walk = 0, walk_rows = 0, n_cells = 0;
   int *d_order = nullptr;
   unsigned *d_queue = nullptr;
   EnsStats *d_stats = nullptr;
@@ -1886,6 +1886,7 @@ struct ins2d_ens {
   std::vector<FdmD> h_fdm;
   std::vector<double *> fdm_z;
   EnsFdmPlan fdm_plan;
+  EnsFdmRun fdm_run{};
 };
 
 namespace {
@@ -2000,17 +2001,66 @@ void ens_build_batch(ins2d_ens *e, const std::vector<int> &order) {
     CK(cudaMemcpy(dr, fr.data(), fr.size() * sizeof(int2), cudaMemcpyHostToDevice));
     e->fdm_plan.tiles = dt;
     e->fdm_plan.rows = dr;
+    std::vector<int4> cells;
+    for (int m : order)
+      for (int k = 0, b = 0; k < e->mem[m]->P.Np; k += kEnsCells, ++b) cells.push_back(make_int4(m, k, b, 0));
+    int4 *dc = ens_alloc<int4>(e, cells.size());
+    CK(cudaMemcpy(dc, cells.data(), cells.size() * sizeof(int4), cudaMemcpyHostToDevice));
+    EnsFdmRun &R = e->fdm_run;
+    R.tiles = dc;
+    R.ntiles = (int)cells.size();
+    R.n = n;
+    R.ticket = ens_alloc<unsigned>(e, 1);
+    CK(cudaMemset(R.ticket, 0, sizeof(unsigned)));
   }
   std::vector<EnsCg> cg(n);
   for (int m = 0; m < n; ++m) {
     cg[m] = EnsCg{};
     cg[m].tol2 = e->tol2;
     cg[m].maxit = e->maxit;
+    if (e->use_fdm) {
+      const DevOps &P = e->mem[m]->P;
+      cg[m].part = ens_alloc<double>(e, ens_fdm_scratch(P.Npx, P.Npy));
+      cg[m].ntiles = (int)((P.Np + kEnsCells - 1) / kEnsCells);
+    }
   }
   e->d_cg = ens_alloc<EnsCg>(e, n);
   CK(cudaMemcpy(e->d_cg, cg.data(), n * sizeof(EnsCg), cudaMemcpyHostToDevice));
   e->d_active = ens_alloc<int>(e, 1);
   CK(cudaMallocHost((void **)&e->h_active, sizeof(int)));
+  if (e->use_fdm) {
+    EnsFdmRun &R = e->fdm_run;
+    R.mem = e->d_mem;
+    R.cg = e->d_cg;
+    R.stats = e->d_stats;
+    R.active = e->d_active;
+    R.loops = e->d_loops;
+  }
+}
+
+// The same with fast diagonalization (ens_fdm.cu), from the velocities: mode 0
+// solves the stage's equation (the projection reads the solution), 1 adds the
+// additional solve's to p.
+void ens_solve_fdm(ins2d_ens *e, int mode, double gamma) {
+  const EnsFdmRun &R = e->fdm_run;
+  cudaStream_t s = e->stream;
+  if (e->dev_loop) {
+    const int limit = (int)std::min<long long>(e->maxit + 4, 1 << 30);
+    capture_while(
+        s, e->body_stream, [&](cudaGraphConditionalHandle h) { ens_fdm_init(R, mode, gamma, h, limit, s); },
+        [&](cudaStream_t bs, cudaGraphConditionalHandle h) { ens_fdm_pass(R, e->fdm_plan, h, limit, bs); });
+  } else {
+    ens_fdm_init(R, mode, gamma, 0, -1, s);
+    for (long long done_it = 0;; ++done_it) {
+      ens_fdm_pass(R, e->fdm_plan, 0, -1, s);
+      CK(cudaGetLastError());
+      CK(cudaMemcpyAsync(e->h_active, e->d_active, sizeof(int), cudaMemcpyDeviceToHost, s));
+      CK(cudaStreamSynchronize(s));
+      if (*e->h_active == 0) break;
+      if (done_it > e->maxit + 2) throw CudaError("ensemble PCG: members still active after CG_maxit");
+    }
+  }
+  if (mode == 1) ens_fdm_finish(R, s);
 }
 
 // All members' Poisson solves, batched across members (one launch per phase;
@@ -2020,21 +2070,14 @@ void ens_solve_batched(ins2d_ens *e, int which) {
   const MgD &M0 = e->mem[0]->mg;
   const double om = M0.omega, al = M0.alpha;
   cudaStream_t s = e->stream;
-  // the preconditioner: fast diagonalization over all members' tiles, or the
-  // members' V-cycles
-  auto precond_on = [&](cudaStream_t st) {
-    if (e->use_fdm)
-      fdm_apply_ens(e->fdm_plan, e->d_cg, st);
-    else
-      ens_vcycle(e->d_mem, e->mgd, e->d_cg, e->plan, om, al, st);
-  };
+  auto precond_on = [&](cudaStream_t st) { ens_vcycle(e->d_mem, e->mgd, e->d_cg, e->plan, om, al, st); };
   auto precond = [&]() { precond_on(s); };
   ens_cg_vec(e->d_mem, e->mgd, e->d_ctiles, e->n_ctiles, e->d_cg, 0, s);
   ens_cg_scalar(e->d_cg, n, 0, nullptr, s);
   precond();
   ens_cg_vec(e->d_mem, e->mgd, e->d_ctiles, e->n_ctiles, e->d_cg, 4, s);
   ens_cg_scalar(e->d_cg, n, 1, nullptr, s);
-  const int chunk = e->use_fdm ? (e->dev_loop ? 1 : 2) : 4;
+  const int chunk = 4;
   auto iterations_on = [&](cudaStream_t st) {
     for (int k = 0; k < chunk; ++k) {
       ens_cg_vec(e->d_mem, e->mgd, e->d_ctiles, e->n_ctiles, e->d_cg, 1, st);
@@ -2086,7 +2129,8 @@ void ens_solve_batched(ins2d_ens *e, int which) {
 void ens_upload(ins2d_ens *e, double dt) {
   const int n = (int)e->mem.size();
   std::vector<EnsMemberD> h(n);
-  std::vector<int4> fast, gen, cells;
+  std::vector<int4> walk, cells;
+  std::vector<const DevOps *> ops;
   for (int m = 0; m < n; ++m) {
     ins2d_ctx *c = e->mem[m];
     EnsMemberD &d = h[m];
@@ -2104,9 +2148,10 @@ void ens_upload(ins2d_ens *e, double dt) {
     d.W = c->pcg;
     d.mg = c->use_mg ? e->d_mg[m] : nullptr;
     d.zf = e->use_fdm ? e->fdm_z[m] : nullptr;
-    walk_tiles(c->P, m, fast, gen);
+    ops.push_back(&c->P);
     cell_tiles(c->P, m, cells);
   }
+  ens_walk_work(ops, walk, e->walk_rows);
   std::vector<int> order(n);
   for (int m = 0; m < n; ++m) order[m] = m;
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return e->mem[a]->P.Np > e->mem[b]->P.Np; });
@@ -2115,18 +2160,15 @@ void ens_upload(ins2d_ens *e, double dt) {
     e->d_order = ens_alloc<int>(e, n);
     e->d_queue = ens_alloc<unsigned>(e, 2);
     e->d_stats = ens_alloc<EnsStats>(e, n);
-    e->d_fast = ens_alloc<int4>(e, fast.size());
-    e->d_gen = ens_alloc<int4>(e, gen.size());
+    e->d_walk = ens_alloc<int4>(e, walk.size());
     e->d_cells = ens_alloc<int4>(e, cells.size());
     CK(cudaMemset(e->d_queue, 0, 2 * sizeof(unsigned)));
   }
   CK(cudaMemcpy(e->d_mem, h.data(), n * sizeof(EnsMemberD), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(e->d_order, order.data(), n * sizeof(int), cudaMemcpyHostToDevice));
-  if (!fast.empty()) CK(cudaMemcpy(e->d_fast, fast.data(), fast.size() * sizeof(int4), cudaMemcpyHostToDevice));
-  if (!gen.empty()) CK(cudaMemcpy(e->d_gen, gen.data(), gen.size() * sizeof(int4), cudaMemcpyHostToDevice));
+  CK(cudaMemcpy(e->d_walk, walk.data(), walk.size() * sizeof(int4), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(e->d_cells, cells.data(), cells.size() * sizeof(int4), cudaMemcpyHostToDevice));
-  e->n_fast = (int)fast.size();
-  e->n_gen = (int)gen.size();
+  e->n_walk = (int)walk.size();
   e->n_cells = (int)cells.size();
   if (e->can_batch && !e->d_cg) ens_build_batch(e, order);
   e->uploaded = true;
@@ -2169,19 +2211,26 @@ void ens_step(ins2d_ens *e, bool k0_cached) {
           ++w.nprev;
         }
       w.aii = c0->A[i][i];
-      launch_walk_ens(e->d_mem, e->d_fast, e->n_fast, e->d_gen, e->n_gen, w, e->fp32, e->stream);
+      launch_walk_ens(e->d_mem, e->d_walk, e->n_walk, e->walk_rows, w, e->fp32, e->stream);
     }
-    if (i > 0) {
+    if (i > 0 && e->use_fdm) {
+      ens_solve_fdm(e, 0, 1.0 / c0->c[i]);
+    } else if (i > 0) {
       launch_div_ens(e->d_mem, e->d_cells, e->n_cells, 0, 1.0 / c0->c[i], e->stream);
       ens_solve(e, 0);
     }
-    launch_project_ens(e->d_mem, e->d_cells, e->n_cells, c0->c[i], i == 0 ? 1 : 0, i == s - 1 ? 1 : 0, e->stream);
+    launch_project_ens(e->d_mem, e->d_cells, e->n_cells, c0->c[i], i == 0 ? 1 : 0, i == s - 1 ? 1 : 0,
+                       e->use_fdm && i > 0 ? e->d_cg : nullptr, e->stream);
   }
   // additional pressure solve; its residual is the next step's first stage
   EnsWalk w{};
   w.mode = 1;
   w.cache = 1;
-  launch_walk_ens(e->d_mem, e->d_fast, e->n_fast, e->d_gen, e->n_gen, w, e->fp32, e->stream);
+  launch_walk_ens(e->d_mem, e->d_walk, e->n_walk, e->walk_rows, w, e->fp32, e->stream);
+  if (e->use_fdm) {
+    ens_solve_fdm(e, 1, 1.0);
+    return;
+  }
   launch_div_ens(e->d_mem, e->d_cells, e->n_cells, 1, 1.0, e->stream);
   ens_solve(e, 1);
 }
@@ -2202,9 +2251,15 @@ void ens_autotune(ins2d_ens *e) {
   for (int k = 0; k < ncand; ++k) {
     e->solve_threads = cand[k];
     e->solve_blocks = cand[k] ? std::min(n, sms * (512 / cand[k])) : 0;
-    ens_solve(e, 0);  // warm-up
+    auto solve = [&] {
+      if (e->use_fdm)
+        ens_solve_fdm(e, 0, 1.0);
+      else
+        ens_solve(e, 0);
+    };
+    solve();  // warm-up
     CK(cudaEventRecord(a, e->stream));
-    ens_solve(e, 0);
+    solve();
     CK(cudaEventRecord(b, e->stream));
     CK(cudaEventSynchronize(b));
     float ms = 0.f;
@@ -2323,6 +2378,7 @@ int ins2d_ens_create(int32_t n, const ins2d_grid_desc *grids, const ins2d_bc_des
           ins2d_ctx *c = e->mem[m];
           FdmD &D = hf[m];
           upload_fdm(c, D);
+          D.f = c->f;
           D.r = c->pcg.r;
           D.z = dalloc<double>(c, (size_t)c->P.Np);
           e->fdm_z.push_back(D.z);

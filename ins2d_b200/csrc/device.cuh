@@ -54,6 +54,32 @@ __device__ __forceinline__ int wrapn(int c, int n) { return c < 0 ? c + n : (c >
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 
+// points [x0, x1) x [y0, y1) of a component's nx x ny; the others ("ring")
+// are numbered: the rows below, the rows above, then the columns left and right
+struct WalkRect {
+  int x0, x1, y0, y1, nx, ny;
+  __host__ __device__ int ring() const { return nx * ny - (x1 - x0) * (y1 - y0); }
+  __device__ void point(int k, int &i, int &j) const {
+    const int below = nx * y0, above = nx * (ny - y1);
+    if (k < below) {
+      j = k / nx;
+      i = k - j * nx;
+    } else if (k < below + above) {
+      k -= below;
+      j = k / nx;
+      i = k - j * nx;
+      j += y1;
+    } else {
+      k -= below + above;
+      const int side = x0 + nx - x1;
+      j = k / side;
+      i = k - j * side;
+      if (i >= x0) i += x1 - x0;
+      j += y0;
+    }
+  }
+};
+
 struct DevOps {
   int Nx, Ny, Nux, Nuy, Nvx, Nvy, Npx, Npy;
   long long Nu, Nv, Np;
@@ -72,6 +98,7 @@ struct DevOps {
   // rectangle [fbx0,fbx1) x [fby0,fby1) whose tiles lie inside all of them
   RegD rAUX, rSUX, rAUY, rSUY, rIVX, rIVY, rMXT, rAVX, rSVX, rAVY, rSVY, rIUX, rIUY, rMYT, rMX, rMY;
   int fbx0, fbx1, fby0, fby1;
+  WalkRect ru, rv;  // the points of each component inside all of them (ensemble walkers)
   int tile_ok;    // the interior tiles may use the shared-memory tiled walkers (FP64 fields)
   int tile_ok32;  // ... on FP32 fields
   int all_fast;   // the rectangle holds every tile of the grid (no table-walker tiles)

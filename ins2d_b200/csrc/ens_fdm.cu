@@ -1,0 +1,242 @@
+// Poisson solves of an ensemble with the fast-diagonalization preconditioner,
+// batched across members: the passes of pcg.cu's single-grid path, every
+// kernel one launch over the work of all members that still iterate.
+//
+// A solve of members of 64 to 256 cells per direction is bound by its
+// launches.  So a member's scalars are advanced by its last block in each
+// reduction (no one-block kernels between), its statistics and the loop
+// condition by the update, the divergence is formed by the initialisation and
+// the solution is read by the projection.  24 members, RK44 step on B200:
+// eleven launches and eleven more per pass before, 0.881 ms; six launches and
+// five more per pass now, @FIG@.
+#include <cfloat>
+
+#include "ins2d.h"
+#include "kernels.cuh"
+#include "reduce.cuh"
+
+namespace ins2d {
+
+namespace {
+
+constexpr int kThreads = 256;
+constexpr int kPer = kEnsCells / kThreads;  // cells per thread
+
+__device__ __forceinline__ RedScratch member_red(EnsCg &C, int nq) {
+  RedScratch r;
+  r.partials = C.part;
+  r.counter = &C.ticket;
+  r.result = C.part + (size_t)C.ntiles * nq;
+  r.max_blocks = C.ntiles;
+  return r;
+}
+
+__device__ __forceinline__ void add_stats(const EnsCg &C, EnsStats &st) {
+  st.n_solves += 1;
+  st.iters_total += C.it;
+  st.iters_max = C.it > st.iters_max ? C.it : st.iters_max;
+  const double n1 = sqrt(C.rr);
+  st.norm1_max = n1 > st.norm1_max ? n1 : st.norm1_max;
+  if (C.status != 0 && st.status == 0) st.status = C.status;
+}
+
+// the last block of a launch: counts the members still iterating and sets the
+// loop condition (first: before any pass)
+__device__ void end_launch(const EnsFdmRun &R, const LoopCond &cond, bool first) {
+  __shared__ bool last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(R.ticket, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  int mine = 0;
+  for (int m = threadIdx.x; m < R.n; m += blockDim.x) mine += *(volatile int *)&R.cg[m].done ? 0 : 1;
+  __shared__ int act;
+  if (threadIdx.x == 0) act = 0;
+  __syncthreads();
+  if (mine) atomicAdd(&act, mine);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    *R.ticket = 0u;
+    *R.active = act;
+    const int loops = first ? 0 : *R.loops + 1;
+    *R.loops = loops;
+    set_cond(cond, act > 0 && loops < cond.limit);
+  }
+}
+
+__device__ __forceinline__ void copy_ops(DevOps *dst, const DevOps *src) {
+  for (int k = threadIdx.x; k < (int)(sizeof(DevOps) / 8); k += blockDim.x)
+    ((long long *)dst)[k] = ((const long long *)src)[k];
+}
+
+// f = (M Wt + yM/dt) gamma (mode 0) or M wres (mode 1); f'f, max|f|
+__global__ void __launch_bounds__(kThreads) k_ef_init(const EnsFdmRun R, int mode, double gamma, const LoopCond cond) {
+  __shared__ __align__(16) DevOps sP;
+  const int4 t = R.tiles[blockIdx.x];
+  const EnsMemberD &M = R.mem[t.x];
+  EnsCg &C = R.cg[t.x];
+  copy_ops(&sP, &M.P);
+  __syncthreads();
+  const double *W = mode == 0 ? M.Wt : M.wres;
+  const double alpha = mode == 0 ? 1.0 / M.dt : 0.0, g = mode == 0 ? gamma : 1.0;
+  double q[2] = {0.0, 0.0};
+  const int ops[2] = {R_SUM, R_MAX};
+#pragma unroll
+  for (int u = 0; u < kPer; ++u) {
+    const int k = t.y + u * kThreads + threadIdx.x;
+    if (k < sP.Np) {
+      const int j = k / sP.Npx, i = k - j * sP.Npx;
+      const double fv = div_cell(sP, W, alpha, 0.0, g, i, j);
+      M.f[k] = fv;
+      q[0] += fv * fv;
+      q[1] = fmax(q[1], fabs(fv));
+    }
+  }
+  double out[2];
+  if (grid_reduce_at<2>(q, ops, member_red(C, 2), out, t.z, C.ntiles)) {
+    C.rr0 = out[0];
+    C.rr = 0.0;
+    C.rz = 0.0;
+    C.it = 0;
+    C.status = 0;
+    // pressure_poisson.m:33-38, cg.F:222-227
+    int done = (out[1] < 1e-14 || C.rr0 <= C.tol2) ? 1 : 0;
+    if (!isfinite(C.rr0)) {
+      C.status = INS2D_ENONFINITE;
+      done = 1;
+    }
+    if (done) add_stats(C, R.stats[t.x]);
+    C.done = done;
+  }
+  end_launch(R, cond, true);
+}
+
+// p = z + beta p (directions alternate between two buffers), q = A p, p'q
+__global__ void __launch_bounds__(kThreads) k_ef_step(const EnsFdmRun R) {
+  __shared__ __align__(16) DevOps sP;
+  const int4 t = R.tiles[blockIdx.x];
+  EnsCg &C = R.cg[t.x];
+  if (*(volatile int *)&C.done) return;
+  const EnsMemberD &M = R.mem[t.x];
+  copy_ops(&sP, &M.P);
+  __syncthreads();
+  const PcgWork &W = M.W;
+  const bool first = C.it == 0, odd = C.it & 1;
+  const double beta = C.beta;
+  const double *__restrict__ z = M.zf, *__restrict__ po = odd ? W.p : W.p2;
+  double *__restrict__ pn = odd ? W.p2 : W.p;
+  auto pv = [&](long long k) {
+    double v = __ldg(z + k);
+    if (!first) v += beta * __ldg(po + k);
+    return v;
+  };
+  double q[1] = {0.0};
+  const int ops[1] = {R_SUM};
+#pragma unroll
+  for (int u = 0; u < kPer; ++u) {
+    const int k = t.y + u * kThreads + threadIdx.x;
+    if (k < sP.Np) {
+      const int j = k / sP.Npx, i = k - j * sP.Npx;
+      const double aq = -(__ldg(sP.hy + j) * tab_x_f(sP.TX, i, pv, (long long)j * sP.Npx) +
+                          __ldg(sP.hx + i) * tab_y_f(sP.TY, j, pv, 0, sP.Npx, i));
+      const double pc = pv(k);
+      W.q[k] = aq;
+      pn[k] = pc;
+      q[0] += pc * aq;
+    }
+  }
+  double out[1];
+  if (grid_reduce_at<1>(q, ops, member_red(C, 1), out, t.z, C.ntiles)) {
+    if (!isfinite(out[0]))
+      C.status = INS2D_ENONFINITE;
+    else if (out[0] == 0.0 && C.status == 0)
+      C.status = INS2D_EBREAKDOWN;
+    C.alpha = C.status ? 0.0 : C.rz / out[0];
+  }
+}
+
+// x += alpha p, r -= alpha q (x = 0, r = f before the first pass), the stopping
+// rule, statistics and loop condition
+__global__ void __launch_bounds__(kThreads) k_ef_update(const EnsFdmRun R, const LoopCond cond) {
+  const int4 t = R.tiles[blockIdx.x];
+  EnsCg &C = R.cg[t.x];
+  if (!*(volatile int *)&C.done) {
+    const EnsMemberD &M = R.mem[t.x];
+    const PcgWork &W = M.W;
+    const bool first = C.it == 0;
+    const double alpha = C.alpha;
+    const double *__restrict__ p = (C.it & 1) ? W.p2 : W.p;
+    const int Np = (int)M.P.Np;
+    double q[1] = {0.0};
+    const int ops[1] = {R_SUM};
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+      const int k = t.y + u * kThreads + threadIdx.x;
+      if (k < Np) {
+        const double x = (first ? 0.0 : W.x[k]) + alpha * __ldg(p + k);
+        const double r = (first ? __ldg(M.f + k) : W.r[k]) - alpha * __ldg(W.q + k);
+        W.x[k] = x;
+        W.r[k] = r;
+        q[0] += r * r;
+      }
+    }
+    double out[1];
+    if (grid_reduce_at<1>(q, ops, member_red(C, 1), out, t.z, C.ntiles)) {
+      int done = 0;
+      if (C.status != 0) {  // found by this pass's reductions (cg.F:240-262)
+        done = 1;
+      } else {
+        C.it += 1;
+        C.rr = out[0] / C.rr0;
+        if (!isfinite(C.rr)) {
+          C.status = INS2D_ENONFINITE;
+          done = 1;
+        } else if (C.rr <= C.tol2) {
+          done = 1;
+        } else if (C.it >= C.maxit) {
+          C.status = INS2D_ENOTCONV;
+          done = 1;
+        }
+      }
+      if (done) add_stats(C, R.stats[t.x]);
+      C.done = done;
+    }
+  }
+  end_launch(R, cond, false);
+}
+
+__global__ void __launch_bounds__(kThreads) k_ef_finish(const EnsFdmRun R) {
+  const int4 t = R.tiles[blockIdx.x];
+  const EnsCg &C = R.cg[t.x];
+  if (C.it == 0 || C.status != 0) return;
+  const EnsMemberD &M = R.mem[t.x];
+#pragma unroll
+  for (int u = 0; u < kPer; ++u) {
+    const int k = t.y + u * kThreads + threadIdx.x;
+    if (k < M.P.Np) M.p[k] += M.W.x[k];
+  }
+}
+
+}  // namespace
+
+size_t ens_fdm_scratch(int nx, int ny) {
+  const size_t cells = ((size_t)nx * ny + kEnsCells - 1) / kEnsCells;
+  const size_t tiles = (size_t)((nx + 31) / 32) * ((ny + 31) / 32);  // fdm.cu's output tiles
+  return 2 * cells + tiles + 8;
+}
+
+void ens_fdm_init(const EnsFdmRun &R, int mode, double gamma, cudaGraphConditionalHandle h, int limit, cudaStream_t s) {
+  k_ef_init<<<R.ntiles, kThreads, 0, s>>>(R, mode, gamma, LoopCond{h, limit});
+}
+void ens_fdm_pass(const EnsFdmRun &R, const EnsFdmPlan &pl, cudaGraphConditionalHandle h, int limit, cudaStream_t s) {
+  fdm_apply_ens(pl, R.cg, s);
+  k_ef_step<<<R.ntiles, kThreads, 0, s>>>(R);
+  k_ef_update<<<R.ntiles, kThreads, 0, s>>>(R, LoopCond{h, limit});
+}
+void ens_fdm_finish(const EnsFdmRun &R, cudaStream_t s) { k_ef_finish<<<R.ntiles, kThreads, 0, s>>>(R); }
+
+}  // namespace ins2d

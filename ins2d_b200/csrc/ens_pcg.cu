@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(kTile) k_ecg_vec(const EnsMemberD *__restrict_
   const long long k = (long long)t.y + threadIdx.x;
   const bool in = k < E.P.Np;
   const PcgWork &W = E.W;
-  const double *z = E.zf ? E.zf : mg_res(G, m, 0);
+  const double *z = mg_res(G, m, 0);
   double a = 0.0, b = 0.0;
   if (op == 1) {  // q = A p, p'q
     for (int w = threadIdx.x; w < (int)(sizeof(DevOps) / 8); w += blockDim.x)

@@ -216,16 +216,39 @@ __global__ void __launch_bounds__(kThreads) k_fdm_fwd_ens(const FdmD *__restrict
   if (*(volatile const int *)&cg[t.x].done) return;
   const FdmD &F = Fs[t.x];
   const int m0 = t.y * kBM, n0 = t.z * kBN;
-  if (m0 < F.nm && n0 < F.n) fdm_forward(F, F.r, m0, n0, sm);
+  if (m0 < F.nm && n0 < F.n) fdm_forward(F, cg[t.x].it == 0 ? F.f : F.r, m0, n0, sm);
 }
 __global__ void __launch_bounds__(kThreads) k_fdm_bwd_ens(const FdmD *__restrict__ Fs, const int4 *__restrict__ tiles,
-                                                          const EnsCg *__restrict__ cg) {
+                                                          EnsCg *__restrict__ cg) {
   __shared__ __align__(16) double sm[2 * kStages * kSlab];
   const int4 t = tiles[blockIdx.x];
-  if (*(volatile const int *)&cg[t.x].done) return;
+  EnsCg &C = cg[t.x];
+  if (*(volatile const int *)&C.done) return;
   const FdmD &F = Fs[t.x];
   const int m0 = t.y * kBM, n0 = t.z * kBN;
-  if (m0 < F.ny && n0 < F.nx) fdm_backward(F, m0, n0, sm, [&](size_t k, double v) { F.z[k] = v; });
+  if (m0 >= F.ny || n0 >= F.nx) return;
+  const double *__restrict__ r = C.it == 0 ? F.f : F.r;
+  double q[1] = {0.0};
+  const int ops[1] = {R_SUM};
+  fdm_backward(F, m0, n0, sm, [&](size_t k, double v) {
+    F.z[k] = v;
+    q[0] += __ldg(r + k) * v;
+  });
+  const int tx = (F.nx + kBN - 1) / kBN, nb = tx * ((F.ny + kBM - 1) / kBM);
+  RedScratch red;
+  red.partials = C.part;
+  red.counter = &C.ticket;
+  red.result = C.part + nb;
+  double out[1];
+  if (grid_reduce_at<1>(q, ops, red, out, t.y * tx + t.z, nb)) {
+    if (!isfinite(out[0])) {
+      C.status = INS2D_ENONFINITE;  // the member's update ends its solve
+      C.beta = 0.0;
+    } else {
+      C.beta = C.it == 0 ? 0.0 : out[0] / C.rz;
+      C.rz = out[0];
+    }
+  }
 }
 template <int W>
 __global__ void __launch_bounds__(128) k_fdm_tri_ens(const FdmD *__restrict__ Fs, const int2 *__restrict__ rows,
@@ -277,7 +300,7 @@ void fdm_ens_lists(const std::vector<FdmD> &F, const std::vector<int> &order, En
   pl.nrows = (int)rows.size();
 }
 
-void fdm_apply_ens(const EnsFdmPlan &pl, const EnsCg *cg, cudaStream_t s) {
+void fdm_apply_ens(const EnsFdmPlan &pl, EnsCg *cg, cudaStream_t s) {
   if (pl.ntiles <= 0) return;
   k_fdm_fwd_ens<<<pl.ntiles, kThreads, 0, s>>>(pl.F, pl.tiles, cg);
   if (pl.warps == 1)

@@ -242,14 +242,15 @@ __global__ void __launch_bounds__(256) k_div_ens(const EnsMemberD *__restrict__ 
 
 __global__ void __launch_bounds__(256) k_project_ens(const EnsMemberD *__restrict__ mem,
                                                     const int4 *__restrict__ tiles, double c, int from_p,
-                                                    int last) {
+                                                    int last, const EnsCg *__restrict__ cg) {
   __shared__ __align__(16) DevOps sP;
   const int4 t = tiles[blockIdx.x];
   const EnsMemberD &M = mem[t.x];
   copy_ops(&sP, &M.P);
   __syncthreads();
-  project_cell(sP, M.Wt, from_p ? M.p : M.dp, M.dt, c, last ? M.V : M.Vs, t.y * BX + threadIdx.x,
-               t.z * BY + threadIdx.y);
+  const bool zero = cg && cg[t.x].it == 0;  // solved without a pass: dp = 0 (any finite field will do)
+  project_cell(sP, M.Wt, from_p ? M.p : (cg ? (zero ? M.f : M.W.x) : M.dp), M.dt, zero ? 0.0 : c, last ? M.V : M.Vs,
+               t.y * BX + threadIdx.x, t.z * BY + threadIdx.y);
 }
 
 __global__ void __launch_bounds__(256) k_stage_cached_ens(const EnsMemberD *__restrict__ mem,
@@ -402,8 +403,8 @@ void launch_div_ens(const EnsMemberD *mem, const int4 *tiles, int n, int mode, d
 }
 
 void launch_project_ens(const EnsMemberD *mem, const int4 *tiles, int n, double c, int from_p, int last,
-                        cudaStream_t s) {
-  if (n > 0) k_project_ens<<<n, dim3(BX, BY), 0, s>>>(mem, tiles, c, from_p, last);
+                        const EnsCg *cg, cudaStream_t s) {
+  if (n > 0) k_project_ens<<<n, dim3(BX, BY), 0, s>>>(mem, tiles, c, from_p, last, cg);
 }
 
 void launch_stage_cached_ens(const EnsMemberD *mem, const int4 *tiles, int n, double aii, cudaStream_t s) {

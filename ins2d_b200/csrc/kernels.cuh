@@ -101,7 +101,7 @@ struct StageArgs {
 // One RK stage right-hand side: kV = Om^-1 (-conv + Diff V + yDiff - y_p),
 // Vtemp = sum_m A(i,m) kV_m, Wt = Vn/dt + Vtemp   (time_ERK.m:90-101,117)
 void launch_stage(const DevOps &P, const StageArgs &a, bool fp32, cudaStream_t s);
-// computes P.fbx0.. (the interior tile rectangle of the stencil walkers)
+// computes P.fbx0.., P.ru, P.rv (the regular tiles and points of the walkers)
 void walker_rectangle(DevOps &P);
 // opts the tiled walkers in to their dynamic shared memory on the current
 // device (once per context); returns the first failure
@@ -163,20 +163,22 @@ struct EnsWalk {
   double aprev[kMaxStages];
   double aii;
 };
-// Host: the walker tiles {member, bx, by, 0} of one member, split into fast
-// (interior) and generic tiles.
-void walk_tiles(const DevOps &P, int member, std::vector<int4> &fast, std::vector<int4> &gen);
-void launch_walk_ens(const EnsMemberD *mem, const int4 *fast, int nfast, const int4 *gen, int ngen, const EnsWalk &w,
-                     bool fp32, cudaStream_t s);
+// Host: the walkers' work items of all members (stencil.cu, k_walk_ens) and the
+// rows per item
+void ens_walk_work(const std::vector<const DevOps *> &P, std::vector<int4> &work, int &rows);
+void launch_walk_ens(const EnsMemberD *mem, const int4 *work, int n, int rows, const EnsWalk &w, bool fp32,
+                     cudaStream_t s);
 // Host: the 32x8 cell tiles {member, bx, by, 0} covering a member's u, v and p
 // index spaces.
 void cell_tiles(const DevOps &P, int member, std::vector<int4> &out);
 // f = (M Wt + yM/dt) gamma (mode 0, stage) or f = M wres (mode 1, residual)
 void launch_div_ens(const EnsMemberD *mem, const int4 *tiles, int n, int mode, double gamma, cudaStream_t s);
-// V_out = dt (Wt - c Om^-1 G dp_src); dp_src = p (from_p) or dp; V_out = V
-// (last stage) or Vs
+// V_out = dt (Wt - c Om^-1 G dp_src); dp_src = p (from_p) or dp, or the CG
+// iterate where cg is given (zero before its first pass); V_out = V (last
+// stage) or Vs
+struct EnsCg;
 void launch_project_ens(const EnsMemberD *mem, const int4 *tiles, int n, double c, int from_p, int last,
-                        cudaStream_t s);
+                        const EnsCg *cg, cudaStream_t s);
 // Wt = V/dt + aii kV[0] (first stage from the cached residual)
 void launch_stage_cached_ens(const EnsMemberD *mem, const int4 *tiles, int n, double aii, cudaStream_t s);
 
@@ -231,7 +233,7 @@ struct FdmD {
   const double *g = nullptr, *cr = nullptr;                 // cyclic systems: nm x n, nm
   int null_mode = -1;
   const double *ng = nullptr, *nmu = nullptr;               // its corrections: n
-  const double *r = nullptr;  // ensembles: the member's CG residual
+  const double *f = nullptr, *r = nullptr;  // ensembles: the member's right-hand side and CG residual
   double *t = nullptr;        // nm x n: transformed residual, then the systems' solutions
   double *z = nullptr;        // the preconditioned residual
   // periodic uniform grids: the Fourier basis, applied by the FFT solve
@@ -255,8 +257,9 @@ struct EnsFdmPlan {
 };
 void fdm_ens_lists(const std::vector<FdmD> &F, const std::vector<int> &order, EnsFdmPlan &pl, std::vector<int4> &tiles,
                    std::vector<int2> &rows);
-// z = A^+ r for every member not yet converged (cg[m].done == 0)
-void fdm_apply_ens(const EnsFdmPlan &pl, const EnsCg *cg, cudaStream_t s);
+// z = A^+ r, r'z and beta for every member not yet converged (cg[m].done == 0);
+// r = f on a member's first pass
+void fdm_apply_ens(const EnsFdmPlan &pl, EnsCg *cg, cudaStream_t s);
 
 // --- PCG (pcg.cu) ---------------------------------------------------------------
 struct PcgScalars {
@@ -308,6 +311,14 @@ void pcg_init_fdm(const DevOps &P, const FdmD &F, const PcgWork &W, const double
 cudaError_t pcg_pass_fdm(const DevOps &P, const FdmD &F, const PcgWork &W, const double *f,
                          cudaGraphConditionalHandle h, int limit, cudaStream_t s);
 void pcg_finish_fdm(const DevOps &P, const PcgWork &W, double *dp, bool accumulate, SolveAccum *acc, cudaStream_t s);
+// condition of the WHILE node around the passes (limit < 0: no graph)
+struct LoopCond {
+  cudaGraphConditionalHandle h;
+  int limit;
+};
+__device__ __forceinline__ void set_cond(const LoopCond &c, bool go) {
+  if (c.limit >= 0) cudaGraphSetConditional(c.h, go ? 1u : 0u);
+}
 // r'z of a new application (one thread): the first one's, or beta
 __device__ __forceinline__ void pcg_new_rz(PcgScalars *s, double rz) {
   if (!isfinite(rz)) {
@@ -358,7 +369,7 @@ struct EnsMemberD {
   double *V, *p, *Vs, *Wt, *kV[kMaxStages], *f, *dp, *wres;
   PcgWork W;
   const MgD *mg;  // device copy of the member's hierarchy, or null (Jacobi)
-  const double *zf;  // batched solves with fast diagonalization: the preconditioned residual
+  const double *zf;  // fast diagonalization: the preconditioned residual
 };
 // per-member solve statistics, accumulated over a run
 struct EnsStats {
@@ -379,7 +390,34 @@ struct EnsCg {
   double rz, rr0, rr, alpha, beta, tol2;
   long long it, maxit;
   int done, status;
+  // fast diagonalization: the member's reduction scratch and its cell tiles
+  double *part;
+  unsigned int ticket;
+  int ntiles;
 };
+// --- ensembles with fast diagonalization (ens_fdm.cu) -----------------------
+// cell tiles {member, first cell, number within the member, 0} of kEnsCells
+// cells, and what the passes share
+constexpr int kEnsCells = 1024;
+struct EnsFdmRun {
+  const EnsMemberD *mem;
+  EnsCg *cg;
+  EnsStats *stats;
+  const int4 *tiles;
+  int ntiles, n;      // cell tiles, members
+  unsigned *ticket;   // blocks of a launch that have finished (zero between launches)
+  int *active;        // members still iterating
+  int *loops;         // passes of the current solve
+};
+// doubles of a member's reduction scratch
+size_t ens_fdm_scratch(int nx, int ny);
+// f = the divergence (mode 0 of a stage, with 1/c = gamma; 1 of the residual),
+// the members' scalars
+void ens_fdm_init(const EnsFdmRun &R, int mode, double gamma, cudaGraphConditionalHandle h, int limit, cudaStream_t s);
+// one pass: application, direction and product, update (cf. pcg_pass_fdm)
+void ens_fdm_pass(const EnsFdmRun &R, const EnsFdmPlan &pl, cudaGraphConditionalHandle h, int limit, cudaStream_t s);
+// p += x (the additional solve; a stage's projection reads x itself)
+void ens_fdm_finish(const EnsFdmRun &R, cudaStream_t s);
 // members' multigrid levels: lev[m * kMgMaxLevels + l]
 struct EnsMgD {
   const MgLevelD *lev;

@@ -503,15 +503,6 @@ __global__ void __launch_bounds__(kVecThreads) k_pupdate_g(const PcgWork W, cons
 // kernels, measured on B200: stretched 512^2 channel step 0.890 -> 0.773 ms,
 // 301 x 257 channel solve 198 -> 163 us.
 
-// condition of the WHILE node around the passes (limit < 0: no graph)
-struct LoopCond {
-  cudaGraphConditionalHandle h;
-  int limit;
-};
-__device__ __forceinline__ void set_cond(const LoopCond &c, bool go) {
-  if (c.limit >= 0) cudaGraphSetConditional(c.h, go ? 1u : 0u);
-}
-
 // sums over f: f'f and max|f|; the solve's scalars (copy: also r = f, the
 // spectral application's input)
 __global__ void __launch_bounds__(kVecThreads) k_init_f(const PcgWork W, const double *__restrict__ f, long long n,

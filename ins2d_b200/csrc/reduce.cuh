@@ -22,9 +22,11 @@ static __host__ __device__ __forceinline__ double red_identity(int op) {
 
 // Block-level reduction of NQ values followed by the grid-level finish: the
 // last block to arrive combines all partials in block order.  Every thread
-// of every block must call it.
+// of every block must call it.  bid, nb: this block's number and their count
+// (a part of the grid may reduce on its own scratch).
 template <int NQ>
-__device__ bool grid_reduce(double (&v)[NQ], const int (&ops)[NQ], const RedScratch &red, double (&out)[NQ]) {
+__device__ bool grid_reduce_at(double (&v)[NQ], const int (&ops)[NQ], const RedScratch &red, double (&out)[NQ], int bid,
+                               int nb) {
   __shared__ double sh[32][NQ];
   __shared__ bool last;
   const int tid = threadIdx.x + blockDim.x * threadIdx.y;
@@ -36,8 +38,6 @@ __device__ bool grid_reduce(double (&v)[NQ], const int (&ops)[NQ], const RedScra
 #pragma unroll
     for (int q = 0; q < NQ; ++q) sh[warp][q] = v[q];
   __syncthreads();
-  const int bid = blockIdx.x + gridDim.x * blockIdx.y;
-  const int nb = gridDim.x * gridDim.y;
   if (tid == 0) {
 #pragma unroll
     for (int q = 0; q < NQ; ++q) {
@@ -87,6 +87,12 @@ __device__ bool grid_reduce(double (&v)[NQ], const int (&ops)[NQ], const RedScra
     *red.counter = 0u;
   }
   return tid == 0;
+}
+
+template <int NQ>
+__device__ __forceinline__ bool grid_reduce(double (&v)[NQ], const int (&ops)[NQ], const RedScratch &red,
+                                            double (&out)[NQ]) {
+  return grid_reduce_at<NQ>(v, ops, red, out, blockIdx.x + gridDim.x * blockIdx.y, gridDim.x * gridDim.y);
 }
 
 // Variant for callers that only need red.result.

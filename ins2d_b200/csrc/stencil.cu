@@ -378,6 +378,43 @@ __device__ __forceinline__ void stage_yrows(const DevOps &P, int j0, YRowsN<NR> 
   }
 }
 
+// the same for a run that may reach past the last row (those faces and rows
+// belong to no walked point)
+template <int NR>
+__device__ __forceinline__ void stage_yrows_cut(const DevOps &P, int j0, YRowsN<NR> &Y, int rows) {
+  const int t = threadIdx.x + blockDim.x * threadIdx.y, j = j0 + t;
+  if (t <= rows) {
+    if (j <= P.Nuy) {
+      Y.auy0[t] = __ldg(P.rAUY.w0 + j);
+      Y.auy1[t] = __ldg(P.rAUY.w1 + j);
+      Y.suy0[t] = __ldg(P.rSUY.w0 + j);
+      Y.suy1[t] = __ldg(P.rSUY.w1 + j);
+      Y.ivy0[t] = __ldg(P.rIVY.w0 + j);
+      Y.ivy1[t] = __ldg(P.rIVY.w1 + j);
+    }
+    if (j <= P.Nvy) {
+      Y.avy0[t] = __ldg(P.rAVY.w0 + j);
+      Y.avy1[t] = __ldg(P.rAVY.w1 + j);
+      Y.svy0[t] = __ldg(P.rSVY.w0 + j);
+      Y.svy1[t] = __ldg(P.rSVY.w1 + j);
+    }
+  }
+  if (t < rows) {
+    if (j < P.Nuy) {
+      Y.hy[t] = __ldg(P.hy + j);
+      Y.rhy[t] = __ldg(P.rhy + j);
+    }
+    if (j < P.Nvy) {
+      Y.iuy0[t] = __ldg(P.rIUY.w0 + j);
+      Y.iuy1[t] = __ldg(P.rIUY.w1 + j);
+      Y.gyi[t] = __ldg(P.gyi + j);
+      Y.rgyi[t] = __ldg(P.rgyi + j);
+      Y.myt0[t] = __ldg(P.rMYT.w0 + j);
+      Y.myt1[t] = __ldg(P.rMYT.w1 + j);
+    }
+  }
+}
+
 // Raw loads of one row of the u walker: the x-face values of row j, the
 // field values of the y-face j+1 and the epilogue input; issued one row ahead
 // of their use so each warp keeps two rows of loads in flight.
@@ -389,7 +426,7 @@ struct URaw {
 
 template <typename S, typename TV>
 __device__ void fast_u(const DevOps &P, const TV *__restrict__ u, const TV *__restrict__ v, const Epi &e,
-                       int i, int j0, int j1, const YRows &Y) {
+                       int i, int j0, int j1, const YRows &Y, int jy) {
   const S ire = S(P.invRe);
   // columns (modulo the row length for periodic wraps)
   const int cA0 = wrapn(i + P.rAUX.s, P.rAUX.n), cA1 = wrapn(cA0 + 1, P.rAUX.n), cA2 = wrapn(cA1 + 1, P.rAUX.n);
@@ -422,7 +459,7 @@ __device__ void fast_u(const DevOps &P, const TV *__restrict__ u, const TV *__re
     }
   };
   auto face = [&](int r, const URaw<S> &q, S &uy, S &sy, S &vf) {
-    const int y = r - j0;
+    const int y = r - jy;
     uy = S(Y.auy0[y]) * q.f0 + S(Y.auy1[y]) * q.f1;
     sy = S(Y.suy0[y]) * q.f0 + S(Y.suy1[y]) * q.f1;
     vf = S(Y.ivy0[y]) * (iv0 * q.va0 + iv1 * q.va1) + S(Y.ivy1[y]) * (iv0 * q.vb0 + iv1 * q.vb1);
@@ -451,14 +488,14 @@ __device__ void fast_u(const DevOps &P, const TV *__restrict__ u, const TV *__re
     face(j + 1, cur, uy1, sy1, vf1);
     const S uxl = a00 * cur.um + a01 * cur.u0, uxr = a10 * cur.u0 + a11 * cur.up;
     const S sxl = s00 * cur.um + s01 * cur.u0, sxr = s10 * cur.u0 + s11 * cur.up;
-    const double hyd = Y.hy[j - j0];
+    const double hyd = Y.hy[j - jy];
     const S hy = S(hyd);
     const S du2dx = (hy * uxr) * uxr - (hy * uxl) * uxl;
     const S duvdy = vf1 * uy1 - vf0 * uy0;
     const S d2u = hy * (ire * sxr - ire * sxl) + gx * (ire * sy1 - ire * sy0);
     const double R = (double)(-(du2dx + duvdy) + d2u);
     const long long idx = (long long)j * Nux + i;
-    const double oi = Y.rhy[j - j0] * rgx;
+    const double oi = Y.rhy[j - jy] * rgx;
     if (e.mode == 0) {
       const double k = oi * R;
       if (e.kV) e.kV[idx] = k;
@@ -487,7 +524,7 @@ struct VRaw {
 
 template <typename S, typename TV>
 __device__ void fast_v(const DevOps &P, const TV *__restrict__ u, const TV *__restrict__ v, const Epi &e,
-                       int i, int j0, int j1, const YRows &Y) {
+                       int i, int j0, int j1, const YRows &Y, int jy) {
   const S ire = S(P.invRe);
   const int cV0 = wrapn(i + P.rAVX.s, P.rAVX.n), cV1 = wrapn(cV0 + 1, P.rAVX.n), cV2 = wrapn(cV1 + 1, P.rAVX.n);
   const int cU0 = wrapn(i + P.rIUX.s, P.rIUX.n), cU1 = wrapn(cU0 + 1, P.rIUX.n), cU2 = wrapn(cU1 + 1, P.rIUX.n);
@@ -509,7 +546,7 @@ __device__ void fast_v(const DevOps &P, const TV *__restrict__ u, const TV *__re
     q.f1 = twoVy ? S(__ldg(v + (long long)wrapn(ra + 1, P.rAVY.n) * Nvx + i)) : S(0);
   };
   auto face = [&](int r, const VRaw<S> &q, S &vy, S &sy) {
-    const int y = r - j0;
+    const int y = r - jy;
     vy = S(Y.avy0[y]) * q.f0 + S(Y.avy1[y]) * q.f1;
     sy = S(Y.svy0[y]) * q.f0 + S(Y.svy1[y]) * q.f1;
   };
@@ -553,15 +590,15 @@ __device__ void fast_v(const DevOps &P, const TV *__restrict__ u, const TV *__re
     // ubar at vx faces i, i+1: IUY row j times IUX rows i, i+1
     const S la = wu00 * cur.ua0 + wu01 * cur.ua1, ra = wu10 * cur.ua1 + wu11 * cur.ua2;
     const S lb = wu00 * cur.ub0 + wu01 * cur.ub1, rb = wu10 * cur.ub1 + wu11 * cur.ub2;
-    const S wy0 = S(Y.iuy0[j - j0]), wy1 = S(Y.iuy1[j - j0]);
+    const S wy0 = S(Y.iuy0[j - jy]), wy1 = S(Y.iuy1[j - jy]);
     const S ufl = wy0 * la + wy1 * lb, ufr = wy0 * ra + wy1 * rb;
     const S duvdx = ufr * vxr - ufl * vxl;
     const S dv2dy = (hx * vy1) * vy1 - (hx * vy0) * vy0;
-    const double gyd = Y.gyi[j - j0];
+    const double gyd = Y.gyi[j - jy];
     const S d2v = S(gyd) * (ire * svr - ire * svl) + hx * (ire * sy1 - ire * sy0);
     const double R = (double)(-(duvdx + dv2dy) + d2v);
     const long long idx = P.Nu + (long long)j * Nvx + i;
-    const double oi = Y.rgyi[j - j0] * rhx;
+    const double oi = Y.rgyi[j - jy] * rhx;
     if (e.mode == 0) {
       const double k = oi * R;
       if (e.kV) e.kV[idx] = k;
@@ -574,8 +611,8 @@ __device__ void fast_v(const DevOps &P, const TV *__restrict__ u, const TV *__re
     } else {
       // (G p)_v = -hx MYT p with the row's weights from shared memory
       const int c0 = wrapn(j + P.rMYT.s, P.rMYT.n);
-      double gy = Y.myt0[j - j0] * __ldg(e.p + (long long)c0 * P.Npx + i);
-      if (P.rMYT.two) gy += Y.myt1[j - j0] * __ldg(e.p + (long long)wrapn(c0 + 1, P.rMYT.n) * P.Npx + i);
+      double gy = Y.myt0[j - jy] * __ldg(e.p + (long long)c0 * P.Npx + i);
+      if (P.rMYT.two) gy += Y.myt1[j - jy] * __ldg(e.p + (long long)wrapn(c0 + 1, P.rMYT.n) * P.Npx + i);
       const double g = -hxd * gy;
       epi_residual(e, idx, oi, R, g);
     }
@@ -900,9 +937,9 @@ __device__ __forceinline__ void tile_fast(const DevOps &P, const TV *__restrict_
   stage_yrows(P, j0, Y, j1 - j0);
   __syncthreads();
   if (threadIdx.y == 0)
-    fast_u<S, TV>(P, u, v, e, i, j0, j1, Y);
+    fast_u<S, TV>(P, u, v, e, i, j0, j1, Y, j0);
   else
-    fast_v<S, TV>(P, u, v, e, i, j0, j1, Y);
+    fast_v<S, TV>(P, u, v, e, i, j0, j1, Y, j0);
 }
 template <typename S, typename TV>
 __device__ __forceinline__ void tile_generic(const DevOps &P, const TV *__restrict__ V, const Epi &e, int bx,
@@ -965,35 +1002,53 @@ __device__ __forceinline__ const double *ens_epi(const EnsMemberD &M, const EnsW
   return M.V;
 }
 
-template <typename S, bool FAST>
-__device__ __forceinline__ void walk_ens_body(const EnsMemberD *__restrict__ mem, const int4 *__restrict__ work,
-                                              const EnsWalk &w, int rows) {
+// Ensemble walkers.  Members are small, so most of their 64-column tiles touch
+// a boundary; a whole tile by the table walker costs several times the fast
+// walker (48 us a launch against 18 us for a fifth of the tiles, 24 members
+// of 64 to 256 cells per direction).  So the split is by point, not by tile:
+// the fast walkers take the points of each component inside its regular
+// rectangle, the table walkers the ring around it, one point per thread, in
+// the same launch.  Work items {member, tile column, tile row, run of rows}
+// and {member, first ring point, -1, 0}.  24-member step on B200: 0.989 ->
+// 0.881 ms.  (On single grids this split was slower than whole tiles: 64^2
+// cavity 0.107 against 0.096 ms, 2048^2 0.917 against 0.879 ms per step.)
+constexpr int kRingThreads = 2 * WX;
+template <typename S>
+__global__ void __launch_bounds__(WX * 2, 4) k_walk_ens(const EnsMemberD *__restrict__ mem,
+                                                        const int4 *__restrict__ work,
+                                                        const __grid_constant__ EnsWalk w, int rows) {
   __shared__ __align__(16) DevOps sP;
   __shared__ __align__(16) Epi sE;
   __shared__ const double *sV;
+  __shared__ YRows Y;
   const int4 it = work[blockIdx.x];
   const EnsMemberD &M = mem[it.x];
   copy_words(&sP, &M.P, (int)sizeof(DevOps));
   if (threadIdx.x == 0 && threadIdx.y == 0) sV = ens_epi(M, w, sE);
   __syncthreads();
-  if (FAST)
-    tile_fast<S, double>(sP, sV, sE, it.y, it.z, blockIdx.y, rows);
-  else
-    tile_generic<S, double>(sP, sV, sE, it.y, it.z, blockIdx.y, rows);
-}
-
-template <typename S>
-__global__ void __launch_bounds__(WX * 2, INS2D_WALK_MINB) k_walk_ens_fast(const EnsMemberD *__restrict__ mem,
-                                                                          const int4 *__restrict__ work,
-                                                                          const __grid_constant__ EnsWalk w,
-                                                                          int rows) {
-  walk_ens_body<S, true>(mem, work, w, rows);
-}
-template <typename S>
-__global__ void __launch_bounds__(WX * 2) k_walk_ens_gen(const EnsMemberD *__restrict__ mem,
-                                                         const int4 *__restrict__ work,
-                                                         const __grid_constant__ EnsWalk w, int rows) {
-  walk_ens_body<S, false>(mem, work, w, rows);
+  const DevOps &P = sP;
+  const double *u = sV, *v = sV + P.Nu;
+  if (it.z >= 0) {
+    const int i = it.y * WX + threadIdx.x, j0 = it.z * RUN + it.w * rows;
+    stage_yrows_cut(P, j0, Y, rows);
+    __syncthreads();
+    const WalkRect &R = threadIdx.y == 0 ? P.ru : P.rv;
+    const int ja = max(j0, R.y0), jb = min(j0 + rows, R.y1);
+    if (i < R.x0 || i >= R.x1 || ja >= jb) return;
+    if (threadIdx.y == 0)
+      fast_u<S, double>(P, u, v, sE, i, ja, jb, Y, j0);
+    else
+      fast_v<S, double>(P, u, v, sE, i, ja, jb, Y, j0);
+  } else {
+    int k = it.y + threadIdx.x + WX * threadIdx.y, i, j;
+    if (k < P.ru.ring()) {
+      P.ru.point(k, i, j);
+      walk_u<S, double>(P, u, v, sE, i, j, j + 1);
+    } else if ((k -= P.ru.ring()) < P.rv.ring()) {
+      P.rv.point(k, i, j);
+      walk_v<S, double>(P, u, v, sE, i, j, j + 1);
+    }
+  }
 }
 
 // MODE 0 and 2 with the count of earlier stages as a template argument (0..3
@@ -1084,9 +1139,43 @@ void launch_walk(const DevOps &P, const double *V, const float *V32, const Epi &
 // walkers on its device.
 cudaError_t walker_prepare() { return cudaSuccess; }
 
+namespace {
+// The rectangles of points whose stencils are regular rows without boundary
+// terms (an empty one: no such point)
+void walker_points(DevOps &P) {
+  auto cut = [](int &lo, int &hi, const RegD &r, int last) {  // rows k .. k + last of r
+    lo = lo > r.lo ? lo : r.lo;
+    hi = hi < r.hi - last ? hi : r.hi - last;
+  };
+  auto rect = [](int nx, int ny, int x0, int x1, int y0, int y1) {
+    WalkRect R{x0, x1, y0, y1, nx, ny};
+    if (x0 >= x1 || y0 >= y1) R.x0 = R.x1 = R.y0 = R.y1 = 0;
+    return R;
+  };
+  int x0 = 0, x1 = P.Nux, y0 = 0, y1 = P.Nuy;
+  cut(x0, x1, P.rAUX, 1);
+  cut(x0, x1, P.rIVX, 0);
+  cut(x0, x1, P.rMXT, 0);
+  cut(y0, y1, P.rAUY, 1);
+  cut(y0, y1, P.rIVY, 1);
+  P.ru = rect(P.Nux, P.Nuy, x0, x1, y0, y1);
+  x0 = y0 = 0;
+  x1 = P.Nvx;
+  y1 = P.Nvy;
+  cut(x0, x1, P.rAVX, 1);
+  cut(x0, x1, P.rIUX, 1);
+  cut(y0, y1, P.rAVY, 1);
+  cut(y0, y1, P.rIUY, 0);
+  cut(y0, y1, P.rMYT, 0);
+  P.rv = rect(P.Nvx, P.Nvy, x0, x1, y0, y1);
+}
+
+}  // namespace
+
 // The rectangle of tiles whose every column and row lies in the regular
 // ranges the fast walkers need (both walkers of a block must qualify).
 void walker_rectangle(DevOps &P) {
+  walker_points(P);
   auto in = [](const RegD &r, int a, int b) { return a >= r.lo && b < r.hi; };  // rows a..b inclusive
   const int nx = P.Nux > P.Nvx ? P.Nux : P.Nvx;
   const int ny = P.Nuy > P.Nvy ? P.Nuy : P.Nvy;
@@ -1125,32 +1214,38 @@ void walker_rectangle(DevOps &P) {
   P.fby1 = by1;
 }
 
-void walk_tiles(const DevOps &P, int member, std::vector<int4> &fast, std::vector<int4> &gen) {
-  const int nx = P.Nux > P.Nvx ? P.Nux : P.Nvx;
-  const int ny = P.Nuy > P.Nvy ? P.Nuy : P.Nvy;
-  const int nbx = (nx + WX - 1) / WX, nby = (ny + RUN - 1) / RUN;
-  for (int by = 0; by < nby; ++by)
-    for (int bx = 0; bx < nbx; ++bx) {
-      const bool f = bx >= P.fbx0 && bx < P.fbx1 && by >= P.fby0 && by < P.fby1;
-      (f ? fast : gen).push_back(make_int4(member, bx, by, 0));
-    }
+namespace {
+// tiles that cover both rectangles
+dim3 tile_grid(const DevOps &P) {
+  const int x1 = P.ru.x1 > P.rv.x1 ? P.ru.x1 : P.rv.x1, y1 = P.ru.y1 > P.rv.y1 ? P.ru.y1 : P.rv.y1;
+  return dim3((x1 + WX - 1) / WX, (y1 + RUN - 1) / RUN);
+}
+int ring_blocks(const DevOps &P) { return (P.ru.ring() + P.rv.ring() + kRingThreads - 1) / kRingThreads; }
+}  // namespace
+
+void ens_walk_work(const std::vector<const DevOps *> &P, std::vector<int4> &work, int &rows) {
+  long long tiles = 0;
+  for (const DevOps *p : P) {
+    const dim3 g = tile_grid(*p);
+    tiles += (long long)g.x * g.y;
+  }
+  rows = walk_rows(tiles);
+  for (int m = 0; m < (int)P.size(); ++m) {
+    const dim3 g = tile_grid(*P[m]);
+    for (int z = 0; z < RUN / rows; ++z)
+      for (int by = 0; by < (int)g.y; ++by)
+        for (int bx = 0; bx < (int)g.x; ++bx) work.push_back(make_int4(m, bx, by, z));
+    for (int b = 0; b < ring_blocks(*P[m]); ++b) work.push_back(make_int4(m, b * kRingThreads, -1, 0));
+  }
 }
 
-void launch_walk_ens(const EnsMemberD *mem, const int4 *fast, int nfast, const int4 *gen, int ngen, const EnsWalk &w,
-                     bool fp32, cudaStream_t s) {
-  const int rf = walk_rows(nfast), rg = walk_rows(ngen);
-  if (nfast > 0) {
-    if (fp32)
-      k_walk_ens_fast<float><<<dim3(nfast, RUN / rf), dim3(WX, 2), 0, s>>>(mem, fast, w, rf);
-    else
-      k_walk_ens_fast<double><<<dim3(nfast, RUN / rf), dim3(WX, 2), 0, s>>>(mem, fast, w, rf);
-  }
-  if (ngen > 0) {
-    if (fp32)
-      k_walk_ens_gen<float><<<dim3(ngen, RUN / rg), dim3(WX, 2), 0, s>>>(mem, gen, w, rg);
-    else
-      k_walk_ens_gen<double><<<dim3(ngen, RUN / rg), dim3(WX, 2), 0, s>>>(mem, gen, w, rg);
-  }
+void launch_walk_ens(const EnsMemberD *mem, const int4 *work, int n, int rows, const EnsWalk &w, bool fp32,
+                     cudaStream_t s) {
+  if (n <= 0) return;
+  if (fp32)
+    k_walk_ens<float><<<n, dim3(WX, 2), 0, s>>>(mem, work, w, rows);
+  else
+    k_walk_ens<double><<<n, dim3(WX, 2), 0, s>>>(mem, work, w, rows);
 }
 
 void launch_stage(const DevOps &P, const StageArgs &a, bool fp32, cudaStream_t s) {
