@@ -1335,10 +1335,9 @@ int ins2d_F(ins2d_ctx *ctx, const double *V, const double *C, const double *p, d
   const double *dP = nopressure ? nullptr : in_dev(ctx, p, ctx->stP, (size_t)ctx->P.Np, mem);
   double *dO = mem == INS2D_MEM_DEVICE ? F_out : ctx->stO;
   if (dP && dC == dV && !ctx->fp32) {
-    // the stencil walkers (the stage kernels' F) and a max|F| reduction
-    Prof pr(ctx, INS2D_PROF_OTHER, 2);
-    launch_F_walk(ctx->P, dV, dP, dO, ctx->stream);
-    launch_maxabs(dO, (long long)NV, ctx->red, ctx->stream);
+    // the stencil walkers (the stage kernels' F), which also take max|F|
+    Prof pr(ctx, INS2D_PROF_OTHER, 1);
+    CK(launch_F_walk(ctx->P, dV, dP, dO, ctx->red.result, ctx->stream));
   } else {
     // C != V (F.m's linearisation point), nopressure, or FP32-stencil
     // contexts (diagnostics stay FP64): one thread per point

@@ -179,32 +179,64 @@ __global__ void __launch_bounds__(256) k_lap(const __grid_constant__ DevOps P, c
   if (i < P.Npx && j < P.Npy) Ap[(long long)j * P.Npx + i] = lap(P, p, i, j);
 }
 
-// each thread takes kConsRows rows (BY apart) of one column, so the grid has
-// kConsRows times fewer blocks (and block partials to reduce)
-constexpr int kConsRows = 16;
+// {max|M V + yM|, sums of Omu u, Omv v, Omu u^2, Omv v^2}; a thread walks
+// `rows` consecutive rows of one column.  Blocks whose cells are all regular
+// two-point rows of Mx and My (no boundary terms, no wrap in y) take a loop
+// with running pointers and weights in registers: three field loads and about
+// 35 instructions per cell, several rows' loads in flight; the general loop
+// (120 instructions a cell, and dependent loads) was bound by issue and
+// latency.  Measured on B200, general loop everywhere with rows 8 apart: 54 us
+// at 2048^2, now 38 us; 18.5 us at 64^2, now 9.5 us (16 rows were one
+// thread's serial work; fewer while the launch has less than two blocks per SM).
 __global__ void __launch_bounds__(256) k_conservation(const __grid_constant__ DevOps P, const double *__restrict__ V,
-                                                     const RedScratch red) {
-  const int i = blockIdx.x * BX + threadIdx.x;
-  const int jb = blockIdx.y * (BY * kConsRows) + threadIdx.y;
+                                                     int rows, const RedScratch red) {
+  const int i0 = blockIdx.x * BX, i = i0 + threadIdx.x;
+  const int jb = blockIdx.y * BY * rows, j0 = jb + threadIdx.y * rows;
   const double *u = V, *v = V + P.Nu;
   double q[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
   const int ops[5] = {R_MAX, R_SUM, R_SUM, R_SUM, R_SUM};
+  const RegD &X = P.rMX, &Y = P.rMY;
+  const int ie = i0 + BX, je = jb + BY * rows;  // end of the block's cells
+  if (i0 >= X.lo && ie <= X.hi && jb >= Y.lo && je <= Y.hi && X.two && Y.two && (X.s == 0 || X.s == -1) &&
+      (Y.s == 0 || Y.s == -1) && jb + Y.s >= 0 && je + Y.s < Y.n && ie <= P.Nux && ie <= P.Nvx && je <= P.Nuy &&
+      je <= P.Nvy) {
+    const double w0 = __ldg(X.w0 + i), w1 = __ldg(X.w1 + i), hx = __ldg(P.hx + i), gx = __ldg(P.gxi + i);
+    const int c0 = wrapn(i + X.s, X.n), c1 = wrapn(c0 + 1, X.n);
+    const double *u0 = u + (long long)j0 * P.Nux + c0, *vp = v + (long long)(j0 + Y.s) * P.Nvx + i;
+    const int du = c1 - c0;
+    const double *hy = P.hy + j0, *gy = P.gyi + j0, *m0 = Y.w0 + j0, *m1 = Y.w1 + j0;
+    double va = __ldg(vp);
 #pragma unroll 4
-  for (int r = 0; r < kConsRows; ++r) {
-    const int j = jb + r * BY;
-    if (i < P.Npx && j < P.Npy)  // M V + yM; interior cells by their regular two-point rows
-      q[0] = fmax(q[0], fabs(div_cell_f(P, WPlain{V}, 1.0, 0.0, 1.0, i, j)));
-    if (i < P.Nux && j < P.Nuy) {
-      const double om = __ldg(P.hy + j) * __ldg(P.gxi + i);
-      const double x = u[(long long)j * P.Nux + i];
-      q[1] += om * x;
-      q[3] += om * x * x;
+    for (int r = 0; r < rows; ++r) {
+      vp += P.Nvx;
+      const double ua = __ldg(u0), ub = __ldg(u0 + du), vb = __ldg(vp);
+      u0 += P.Nux;
+      const double h = __ldg(hy + r);
+      q[0] = fmax(q[0], fabs(h * (w0 * ua + w1 * ub) + hx * (__ldg(m0 + r) * va + __ldg(m1 + r) * vb)));
+      const double x = X.s == 0 ? ua : ub, y = Y.s == 0 ? va : vb;
+      const double ou = h * gx, ov = __ldg(gy + r) * hx;
+      q[1] += ou * x;
+      q[3] += ou * x * x;
+      q[2] += ov * y;
+      q[4] += ov * y * y;
+      va = vb;
     }
-    if (i < P.Nvx && j < P.Nvy) {
-      const double om = __ldg(P.gyi + j) * __ldg(P.hx + i);
-      const double x = v[(long long)j * P.Nvx + i];
-      q[2] += om * x;
-      q[4] += om * x * x;
+  } else {
+    for (int r = 0; r < rows; ++r) {
+      const int j = j0 + r;
+      if (i < P.Npx && j < P.Npy) q[0] = fmax(q[0], fabs(div_cell_f(P, WPlain{V}, 1.0, 0.0, 1.0, i, j)));
+      if (i < P.Nux && j < P.Nuy) {
+        const double om = __ldg(P.hy + j) * __ldg(P.gxi + i);
+        const double x = __ldg(u + (long long)j * P.Nux + i);
+        q[1] += om * x;
+        q[3] += om * x * x;
+      }
+      if (i < P.Nvx && j < P.Nvy) {
+        const double om = __ldg(P.gyi + j) * __ldg(P.hx + i);
+        const double x = __ldg(v + (long long)j * P.Nvx + i);
+        q[2] += om * x;
+        q[4] += om * x * x;
+      }
     }
   }
   grid_reduce<5>(q, ops, red);
@@ -272,38 +304,6 @@ __global__ void __launch_bounds__(256) k_stage_cached_ens(const EnsMemberD *__re
 
 }  // namespace
 
-namespace {
-// VEC: x is 16-byte aligned and read two values at a time
-template <bool VEC>
-__global__ void __launch_bounds__(256) k_maxabs(const double *__restrict__ x, long long n, const RedScratch red) {
-  double m[1] = {0.0};
-  const int ops[1] = {R_MAX};
-  constexpr int W = VEC ? 2 : 1;
-  const long long stride = (long long)gridDim.x * blockDim.x * W;
-  for (long long k = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * W; k < n; k += stride) {
-    if (VEC && k + 1 < n) {
-      const double2 v = __ldg(reinterpret_cast<const double2 *>(x + k));
-      m[0] = fmax(m[0], fmax(fabs(v.x), fabs(v.y)));
-    } else {
-      m[0] = fmax(m[0], fabs(__ldg(x + k)));
-    }
-  }
-  grid_reduce<1>(m, ops, red);
-}
-}  // namespace
-
-void launch_maxabs(const double *x, long long n, const RedScratch &red, cudaStream_t s) {
-  const bool vec = ((uintptr_t)x & 15) == 0;
-  long long b = ((vec ? n / 2 : n) + 255) / 256;
-  if (b > 148LL * 8) b = 148LL * 8;
-  if (b > red.max_blocks) b = red.max_blocks;
-  if (b < 1) b = 1;
-  if (vec)
-    k_maxabs<true><<<(unsigned)b, 256, 0, s>>>(x, n, red);
-  else
-    k_maxabs<false><<<(unsigned)b, 256, 0, s>>>(x, n, red);
-}
-
 void launch_F(const DevOps &P, const double *V, const double *C, const double *p, double *F_out,
               const RedScratch &red, cudaStream_t s) {
   dim3 g = grid_for(P.Nux > P.Nvx ? P.Nux : P.Nvx, P.Nuy > P.Nvy ? P.Nuy : P.Nvy);
@@ -368,10 +368,11 @@ void launch_lap(const DevOps &P, const double *p, double *Ap, cudaStream_t s) {
 }
 
 void launch_conservation(const DevOps &P, const double *V, const RedScratch &red, cudaStream_t s) {
-  int nx = P.Nux > P.Nvx ? P.Nux : P.Nvx;
-  int ny = P.Nuy > P.Nvy ? P.Nuy : P.Nvy;
-  const dim3 g((nx + BX - 1) / BX, (ny + BY * kConsRows - 1) / (BY * kConsRows));
-  k_conservation<<<g, dim3(BX, BY), 0, s>>>(P, V, red);
+  const int nx = P.Nux > P.Nvx ? P.Nux : P.Nvx, ny = P.Nuy > P.Nvy ? P.Nuy : P.Nvy;
+  int rows = 16;
+  auto grid = [&](int r) { return dim3((nx + BX - 1) / BX, (ny + BY * r - 1) / (BY * r)); };
+  while (rows > 1 && (long long)grid(rows).x * grid(rows).y < 2LL * P.nsm) rows >>= 1;
+  k_conservation<<<grid(rows), dim3(BX, BY), 0, s>>>(P, V, rows, red);
 }
 
 void launch_stage_cached(const double *kV0, const double *Vn, double aii, double inv_dt, double *Wt, long long n,

@@ -111,10 +111,10 @@ cudaError_t walker_prepare();
 void launch_residual(const DevOps &P, const double *V, const double *p, double *w, double *kV_next,
                      float *kV_next32, bool fp32, cudaStream_t s);
 // F_out = -conv(V) + Diff V + yDiff - (G p + y_p) (F.m:137-145 with C = V and
-// the pressure) by the stencil walkers, FP64 fields and arithmetic
-void launch_F_walk(const DevOps &P, const double *V, const double *p, double *F_out, cudaStream_t s);
-// red.result[0] = max |x| over n values (deterministic)
-void launch_maxabs(const double *x, long long n, const RedScratch &red, cudaStream_t s);
+// the pressure) by the stencil walkers, FP64 fields and arithmetic; max|F| into
+// *maxres (zeroed on the stream first; a maximum, so its order is immaterial)
+cudaError_t launch_F_walk(const DevOps &P, const double *V, const double *p, double *F_out, double *maxres,
+                          cudaStream_t s);
 // F_out = -conv(V;C) + Diff V + yDiff - (G p + y_p) (F.m); maxres into red.result[0]
 void launch_F(const DevOps &P, const double *V, const double *C, const double *p, double *F_out,
               const RedScratch &red, cudaStream_t s);

@@ -132,7 +132,17 @@ struct Epi {
   double *w;
   double *kV_next;
   float *kV_next32;
+  // F: max|F| as the bits of a non-negative double
+  unsigned long long *fmax;
 };
+
+// mode 3: max|F| of the block's points into *e.fmax (every thread calls it; m:
+// its own points' maximum, 0 for none)
+__device__ __forceinline__ void block_fmax(const Epi &e, double m) {
+  for (int off = 16; off > 0; off >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, off));
+  if (((threadIdx.x + blockDim.x * threadIdx.y) & 31) == 0 && m > 0.0)
+    atomicMax(e.fmax, (unsigned long long)__double_as_longlong(m));
+}
 
 // NP >= 0: that many earlier stages, unrolled; NP < 0: e.nprev
 template <int NP = -1>
@@ -165,9 +175,10 @@ __device__ __forceinline__ void epilogue_stage(const Epi &e, long long idx, doub
   e.Wt[idx] = e.Vn[idx] * e.inv_dt + vt;
 }
 
-__device__ __forceinline__ void epi_residual(const Epi &e, long long idx, double oi, double R, double g) {
+__device__ __forceinline__ void epi_residual(const Epi &e, long long idx, double oi, double R, double g, double &fm) {
   if (e.mode == 3) {  // F (F.m): the momentum right-hand side with the pressure gradient
     e.w[idx] = R - g;
+    fm = fmax(fm, fabs(R - g));
     return;
   }
   e.w[idx] = oi * (R - g);
@@ -179,7 +190,7 @@ __device__ __forceinline__ void epi_residual(const Epi &e, long long idx, double
 // u walker
 template <typename S, typename TV>
 __device__ void walk_u(const DevOps &P, const TV *__restrict__ u, const TV *__restrict__ v, const Epi &e,
-                       int i, int j0, int j1) {
+                       int i, int j0, int j1, double &fm) {
   if (i >= P.Nux) return;
   j1 = min(j1, P.Nuy);
   if (j0 >= j1) return;
@@ -238,7 +249,7 @@ __device__ void walk_u(const DevOps &P, const TV *__restrict__ u, const TV *__re
       const double *prow = e.p + (long long)j * P.Npx;
       const double g = -hyd * (gt.w0 * __ldg(prow + gt.c0) + gt.w1 * __ldg(prow + gt.c1) +
                                (gt.w2 != 0.0 ? gt.w2 * __ldg(prow + gt.c2) : 0.0));
-      epi_residual(e, idx, oi, R, g);
+      epi_residual(e, idx, oi, R, g, fm);
     }
     uy0 = uy1;
     sy0 = sy1;
@@ -250,7 +261,7 @@ __device__ void walk_u(const DevOps &P, const TV *__restrict__ u, const TV *__re
 // v walker
 template <typename S, typename TV>
 __device__ void walk_v(const DevOps &P, const TV *__restrict__ u, const TV *__restrict__ v, const Epi &e,
-                       int i, int j0, int j1) {
+                       int i, int j0, int j1, double &fm) {
   if (i >= P.Nvx) return;
   j1 = min(j1, P.Nvy);
   if (j0 >= j1) return;
@@ -320,7 +331,7 @@ __device__ void walk_v(const DevOps &P, const TV *__restrict__ u, const TV *__re
       const double g = -__ldg(P.hx + i) *
                        (gy.w0 * __ldg(e.p + (long long)gy.c0 * P.Npx + i) + gy.w1 * __ldg(e.p + (long long)gy.c1 * P.Npx + i) +
                         (gy.w2 != 0.0 ? gy.w2 * __ldg(e.p + (long long)gy.c2 * P.Npx + i) : 0.0));
-      epi_residual(e, idx, oi, R, g);
+      epi_residual(e, idx, oi, R, g, fm);
     }
     vy0 = vy1;
     sy0 = sy1;
@@ -426,7 +437,7 @@ struct URaw {
 
 template <typename S, typename TV>
 __device__ void fast_u(const DevOps &P, const TV *__restrict__ u, const TV *__restrict__ v, const Epi &e,
-                       int i, int j0, int j1, const YRows &Y, int jy) {
+                       int i, int j0, int j1, const YRows &Y, int jy, double &fm) {
   const S ire = S(P.invRe);
   // columns (modulo the row length for periodic wraps)
   const int cA0 = wrapn(i + P.rAUX.s, P.rAUX.n), cA1 = wrapn(cA0 + 1, P.rAUX.n), cA2 = wrapn(cA1 + 1, P.rAUX.n);
@@ -507,7 +518,7 @@ __device__ void fast_u(const DevOps &P, const TV *__restrict__ u, const TV *__re
       epi_stage32(e, idx, oi * R);
     } else {
       const double g = -hyd * reg_x(P.rMXT, i, e.p, (long long)j * P.Npx);
-      epi_residual(e, idx, oi, R, g);
+      epi_residual(e, idx, oi, R, g, fm);
     }
     uy0 = uy1;
     sy0 = sy1;
@@ -524,7 +535,7 @@ struct VRaw {
 
 template <typename S, typename TV>
 __device__ void fast_v(const DevOps &P, const TV *__restrict__ u, const TV *__restrict__ v, const Epi &e,
-                       int i, int j0, int j1, const YRows &Y, int jy) {
+                       int i, int j0, int j1, const YRows &Y, int jy, double &fm) {
   const S ire = S(P.invRe);
   const int cV0 = wrapn(i + P.rAVX.s, P.rAVX.n), cV1 = wrapn(cV0 + 1, P.rAVX.n), cV2 = wrapn(cV1 + 1, P.rAVX.n);
   const int cU0 = wrapn(i + P.rIUX.s, P.rIUX.n), cU1 = wrapn(cU0 + 1, P.rIUX.n), cU2 = wrapn(cU1 + 1, P.rIUX.n);
@@ -614,7 +625,7 @@ __device__ void fast_v(const DevOps &P, const TV *__restrict__ u, const TV *__re
       double gy = Y.myt0[j - jy] * __ldg(e.p + (long long)c0 * P.Npx + i);
       if (P.rMYT.two) gy += Y.myt1[j - jy] * __ldg(e.p + (long long)wrapn(c0 + 1, P.rMYT.n) * P.Npx + i);
       const double g = -hxd * gy;
-      epi_residual(e, idx, oi, R, g);
+      epi_residual(e, idx, oi, R, g, fm);
     }
     vy0 = vy1;
     sy0 = sy1;
@@ -710,7 +721,7 @@ __device__ __forceinline__ void stage_store(const Epi &e, long long idx, double 
 // MODE 0: FP64-storage stage, 1: residual, 2: FP32-storage stage
 template <typename S, int MODE, typename TV, int NP>
 __device__ void tile_u(const DevOps &P, const TileSm<TV> &T, const Epi &e, int i, int i0, int j0, int ja, int jb,
-                       const YRowsN<RUN> &Y) {
+                       const YRowsN<RUN> &Y, double &fm) {
   const S ire = S(P.invRe);
   const int ci = i - i0 + TileGeo<TV>::HL;  // shared-memory column of u(i, .)
   const int cA0 = ci + P.rAUX.s, cA1 = cA0 + 1, cA2 = cA1 + 1;
@@ -783,7 +794,7 @@ __device__ void tile_u(const DevOps &P, const TileSm<TV> &T, const Epi &e, int i
     } else {
       double gp = gw0 * cur.a;
       if (twoG) gp += gw1 * cur.b;
-      epi_residual(e, idx, oi, R, -hyd * gp);
+      epi_residual(e, idx, oi, R, -hyd * gp, fm);
     }
     uy0 = uy1;
     sy0 = sy1;
@@ -793,7 +804,7 @@ __device__ void tile_u(const DevOps &P, const TileSm<TV> &T, const Epi &e, int i
 
 template <typename S, int MODE, typename TV, int NP>
 __device__ void tile_v(const DevOps &P, const TileSm<TV> &T, const Epi &e, int i, int i0, int j0, int ja, int jb,
-                       const YRowsN<RUN> &Y) {
+                       const YRowsN<RUN> &Y, double &fm) {
   const S ire = S(P.invRe);
   const int ci = i - i0 + TileGeo<TV>::HL;
   const int cV0 = ci + P.rAVX.s, cV1 = cV0 + 1, cV2 = cV1 + 1;
@@ -868,7 +879,7 @@ __device__ void tile_v(const DevOps &P, const TileSm<TV> &T, const Epi &e, int i
     } else {
       double gy = Y.myt0[j - j0] * cur.a;
       if (twoG) gy += Y.myt1[j - j0] * cur.b;
-      epi_residual(e, idx, oi, R, -hxd * gy);
+      epi_residual(e, idx, oi, R, -hxd * gy, fm);
     }
     vy0 = vy1;
     sy0 = sy1;
@@ -919,10 +930,12 @@ __global__ void __launch_bounds__(kTileThreads, INS2D_TILE_MINB)
   const int i = i0 + threadIdx.x;
   const int seg = threadIdx.y & 1;
   const int ja = j0 + seg * kTileSeg, jb = ja + kTileSeg;
+  double fm = 0.0;
   if (threadIdx.y < 2)
-    tile_u<S, MODE, TV, NP>(P, T, e, i, i0, j0, ja, jb, Y);
+    tile_u<S, MODE, TV, NP>(P, T, e, i, i0, j0, ja, jb, Y, fm);
   else
-    tile_v<S, MODE, TV, NP>(P, T, e, i, i0, j0, ja, jb, Y);
+    tile_v<S, MODE, TV, NP>(P, T, e, i, i0, j0, ja, jb, Y, fm);
+  if (MODE == 1 && e.mode == 3) block_fmax(e, fm);
 }
 
 // rows [z rows, (z + 1) rows) of one WX x RUN tile (bx, by): u walkers in
@@ -936,10 +949,12 @@ __device__ __forceinline__ void tile_fast(const DevOps &P, const TV *__restrict_
   const TV *u = V, *v = V + P.Nu;
   stage_yrows(P, j0, Y, j1 - j0);
   __syncthreads();
+  double fm = 0.0;
   if (threadIdx.y == 0)
-    fast_u<S, TV>(P, u, v, e, i, j0, j1, Y, j0);
+    fast_u<S, TV>(P, u, v, e, i, j0, j1, Y, j0, fm);
   else
-    fast_v<S, TV>(P, u, v, e, i, j0, j1, Y, j0);
+    fast_v<S, TV>(P, u, v, e, i, j0, j1, Y, j0, fm);
+  if (e.mode == 3) block_fmax(e, fm);
 }
 template <typename S, typename TV>
 __device__ __forceinline__ void tile_generic(const DevOps &P, const TV *__restrict__ V, const Epi &e, int bx,
@@ -947,10 +962,12 @@ __device__ __forceinline__ void tile_generic(const DevOps &P, const TV *__restri
   const int i = bx * WX + threadIdx.x;
   const int j0 = by * RUN + z * rows, j1 = min(j0 + rows, (by + 1) * RUN);
   const TV *u = V, *v = V + P.Nu;
+  double fm = 0.0;
   if (threadIdx.y == 0)
-    walk_u<S, TV>(P, u, v, e, i, j0, j1);
+    walk_u<S, TV>(P, u, v, e, i, j0, j1, fm);
   else
-    walk_v<S, TV>(P, u, v, e, i, j0, j1);
+    walk_v<S, TV>(P, u, v, e, i, j0, j1, fm);
+  if (e.mode == 3) block_fmax(e, fm);
 }
 
 template <typename S, typename TV>
@@ -1028,6 +1045,7 @@ __global__ void __launch_bounds__(WX * 2, 4) k_walk_ens(const EnsMemberD *__rest
   __syncthreads();
   const DevOps &P = sP;
   const double *u = sV, *v = sV + P.Nu;
+  double fm = 0.0;  // F only (not an ensemble's mode)
   if (it.z >= 0) {
     const int i = it.y * WX + threadIdx.x, j0 = it.z * RUN + it.w * rows;
     stage_yrows_cut(P, j0, Y, rows);
@@ -1036,17 +1054,17 @@ __global__ void __launch_bounds__(WX * 2, 4) k_walk_ens(const EnsMemberD *__rest
     const int ja = max(j0, R.y0), jb = min(j0 + rows, R.y1);
     if (i < R.x0 || i >= R.x1 || ja >= jb) return;
     if (threadIdx.y == 0)
-      fast_u<S, double>(P, u, v, sE, i, ja, jb, Y, j0);
+      fast_u<S, double>(P, u, v, sE, i, ja, jb, Y, j0, fm);
     else
-      fast_v<S, double>(P, u, v, sE, i, ja, jb, Y, j0);
+      fast_v<S, double>(P, u, v, sE, i, ja, jb, Y, j0, fm);
   } else {
     int k = it.y + threadIdx.x + WX * threadIdx.y, i, j;
     if (k < P.ru.ring()) {
       P.ru.point(k, i, j);
-      walk_u<S, double>(P, u, v, sE, i, j, j + 1);
+      walk_u<S, double>(P, u, v, sE, i, j, j + 1, fm);
     } else if ((k -= P.ru.ring()) < P.rv.ring()) {
       P.rv.point(k, i, j);
-      walk_v<S, double>(P, u, v, sE, i, j, j + 1);
+      walk_v<S, double>(P, u, v, sE, i, j, j + 1, fm);
     }
   }
 }
@@ -1267,12 +1285,17 @@ void launch_stage(const DevOps &P, const StageArgs &a, bool fp32, cudaStream_t s
   launch_walk(P, a.V, a.V32, e, fp32, s);
 }
 
-void launch_F_walk(const DevOps &P, const double *V, const double *p, double *F_out, cudaStream_t s) {
+cudaError_t launch_F_walk(const DevOps &P, const double *V, const double *p, double *F_out, double *maxres,
+                          cudaStream_t s) {
+  const cudaError_t ms = cudaMemsetAsync(maxres, 0, sizeof(double), s);
+  if (ms != cudaSuccess) return ms;
   Epi e{};
   e.mode = 3;
   e.p = p;
   e.w = F_out;
+  e.fmax = reinterpret_cast<unsigned long long *>(maxres);
   launch_walk(P, V, nullptr, e, false, s);
+  return cudaSuccess;
 }
 
 void launch_residual(const DevOps &P, const double *V, const double *p, double *w, double *kV_next,
