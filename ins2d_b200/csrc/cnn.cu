@@ -20,14 +20,15 @@
 //   forward        Z[p][co]   = sum_{t,ci} W[co][t][ci] A[p+t][ci]    M = pixels, N = 32, K = 288
 //   backward-data  dA[p][ci]  = sum_{t,co} W[co][8-t][ci] dZ[p+t][co] (the same kernel, transposed weights)
 //   weight grad    dW[co][t,ci] = sum_p dZ[p][co] A[p+t][ci]          M = 32, N = 288, K = pixels
-// The first two run on tcgen05.mma with TMEM accumulators (k_conv_mid_tc,
-// the default) or on mma.sync m16n8k16 (k_conv_mid); the weight gradient on
-// mma.sync (k_wgrad_mid).  The 1 -> 32 and 32 -> 1 layers (2 x 288 MACs per
-// pixel), the losses (squared error; the residual loss with the context's
-// operator tables), the solver's odd-part application and Adam are FP32 /
-// FP64 CUDA-core kernels.  Per pixel and 32 -> 32 layer the traffic is one
-// read of the input activations and one write of the output (64 bytes each
-// in BF16).
+// The default path runs on tcgen05.mma with TMEM accumulators: the first two by
+// k_conv_row_tc (k_conv_mid_tc on narrow fields), the weight gradient by
+// k_wgrad_tc.  The other path runs on mma.sync m16n8k16 (k_conv_mid,
+// k_wgrad_mid).  The 1 -> 32 and 32 -> 1 layers (2 x 288 MACs per pixel), the
+// losses (squared error; the residual loss with the context's operator tables),
+// the solver's odd-part application and Adam are FP32 / FP64 CUDA-core kernels.
+// Per pixel and 32 -> 32 layer the traffic is one read of the input activations
+// and one write of the output (64 bytes each in BF16).
+#include <cuda.h>
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -300,6 +301,44 @@ __global__ void __launch_bounds__(kEThreads, kEBlocksPerSm)
 // 32 input channels in 18 steps of 16.  The halo tile and the weights sit in
 // shared memory with padded strides so that the 32-bit fragment loads of a
 // warp hit 32 different banks.
+// 32 bytes to and from global memory in one instruction
+__device__ __forceinline__ void ldg32(const void *p, uint32_t (&r)[8]) {
+  asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "l"(p)
+               : "memory");
+}
+__device__ __forceinline__ void stg32(void *p, const uint32_t (&r)[8]) {
+  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n" ::"l"(p), "r"(r[0]), "r"(r[1]), "r"(r[2]),
+               "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
+}
+// 32 accumulators of a pixel -> BF16: ReLU, or the mask of the layer's
+// activation.  A lane holds a whole pixel (64 bytes): 16-byte stores write each
+// sector in two halves, 32-byte ones (pixels are 64-byte aligned) 8 us a layer
+// faster for 4 fields of 512^2.
+template <int MODE>
+__device__ __forceinline__ void store_mid(const uint32_t (&r)[2][16], const uint32_t (&mk)[2][8], bf16 *out) {
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    uint32_t o[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      float v0 = __uint_as_float(r[q][2 * j]), v1 = __uint_as_float(r[q][2 * j + 1]);
+      if (MODE == 0) {
+        v0 = fmaxf(v0, 0.0f);
+        v1 = fmaxf(v1, 0.0f);
+      } else {
+        const __nv_bfloat162 m = *reinterpret_cast<const __nv_bfloat162 *>(&mk[q][j]);
+        if (!(__low2float(m) > 0.0f)) v0 = 0.0f;
+        if (!(__high2float(m) > 0.0f)) v1 = 0.0f;
+      }
+      o[j] = pack2(v0, v1);
+    }
+    stg32(out + 16 * q, o);
+  }
+}
+
 // MODE 0: out = bf16(ReLU(Z)).  MODE 1 (backward-data): out = bf16(Z * [mask > 0]).
 template <int MODE>
 __global__ void __launch_bounds__(256) k_conv_mid(const bf16 *__restrict__ in, const bf16 *__restrict__ wt,
@@ -390,13 +429,13 @@ __global__ void __launch_bounds__(256) k_conv_mid(const bf16 *__restrict__ in, c
 // planes fall on distinct banks.  The weights (B: 32 x 288; core matrices of 8
 // output channels, next 8 input channels kBLbo bytes further) are loaded once
 // per block.
-// What bounds it: with N = 32 an MMA reads 4 KB of A for 65536 multiply-adds,
-// which takes the tensor core 64 cycles (counted; 16 at its full rate): 33 us
-// for 4 fields of 512^2, against 20 us for the 128 bytes per pixel of memory
-// traffic.  There on B200: all 256 threads of a block loading, waiting and
-// storing in turn, five blocks per SM, 65 us (72 us with the mask; half the
-// issue slots went to polling and per-chunk index arithmetic); this form 51
-// and 55 us.
+// What bounds it: with N = 32 an MMA reads 5 KB of operands for 131072
+// multiply-adds, 40 cycles of shared memory against 32 of arithmetic: 22 us for
+// 4 fields of 512^2, beside 20 us for the 128 bytes per pixel of memory traffic
+// and the producers' copies and fences (about 1300 cycles a tile row of warps).
+// There on B200: all 256 threads of a block loading, waiting and storing in
+// turn, five blocks per SM, 65 us (72 us with the mask); this form 41 and 46
+// us.  Fields wide enough go by rows instead (k_conv_row_tc, 27.5 and 33 us).
 constexpr int kTcM = 128;
 constexpr int kTcT = 16;                        // tile: 16 x 16 pixels
 constexpr int kTcH = kTcT + 2;
@@ -431,11 +470,15 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
   return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
          ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
 }
-__device__ __forceinline__ void tc_mma(uint32_t tmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
+// an MMA from its descriptors' halves: the offsets of an unrolled sequence stay
+// immediate 32-bit additions for the one thread that issues it
+constexpr uint64_t kSwizzle64 = 4ull << 61;  // layout type, with 8 rows of 64 bytes as the core matrix
+__device__ __forceinline__ void tc_mma_lo(uint32_t tmem, uint32_t alo, uint32_t ahi, uint32_t blo, uint32_t bhi,
+                                          uint32_t idesc, uint32_t acc) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem),
-      "l"(a), "l"(b), "r"(idesc), "r"(acc)
+      "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\tmov.b64 a, {%1, %2};\n\tmov.b64 b, {%3, %4};\n\t"
+      "setp.ne.b32 p, %6, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %5, p;\n\t}\n" ::"r"(tmem),
+      "r"(alo), "r"(ahi), "r"(blo), "r"(bhi), "r"(idesc), "r"(acc)
       : "memory");
 }
 // 16-byte asynchronous copy global -> shared; src_bytes = 0 writes zeros
@@ -460,8 +503,33 @@ __device__ __forceinline__ bool mbar_wait(uint32_t addr, uint32_t parity) {
 __device__ __forceinline__ void mbar_arrive(uint32_t addr) {
   asm volatile("{\n\t.reg .b64 s;\n\tmbarrier.arrive.shared::cta.b64 s, [%0];\n\t}\n" ::"r"(addr) : "memory");
 }
+// one arrival for a converged warp, after all its lanes' work (an arrival per
+// lane is a serial chain of shared-memory updates)
+__device__ __forceinline__ void mbar_arrive_warp(uint32_t addr) {
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) mbar_arrive(addr);
+}
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar) : "memory");
+}
+// one lane of a converged warp
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(p));
+  return p != 0;
+}
+// a box of the activations (act_map) into shared memory from pixel x, row y of
+// field b on; completes on bar (bytes announced by tma_expect)
+__device__ __forceinline__ void tma_box(uint32_t dst, const CUtensorMap *map, int x, int y, int b, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
+      "[%6];\n" ::"r"(dst),
+      "l"(map), "r"(0), "r"(x), "r"(y), "r"(b), "r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ void tma_expect(uint32_t bar, uint32_t bytes) {
+  asm volatile("{\n\t.reg .b64 s;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 s, [%0], %1;\n\t}\n" ::"r"(bar), "r"(bytes)
+               : "memory");
 }
 // 16 accumulator columns of this warp's 32 lanes
 __device__ __forceinline__ void tmem_ld16(uint32_t addr, uint32_t (&r)[16]) {
@@ -499,8 +567,8 @@ __global__ void __launch_bounds__(kTcThreads, kTcBlocksPerSm)
   }
   if (tid == 0) {
     for (int k = 0; k < kTcBars; ++k) {
-      // full: the producers; empty and tfull: one commit; tempty: the epilogue threads
-      const int count = k < kTcStages ? kTcProd : (k < 2 * kTcStages + 2 ? 1 : kTcEpi);
+      // full: the producer warps; empty and tfull: one commit; tempty: the epilogue warps
+      const int count = k < kTcStages ? kTcProd / 32 : (k < 2 * kTcStages + 2 ? 1 : kTcEpi / 32);
       asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bars + 8 * k), "r"(count) : "memory");
     }
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -524,10 +592,10 @@ __global__ void __launch_bounds__(kTcThreads, kTcBlocksPerSm)
       const int gx = (rem % tiles_x) * kTcT + px, gy = (rem / tiles_x) * kTcT + py;
       const bool in_f = gx < W && gy < H;
       const long long pix = (long long)b * H * W + (long long)gy * W + gx;
-      uint4 mk[4];
+      uint32_t mk[2][8];
       if (MODE == 1 && in_f)
 #pragma unroll
-        for (int q = 0; q < 4; ++q) mk[q] = __ldg(reinterpret_cast<const uint4 *>(mask + pix * kC) + q);
+        for (int q = 0; q < 2; ++q) ldg32(mask + pix * kC + 16 * q, mk[q]);
       ok = __all_sync(0xffffffffu, mbar_wait(tfull + 8 * acc, (it >> 1) & 1));  // the warp stays converged
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
@@ -537,26 +605,8 @@ __global__ void __launch_bounds__(kTcThreads, kTcBlocksPerSm)
       tmem_ld16(ta + 16, r[1]);
       asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-      mbar_arrive(tempty + 8 * acc);
-      if (!in_f) continue;
-      uint4 *dst = reinterpret_cast<uint4 *>(out + pix * kC);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        float v[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(r[q >> 1][8 * (q & 1) + j]);
-        if (MODE == 0) {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) v[j] = fmaxf(v[j], 0.0f);
-        } else {
-          float mv[8];
-          unpack8(mk[q], mv);
-#pragma unroll
-          for (int j = 0; j < 8; ++j)
-            if (!(mv[j] > 0.0f)) v[j] = 0.0f;
-        }
-        dst[q] = make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7]));
-      }
+      mbar_arrive_warp(tempty + 8 * acc);
+      if (in_f) store_mid<MODE>(r, mk, out + pix * kC);
     }
   } else if (tid < kTcEpi + kTcProd) {
     // chunk j of this thread: plane c8 of halo pixel hp0 + 32 j
@@ -571,11 +621,11 @@ __global__ void __launch_bounds__(kTcThreads, kTcBlocksPerSm)
     int it = 0;
     auto publish = [&](int k) {  // tile k's copies by this thread are complete
       asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-      mbar_arrive(full + 8 * (k % kTcStages));
+      mbar_arrive_warp(full + 8 * (k % kTcStages));
     };
     for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++it) {
       const int st = it % kTcStages;
-      if (!(ok = mbar_wait(empty + 8 * st, ((it / kTcStages) & 1) ^ 1))) break;
+      if (!(ok = __all_sync(0xffffffffu, mbar_wait(empty + 8 * st, ((it / kTcStages) & 1) ^ 1)))) break;
       const int b = (int)(tile / per_field), rem = (int)(tile % per_field);
       const int hx0 = (rem % tiles_x) * kTcT - 1, hy0 = (rem / tiles_x) * kTcT - 1;
       const bf16 *src = in + ((long long)b * H * W + (long long)hy0 * W + hx0) * kC + 8 * c8;
@@ -601,6 +651,8 @@ __global__ void __launch_bounds__(kTcThreads, kTcBlocksPerSm)
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     if (ok && it > 0) publish(it - 1);
   } else if (lane == 0) {
+    const uint64_t a0 = smem_desc(aBase, kTcLbo, kTcSbo), b0 = smem_desc(bBase, kBLbo, 128);
+    const uint32_t alo = (uint32_t)a0, ahi = (uint32_t)(a0 >> 32), blo = (uint32_t)b0, bhi = (uint32_t)(b0 >> 32);
     int it = 0;
     for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++it) {
       const int st = it % kTcStages, acc = it & 1;
@@ -612,9 +664,9 @@ __global__ void __launch_bounds__(kTcThreads, kTcBlocksPerSm)
 #pragma unroll
         for (int ks = 0; ks < kK / 16; ++ks) {
           const int t = ks >> 1, h = ks & 1;
-          const uint32_t a0 = aBase + st * kABytes + 2 * h * kTcLbo + ((t / 3) * kTcH + t % 3 + 8 * half) * 16;
-          tc_mma(taddr + 2 * kC * acc + kC * half, smem_desc(a0, kTcLbo, kTcSbo),
-                 smem_desc(bBase + 2 * ks * kBLbo, kBLbo, 128), kIdesc, ks > 0 ? 1u : 0u);
+          tc_mma_lo(taddr + 2 * kC * acc + kC * half,
+                    alo + st * (kABytes / 16) + 2 * h * (kTcLbo / 16) + (t / 3) * kTcH + t % 3 + 8 * half, ahi,
+                    blo + 2 * ks * (kBLbo / 16), bhi, kIdesc, ks > 0 ? 1u : 0u);
         }
       tc_commit(empty + 8 * st);
       tc_commit(tfull + 8 * acc);
@@ -627,6 +679,217 @@ __global__ void __launch_bounds__(kTcThreads, kTcBlocksPerSm)
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
   if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(taddr), "r"(kTcTmemCols) : "memory");
+}
+
+// --- 32 -> 32, 128 pixels of a row per MMA ------------------------------------------
+// The tile kernel above spends an MMA on every tap; here one MMA does three.
+// A is 128 consecutive pixels of one input row as a TMA copy leaves them: 64
+// bytes per pixel with the 64-byte swizzle, core matrices of 8 pixels (512
+// bytes); tap dx moves the start address by a pixel (the swizzle follows the
+// address, so it moves along).  B stacks the three dy taps along N = 96: its
+// products belong to three consecutive output rows, whose accumulators (32
+// TMEM columns each) lie side by side in a ring of kRSlots rows.  Input row q
+// of a strip takes 6 MMAs (3 dx x 2 channel halves) and one more to start
+// output row q from zero; where the ring wraps an MMA splits in two, and the
+// first and last two input rows take the N = 32 and 64 parts they need.  Rows,
+// their accumulators and the unrolled MMA sequence share the index it %
+// kRStages, so every offset is an immediate.  Blocks walk down strips of 128
+// columns; one thread issues the copies, one the MMAs, and two groups of four
+// warps turn alternate output rows into BF16.
+// What bounds it: 7 KB of operands per MMA (N = 96) are 56 cycles, 13 us of the
+// tensor core for 4 fields of 512^2; the memory traffic is 20 us, and about 7
+// us pass before the first row and after the last.  On B200 (ReLU, mask):
+// the tile kernel 51 and 55 us; rows staged by cp.async into planes of 8
+// channels (no swizzle) 42 us, with every thread's proxy fence and arrival
+// per row on the critical path; by TMA into such planes, 16 bytes at a time,
+// 36 us; this form 27.5 and 33 us.
+constexpr int kRM = 128;
+constexpr int kRBytes = (kRM + 2) * 2 * kC;     // 8320 per input row
+constexpr int kRRow = 9216;                     // staged, 1024-byte aligned
+constexpr int kRStages = 8;
+constexpr int kRSlots = kRStages;               // row it: stage and accumulator it % kRStages
+constexpr int kRBLbo = 3 * kC * 16;             // 1536: next 8 K-elements of B
+constexpr int kRBBytes = 3 * (kC / 8) * kRBLbo; // 18432
+constexpr int kRBars = 2 * kRStages + 2 * kRSlots + 1;
+constexpr int kRSmem = kRStages * kRRow + kRBBytes + 8 * kRBars + 16;
+constexpr int kRTmemCols = kRSlots * kC;
+constexpr uint32_t kRIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kRM >> 4) << 24);  // N is added
+static_assert(kRRow >= kRBytes && kRRow % 1024 == 0, "the swizzle repeats every 512 bytes of address");
+// Rows of 128 pixels or tiles of 16: by the pixels each computes, a tile's
+// costing half as much again (4 fields of 512 rows: 64 columns 12.0 and 11.4 us,
+// 96 columns 12.2 and 14.2, 512 columns 27.5 and 41).
+inline bool by_rows(int W) { return 2 * ((W + kRM - 1) / kRM) * kRM < 3 * ((W + kTcT - 1) / kTcT) * kTcT; }
+constexpr int kRThreads = kTcEpi + 64;          // epilogue warps, the producer's and the MMAs'
+
+// the MMAs of an input row in stage PH that ends output row it - 2, continues
+// it - 1 and starts it (slots PH - 2 .. PH of the ring)
+template <int PH>
+__device__ __forceinline__ void row_mmas(uint32_t taddr, uint32_t alo, uint32_t ahi, uint32_t blo, uint32_t bhi) {
+  constexpr int s0 = (PH + kRSlots - 2) % kRSlots, n1 = s0 + 3 <= kRSlots ? 3 : kRSlots - s0;
+  auto mm = [&](int ks, int j, int cnt, int slot, uint32_t acc) {
+    tc_mma_lo(taddr + kC * slot, alo + PH * (kRRow / 16) + 2 * (ks & 1) + 2 * kC / 16 * (ks >> 1), ahi,
+              blo + 2 * ks * (kRBLbo / 16) + j * kC, bhi, kRIdesc | ((uint32_t)(cnt * (kC >> 3)) << 17), acc);
+  };
+  mm(0, 2, 1, PH, 0u);
+  if (n1 == 1) {
+    mm(0, 0, 1, s0, 1u);
+    mm(0, 1, 1, 0, 1u);
+  } else {
+    mm(0, 0, 2, s0, 1u);
+  }
+#pragma unroll
+  for (int ks = 1; ks < 6; ++ks) {
+    mm(ks, 0, n1, s0, 1u);
+    if (n1 < 3) mm(ks, n1, 3 - n1, 0, 1u);
+  }
+}
+
+// MODE as k_conv_mid_tc; item = strip of 128 columns, rows [R chunk, R (chunk + 1))
+template <int MODE>
+__global__ void __launch_bounds__(kRThreads, kTcBlocksPerSm)
+    k_conv_row_tc(const __grid_constant__ CUtensorMap in, const bf16 *__restrict__ wt, const bf16 *__restrict__ mask,
+                  bf16 *__restrict__ out, int H, int W, int strips, int chunks, int R, int nitems,
+                  unsigned *__restrict__ err) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  uint8_t *sB = smem + kRStages * kRRow;
+  const uint32_t aBase = smem_u32(smem), bBase = smem_u32(sB), bars = bBase + kRBBytes;
+  uint32_t *tslot = reinterpret_cast<uint32_t *>(sB + kRBBytes + 8 * kRBars);
+  const uint32_t full = bars, empty = bars + 8 * kRStages, tfull = bars + 16 * kRStages, tempty = tfull + 8 * kRSlots,
+                 drain = tempty + 8 * kRSlots;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // B: column n = 32 j + co is tap row dy = 2 - j; element (n, k = 32 dx + ci)
+  // at (k / 8) * kRBLbo + n * 16 + (k % 8) * 2
+  for (int i = tid; i < kC * (kK / 8); i += kRThreads) {
+    const int co = i % kC, r = i / kC, t = r >> 2, c8 = r & 3, dy = t / 3, dx = t % 3;
+    *reinterpret_cast<uint4 *>(sB + (4 * dx + c8) * kRBLbo + ((2 - dy) * kC + co) * 16) =
+        *reinterpret_cast<const uint4 *>(&wt[co * kK + t * kC + c8 * 8]);
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(tslot)),
+                 "r"(kRTmemCols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+  }
+  if (tid == 0) {
+    for (int k = 0; k < kRBars; ++k) {
+      // full: the producer; empty, tfull and drain: one commit; tempty: a group of epilogue warps
+      const int te = 2 * kRStages + kRSlots;
+      const int count = k >= te && k < te + kRSlots ? kTcEpi / 64 : 1;
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bars + 8 * k), "r"(count) : "memory");
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+  const uint32_t taddr = *tslot;
+  bool ok = true;
+  // item -> field, first column and row, rows
+  struct Item {
+    int x0, y0, rows, b;
+  };
+  auto item_at = [&](int item) {
+    const int sx = item % strips, r = item / strips, c = r % chunks, b = r / chunks;
+    return Item{sx * kRM, c * R, min(R, H - c * R), b};
+  };
+  if (tid < kTcEpi) {
+    const int group = warp >> 2, px = 32 * (warp & 3) + lane;
+    int it = 0;  // input rows so far: output row k of an item is its slot's row it + k
+    for (int item = blockIdx.x; ok && item < nitems; item += gridDim.x) {
+      const Item t = item_at(item);
+      const int gx = t.x0 + px;
+      const int first = it;
+      it += t.rows + 2;
+      for (int k = first + ((first ^ group) & 1); k < it; k += 2) {
+        const int slot = k & (kRSlots - 1);
+        const bool in_f = gx < W && k - first < t.rows;  // the last two rows start no output
+        const long long pix = ((long long)t.b * H + t.y0 + k - first) * W + gx;
+        uint32_t mk[2][8];
+        if (MODE == 1 && in_f)
+#pragma unroll
+          for (int q = 0; q < 2; ++q) ldg32(mask + pix * kC + 16 * q, mk[q]);
+        ok = __all_sync(0xffffffffu, mbar_wait(tfull + 8 * slot, (k / kRSlots) & 1));  // the warp stays converged
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        uint32_t r[2][16];
+        const uint32_t ta = taddr + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(kC * slot);
+        tmem_ld16(ta, r[0]);
+        tmem_ld16(ta + 16, r[1]);
+        asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+        mbar_arrive_warp(tempty + 8 * slot);
+        if (in_f) store_mid<MODE>(r, mk, out + pix * kC);
+      }
+    }
+  } else if (warp == kTcEpi / 32) {
+    if (elect_one()) {
+      int it = 0;
+      for (int item = blockIdx.x; ok && item < nitems; item += gridDim.x) {
+        const Item t = item_at(item);
+        for (int q = 0; q < t.rows + 2; ++q, ++it) {
+          const int st = it % kRStages;
+          if (!(ok = mbar_wait(empty + 8 * st, ((it / kRStages) & 1) ^ 1))) break;
+          tma_expect(full + 8 * st, kRBytes);
+          tma_box(aBase + st * kRRow, &in, t.x0 - 1, t.y0 - 1 + q, t.b, full + 8 * st);
+        }
+      }
+      // the last copies have landed before the block leaves, whatever the other roles met
+      for (int k = max(0, it - kRStages); k < it; ++k) ok &= mbar_wait(full + 8 * (k % kRStages), (k / kRStages) & 1);
+    }
+    ok = __all_sync(0xffffffffu, ok);
+  } else {
+    const bool leader = elect_one();
+    const uint64_t a0 = smem_desc(aBase, 16, 8 * 2 * kC) | kSwizzle64, b0 = smem_desc(bBase, kRBLbo, 128);
+    const uint32_t alo = (uint32_t)a0, ahi = (uint32_t)(a0 >> 32), blo = (uint32_t)b0, bhi = (uint32_t)(b0 >> 32);
+    int it = 0;
+    for (int item = blockIdx.x; ok && item < nitems; item += gridDim.x) {
+      const int rows = item_at(item).rows;
+      for (int q = 0; q < rows + 2; ++q, ++it) {
+        const int ph = it & (kRSlots - 1), par = (it / kRSlots) & 1;
+        ok = mbar_wait(full + 8 * ph, par) && mbar_wait(tempty + 8 * ph, par ^ 1);
+        if (!(ok = __all_sync(0xffffffffu, ok))) break;
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        if (!leader) continue;
+        if (q >= 2 && q < rows) {
+          switch (ph) {
+            case 0: row_mmas<0>(taddr, alo, ahi, blo, bhi); break;
+            case 1: row_mmas<1>(taddr, alo, ahi, blo, bhi); break;
+            case 2: row_mmas<2>(taddr, alo, ahi, blo, bhi); break;
+            case 3: row_mmas<3>(taddr, alo, ahi, blo, bhi); break;
+            case 4: row_mmas<4>(taddr, alo, ahi, blo, bhi); break;
+            case 5: row_mmas<5>(taddr, alo, ahi, blo, bhi); break;
+            case 6: row_mmas<6>(taddr, alo, ahi, blo, bhi); break;
+            default: row_mmas<7>(taddr, alo, ahi, blo, bhi); break;
+          }
+        } else {  // one or two of the three output rows, an MMA each
+          for (int j = max(2 - q, 0); j <= min(2, rows + 1 - q); ++j)
+            for (int ks = 0; ks < 6; ++ks)
+              tc_mma_lo(taddr + kC * ((ph + j + kRSlots - 2) & (kRSlots - 1)),
+                        alo + ph * (kRRow / 16) + 2 * (ks & 1) + 2 * kC / 16 * (ks >> 1), ahi,
+                        blo + 2 * ks * (kRBLbo / 16) + j * kC, bhi, kRIdesc | ((uint32_t)(kC >> 3) << 17),
+                        j < 2 || ks > 0 ? 1u : 0u);
+        }
+        tc_commit(empty + 8 * ph);
+        if (q >= 2) tc_commit(tfull + 8 * ((ph + kRSlots - 2) & (kRSlots - 1)));
+      }
+      if (!ok) break;
+      if (!leader) continue;
+      // the slots of the last two rows hold no output
+      tc_commit(tfull + 8 * ((it + kRSlots - 2) & (kRSlots - 1)));
+      tc_commit(tfull + 8 * ((it + kRSlots - 1) & (kRSlots - 1)));
+    }
+    if (!ok && leader) {  // MMAs in flight, before the TMEM is freed
+      tc_commit(drain);
+      mbar_wait(drain, 0);
+    }
+  }
+  if (!ok) atomicExch(err, 1u);
+  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+  if (warp == 0)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(taddr), "r"(kRTmemCols) : "memory");
 }
 
 // --- block reductions (fixed order: deterministic) ----------------------------
@@ -838,6 +1101,133 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_wgrad_mid(const bf16 *__restr
   for (int i = tid; i < kSzWm; i += kWgThreads) part[(long long)blockIdx.x * kSzWm + i] = sum[i];
 }
 
+// The same on tcgen05 (the default path).  K = 16 pixels of a row; A is four rows
+// of dZ (M = 4 rows x 32 channels), B five rows of the activations (N = 160),
+// shifted by tap dx: the accumulator of dZ row i and activation row q is tap
+// row dy = q - i of the gradient.  The first three dZ rows use their three taps
+// of the five rows, so an MMA does nine useful row pairs of twenty; what the
+// others hold (the fourth dZ row is whatever follows in shared memory) is never
+// read.  Both operands lie as the copies leave them, 64 bytes per pixel with
+// the 64-byte swizzle, M/N-major: 8 pixels 512 bytes, the next image row a row
+// pitch further, dx 64 bytes.  The three dx accumulators (480 TMEM columns) stay
+// for all of a block's tiles of 64 x 6 pixels (kGStages in flight); at the end
+// three warps read their dZ row's lanes and the three rows are added in order.
+// What bounds it: 9 KB of operands per MMA, 72 cycles: 17 us of the tensor core
+// for 4 fields of 512^2, and 20 us of memory traffic.  There on B200: the
+// mma.sync form 104 us, this one 32 us.
+constexpr int kGW = 64, kGRows = 6;                   // dZ tile
+constexpr int kGPitch = kGW * 2 * kC;                 // 4096 per dZ row
+constexpr int kGXPitch = (kGW + 2) * 2 * kC;          // 4224 per activation row
+constexpr int kGOff = kGRows * kGPitch;               // the activation rows of a stage
+constexpr int kGStage = kGOff + (kGRows + 2) * kGXPitch;
+constexpr int kGStages = 3;
+constexpr int kGN = 5 * kC;                           // 160
+constexpr int kGSumLd = kK + 1;
+constexpr int kGBars = 2 * kGStages + 1;
+constexpr int kGSmem = kGStages * kGStage + 8 * kGBars + 16;
+constexpr int kGThreads = 192;                        // four epilogue warps, the producer's and the MMAs'
+constexpr uint32_t kGIdesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) |
+                             ((uint32_t)(kGN >> 3) << 17) | ((uint32_t)(kTcM >> 4) << 24);  // both M/N-major
+static_assert(kGStage % 1024 == 0 && kGOff % 1024 == 0, "the swizzle repeats every 512 bytes of address");
+static_assert(kGPitch <= (kGRows + 2) * kGXPitch, "the unused fourth dZ row lies within the stage");
+static_assert(3 * kC * kGSumLd * (int)sizeof(float) <= kGStages * kGStage, "the row sums reuse the stages");
+
+__global__ void __launch_bounds__(kGThreads, 1)
+    k_wgrad_tc(const __grid_constant__ CUtensorMap dz, const __grid_constant__ CUtensorMap a, float *__restrict__ part,
+               int tiles_x, int tiles_y, int ntiles, unsigned *__restrict__ err) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  const uint32_t base = smem_u32(smem), bars = base + kGStages * kGStage;
+  uint32_t *tslot = reinterpret_cast<uint32_t *>(smem + kGStages * kGStage + 8 * kGBars);
+  const uint32_t full = bars, empty = bars + 8 * kGStages, done = bars + 16 * kGStages;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;\n" ::"r"(smem_u32(tslot))
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+  }
+  if (tid == 0) {
+    for (int k = 0; k < kGBars; ++k)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(bars + 8 * k) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+  const uint32_t taddr = *tslot;
+  bool ok = true;
+  if (warp == 4) {
+    if (elect_one()) {
+      int it = 0;
+      for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++it) {
+        const int st = it % kGStages, r = tile / tiles_x, b = r / tiles_y;
+        const int x = (tile % tiles_x) * kGW, y = (r % tiles_y) * kGRows;
+        if (!(ok = mbar_wait(empty + 8 * st, ((it / kGStages) & 1) ^ 1))) break;
+        tma_expect(full + 8 * st, kGStage);
+        tma_box(base + st * kGStage, &dz, x, y, b, full + 8 * st);
+        tma_box(base + st * kGStage + kGOff, &a, x - 1, y - 1, b, full + 8 * st);
+      }
+      // the last copies have landed before the block leaves, whatever the other roles met
+      for (int k = max(0, it - kGStages); k < it; ++k) ok &= mbar_wait(full + 8 * (k % kGStages), (k / kGStages) & 1);
+    }
+    ok = __all_sync(0xffffffffu, ok);
+  } else if (warp == 5) {
+    const bool leader = elect_one();
+    const uint64_t a0 = smem_desc(base, kGPitch, 512) | kSwizzle64, b0 = smem_desc(base + kGOff, kGXPitch, 512) | kSwizzle64;
+    const uint32_t alo = (uint32_t)a0, ahi = (uint32_t)(a0 >> 32), blo = (uint32_t)b0, bhi = (uint32_t)(b0 >> 32);
+    int it = 0;
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++it) {
+      const int st = it % kGStages;
+      if (!(ok = __all_sync(0xffffffffu, mbar_wait(full + 8 * st, (it / kGStages) & 1)))) break;
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+      if (!leader) continue;
+      const uint32_t as = alo + st * (kGStage / 16), bs = blo + st * (kGStage / 16);
+#pragma unroll
+      for (int u = 0; u < kGRows / 3; ++u)
+#pragma unroll
+        for (int kb = 0; kb < kGW / 16; ++kb)
+#pragma unroll
+          for (int dx = 0; dx < 3; ++dx)
+            tc_mma_lo(taddr + kGN * dx, as + (3 * u * kGPitch + 1024 * kb) / 16, ahi,
+                      bs + (3 * u * kGXPitch + 1024 * kb + 64 * dx) / 16, bhi, kGIdesc,
+                      it > 0 || u > 0 || kb > 0 ? 1u : 0u);
+      tc_commit(empty + 8 * st);
+    }
+    if (leader) tc_commit(done);
+  }
+  if (warp != 4) {  // every MMA, before the TMEM is freed; the wait spans all tiles
+    bool fin = false;
+    for (int k = 0; k < 64 && !fin; ++k) fin = __all_sync(0xffffffffu, mbar_wait(done, 0));
+    ok &= fin;
+  }
+  __syncthreads();
+  float *sum = reinterpret_cast<float *>(smem);
+  if (warp < 3) {
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    float *d = sum + (warp * kC + lane) * kGSumLd;  // dZ row i = warp, co = lane
+#pragma unroll 1
+    for (int dx = 0; dx < 3; ++dx)
+#pragma unroll
+      for (int dy = 0; dy < 3; ++dy) {
+        uint32_t r[2][16];
+        const uint32_t ta = taddr + ((uint32_t)(32 * warp) << 16) + (uint32_t)(kGN * dx + kC * (warp + dy));
+        tmem_ld16(ta, r[0]);
+        tmem_ld16(ta + 16, r[1]);
+        asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+#pragma unroll
+        for (int ci = 0; ci < kC; ++ci) d[(3 * dy + dx) * kC + ci] = __uint_as_float(r[ci >> 4][ci & 15]);
+      }
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+  }
+  if (!ok) atomicExch(err, 1u);
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;\n" ::"r"(taddr) : "memory");
+  for (int i = tid; i < kSzWm; i += kGThreads) {
+    const float *d = sum + (i / kK) * kGSumLd + i % kK;
+    part[(long long)blockIdx.x * kSzWm + i] = (d[0] + d[kC * kGSumLd]) + d[2 * kC * kGSumLd];
+  }
+}
+
 // out[j] = sum over rows of part[row * cols + j]: a block takes 32 columns, its
 // eight warps every eighth row each, combined in a fixed order (one thread per
 // column summing its rows waited for each load: 41 us for 592 rows of 9216
@@ -984,10 +1374,51 @@ EdgeGrid edge_grid(const ins2d_cnn *net, int B, int H, int W, int step_x) {
   return g;
 }
 
+// A BF16 activation array of B fields as {channel, pixel, row, field} for copies
+// of npx pixels by nrows rows, 64 bytes a pixel with the 64-byte swizzle; zeros
+// outside the field
+CUtensorMap act_map(const bf16 *p, int B, int H, int W, int npx, int nrows) {
+  using Encode = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
+                              const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
+                              CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+  static const Encode encode = [] {
+    void *f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    CK(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q));
+    if (q != cudaDriverEntryPointSuccess || !f) throw CudaError("cnn: no cuTensorMapEncodeTiled in this driver");
+    return (Encode)f;
+  }();
+  CUtensorMap m;
+  const cuuint64_t w = (cuuint64_t)W, h = (cuuint64_t)H;
+  const cuuint64_t dims[4] = {kC, w, h, (cuuint64_t)B};
+  const cuuint64_t strides[3] = {2 * kC, 2 * kC * w, 2 * kC * w * h};
+  const cuuint32_t box[4] = {kC, (cuuint32_t)npx, (cuuint32_t)nrows, 1}, es[4] = {1, 1, 1, 1};
+  if (encode(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<bf16 *>(p), dims, strides, box, es,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+    throw CudaError("cnn: the activations' tensor map was refused");
+  return m;
+}
+
 template <int MODE>
 void launch_mid(ins2d_cnn *net, const bf16 *in, const bf16 *wt, const bf16 *mask, bf16 *out, int B, int H, int W,
                 cudaStream_t s) {
-  if (net->path == INS2D_CNN_PATH_TCGEN05) {
+  if (net->path == INS2D_CNN_PATH_TCGEN05 && by_rows(W)) {
+    const int strips = (W + kRM - 1) / kRM, cap = kTcBlocksPerSm * net->sms;
+    // rows per item: the fewest row steps (R + 2 an item) of the busiest block
+    const long long per = (long long)strips * B;
+    int R = H;
+    long long best = -1;
+    for (int c = 1; c <= (H + 3) / 4 && (c == 1 || per * (c - 1) < 2LL * cap); ++c) {
+      const int r = (H + c - 1) / c;
+      const long long cost = ((per * ((H + r - 1) / r) + cap - 1) / cap) * (r + 2);
+      if (best < 0 || cost < best) best = cost, R = r;
+    }
+    const int chunks = (H + R - 1) / R;
+    const int nitems = (int)(per * chunks), grid = std::min(nitems, cap);
+    k_conv_row_tc<MODE><<<grid, kRThreads, kRSmem, s>>>(act_map(in, B, H, W, kRM + 2, 1), wt, mask, out, H, W, strips,
+                                                        chunks, R, nitems, net->flag);
+  } else if (net->path == INS2D_CNN_PATH_TCGEN05) {
     const int tx = (W + kTcT - 1) / kTcT, ty = (H + kTcT - 1) / kTcT;
     const long long nt = (long long)tx * ty * B;
     const int grid = (int)std::min<long long>(nt, (long long)kTcBlocksPerSm * net->sms);
@@ -1124,13 +1555,20 @@ double loss_grad(ins2d_cnn *net, const float *in, const float *tgt, int B, int H
   k_wgrad_edge<6><<<e.blocks, kEThreads, 0, s>>>(net->act[4], net->dy, net->partials, B, H, W, e.tx, e.ty);
   k_reduce_rows<<<kK / 32, 256, 0, s>>>(net->partials, (int)e.blocks, kK, net->g + kOffW6, 0);
   // layers 5..2: dZ_l in dz[cur]; weight gradient from (dZ_l, A_{l-1}); dZ_{l-1}
-  const int tiles_x = (W + TW - 1) / TW, tiles_y = (H + TH - 1) / TH;
+  const bool tc = net->path == INS2D_CNN_PATH_TCGEN05;
+  const int tw = tc ? kGW : TW, th = tc ? kGRows : TH;
+  const int tiles_x = (W + tw - 1) / tw, tiles_y = (H + th - 1) / th;
   const long long ntiles = (long long)tiles_x * tiles_y * B;
   const int wb = (int)std::min({(long long)kWgBlocks, (long long)net->sms, ntiles});
   int cur = 0;
   for (int l = kMid - 1; l >= 0; --l) {
     // layer index l: input act[l], output act[l + 1], gradient dZ in dz[cur]
-    k_wgrad_mid<<<wb, kWgThreads, kWgSmem, s>>>(net->dz[cur], net->act[l], net->partials, B, H, W, tiles_x, tiles_y);
+    if (tc)
+      k_wgrad_tc<<<wb, kGThreads, kGSmem, s>>>(act_map(net->dz[cur], B, H, W, kGW, kGRows),
+                                               act_map(net->act[l], B, H, W, kGW + 2, kGRows + 2), net->partials,
+                                               tiles_x, tiles_y, (int)ntiles, net->flag);
+    else
+      k_wgrad_mid<<<wb, kWgThreads, kWgSmem, s>>>(net->dz[cur], net->act[l], net->partials, B, H, W, tiles_x, tiles_y);
     k_reduce_rows<<<kSzWm / 32, 256, 0, s>>>(net->partials, wb, kSzWm, net->g + kOffWm + l * kSzWm, 0);
     launch_mid<1>(net, net->dz[cur], net->wb + l * kSzWm, net->act[l], net->dz[cur ^ 1], B, H, W, s);
     cur ^= 1;
@@ -1292,8 +1730,11 @@ cudaError_t prepare_kernels() {
     if (e == cudaSuccess) e = r;
   };
   opt_in((const void *)k_wgrad_mid, kWgSmem);
+  opt_in((const void *)k_wgrad_tc, kGSmem);
   opt_in((const void *)k_conv_mid_tc<0>, kTcSmem);
   opt_in((const void *)k_conv_mid_tc<1>, kTcSmem);
+  opt_in((const void *)k_conv_row_tc<0>, kRSmem);
+  opt_in((const void *)k_conv_row_tc<1>, kRSmem);
   return e;
 }
 

@@ -95,10 +95,12 @@ def test_line_transforms(shape):
     assert _rel(m.time_ERK(V, np.zeros(m.Np), 0.0, 1e-4)[0], ref) < 1e-5
 
 
-# the network's edge layers and weight gradients: tile edges of 62, 64 and 16,
-# one column or row left over, several fields; the learned tests' bounds
+# the network's layers and weight gradients: tile edges of 62, 64 and 16, strips
+# of 128 columns (one row, one column over, several strips per block), one
+# column or row left over, several fields; the learned tests' bounds
 @pytest.mark.parametrize("path", ["tcgen05", "mma_sync"])
-@pytest.mark.parametrize("shape", [(1, 1, 62), (1, 16, 63), (2, 17, 64), (1, 15, 65), (3, 33, 124), (1, 129, 130)])
+@pytest.mark.parametrize("shape", [(1, 1, 62), (1, 16, 63), (2, 17, 64), (1, 15, 65), (3, 33, 124), (1, 129, 130),
+                                   (1, 1, 96), (2, 3, 128), (1, 40, 200), (300, 5, 97), (2, 150, 257)])
 def test_network_tiles(shape, path):
     from oracle import cnn_ref as N
     from tests import test_gpu_learned as L
