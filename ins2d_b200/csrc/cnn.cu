@@ -301,12 +301,6 @@ __global__ void __launch_bounds__(kEThreads, kEBlocksPerSm)
   }
 }
 
-// --- 32 -> 32 on tensor cores ---------------------------------------------------
-// One block: a 16 x 8 pixel tile of one field; warp w computes tile row w
-// (M = 16 pixels) for all 32 output channels (4 n-tiles of 8), K = 9 taps x
-// 32 input channels in 18 steps of 16.  The halo tile and the weights sit in
-// shared memory with padded strides so that the 32-bit fragment loads of a
-// warp hit 32 different banks.
 // 32 bytes to and from global memory in one instruction
 __device__ __forceinline__ void ldg32(const void *p, uint32_t (&r)[8]) {
   asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
@@ -345,6 +339,12 @@ __device__ __forceinline__ void store_mid(const uint32_t (&r)[2][16], const uint
   }
 }
 
+// --- 32 -> 32 on tensor cores ---------------------------------------------------
+// One block: a 16 x 8 pixel tile of one field; warp w computes tile row w
+// (M = 16 pixels) for all 32 output channels (4 n-tiles of 8), K = 9 taps x
+// 32 input channels in 18 steps of 16.  The halo tile and the weights sit in
+// shared memory with padded strides so that the 32-bit fragment loads of a
+// warp hit 32 different banks.
 // MODE 0: out = bf16(ReLU(Z)).  MODE 1 (backward-data): out = bf16(Z * [mask > 0]).
 template <int MODE>
 __global__ void __launch_bounds__(256) k_conv_mid(const bf16 *__restrict__ in, const bf16 *__restrict__ wt,
