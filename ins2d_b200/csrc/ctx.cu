@@ -2009,8 +2009,8 @@ void ens_build_batch(ins2d_ens *e, const std::vector<int> &order) {
     R.tiles = dc;
     R.ntiles = (int)cells.size();
     R.n = n;
-    R.ticket = ens_alloc<unsigned>(e, 1);
-    CK(cudaMemset(R.ticket, 0, sizeof(unsigned)));
+    R.ticket = ens_alloc<unsigned long long>(e, 1);
+    CK(cudaMemset(R.ticket, 0, sizeof(unsigned long long)));
   }
   std::vector<EnsCg> cg(n);
   for (int m = 0; m < n; ++m) {

@@ -8,7 +8,7 @@
 // condition by the update, the divergence is formed by the initialisation and
 // the solution is read by the projection.  24 members, RK44 step on B200:
 // eleven launches and eleven more per pass before, 0.881 ms; six launches and
-// five more per pass now, 0.787 ms.
+// five more per pass, 0.787 ms; with the members' ends below, 0.748 ms.
 #include <cfloat>
 
 #include "ins2d.h"
@@ -40,32 +40,20 @@ __device__ __forceinline__ void add_stats(const EnsCg &C, EnsStats &st) {
   if (C.status != 0 && st.status == 0) st.status = C.status;
 }
 
-// the last block of a launch: counts the members still iterating and sets the
-// loop condition (first: before any pass)
-__device__ void end_launch(const EnsFdmRun &R, const LoopCond &cond, bool first) {
-  __shared__ bool last;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    last = atomicAdd(R.ticket, 1u) == gridDim.x - 1;
-  }
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  int mine = 0;
-  for (int m = threadIdx.x; m < R.n; m += blockDim.x) mine += *(volatile int *)&R.cg[m].done ? 0 : 1;
-  __shared__ int act;
-  if (threadIdx.x == 0) act = 0;
-  __syncthreads();
-  if (mine) atomicAdd(&act, mine);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    *R.ticket = 0u;
-    *R.active = act;
-    const int loops = first ? 0 : *R.loops + 1;
-    *R.loops = loops;
-    set_cond(cond, act > 0 && loops < cond.limit);
-  }
+// One thread per member and launch, when the member's scalars are final; the
+// last member's sets the loop condition (first: before any pass).  The ticket
+// counts members in its low and those still iterating in its high half: a
+// ticket per block and a scan of the members' flags were 511 atomics on one
+// word and another round of loads for 24 members (k_ef_update 11.9 -> 9.4 us, ten steps 7.75 ->
+// 7.48 ms).
+__device__ __forceinline__ void end_member(const EnsFdmRun &R, const LoopCond &cond, bool active, bool first) {
+  const unsigned long long t = atomicAdd(R.ticket, 1ull + (active ? 1ull << 32 : 0ull)) + 1ull + (active ? 1ull << 32 : 0ull);
+  if ((unsigned)t != (unsigned)R.n) return;
+  const int act = (int)(t >> 32), loops = first ? 0 : *R.loops + 1;
+  *R.ticket = 0ull;
+  *R.active = act;
+  *R.loops = loops;
+  set_cond(cond, act > 0 && loops < cond.limit);
 }
 
 __device__ __forceinline__ void copy_ops(DevOps *dst, const DevOps *src) {
@@ -111,22 +99,24 @@ __global__ void __launch_bounds__(kThreads) k_ef_init(const EnsFdmRun R, int mod
     }
     if (done) add_stats(C, R.stats[t.x]);
     C.done = done;
+    end_member(R, cond, !done, true);
   }
-  end_launch(R, cond, true);
 }
 
 // p = z + beta p (directions alternate between two buffers), q = A p, p'q
 __global__ void __launch_bounds__(kThreads) k_ef_step(const EnsFdmRun R) {
-  __shared__ __align__(16) DevOps sP;
   const int4 t = R.tiles[blockIdx.x];
   EnsCg &C = R.cg[t.x];
-  if (*(volatile int *)&C.done) return;
   const EnsMemberD &M = R.mem[t.x];
-  copy_ops(&sP, &M.P);
-  __syncthreads();
-  const PcgWork &W = M.W;
-  const bool first = C.it == 0, odd = C.it & 1;
+  const int stop = *(volatile int *)&C.done;  // with the other scalars: one latency
+  const long long it = C.it;
   const double beta = C.beta;
+  const PcgWork W = M.W;
+  const auto TX = M.P.TX, TY = M.P.TY;
+  const double *__restrict__ hx = M.P.hx, *__restrict__ hy = M.P.hy;
+  const int Npx = M.P.Npx, Np = (int)M.P.Np;
+  if (stop) return;
+  const bool first = it == 0, odd = it & 1;
   const double *__restrict__ z = M.zf, *__restrict__ po = odd ? W.p : W.p2;
   double *__restrict__ pn = odd ? W.p2 : W.p;
   auto pv = [&](long long k) {
@@ -139,10 +129,10 @@ __global__ void __launch_bounds__(kThreads) k_ef_step(const EnsFdmRun R) {
 #pragma unroll
   for (int u = 0; u < kPer; ++u) {
     const int k = t.y + u * kThreads + threadIdx.x;
-    if (k < sP.Np) {
-      const int j = k / sP.Npx, i = k - j * sP.Npx;
-      const double aq = -(__ldg(sP.hy + j) * tab_x_f(sP.TX, i, pv, (long long)j * sP.Npx) +
-                          __ldg(sP.hx + i) * tab_y_f(sP.TY, j, pv, 0, sP.Npx, i));
+    if (k < Np) {
+      const int j = k / Npx, i = k - j * Npx;
+      const double aq = -(__ldg(hy + j) * tab_x_f(TX, i, pv, (long long)j * Npx) +
+                          __ldg(hx + i) * tab_y_f(TY, j, pv, 0, Npx, i));
       const double pc = pv(k);
       W.q[k] = aq;
       pn[k] = pc;
@@ -164,49 +154,54 @@ __global__ void __launch_bounds__(kThreads) k_ef_step(const EnsFdmRun R) {
 __global__ void __launch_bounds__(kThreads) k_ef_update(const EnsFdmRun R, const LoopCond cond) {
   const int4 t = R.tiles[blockIdx.x];
   EnsCg &C = R.cg[t.x];
-  if (!*(volatile int *)&C.done) {
-    const EnsMemberD &M = R.mem[t.x];
-    const PcgWork &W = M.W;
-    const bool first = C.it == 0;
-    const double alpha = C.alpha;
-    const double *__restrict__ p = (C.it & 1) ? W.p2 : W.p;
-    const int Np = (int)M.P.Np;
-    double q[1] = {0.0};
-    const int ops[1] = {R_SUM};
+  const EnsMemberD &M = R.mem[t.x];
+  const int stop = *(volatile int *)&C.done;  // with the other scalars: one latency
+  const long long it = C.it;
+  const double alpha = C.alpha;
+  const PcgWork W = M.W;
+  const double *__restrict__ f = M.f;
+  const int Np = (int)M.P.Np;
+  if (stop) {
+    if (t.z == 0 && threadIdx.x == 0) end_member(R, cond, false, false);
+    return;
+  }
+  const bool first = it == 0;
+  const double *__restrict__ p = (it & 1) ? W.p2 : W.p;
+  double q[1] = {0.0};
+  const int ops[1] = {R_SUM};
 #pragma unroll
-    for (int u = 0; u < kPer; ++u) {
-      const int k = t.y + u * kThreads + threadIdx.x;
-      if (k < Np) {
-        const double x = (first ? 0.0 : W.x[k]) + alpha * __ldg(p + k);
-        const double r = (first ? __ldg(M.f + k) : W.r[k]) - alpha * __ldg(W.q + k);
-        W.x[k] = x;
-        W.r[k] = r;
-        q[0] += r * r;
-      }
-    }
-    double out[1];
-    if (grid_reduce_at<1>(q, ops, member_red(C, 1), out, t.z, C.ntiles)) {
-      int done = 0;
-      if (C.status != 0) {  // found by this pass's reductions (cg.F:240-262)
-        done = 1;
-      } else {
-        C.it += 1;
-        C.rr = out[0] / C.rr0;
-        if (!isfinite(C.rr)) {
-          C.status = INS2D_ENONFINITE;
-          done = 1;
-        } else if (C.rr <= C.tol2) {
-          done = 1;
-        } else if (C.it >= C.maxit) {
-          C.status = INS2D_ENOTCONV;
-          done = 1;
-        }
-      }
-      if (done) add_stats(C, R.stats[t.x]);
-      C.done = done;
+  for (int u = 0; u < kPer; ++u) {
+    const int k = t.y + u * kThreads + threadIdx.x;
+    if (k < Np) {
+      const double x = (first ? 0.0 : W.x[k]) + alpha * __ldg(p + k);
+      const double r = (first ? __ldg(f + k) : W.r[k]) - alpha * __ldg(W.q + k);
+      W.x[k] = x;
+      W.r[k] = r;
+      q[0] += r * r;
     }
   }
-  end_launch(R, cond, false);
+  double out[1];
+  if (grid_reduce_at<1>(q, ops, member_red(C, 1), out, t.z, C.ntiles)) {
+    int done = 0;
+    if (C.status != 0) {  // found by this pass's reductions (cg.F:240-262)
+      done = 1;
+    } else {
+      C.it += 1;
+      C.rr = out[0] / C.rr0;
+      if (!isfinite(C.rr)) {
+        C.status = INS2D_ENONFINITE;
+        done = 1;
+      } else if (C.rr <= C.tol2) {
+        done = 1;
+      } else if (C.it >= C.maxit) {
+        C.status = INS2D_ENOTCONV;
+        done = 1;
+      }
+    }
+    if (done) add_stats(C, R.stats[t.x]);
+    C.done = done;
+    end_member(R, cond, !done, false);
+  }
 }
 
 __global__ void __launch_bounds__(kThreads) k_ef_finish(const EnsFdmRun R) {

@@ -405,7 +405,7 @@ struct EnsFdmRun {
   EnsStats *stats;
   const int4 *tiles;
   int ntiles, n;      // cell tiles, members
-  unsigned *ticket;   // blocks of a launch that have finished (zero between launches)
+  unsigned long long *ticket;  // members finished (low half) and still iterating (high half) in a launch; else zero
   int *active;        // members still iterating
   int *loops;         // passes of the current solve
 };

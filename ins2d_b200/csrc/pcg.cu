@@ -559,12 +559,15 @@ __global__ void __launch_bounds__(kVecThreads) k_rz_f(const PcgWork W, const dou
 // k_spmv_cols does
 __global__ void __launch_bounds__(256) k_step_f(const __grid_constant__ DevOps P, const PcgWork W,
                                                 const double *__restrict__ z, int rows) {
-  if (*(volatile int *)&W.sc->done) return;
+  const int done = *(volatile int *)&W.sc->done;
+  const long long it = W.sc->it;  // read together with done: one latency
+  const double bt = W.sc->beta;
+  if (done) return;
   const int i = blockIdx.x * BX + threadIdx.x;
   const int j0 = (blockIdx.y * BY + threadIdx.y) * rows;
-  const bool first = W.sc->it == 0;
-  const bool odd = W.sc->it & 1;
-  const double beta = first ? 0.0 : W.sc->beta;
+  const bool first = it == 0;
+  const bool odd = it & 1;
+  const double beta = first ? 0.0 : bt;
   const double *__restrict__ po = odd ? W.p : W.p2;
   double *__restrict__ pn = odd ? W.p2 : W.p;
   auto pv = [&](long long k) {
@@ -617,13 +620,15 @@ __global__ void __launch_bounds__(256) k_step_f(const __grid_constant__ DevOps P
 // stopping rule and the loop condition
 __global__ void __launch_bounds__(kVecThreads) k_update_f(const PcgWork W, const double *__restrict__ f, long long n,
                                                           const LoopCond cond) {
-  if (*(volatile int *)&W.sc->done) {  // an earlier kernel of this pass found an error
+  const int done = *(volatile int *)&W.sc->done;
+  const double alpha = W.sc->alpha;  // read together with done: one latency
+  const long long it = W.sc->it;
+  if (done) {  // an earlier kernel of this pass found an error
     if (blockIdx.x == 0 && threadIdx.x == 0) set_cond(cond, false);
     return;
   }
-  const double alpha = W.sc->alpha;
-  const bool first = W.sc->it == 0;
-  const double *__restrict__ p = (W.sc->it & 1) ? W.p2 : W.p;
+  const bool first = it == 0;
+  const double *__restrict__ p = (it & 1) ? W.p2 : W.p;
   double q[4] = {0.0, -DBL_MAX, DBL_MAX, 0.0};
   const int ops[4] = {R_SUM, R_MAX, R_MIN, R_MAX};
   const long long stride = (long long)gridDim.x * blockDim.x;
