@@ -73,16 +73,22 @@ __global__ void __launch_bounds__(kThreads) k_ef_init(const EnsFdmRun R, int mod
   const double alpha = mode == 0 ? 1.0 / M.dt : 0.0, g = mode == 0 ? gamma : 1.0;
   double q[2] = {0.0, 0.0};
   const int ops[2] = {R_SUM, R_MAX};
+  // loads of all the thread's cells before the first store, here and below: a
+  // store in between orders the next cell's loads behind it
+  const int Np = (int)sP.Np, Npx = sP.Npx;
+  double *__restrict__ f = M.f;
+  double fv[kPer];
+#pragma unroll
+  for (int u = 0; u < kPer; ++u) {
+    const int k = t.y + u * kThreads + threadIdx.x, j = k / Npx;
+    fv[u] = k < Np ? div_cell(sP, W, alpha, 0.0, g, k - j * Npx, j) : 0.0;
+  }
 #pragma unroll
   for (int u = 0; u < kPer; ++u) {
     const int k = t.y + u * kThreads + threadIdx.x;
-    if (k < sP.Np) {
-      const int j = k / sP.Npx, i = k - j * sP.Npx;
-      const double fv = div_cell(sP, W, alpha, 0.0, g, i, j);
-      M.f[k] = fv;
-      q[0] += fv * fv;
-      q[1] = fmax(q[1], fabs(fv));
-    }
+    if (k < Np) f[k] = fv[u];
+    q[0] += fv[u] * fv[u];
+    q[1] = fmax(q[1], fabs(fv[u]));
   }
   double out[2];
   if (grid_reduce_at<2>(q, ops, member_red(C, 2), out, t.z, C.ntiles)) {
@@ -126,17 +132,24 @@ __global__ void __launch_bounds__(kThreads) k_ef_step(const EnsFdmRun R) {
   };
   double q[1] = {0.0};
   const int ops[1] = {R_SUM};
+  double aq[kPer], pc[kPer];
+#pragma unroll
+  for (int u = 0; u < kPer; ++u) {
+    const int k = t.y + u * kThreads + threadIdx.x, j = k / Npx, i = k - j * Npx;
+    aq[u] = pc[u] = 0.0;
+    if (k < Np) {
+      aq[u] = -(__ldg(hy + j) * tab_x_f(TX, i, pv, (long long)j * Npx) +
+                __ldg(hx + i) * tab_y_f(TY, j, pv, 0, Npx, i));
+      pc[u] = pv(k);
+    }
+  }
 #pragma unroll
   for (int u = 0; u < kPer; ++u) {
     const int k = t.y + u * kThreads + threadIdx.x;
     if (k < Np) {
-      const int j = k / Npx, i = k - j * Npx;
-      const double aq = -(__ldg(hy + j) * tab_x_f(TX, i, pv, (long long)j * Npx) +
-                          __ldg(hx + i) * tab_y_f(TY, j, pv, 0, Npx, i));
-      const double pc = pv(k);
-      W.q[k] = aq;
-      pn[k] = pc;
-      q[0] += pc * aq;
+      W.q[k] = aq[u];
+      pn[k] = pc[u];
+      q[0] += pc[u] * aq[u];
     }
   }
   double out[1];
@@ -169,15 +182,24 @@ __global__ void __launch_bounds__(kThreads) k_ef_update(const EnsFdmRun R, const
   const double *__restrict__ p = (it & 1) ? W.p2 : W.p;
   double q[1] = {0.0};
   const int ops[1] = {R_SUM};
+  double x[kPer], r[kPer];
+  const double *ro = first ? f : W.r;
+#pragma unroll
+  for (int u = 0; u < kPer; ++u) {
+    const int k = t.y + u * kThreads + threadIdx.x;
+    x[u] = r[u] = 0.0;
+    if (k < Np) {
+      x[u] = (first ? 0.0 : W.x[k]) + alpha * __ldg(p + k);
+      r[u] = ro[k] - alpha * __ldg(W.q + k);
+    }
+  }
 #pragma unroll
   for (int u = 0; u < kPer; ++u) {
     const int k = t.y + u * kThreads + threadIdx.x;
     if (k < Np) {
-      const double x = (first ? 0.0 : W.x[k]) + alpha * __ldg(p + k);
-      const double r = (first ? __ldg(f + k) : W.r[k]) - alpha * __ldg(W.q + k);
-      W.x[k] = x;
-      W.r[k] = r;
-      q[0] += r * r;
+      W.x[k] = x[u];
+      W.r[k] = r[u];
+      q[0] += r[u] * r[u];
     }
   }
   double out[1];

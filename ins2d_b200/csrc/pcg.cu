@@ -632,16 +632,31 @@ __global__ void __launch_bounds__(kVecThreads) k_update_f(const PcgWork W, const
   double q[4] = {0.0, -DBL_MAX, DBL_MAX, 0.0};
   const int ops[4] = {R_SUM, R_MAX, R_MIN, R_MAX};
   const long long stride = (long long)gridDim.x * blockDim.x;
-#pragma unroll 4
-  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += stride) {
-    const double x = (first ? 0.0 : W.x[k]) + alpha * __ldg(p + k);
-    const double r = (first ? __ldg(f + k) : W.r[k]) - alpha * __ldg(W.q + k);
-    W.x[k] = x;
-    W.r[k] = r;
-    q[0] += r * r;
-    q[1] = fmax(q[1], x);
-    q[2] = fmin(q[2], x);
-    q[3] = fmax(q[3], fabs(r));
+  const double *ro = first ? f : W.r;
+  // four points' loads before the first store, which would order the next
+  // points' loads behind it
+  for (long long k0 = blockIdx.x * (long long)blockDim.x + threadIdx.x; k0 < n; k0 += 4 * stride) {
+    double x[4], r[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const long long k = k0 + u * stride;
+      if (k < n) {
+        x[u] = (first ? 0.0 : W.x[k]) + alpha * __ldg(p + k);
+        r[u] = ro[k] - alpha * __ldg(W.q + k);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const long long k = k0 + u * stride;
+      if (k < n) {
+        W.x[k] = x[u];
+        W.r[k] = r[u];
+        q[0] += r[u] * r[u];
+        q[1] = fmax(q[1], x[u]);
+        q[2] = fmin(q[2], x[u]);
+        q[3] = fmax(q[3], fabs(r[u]));
+      }
+    }
   }
   double out[4];
   if (grid_reduce<4>(q, ops, red_of(W), out)) {
