@@ -85,7 +85,9 @@ struct ins2d_ctx {
   bool p_pending = false;
   double *v_out_host = nullptr;  // erk_step copies V there after its last projection
   bool v_out_done = false;
-  double *h_red = nullptr;      // pinned
+  double *h_red = nullptr;      // pinned: the last reduction's results (valid after a stream synchronisation)
+  unsigned long long *fmax = nullptr;  // F's running maximum and its finished blocks, zero between calls
+  unsigned *fcount = nullptr;
   // host copies of boundary samples (check_conservation.m boundary terms)
   std::vector<double> uLe_i, uRi_i, vLo_i, vUp_i;
   ins2d_bc_sampler_fn sampler = nullptr;
@@ -1055,7 +1057,10 @@ int ins2d_ctx_create(const ins2d_grid_desc *grid, const ins2d_bc_desc *bc, const
     const int maxb = ((nx + 31) / 32) * ((ny + 7) / 8) + 64;
     c->red.partials = dalloc<double>(c, (size_t)maxb * kRedQ);
     c->red.counter = dalloc<unsigned int>(c, 1);
-    c->red.result = dalloc<double>(c, kRedQ);
+    c->fmax = dalloc<unsigned long long>(c, 1);
+    c->fcount = dalloc<unsigned>(c, 1);
+    CK(cudaMemset(c->fmax, 0, sizeof(unsigned long long)));
+    CK(cudaMemset(c->fcount, 0, sizeof(unsigned)));
     c->red.max_blocks = maxb;
     CK(cudaMemset(c->red.counter, 0, sizeof(unsigned int)));
     if (c->poisson == INS2D_POISSON_FFT) {
@@ -1139,6 +1144,7 @@ int ins2d_ctx_create(const ins2d_grid_desc *grid, const ins2d_bc_desc *bc, const
     }
     CK(cudaMallocHost((void **)&c->h_sc, sizeof(PcgScalars)));
     CK(cudaMallocHost((void **)&c->h_red, sizeof(double) * kRedQ));
+    c->red.result = c->h_red;  // the last block of a reduction writes to the host itself
     CK(cudaMallocHost((void **)&c->h_accum, sizeof(SolveAccum)));
     c->accum = dalloc<SolveAccum>(c, 1);
     CK(cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking));
@@ -1337,7 +1343,7 @@ int ins2d_F(ins2d_ctx *ctx, const double *V, const double *C, const double *p, d
   if (dP && dC == dV && !ctx->fp32) {
     // the stencil walkers (the stage kernels' F), which also take max|F|
     Prof pr(ctx, INS2D_PROF_OTHER, 1);
-    CK(launch_F_walk(ctx->P, dV, dP, dO, ctx->red.result, ctx->stream));
+    launch_F_walk(ctx->P, dV, dP, dO, ctx->fmax, ctx->fcount, ctx->h_red, ctx->stream);
   } else {
     // C != V (F.m's linearisation point), nopressure, or FP32-stencil
     // contexts (diagnostics stay FP64): one thread per point
@@ -1345,7 +1351,6 @@ int ins2d_F(ins2d_ctx *ctx, const double *V, const double *C, const double *p, d
     launch_F(ctx->P, dV, dC, dP, dO, ctx->red, ctx->stream);
   }
   CK(cudaGetLastError());
-  CK(cudaMemcpyAsync(ctx->h_red, ctx->red.result, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
   if (mem == INS2D_MEM_HOST) CK(cudaMemcpyAsync(F_out, dO, NV * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   if (maxres) *maxres = ctx->h_red[0];
@@ -1363,7 +1368,6 @@ int ins2d_divergence(ins2d_ctx *ctx, const double *V, double *f_out, double *max
   Prof pr(ctx, INS2D_PROF_OTHER, 1);
   launch_div(ctx->P, dV, 1.0, 0.0, 1.0, dO, true, ctx->red, ctx->stream);
   CK(cudaGetLastError());
-  CK(cudaMemcpyAsync(ctx->h_red, ctx->red.result, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
   if (mem == INS2D_MEM_HOST)
     CK(cudaMemcpyAsync(f_out, dO, (size_t)ctx->P.Np * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
@@ -1585,7 +1589,6 @@ int ins2d_initial_projection(ins2d_ctx *ctx, double *V, double t, double *maxdiv
     launch_div(ctx->P, dV, 1.0, 0.0, 1.0, ctx->f, true, ctx->red, ctx->stream);
   }
   CK(cudaGetLastError());
-  CK(cudaMemcpyAsync(ctx->h_red, ctx->red.result, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   const double md = ctx->h_red[0];
   if (maxdiv) *maxdiv = md;
@@ -1616,7 +1619,6 @@ int ins2d_conservation(ins2d_ctx *ctx, const double *V, double t, double out[4],
   Prof pr(ctx, INS2D_PROF_OTHER, 1);
   launch_conservation(ctx->P, dV, ctx->red, ctx->stream);
   CK(cudaGetLastError());
-  CK(cudaMemcpyAsync(ctx->h_red, ctx->red.result, 5 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   const HostOps &H = ctx->H;
   const double *r = ctx->h_red;

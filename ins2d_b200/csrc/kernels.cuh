@@ -112,9 +112,10 @@ void launch_residual(const DevOps &P, const double *V, const double *p, double *
                      float *kV_next32, bool fp32, cudaStream_t s);
 // F_out = -conv(V) + Diff V + yDiff - (G p + y_p) (F.m:137-145 with C = V and
 // the pressure) by the stencil walkers, FP64 fields and arithmetic; max|F| into
-// *maxres (zeroed on the stream first; a maximum, so its order is immaterial)
-cudaError_t launch_F_walk(const DevOps &P, const double *V, const double *p, double *F_out, double *maxres,
-                          cudaStream_t s);
+// *maxres (host memory), by way of *fmax and *fcount (zero between calls; a
+// maximum, so its order is immaterial)
+void launch_F_walk(const DevOps &P, const double *V, const double *p, double *F_out, unsigned long long *fmax,
+                   unsigned *fcount, double *maxres, cudaStream_t s);
 // F_out = -conv(V;C) + Diff V + yDiff - (G p + y_p) (F.m); maxres into red.result[0]
 void launch_F(const DevOps &P, const double *V, const double *C, const double *p, double *F_out,
               const RedScratch &red, cudaStream_t s);

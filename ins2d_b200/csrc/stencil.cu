@@ -134,14 +134,32 @@ struct Epi {
   float *kV_next32;
   // F: max|F| as the bits of a non-negative double
   unsigned long long *fmax;
+  // in the last launch of an F: the launch's blocks that have finished, and
+  // where its last block writes the maximum (host memory; fmax and the count
+  // are zero again afterwards)
+  unsigned *fcount;
+  double *fhost;
 };
 
+__device__ __forceinline__ void finish_fmax(const Epi &e) {  // one thread per block
+  __threadfence();
+  if (atomicAdd(e.fcount, 1u) != gridDim.x * gridDim.y * gridDim.z - 1) return;
+  *e.fhost = __longlong_as_double((long long)atomicExch(e.fmax, 0ull));
+  *e.fcount = 0u;
+}
 // mode 3: max|F| of the block's points into *e.fmax (every thread calls it; m:
-// its own points' maximum, 0 for none)
+// its own points' maximum, 0 for none).  The result goes to the host from the
+// last block: with a memset before and a copy after the walkers, F and the
+// conservation sums of a 64^2 cavity took 69 us, now 47 (and 2048^2 periodic
+// 159, now 147).
 __device__ __forceinline__ void block_fmax(const Epi &e, double m) {
   for (int off = 16; off > 0; off >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, off));
   if (((threadIdx.x + blockDim.x * threadIdx.y) & 31) == 0 && m > 0.0)
     atomicMax(e.fmax, (unsigned long long)__double_as_longlong(m));
+  if (e.fhost) {
+    __syncthreads();
+    if (threadIdx.x == 0 && threadIdx.y == 0) finish_fmax(e);
+  }
 }
 
 // NP >= 0: that many earlier stages, unrolled; NP < 0: e.nprev
@@ -984,8 +1002,10 @@ __global__ void __launch_bounds__(WX * 2) k_walk(const __grid_constant__ DevOps 
   pdl_wait();
   pdl_trigger();
   if ((int)blockIdx.x >= P.fbx0 && (int)blockIdx.x < P.fbx1 && (int)blockIdx.y >= P.fby0 &&
-      (int)blockIdx.y < P.fby1)
-    return;  // interior tile: handled by k_walk_fast / k_walk_tile
+      (int)blockIdx.y < P.fby1) {  // interior tile: handled by k_walk_fast / k_walk_tile
+    if (e.mode == 3 && e.fhost && threadIdx.x == 0 && threadIdx.y == 0) finish_fmax(e);
+    return;
+  }
   tile_generic<S, TV>(P, V, e, blockIdx.x, blockIdx.y, blockIdx.z, rows);
 }
 
@@ -1120,16 +1140,18 @@ void launch_walk_t(const DevOps &P, const TV *V, const Epi &e, cudaStream_t s) {
   const bool tiled = (sizeof(TV) == 8 ? P.tile_ok : P.tile_ok32) && (((uintptr_t)V & 15) == 0);
   if (has_fast) {
     const dim3 gf(P.fbx1 - P.fbx0, P.fby1 - P.fby0);
+    Epi ef = e;
+    if (!P.all_fast) ef.fhost = nullptr;  // not the last launch
     if (tiled) {
       if (e.mode == 0)
-        launch_tile<S, 0, TV>(P, V, e, s);
+        launch_tile<S, 0, TV>(P, V, ef, s);
       else if (e.mode == 2)
-        launch_tile<S, 2, TV>(P, V, e, s);
+        launch_tile<S, 2, TV>(P, V, ef, s);
       else
-        launch_tile<S, 1, TV>(P, V, e, s);  // residual and F
+        launch_tile<S, 1, TV>(P, V, ef, s);  // residual and F
     } else {
       const int r = walk_rows((long long)gf.x * gf.y);
-      launch_kp(P.pdl, k_walk_fast<S, TV>, dim3(gf.x, gf.y, RUN / r), dim3(WX, 2), 0, s, P, V, e, r);
+      launch_kp(P.pdl, k_walk_fast<S, TV>, dim3(gf.x, gf.y, RUN / r), dim3(WX, 2), 0, s, P, V, ef, r);
     }
   }
   if (!P.all_fast) {
@@ -1285,17 +1307,16 @@ void launch_stage(const DevOps &P, const StageArgs &a, bool fp32, cudaStream_t s
   launch_walk(P, a.V, a.V32, e, fp32, s);
 }
 
-cudaError_t launch_F_walk(const DevOps &P, const double *V, const double *p, double *F_out, double *maxres,
-                          cudaStream_t s) {
-  const cudaError_t ms = cudaMemsetAsync(maxres, 0, sizeof(double), s);
-  if (ms != cudaSuccess) return ms;
+void launch_F_walk(const DevOps &P, const double *V, const double *p, double *F_out, unsigned long long *fmax,
+                   unsigned *fcount, double *maxres, cudaStream_t s) {
   Epi e{};
   e.mode = 3;
   e.p = p;
   e.w = F_out;
-  e.fmax = reinterpret_cast<unsigned long long *>(maxres);
+  e.fmax = fmax;
+  e.fcount = fcount;
+  e.fhost = maxres;
   launch_walk(P, V, nullptr, e, false, s);
-  return cudaSuccess;
 }
 
 void launch_residual(const DevOps &P, const double *V, const double *p, double *w, double *kV_next,
