@@ -357,7 +357,7 @@ int solve_pcg_graph(ins2d_ctx *c, const double *f, double *dp, bool accumulate, 
           CK(pcg_pass_fdm(c->P, c->fdm, c->pcg, f, h, limit, bs));
           c->launches[INS2D_PROF_POISSON] += fdm_pass_kernels(c);
         });
-    pcg_finish_fdm(c->P, c->pcg, dp, accumulate, c->accum, c->stream);
+    pcg_finish_fdm(c->P, c->pcg, dp, accumulate, false, c->accum, c->stream);
     CK(cudaGetLastError());
     return INS2D_OK;
   }
@@ -411,6 +411,13 @@ int read_solve(ins2d_ctx *c, ins2d_solve_stats *st) {
   return solve_outcome(c, st);
 }
 
+// the PCG workspace of a solve whose scalars the host reads
+PcgWork host_work(const ins2d_ctx *c) {
+  PcgWork W = c->pcg;
+  W.hsc = c->h_sc;
+  return W;
+}
+
 bool cluster_solver(const ins2d_ctx *c) { return c->use_fdm && pcg_use_cluster(c->fdm); }
 
 // a small grid's whole solve in one launch (inside a step graph its statistics
@@ -419,10 +426,40 @@ int solve_cluster(ins2d_ctx *c, const SolveSrc &src, double *dp, bool accumulate
   if (st) *st = ins2d_solve_stats{0, 0.0, 0.0};
   {
     Prof pr(c, INS2D_PROF_POISSON, 1);
-    CK(pcg_solve_cluster(c->P, c->fdm, c->pcg, src, dp, tol, c->opts.CG_maxit, accumulate,
+    CK(pcg_solve_cluster(c->P, c->fdm, c->dev_loop ? c->pcg : host_work(c), src, dp, tol, c->opts.CG_maxit, accumulate,
                          c->dev_loop ? c->accum : nullptr, c->stream));
   }
-  return c->dev_loop ? INS2D_OK : read_solve(c, st);
+  if (c->dev_loop) return INS2D_OK;
+  CK(cudaStreamSynchronize(c->stream));
+  return solve_outcome(c, st);
+}
+
+// The fast-diagonalization solve from the host.  Its application is exact up
+// to rounding, so two passes and the (guarded) result are enqueued before the
+// host looks for the first time, and the kernels write the scalars it reads to
+// host memory themselves; passes after convergence return at once.  Against a
+// copy and a synchronisation after each pass, 301 x 257 channel solve: 146 ->
+// 126 us.
+int solve_fdm_host(ins2d_ctx *c, const double *f, double *dp, bool accumulate, ins2d_solve_stats *st, double tol) {
+  const PcgWork W = host_work(c);
+  Prof pr(c, INS2D_PROF_POISSON, 1);
+  pcg_init_fdm(c->P, c->fdm, W, f, tol, c->opts.CG_maxit, 0, -1, c->stream);
+  const long long limit = c->poll_limit >= 0 ? c->poll_limit : (long long)c->opts.CG_maxit + 1024;
+  long long launched = 0;
+  for (long long chunk = std::min(2LL, limit);; chunk = 1) {
+    for (long long k = 0; k < chunk; ++k) {
+      CK(pcg_pass_fdm(c->P, c->fdm, W, f, 0, -1, c->stream));
+      c->launches[INS2D_PROF_POISSON] += fdm_pass_kernels(c);
+    }
+    pcg_finish_fdm(c->P, W, dp, accumulate, true, nullptr, c->stream);
+    c->launches[INS2D_PROF_POISSON] += 1;
+    CK(cudaGetLastError());
+    launched += chunk;
+    CK(cudaStreamSynchronize(c->stream));
+    if (c->h_sc->done) return solve_outcome(c, st);
+    if (launched >= limit)
+      return fail(c, INS2D_ETIMEOUT, "PCG: device convergence flag not set within the host's iteration limit");
+  }
 }
 
 // PCG to the relative residual tol (cg.F's rule ||r|| <= tol ||f||)
@@ -436,7 +473,8 @@ int solve_pcg(ins2d_ctx *c, const double *f, double *dp, bool accumulate, ins2d_
     if (st) *st = ins2d_solve_stats{0, 0.0, 0.0};
     return solve_pcg_graph(c, f, dp, accumulate, tol);
   }
-  const bool block = !c->use_fdm && (c->use_mg ? (c->P.Np <= kPcgBlockMgMaxCells) : pcg_use_block(c->P));
+  if (c->use_fdm) return solve_fdm_host(c, f, dp, accumulate, st, tol);
+  const bool block = (c->use_mg ? (c->P.Np <= kPcgBlockMgMaxCells) : pcg_use_block(c->P));
   Prof pr(c, INS2D_PROF_POISSON, block ? 1 : 2);
   if (block) {
     if (c->use_mg)
@@ -446,31 +484,21 @@ int solve_pcg(ins2d_ctx *c, const double *f, double *dp, bool accumulate, ins2d_
     CK(cudaGetLastError());
     return read_solve(c, st);
   }
-  if (c->use_fdm)
-    pcg_init_fdm(c->P, c->fdm, c->pcg, f, tol, c->opts.CG_maxit, 0, -1, c->stream);
-  else if (c->use_mg)
+  if (c->use_mg)
     pcg_init_mg(c->P, c->mg, c->pcg, f, tol, c->opts.CG_maxit, c->stream);
   else
     pcg_init(c->P, c->pcg, f, tol, c->opts.CG_maxit, c->stream);
   CK(cudaGetLastError());
-  // the fast-diagonalization preconditioner is exact up to rounding: one
-  // iteration at a time between the polls, the first one before any poll
-  // (its kernels return at once when there is nothing to solve)
   const long long limit = c->poll_limit >= 0 ? c->poll_limit : (long long)c->opts.CG_maxit + 1024;
-  int chunk = c->use_fdm ? 1 : (c->use_mg ? 2 : 4);
+  int chunk = c->use_mg ? 2 : 4;
   long long launched = 0;
   for (;;) {
-    if (!(c->use_fdm && launched == 0 && limit > 0)) {
-      CK(cudaMemcpyAsync(c->h_sc, c->pcg.sc, sizeof(PcgScalars), cudaMemcpyDeviceToHost, c->stream));
-      CK(cudaStreamSynchronize(c->stream));
-      if (c->h_sc->done) break;
-      if (launched >= limit)
-        return fail(c, INS2D_ETIMEOUT, "PCG: device convergence flag not set within the host's iteration limit");
-    }
-    if (c->use_fdm) {
-      CK(pcg_pass_fdm(c->P, c->fdm, c->pcg, f, 0, -1, c->stream));
-      c->launches[INS2D_PROF_POISSON] += fdm_pass_kernels(c);
-    } else if (c->use_mg) {
+    CK(cudaMemcpyAsync(c->h_sc, c->pcg.sc, sizeof(PcgScalars), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    if (c->h_sc->done) break;
+    if (launched >= limit)
+      return fail(c, INS2D_ETIMEOUT, "PCG: device convergence flag not set within the host's iteration limit");
+    if (c->use_mg) {
       pcg_iterations_mg(c->P, c->mg, c->pcg, chunk, c->stream);
       c->launches[INS2D_PROF_POISSON] += (long long)(4 + 6 * mg_tail_level(c->mg) + 1) * chunk;
     } else {
@@ -479,14 +507,11 @@ int solve_pcg(ins2d_ctx *c, const double *f, double *dp, bool accumulate, ins2d_
     }
     CK(cudaGetLastError());
     launched += chunk;
-    chunk = c->use_fdm ? 1 : (c->use_mg ? 4 : std::min(chunk * 2, 128));
+    chunk = c->use_mg ? 4 : std::min(chunk * 2, 128);
   }
   const int rc = solve_outcome(c, st);
   if (rc) return rc;
-  if (c->use_fdm)
-    pcg_finish_fdm(c->P, c->pcg, dp, accumulate, nullptr, c->stream);
-  else
-    pcg_finish(c->P, c->pcg, dp, accumulate, c->stream);
+  pcg_finish(c->P, c->pcg, dp, accumulate, c->stream);
   c->launches[INS2D_PROF_POISSON] += 1;
   CK(cudaGetLastError());
   return INS2D_OK;

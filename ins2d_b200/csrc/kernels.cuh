@@ -292,6 +292,7 @@ struct PcgWork {
   PcgScalars *sc;      // device
   double *partials;    // >= blocks * 4
   int blocks;
+  PcgScalars *hsc;     // fast diagonalization: also the solve's scalars as they end a kernel (host memory; may be null)
 };
 void pcg_init(const DevOps &P, const PcgWork &W, const double *f, double tol, long long maxit, cudaStream_t s);
 void pcg_iterations(const DevOps &P, const PcgWork &W, int n, cudaStream_t s);
@@ -311,7 +312,9 @@ void pcg_init_fdm(const DevOps &P, const FdmD &F, const PcgWork &W, const double
                   cudaGraphConditionalHandle h, int limit, cudaStream_t s);
 cudaError_t pcg_pass_fdm(const DevOps &P, const FdmD &F, const PcgWork &W, const double *f,
                          cudaGraphConditionalHandle h, int limit, cudaStream_t s);
-void pcg_finish_fdm(const DevOps &P, const PcgWork &W, double *dp, bool accumulate, SolveAccum *acc, cudaStream_t s);
+// guarded: only when the solve has converged (dp untouched otherwise)
+void pcg_finish_fdm(const DevOps &P, const PcgWork &W, double *dp, bool accumulate, bool guarded, SolveAccum *acc,
+                    cudaStream_t s);
 // condition of the WHILE node around the passes (limit < 0: no graph)
 struct LoopCond {
   cudaGraphConditionalHandle h;

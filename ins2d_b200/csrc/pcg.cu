@@ -537,6 +537,7 @@ __global__ void __launch_bounds__(kVecThreads) k_init_f(const PcgWork W, const d
       s->done = 1;
     }
     set_cond(cond, !s->done && 0 < cond.limit);
+    if (W.hsc) *W.hsc = *s;
   }
 }
 
@@ -624,7 +625,10 @@ __global__ void __launch_bounds__(kVecThreads) k_update_f(const PcgWork W, const
   const double alpha = W.sc->alpha;  // read together with done: one latency
   const long long it = W.sc->it;
   if (done) {  // an earlier kernel of this pass found an error
-    if (blockIdx.x == 0 && threadIdx.x == 0) set_cond(cond, false);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      set_cond(cond, false);
+      if (W.hsc) *W.hsc = *W.sc;
+    }
     return;
   }
   const bool first = it == 0;
@@ -678,13 +682,15 @@ __global__ void __launch_bounds__(kVecThreads) k_update_f(const PcgWork W, const
     const int loops = s->loops + 1;
     s->loops = loops;
     set_cond(cond, !s->done && loops < cond.limit);
+    if (W.hsc) *W.hsc = *s;
   }
 }
 
 // dp = x or dp += x (x = 0 when no pass ran); acc (may be null): the solve's
 // statistics
 __global__ void __launch_bounds__(kVecThreads) k_finish_f(const PcgWork W, double *__restrict__ dp, long long n,
-                                                          int accumulate, SolveAccum *acc) {
+                                                          int accumulate, int guarded, SolveAccum *acc) {
+  if (guarded && (!W.sc->done || W.sc->status != 0)) return;
   const bool none = W.sc->it == 0;
   const long long stride = (long long)gridDim.x * blockDim.x;
 #pragma unroll 4
@@ -858,8 +864,9 @@ cudaError_t pcg_pass_fdm(const DevOps &P, const FdmD &F, const PcgWork &W, const
   return cudaSuccess;
 }
 
-void pcg_finish_fdm(const DevOps &P, const PcgWork &W, double *dp, bool accumulate, SolveAccum *acc, cudaStream_t s) {
-  k_finish_f<<<vec_blocks_f(P, W), kVecThreads, 0, s>>>(W, dp, P.Np, accumulate ? 1 : 0, acc);
+void pcg_finish_fdm(const DevOps &P, const PcgWork &W, double *dp, bool accumulate, bool guarded, SolveAccum *acc,
+                    cudaStream_t s) {
+  k_finish_f<<<vec_blocks_f(P, W), kVecThreads, 0, s>>>(W, dp, P.Np, accumulate ? 1 : 0, guarded ? 1 : 0, acc);
 }
 
 namespace {

@@ -458,6 +458,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     out->tol2 = tol2;
     out->maxit = maxit;
     if (acc) solve_accum(out, acc);
+    if (W.hsc) *W.hsc = *out;
   }
   cl.sync();  // no block leaves while another may still write to its shared memory
 }
