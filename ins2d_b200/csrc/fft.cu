@@ -180,6 +180,100 @@ __global__ void __launch_bounds__(kThreads) k_rows_c2r(const __grid_constant__ F
   }
 }
 
+// The whole solve in one block: every line of a pass at once in shared memory,
+// the arithmetic of the three kernels above.  For grids whose three launches
+// are bound by their latency (fft_small).
+constexpr int kSmallThreads = 512;  // 256, 768 and 1024: a step of 40 x 40 in 101, 95 and 106 us instead of 93
+template <int SRC>
+__global__ void __launch_bounds__(kSmallThreads) k_fft_small(const __grid_constant__ FftLine Lx,
+                                                             const __grid_constant__ FftLine Ly, int cap,
+                                                             const double2 *__restrict__ tx,
+                                                             const double2 *__restrict__ ty,
+                                                             const double *__restrict__ f, const WSplit ws,
+                                                             const __grid_constant__ DevOps P, double alpha,
+                                                             double beta, double gamma, double *__restrict__ out,
+                                                             int accumulate, unsigned long long *__restrict__ maxbits,
+                                                             const unsigned long long *__restrict__ gate,
+                                                             const int *__restrict__ skip) {
+  extern __shared__ double2 sm[];
+  __shared__ double wmax[kSmallThreads / 32];
+  if (skip && *(volatile const int *)skip) return;
+  const int Nx = Lx.n, Ny = Ly.n, H = Nx / 2 + 1, pairs = (Ny + 1) / 2;
+  const int ldx = line_ld(Nx), ldy = line_ld(Ny);
+  double2 *a = sm, *b = sm + cap;
+  for (int o = threadIdx.x; o < pairs * Nx; o += kSmallThreads) {
+    const int q = o / Nx, k = o - q * Nx, j0 = 2 * q, j1 = j0 + 1;
+    const bool has1 = j1 < Ny;
+    double2 v;
+    if constexpr (SRC == 0)
+      v = make_double2(__ldg(f + (size_t)j0 * Nx + k), has1 ? __ldg(f + (size_t)j1 * Nx + k) : 0.0);
+    else if constexpr (SRC == 1)
+      v = make_double2(div_cell(P, f, alpha, beta, gamma, k, j0), has1 ? div_cell(P, f, alpha, beta, gamma, k, j1) : 0.0);
+    else
+      v = make_double2(div_cell_f(P, ws, alpha, beta, gamma, k, j0),
+                       has1 ? div_cell_f(P, ws, alpha, beta, gamma, k, j1) : 0.0);
+    a[q * ldx + line_slot(k)] = v;
+  }
+  __syncthreads();
+  const double2 *Z = line_transform(Lx, a, b, pairs, ldx, tx);
+  double2 *c = Z == a ? b : a, *d = Z == a ? a : b;
+  for (int o = threadIdx.x; o < pairs * H; o += kSmallThreads) {
+    const int q = o / H, I = o - q * H, j0 = 2 * q;
+    const double2 z = Z[q * ldx + line_slot(I)], m = Z[q * ldx + line_slot(I ? Nx - I : 0)];
+    c[I * ldy + line_slot(j0)] = make_double2(0.5 * (z.x + m.x), 0.5 * (z.y - m.y));
+    if (j0 + 1 < Ny) c[I * ldy + line_slot(j0 + 1)] = make_double2(0.5 * (z.y + m.y), 0.5 * (m.x - z.x));
+  }
+  __syncthreads();
+  double2 *F = line_transform(Ly, c, d, H, ldy, ty);
+  double lmax = 0.0;
+  for (int o = threadIdx.x; o < H * Ny; o += kSmallThreads) {
+    const int I = o / Ny, J = o - I * Ny;
+    double2 *slot = F + I * ldy + line_slot(J);
+    const double2 v = *slot;
+    lmax = fmax(lmax, v.x * v.x + v.y * v.y);
+    const double lam = (I == 0 && J == 0) ? 1.0 : (P.fft_dxdy * 4.0) * (__ldg(P.fft_ax + I) + __ldg(P.fft_ay + J));
+    const double r = -1.0 / lam;
+    *slot = make_double2(v.y * r, v.x * r);  // exchanged: the next transform is the inverse
+  }
+  for (int off = 16; off > 0; off >>= 1) lmax = fmax(lmax, __shfl_xor_sync(0xffffffffu, lmax, off));
+  if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = lmax;
+  __syncthreads();
+  double mx = wmax[0];
+#pragma unroll
+  for (int w = 1; w < kSmallThreads / 32; ++w) mx = fmax(mx, wmax[w]);
+  mx = sqrt(mx);
+  if (threadIdx.x == 0) *maxbits = (unsigned long long)__double_as_longlong(mx);
+  if (gate) mx = __longlong_as_double((long long)*gate);
+  const size_t n = (size_t)Nx * Ny;
+  if (mx < 1e-14) {  // pressure_poisson.m:21-32: dp stays zero
+    if (!accumulate)
+      for (size_t k = threadIdx.x; k < n; k += kSmallThreads) out[k] = 0.0;
+    return;
+  }
+  const double2 *B = line_transform(Ly, F, F == a ? b : a, H, ldy, ty);
+  double2 *e = B == a ? b : a, *g = B == a ? a : b;
+  const double sy = 1.0 / Ny, sx = 1.0 / Nx;
+  for (int o = threadIdx.x; o < pairs * Nx; o += kSmallThreads) {
+    const int q = o / Nx, k = o - q * Nx, j0 = 2 * q, I = k < H ? k : Nx - k;
+    const double2 u = B[I * ldy + line_slot(j0)];
+    double2 g0 = make_double2(u.y * sy, u.x * sy), g1 = make_double2(0.0, 0.0);
+    if (j0 + 1 < Ny) {
+      const double2 w = B[I * ldy + line_slot(j0 + 1)];
+      g1 = make_double2(w.y * sy, w.x * sy);
+    }
+    if (k >= H) g0.y = -g0.y, g1.y = -g1.y;
+    e[q * ldx + line_slot(k)] = make_double2(g0.y + g1.x, g0.x - g1.y);  // exchanged: inverse transform
+  }
+  __syncthreads();
+  const double2 *R = line_transform(Lx, e, g, pairs, ldx, tx);
+  for (int o = threadIdx.x; o < (int)n; o += kSmallThreads) {
+    const int j = o / Nx, k = o - j * Nx;
+    const double2 w = R[(j >> 1) * ldx + line_slot(k)];
+    const double v = (j & 1 ? w.x : w.y) * sx;
+    out[o] = accumulate ? out[o] + v : v;
+  }
+}
+
 // ---------------------------------------------------------------------------
 // Register groups of up to three radix-2 stages on 8 values x[m] at positions
 // base + m*h (h = half size of the smallest stage of the group, k = base mod h).
@@ -819,6 +913,23 @@ int cols_group(const FftLine &L) {
   const size_t per = 2 * (size_t)line_ld(L.m) * sizeof(double2);
   return (int)std::max<size_t>(1, std::min<size_t>(4, (INS2D_FFT_COLS_BUDGET * 1024) / per));
 }
+// One block for the whole solve: both sides of general length without
+// Bluestein's algorithm, at most INS2D_FFT_SMALL_MAX cells.  Four solves of a
+// step against three kernels each, B200, us per step: 24 x 24 80.6 and 88.8,
+// 40 x 40 92.9 and 96.9 (called from the host a step at a time 181 and 204),
+// 48 x 60 110 and 99: one SM's throughput takes over from the launches' latency.
+#ifndef INS2D_FFT_SMALL_MAX
+#define INS2D_FFT_SMALL_MAX 1800
+#endif
+int fft_small_cap(const FftLine &Lx, const FftLine &Ly) {  // complex values per buffer
+  return std::max((Ly.n + 1) / 2 * line_ld(Lx.n), (Lx.n / 2 + 1) * line_ld(Ly.n));
+}
+bool fft_small(const FftPlan &plan) {
+  if (plan.logx >= kFusedMinLog || plan.logy >= kFusedMinLog || plan.Nx * (long long)plan.Ny > INS2D_FFT_SMALL_MAX)
+    return false;
+  const FftLine Lx = fft_line(plan.Nx), Ly = fft_line(plan.Ny);
+  return Lx.m == Lx.n && Ly.m == Ly.n && 32 * (size_t)fft_small_cap(Lx, Ly) <= 200 * 1024;
+}
 // threads per block for `lines` lines: about one butterfly of radix 4 each
 int line_threads(const FftLine &L, int lines) {
   int t = 32;
@@ -971,6 +1082,9 @@ cudaError_t fft_prepare() {
   opt_in((const void *)k_rows_r2c<1>);
   opt_in((const void *)k_rows_r2c<2>);
   opt_in((const void *)k_cols);
+  opt_in((const void *)k_fft_small<0>);
+  opt_in((const void *)k_fft_small<1>);
+  opt_in((const void *)k_fft_small<2>);
   opt_in((const void *)k_rows_c2r);
   return first;
 }
@@ -985,6 +1099,21 @@ cudaError_t fft_passes(const DevOps &P, const FftPlan &plan, const double *src, 
   const int pairs = (Ny + 1) / 2;
   const int H = Nx / 2 + 1;
   unsigned long long *maxbits = (unsigned long long *)plan.maxabs;
+  if (fft_small(plan)) {
+    const FftLine Lx = fft_line(Nx), Ly = fft_line(Ny);
+    const int cap = fft_small_cap(Lx, Ly), acc = accumulate ? 1 : 0;
+    const size_t sm = 2 * (size_t)cap * sizeof(double2);
+    if (ws)
+      k_fft_small<2><<<1, kSmallThreads, sm, s>>>(Lx, Ly, cap, plan.twx, plan.twy, nullptr, *ws, P, alpha, beta, gamma,
+                                                  dp, acc, maxbits, gate, skip);
+    else if (div)
+      k_fft_small<1><<<1, kSmallThreads, sm, s>>>(Lx, Ly, cap, plan.twx, plan.twy, src, WSplit{}, P, alpha, beta,
+                                                  gamma, dp, acc, maxbits, gate, skip);
+    else
+      k_fft_small<0><<<1, kSmallThreads, sm, s>>>(Lx, Ly, cap, plan.twx, plan.twy, src, WSplit{}, P, 0.0, 0.0, 0.0, dp,
+                                                  acc, maxbits, gate, skip);
+    return cudaSuccess;
+  }
   // rows, real -> half spectrum (the first pass also zeroes max |fhat|: no
   // memset node between the passes)
   const int fastdiv = P.rMX.lo <= 0 && P.rMX.hi >= Nx && P.rMY.lo <= 0 && P.rMY.hi >= Ny && P.rMX.two && P.rMY.two;
@@ -1052,7 +1181,7 @@ cudaError_t launch_fft_poisson(const DevOps &P, const FftPlan &plan, const doubl
   return fft_passes(P, plan, f, nullptr, false, 0.0, 0.0, 0.0, dp, accumulate, s);
 }
 
-int fft_kernels(const FftPlan &) { return 3; }
+int fft_kernels(const FftPlan &plan) { return fft_small(plan) ? 1 : 3; }
 
 cudaError_t launch_fft_poisson_div(const DevOps &P, const FftPlan &plan, const double *W, double alpha,
                                    double beta, double gamma, double *dp, bool accumulate, cudaStream_t s) {

@@ -63,11 +63,13 @@ def test_small_grid_solve(shape, combo):
 # line transforms: every radix and leftover, primes by direct sums (up to 31)
 # and by Bluestein's algorithm (37 and more, up to the longest length), odd
 # lengths, one side a compile-time power of two; right-hand sides given, and
-# formed from a velocity inside the first pass (FP64 and FP32 stages); the last
-# three take a quarter, half and all of the columns a block can hold
+# formed from a velocity inside the first pass (FP64 and FP32 stages); (256, 256) to
+# (4096, 32) take a quarter, half and all of the columns a block can hold, then
+# the largest whole solve in one block and the first in three kernels, and lines
+# of 3 by 500
 @pytest.mark.parametrize("shape", [(2, 3), (6, 2), (12, 10), (40, 32), (31, 29), (49, 37), (125, 343), (74, 961), (64, 1009),
                                    (2039, 64), (2047, 17), (24, 2039), (1000, 600), (1536, 640), (375, 2000), (256, 256), (2048, 128),
-                                   (4096, 32)])
+                                   (4096, 32), (45, 40), (40, 46), (3, 500)])
 def test_line_transforms(shape):
     nx, ny = shape
     x, y = np.arange(nx + 1) / nx * 1.5, np.arange(ny + 1) / ny
