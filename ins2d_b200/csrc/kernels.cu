@@ -85,51 +85,98 @@ __device__ __forceinline__ void project_cell(const DevOps &P, const double *__re
   }
 }
 
-// Each thread projects kProjRows rows (BY apart) of one column, so a warp
-// has that many independent rows of loads in flight and the column's x
-// weights are read once.
+// Each thread projects kProjRows rows (BY apart) of one column: src.load(idx)
+// what it reads at a point, src.store(idx, that, c Om^-1 (G dp)).  A block
+// whose every row of both gradients is regular issues the loads of all its
+// points before the first store; a store between them, or a branch per point,
+// leaves one point's loads in flight at a time.  Ten steps at 512^2 1.052 ->
+// 0.953 ms, two at 2048^2 1.752 -> 1.736 ms; two rows a thread 0.972 and 1.738,
+// four blocks per SM (spills) 0.974 and 1.754.
 #ifndef INS2D_PROJ_ROWS
 #define INS2D_PROJ_ROWS 4
 #endif
+#ifndef INS2D_PROJ_MINB
+#define INS2D_PROJ_MINB 3
+#endif
 constexpr int kProjRows = INS2D_PROJ_ROWS;
-__global__ void __launch_bounds__(256) k_project(const __grid_constant__ DevOps P, const double *__restrict__ Wt,
-                                                const double *__restrict__ dp, double dt, double c,
-                                                double *__restrict__ Vo) {
+template <typename Src>
+__device__ __forceinline__ void project_rows(const DevOps &P, const Src &src, const double *__restrict__ dp, double c) {
+  const int i0 = blockIdx.x * BX, jb = blockIdx.y * (BY * kProjRows), ie = i0 + BX, je = jb + BY * kProjRows;
+  const int i = i0 + threadIdx.x, j0 = jb + threadIdx.y;
+  const RegD &X = P.rMXT, &Y = P.rMYT;
+  if (ie <= P.Nux && ie <= P.Nvx && je <= P.Nuy && je <= P.Nvy && i0 >= X.lo && ie <= X.hi && jb >= Y.lo &&
+      je <= Y.hi) {
+    typename Src::Raw u[kProjRows], v[kProjRows];
+    double gu[kProjRows], gv[kProjRows];
+#pragma unroll
+    for (int r = 0; r < kProjRows; ++r) {
+      const int j = j0 + r * BY;
+      u[r] = src.load((long long)j * P.Nux + i);
+      v[r] = src.load(P.Nu + (long long)j * P.Nvx + i);
+      gu[r] = c * om_inv_u(P, i, j) * (-__ldg(P.hy + j) * reg_x(X, i, dp, (long long)j * P.Npx));
+      gv[r] = c * om_inv_v(P, i, j) * (-__ldg(P.hx + i) * reg_y(Y, j, dp, P.Npx, i));
+    }
+#pragma unroll
+    for (int r = 0; r < kProjRows; ++r) {
+      const int j = j0 + r * BY;
+      src.store((long long)j * P.Nux + i, u[r], gu[r]);
+      src.store(P.Nu + (long long)j * P.Nvx + i, v[r], gv[r]);
+    }
+    return;
+  }
+#pragma unroll 1
+  for (int r = 0; r < kProjRows; ++r) {
+    const int j = j0 + r * BY;
+    if (i < P.Nux && j < P.Nuy) {
+      const long long k = (long long)j * P.Nux + i;
+      src.store(k, src.load(k), c * om_inv_u(P, i, j) * grad_x_fast(P, dp, i, j));
+    }
+    if (i < P.Nvx && j < P.Nvy) {
+      const long long k = P.Nu + (long long)j * P.Nvx + i;
+      src.store(k, src.load(k), c * om_inv_v(P, i, j) * grad_y_fast(P, dp, i, j));
+    }
+  }
+}
+
+struct ProjPlain {
+  const double *Wt;
+  double *Vo;
+  double dt;
+  using Raw = double;
+  __device__ __forceinline__ Raw load(long long k) const { return __ldg(Wt + k); }
+  __device__ __forceinline__ void store(long long k, Raw w, double g) const { Vo[k] = dt * (w - g); }
+};
+__global__ void __launch_bounds__(256, INS2D_PROJ_MINB) k_project(const __grid_constant__ DevOps P,
+                                                                  const double *__restrict__ Wt,
+                                                                  const double *__restrict__ dp, double dt, double c,
+                                                                  double *__restrict__ Vo) {
   pdl_wait();
   pdl_trigger();
-  const int i = blockIdx.x * BX + threadIdx.x;
-  const int j0 = blockIdx.y * (BY * kProjRows) + threadIdx.y;
-#pragma unroll
-  for (int r = 0; r < kProjRows; ++r) project_cell(P, Wt, dp, dt, c, Vo, i, j0 + r * BY);
+  project_rows(P, ProjPlain{Wt, Vo, dt}, dp, c);
 }
 
 // the first stage from the cached residual fused into its projection:
 // Wt = Vn/dt + aii kV0 (k_stage_cached's expression) formed in registers, so
 // Wt is neither written nor read again (the first stage solves no Poisson
 // equation when the boundary conditions are steady: dp = p)
-__global__ void __launch_bounds__(256) k_project_cached(const __grid_constant__ DevOps P,
-                                                       const double *__restrict__ Vn,
-                                                       const double *__restrict__ kV0, double aii, double inv_dt,
-                                                       const double *__restrict__ dp, double dt, double c,
-                                                       double *__restrict__ Vo) {
+struct ProjCached {
+  const double *Vn, *kV0;
+  double *Vo;
+  double aii, inv_dt, dt;
+  struct Raw {
+    double v, k;
+  };
+  __device__ __forceinline__ Raw load(long long k) const { return Raw{__ldg(Vn + k), __ldg(kV0 + k)}; }
+  __device__ __forceinline__ void store(long long k, Raw w, double g) const {
+    Vo[k] = dt * ((w.v * inv_dt + aii * w.k) - g);
+  }
+};
+__global__ void __launch_bounds__(256, INS2D_PROJ_MINB) k_project_cached(
+    const __grid_constant__ DevOps P, const double *__restrict__ Vn, const double *__restrict__ kV0, double aii,
+    double inv_dt, const double *__restrict__ dp, double dt, double c, double *__restrict__ Vo) {
   pdl_wait();
   pdl_trigger();
-  const int i = blockIdx.x * BX + threadIdx.x;
-  const int j0 = blockIdx.y * (BY * kProjRows) + threadIdx.y;
-#pragma unroll
-  for (int r = 0; r < kProjRows; ++r) {
-    const int j = j0 + r * BY;
-    if (i < P.Nux && j < P.Nuy) {
-      const long long idx = (long long)j * P.Nux + i;
-      const double w = Vn[idx] * inv_dt + aii * kV0[idx];
-      Vo[idx] = dt * (w - c * om_inv_u(P, i, j) * grad_x_fast(P, dp, i, j));
-    }
-    if (i < P.Nvx && j < P.Nvy) {
-      const long long idx = P.Nu + (long long)j * P.Nvx + i;
-      const double w = Vn[idx] * inv_dt + aii * kV0[idx];
-      Vo[idx] = dt * (w - c * om_inv_v(P, i, j) * grad_y_fast(P, dp, i, j));
-    }
-  }
+  project_rows(P, ProjCached{Vn, kV0, Vo, aii, inv_dt, dt}, dp, c);
 }
 
 // FP32-storage stages: V_out = Vn + dt (a T - c Om^-1 G dp) in FP64 (T = the
@@ -137,25 +184,28 @@ __global__ void __launch_bounds__(256) k_project_cached(const __grid_constant__ 
 // for the new state (then V_out may be Vn itself: each point is read before it
 // is written by the same thread)
 template <typename TO>
-__global__ void __launch_bounds__(256) k_project32(const __grid_constant__ DevOps P, const double *Vn,
-                                                  const float *__restrict__ T, double a, const double *__restrict__ dp,
-                                                  double dt, double c, TO *Vo) {
+struct Proj32 {
+  const double *Vn;
+  const float *T;
+  TO *Vo;
+  double a, dt;
+  struct Raw {
+    double v;
+    float t;
+  };
+  __device__ __forceinline__ Raw load(long long k) const { return Raw{Vn[k], __ldg(T + k)}; }
+  __device__ __forceinline__ void store(long long k, Raw w, double g) const {
+    Vo[k] = (TO)(w.v + dt * (a * (double)w.t - g));
+  }
+};
+template <typename TO>
+__global__ void __launch_bounds__(256, INS2D_PROJ_MINB) k_project32(const __grid_constant__ DevOps P, const double *Vn,
+                                                                    const float *__restrict__ T, double a,
+                                                                    const double *__restrict__ dp, double dt, double c,
+                                                                    TO *Vo) {
   pdl_wait();
   pdl_trigger();
-  const int i = blockIdx.x * BX + threadIdx.x;
-  const int j0 = blockIdx.y * (BY * kProjRows) + threadIdx.y;
-#pragma unroll
-  for (int r = 0; r < kProjRows; ++r) {
-    const int j = j0 + r * BY;
-    if (i < P.Nux && j < P.Nuy) {
-      const long long idx = (long long)j * P.Nux + i;
-      Vo[idx] = (TO)(Vn[idx] + dt * (a * (double)T[idx] - c * om_inv_u(P, i, j) * grad_x_fast(P, dp, i, j)));
-    }
-    if (i < P.Nvx && j < P.Nvy) {
-      const long long idx = P.Nu + (long long)j * P.Nvx + i;
-      Vo[idx] = (TO)(Vn[idx] + dt * (a * (double)T[idx] - c * om_inv_v(P, i, j) * grad_y_fast(P, dp, i, j)));
-    }
-  }
+  project_rows(P, Proj32<TO>{Vn, T, Vo, a, dt}, dp, c);
 }
 
 __global__ void __launch_bounds__(256) k_correct(const __grid_constant__ DevOps P, const double *__restrict__ Vi,
