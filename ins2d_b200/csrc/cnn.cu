@@ -22,9 +22,10 @@
 //   weight grad    dW[co][t,ci] = sum_p dZ[p][co] A[p+t][ci]          M = 32, N = 288, K = pixels
 // The default path runs on tcgen05.mma with TMEM accumulators: the first two by
 // k_conv_row_tc (k_conv_mid_tc on narrow fields), the weight gradient by
-// k_wgrad_tc.  The other path runs on mma.sync m16n8k16 (k_conv_mid,
-// k_wgrad_mid).  The 1 -> 32 and 32 -> 1 layers (2 x 288 MACs per pixel), the
-// losses (squared error; the residual loss with the context's operator tables),
+// k_wgrad_tc, and the 32 -> 1 layer by k_conv_out_tc, whose FP32 weights are three
+// BF16 parts each.  The other path runs on mma.sync m16n8k16 (k_conv_mid,
+// k_wgrad_mid).  The 1 -> 32 layer, the edge layers' gradients (2 x 288 MACs per
+// pixel), the losses (squared error; the residual loss with the context's operator tables),
 // the solver's odd-part application and Adam are FP32 / FP64 CUDA-core kernels.
 // Per pixel and 32 -> 32 layer the traffic is one read of the input activations
 // and one write of the output (64 bytes each in BF16).
@@ -904,6 +905,158 @@ __global__ void __launch_bounds__(kRThreads, kTcBlocksPerSm)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(taddr), "r"(kRTmemCols) : "memory");
 }
 
+// --- 32 -> 1 on tensor cores (the default path) --------------------------------------
+// y = scale sum_t sum_c W6[t][c] a5[p + t][c] with FP32 weights: each weight is
+// the sum of three BF16 values (24 bits, exact up to its last), so one row of
+// 128 pixels is two MMAs (K = 32 channels) with N = 32 columns: tap t's parts at
+// 3 t .. 3 t + 2, products exact, sums in FP32.  An epilogue thread adds a
+// pixel's parts, keeps per dx the running sums of the three rows it belongs to
+// and exchanges the finished row's with its neighbours through shared memory.
+// Rows come by TMA as in k_conv_row_tc; 126 outputs of 128 columns.  Bound by
+// the epilogue's adds and barriers, near its 67 MB of reads (10 us) for 4 fields
+// of 512^2: 15.5 us on B200, against 40 us on the FP32 cores (k_conv_out).
+constexpr int kOStages = 4;                     // staged rows and accumulators
+constexpr int kORow = kRM * 2 * kC;             // 8192
+constexpr int kOBBytes = kC * kC * 2;
+constexpr int kOW = kRM - 2;                    // output columns of a strip
+constexpr int kOBars = 4 * kOStages + 1;
+constexpr int kOSmem = kOStages * kORow + kOBBytes + 2 * 3 * kRM * 4 + 8 * kOBars + 16;
+constexpr int kOThreads = 192, kOBlocksPerSm = 4;
+__global__ void __launch_bounds__(kOThreads, kOBlocksPerSm)
+    k_conv_out_tc(const __grid_constant__ CUtensorMap a5, const float *__restrict__ w6, float scale,
+                  float *__restrict__ y, int H, int W, int strips, int chunks, int R, int nitems,
+                  unsigned *__restrict__ err) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  uint8_t *sB = smem + kOStages * kORow;
+  float(*sv)[3][kRM] = reinterpret_cast<float(*)[3][kRM]>(sB + kOBBytes);
+  const uint32_t aBase = smem_u32(smem), bBase = smem_u32(sB), bars = bBase + kOBBytes + 2 * 3 * kRM * 4;
+  uint32_t *tslot = reinterpret_cast<uint32_t *>(sB + kOBBytes + 2 * 3 * kRM * 4 + 8 * kOBars);
+  const uint32_t full = bars, empty = bars + 8 * kOStages, tfull = bars + 16 * kOStages, tempty = bars + 24 * kOStages,
+                 drain = bars + 32 * kOStages;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(tslot)),
+                 "r"(kOStages * kC)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+  }
+  if (tid == 0) {
+    for (int k = 0; k < kOBars; ++k)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bars + 8 * k),
+                   "r"(k >= 3 * kOStages && k < 4 * kOStages ? 4 : 1)
+                   : "memory");  // tempty: the four epilogue warps
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  // B: element (n = 3 t + part, k = c) at (c / 8) * 512 + n * 16 + (c % 8) * 2
+  for (int i = tid; i < kC * kC; i += kOThreads) {
+    const int n = i / kC, c = i % kC, t = n / 3, part = n % 3;
+    float w = t < kTaps ? __ldg(w6 + t * kC + c) : 0.0f;
+    for (int q = 0; q < part; ++q) w -= __bfloat162float(__float2bfloat16_rn(w));
+    *reinterpret_cast<bf16 *>(sB + (c >> 3) * 512 + n * 16 + (c & 7) * 2) = __float2bfloat16_rn(w);
+  }
+  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+  const uint32_t taddr = *tslot;
+  pdl_wait();
+  pdl_trigger();
+  bool ok = true;
+  int it = 0;  // rows so far: stage and accumulator it % kOStages
+  struct Item {
+    int x0, y0, rows, b;
+  };
+  auto item_at = [&](int item) {
+    const int sx = item % strips, r = item / strips, c = r % chunks, b = r / chunks;
+    return Item{sx * kOW, c * R, min(R, H - c * R), b};
+  };
+  if (warp < 4) {
+    // a wait that gave up leaves the loop running without waits: the four
+    // warps meet at every row's barrier
+    for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
+      const Item t = item_at(item);
+      float up[3] = {0.0f, 0.0f, 0.0f}, mid[3] = {0.0f, 0.0f, 0.0f};  // rows q - 1 and q without their later taps
+      float *dst = y + ((long long)t.b * H + t.y0) * W + t.x0 + tid;
+      const bool store = tid < kOW && t.x0 + tid < W;
+      for (int q = 0; q < t.rows + 2; ++q, ++it) {
+        const int st = it % kOStages;
+        if (ok) ok = __all_sync(0xffffffffu, mbar_wait(tfull + 8 * st, (it / kOStages) & 1));
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        uint32_t r[2][16];
+        const uint32_t ta = taddr + ((uint32_t)(32 * warp) << 16) + (uint32_t)(kC * st);
+        tmem_ld16(ta, r[0]);
+        tmem_ld16(ta + 16, r[1]);
+        asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+        mbar_arrive_warp(tempty + 8 * st);
+        float v[kTaps];
+#pragma unroll
+        for (int k = 0; k < kTaps; ++k) {
+          auto d = [&](int n) { return __uint_as_float(r[n >> 4][n & 15]); };
+          v[k] = (d(3 * k + 2) + d(3 * k + 1)) + d(3 * k);
+        }
+        float o[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          o[k] = up[k] + v[6 + k];  // this row is dy = +1 of output row q - 2
+          up[k] = mid[k] + v[3 + k];
+          mid[k] = v[k];
+        }
+        if (q < 2) continue;  // the same for all four warps
+#pragma unroll
+        for (int k = 0; k < 3; ++k) sv[it & 1][k][tid] = o[k];
+        asm volatile("bar.sync 1, 128;\n" ::: "memory");
+        if (store)
+          dst[(long long)(q - 2) * W] = scale * (sv[it & 1][0][tid] + sv[it & 1][1][tid + 1] + sv[it & 1][2][tid + 2]);
+      }
+    }
+  } else if (warp == 4) {
+    if (elect_one()) {
+      for (int item = blockIdx.x; ok && item < nitems; item += gridDim.x) {
+        const Item t = item_at(item);
+        for (int q = 0; q < t.rows + 2; ++q, ++it) {
+          const int st = it % kOStages;
+          if (!(ok = mbar_wait(empty + 8 * st, ((it / kOStages) & 1) ^ 1))) break;
+          tma_expect(full + 8 * st, kORow);
+          tma_box(aBase + st * kORow, &a5, t.x0 - 1, t.y0 - 1 + q, t.b, full + 8 * st);
+        }
+      }
+      // the last copies have landed before the block leaves, whatever the other roles met
+      for (int k = max(0, it - kOStages); k < it; ++k) ok &= mbar_wait(full + 8 * (k % kOStages), (k / kOStages) & 1);
+    }
+    ok = __all_sync(0xffffffffu, ok);
+  } else {
+    const bool leader = elect_one();
+    const uint64_t a0 = smem_desc(aBase, 16, 8 * 2 * kC) | kSwizzle64, b0 = smem_desc(bBase, 512, 128);
+    const uint32_t alo = (uint32_t)a0, ahi = (uint32_t)(a0 >> 32), blo = (uint32_t)b0, bhi = (uint32_t)(b0 >> 32);
+    for (int item = blockIdx.x; ok && item < nitems; item += gridDim.x) {
+      const int rows = item_at(item).rows;
+      for (int q = 0; q < rows + 2; ++q, ++it) {
+        const int st = it % kOStages, par = (it / kOStages) & 1;
+        ok = mbar_wait(full + 8 * st, par) && mbar_wait(tempty + 8 * st, par ^ 1);
+        if (!(ok = __all_sync(0xffffffffu, ok))) break;
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        if (!leader) continue;
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          tc_mma_lo(taddr + kC * st, alo + st * (kORow / 16) + 2 * h, ahi, blo + 2 * h * (512 / 16), bhi, kIdesc, (uint32_t)h);
+        tc_commit(empty + 8 * st);
+        tc_commit(tfull + 8 * st);
+      }
+    }
+    if (!ok && leader) {  // MMAs in flight, before the TMEM is freed
+      tc_commit(drain);
+      mbar_wait(drain, 0);
+    }
+  }
+  if (!ok) atomicExch(err, 1u);
+  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+  if (warp == 0)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(taddr), "r"(kOStages * kC) : "memory");
+}
+
 // --- block reductions (fixed order: deterministic) ----------------------------
 template <int NQ>
 __device__ void block_sum(double (&v)[NQ], const bool (&is_max)[NQ], double *out) {
@@ -1422,20 +1575,26 @@ CUtensorMap act_map(const bf16 *p, int B, int H, int W, int npx, int nrows) {
   return m;
 }
 
+// Rows per item for `per` strips of H rows on up to cap blocks: the fewest row
+// steps (R + 2 an item) of the busiest block
+int item_rows(long long per, int H, int cap) {
+  int R = H;
+  long long best = -1;
+  for (int c = 1; c <= (H + 3) / 4 && (c == 1 || per * (c - 1) < 2LL * cap); ++c) {
+    const int r = (H + c - 1) / c;
+    const long long cost = ((per * ((H + r - 1) / r) + cap - 1) / cap) * (r + 2);
+    if (best < 0 || cost < best) best = cost, R = r;
+  }
+  return R;
+}
+
 template <int MODE>
 void launch_mid(ins2d_cnn *net, const bf16 *in, const bf16 *wt, const bf16 *mask, bf16 *out, int B, int H, int W,
                 cudaStream_t s) {
   if (net->path == INS2D_CNN_PATH_TCGEN05 && by_rows(W)) {
     const int strips = (W + kRM - 1) / kRM, cap = kTcBlocksPerSm * net->sms;
-    // rows per item: the fewest row steps (R + 2 an item) of the busiest block
     const long long per = (long long)strips * B;
-    int R = H;
-    long long best = -1;
-    for (int c = 1; c <= (H + 3) / 4 && (c == 1 || per * (c - 1) < 2LL * cap); ++c) {
-      const int r = (H + c - 1) / c;
-      const long long cost = ((per * ((H + r - 1) / r) + cap - 1) / cap) * (r + 2);
-      if (best < 0 || cost < best) best = cost, R = r;
-    }
+    const int R = item_rows(per, H, cap);
     const int chunks = (H + R - 1) / R;
     const int nitems = (int)(per * chunks), grid = std::min(nitems, cap);
     launch_kp(true, k_conv_row_tc<MODE>, grid, kRThreads, kRSmem, s, act_map(in, B, H, W, kRM + 2, 1), wt, mask, out, H,
@@ -1552,12 +1711,21 @@ void forward(ins2d_cnn *net, const float *in, int B, int H, int W, cudaStream_t 
   const long long n = (long long)B * H * W;
   reserve(net, n);
   pack(net, s);
-  const EdgeGrid e = edge_grid(net, B, H, W, kEC), eo = edge_grid(net, B, H, W, kEC - 2);
+  const EdgeGrid e = edge_grid(net, B, H, W, kEC);
   launch_kp(true, k_expand<0>, e.blocks, kEThreads, 0, s, in, net->w + kOffW1, nullptr, net->act[0], B, H, W, e.tx, e.ty);
   for (int l = 0; l < kMid; ++l)
     launch_mid<0>(net, net->act[l], net->wf + l * kSzWm, nullptr, net->act[l + 1], B, H, W, s);
-  launch_kp(true, k_conv_out, eo.blocks, kEThreads, 0, s, net->act[4], net->w + kOffW6, net->out_scale, net->y, B, H,
-            W, eo.tx, eo.ty);
+  if (net->path == INS2D_CNN_PATH_TCGEN05) {
+    const int strips = (W + kOW - 1) / kOW, cap = kOBlocksPerSm * net->sms;
+    const long long per = (long long)strips * B;
+    const int R = item_rows(per, H, cap), chunks = (H + R - 1) / R, nitems = (int)(per * chunks);
+    launch_kp(true, k_conv_out_tc, std::min(nitems, cap), kOThreads, kOSmem, s, act_map(net->act[4], B, H, W, kRM, 1),
+              net->w + kOffW6, net->out_scale, net->y, H, W, strips, chunks, R, nitems, net->flag);
+  } else {
+    const EdgeGrid eo = edge_grid(net, B, H, W, kEC - 2);
+    launch_kp(true, k_conv_out, eo.blocks, kEThreads, 0, s, net->act[4], net->w + kOffW6, net->out_scale, net->y, B, H,
+              W, eo.tx, eo.ty);
+  }
   CK(cudaGetLastError());
 }
 
@@ -1763,6 +1931,7 @@ cudaError_t prepare_kernels() {
   opt_in((const void *)k_conv_mid_tc<0>, kTcSmem);
   opt_in((const void *)k_conv_mid_tc<1>, kTcSmem);
   opt_in((const void *)k_conv_row_tc<0>, kRSmem);
+  opt_in((const void *)k_conv_out_tc, kOSmem);
   opt_in((const void *)k_conv_row_tc<1>, kRSmem);
   return e;
 }
