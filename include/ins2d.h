@@ -70,13 +70,14 @@ extern "C" {
  * the device offers fast diagonalization, a multigrid V-cycle or the Jacobi
  * diagonal.  Either way CG iterates to the same relative residual CG_acc. */
 #define INS2D_PRECOND_DEFAULT 0 /* fast diagonalization where it applies, else multigrid, else Jacobi;
-                                   ensemble members: multigrid */
+                                   ensembles: fast diagonalization where it applies to every member */
 #define INS2D_PRECOND_JACOBI 1
 #define INS2D_PRECOND_MG 2
 /* fast diagonalization: A is separable, A = -(diag(hy) (x) TX + TY (x)
- * diag(hx)), so the generalized eigenbases of the 1D factors TX, TY give its
- * inverse on the range of A as four dense transforms (periodic uniform grids:
- * the Fourier basis, i.e. the FFT solve).  CG then converges in one or two
+ * diag(hx)), so the generalized eigenbasis of one 1D factor and tridiagonal
+ * systems in the other direction give its inverse on the range of A: two dense
+ * transforms and the systems between them (periodic uniform grids: the Fourier
+ * basis, i.e. the FFT solve).  CG then converges in one or two
  * iterations.  Grids up to 1024 cells per direction (set-up O(n^3) on the
  * host), or any periodic uniform grid the FFT solver takes. */
 #define INS2D_PRECOND_FDM 3

@@ -1060,23 +1060,25 @@ bool fft_supported(int Nx, int Ny) {
 // device (called once per context); returns the first failure.
 cudaError_t fft_prepare() {
   cudaError_t first = cudaSuccess;
-  auto opt_in = [&](const void *k) {
+  auto opt_in = [&](const void *k, size_t bytes = 200 * 1024) {
+    if (bytes <= 47 * 1024) return;  // within every kernel's default; the call would load the kernel (about 0.1 ms)
     const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     if (first == cudaSuccess) first = e;
   };
   for (int l = kFusedMinLog; l <= 13; ++l)
     with_log2<kFusedMinLog>(l, [&](auto c) {
       constexpr int L = decltype(c)::value;
-      opt_in((const void *)k_rows_r2c_t<L, 0>);
-      opt_in((const void *)k_rows_r2c_t<L, 1>);
-      opt_in((const void *)k_rows_r2c_t<L, 2>);
+      constexpr size_t rows = (size_t)paddedl<L>() * sizeof(double2);
+      opt_in((const void *)k_rows_r2c_t<L, 0>, rows);
+      opt_in((const void *)k_rows_r2c_t<L, 1>, rows);
+      opt_in((const void *)k_rows_r2c_t<L, 2>, rows);
       constexpr int G = cols_per_block<L>();
-      opt_in((const void *)k_cols_t<L, G, cols_radix<L>()>);
+      opt_in((const void *)k_cols_t<L, G, cols_radix<L>()>, cols_smem<L, G>());
       if constexpr (G >= 4) {
-        opt_in((const void *)k_cols_t<L, G / 2, cols_radix<L>()>);
-        opt_in((const void *)k_cols_t<L, G / 4, cols_radix<L>()>);
+        opt_in((const void *)k_cols_t<L, G / 2, cols_radix<L>()>, cols_smem<L, G / 2>());
+        opt_in((const void *)k_cols_t<L, G / 4, cols_radix<L>()>, cols_smem<L, G / 4>());
       }
-      opt_in((const void *)k_rows_c2r_t<L>);
+      opt_in((const void *)k_rows_c2r_t<L>, rows);
     });
   opt_in((const void *)k_rows_r2c<0>);
   opt_in((const void *)k_rows_r2c<1>);

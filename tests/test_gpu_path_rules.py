@@ -116,3 +116,78 @@ def test_network_tiles(shape, path):
     for a, b in zip(bounds[:-1], bounds[1:]):
         assert L._rel(g[a:b], g_ref[a:b]) < 1e-2, (a, b)
     assert L._rel(g[N.OFF_W6:], g_ref[N.OFF_W6:]) < 1e-5
+
+
+# F's maximum and the conservation sums, written to the host by the last block
+# of the last launch: no interior tile, interior and boundary tiles, interior
+# tiles only; a later call's smaller maximum.  Sums of n terms: n rounding
+# errors of the sum of their sizes at the most, far fewer in blocks of 256
+@pytest.mark.parametrize("shape,bc", [((3, 2), "cavity"), ((64, 32), "periodic"), ((128, 64), "periodic"),
+                                      ((300, 260), "cavity"), ((257, 321), "channel"), ((320, 96), "per_x_walls")])
+def test_results_to_host(shape, bc):
+    uBC, vBC = smooth_bc(3)
+    kw = dict(Re=50.0) if bc == "periodic" else dict(Re=50.0, uBC=uBC, vBC=vBC)
+    x, y = np.linspace(0.0, 2.0, shape[0] + 1), np.linspace(0.0, 1.0, shape[1] + 1)
+    m = api.Options(x, y, BC_COMBOS[bc], poisson=6 if bc == "periodic" else 4, **kw)
+    o = R.make_options(x, y, BC_COMBOS[bc], poisson=6 if bc == "periodic" else 4, **kw)
+    rng = np.random.default_rng(shape[1])
+    for scale in (1.0, 1e-2):
+        V, p = scale * rng.standard_normal(m.NV), scale * rng.standard_normal(m.Np)
+        mr, F = m.F(V, None, p)
+        mr_ref, F_ref = R.F(V, V, p, 0.0, o)
+        assert _rel(F, F_ref) < 1e-12 and abs(mr - mr_ref) < 1e-12 * mr_ref
+        got, ref = m.check_conservation(V, 0.0), R.check_conservation(V, 0.0, o)
+        top = np.max(np.abs(V)) + 2.0  # and the boundary values
+        assert abs(got[0] - ref[0]) < 1e-12 * top
+        for a, b, s in zip(got[1:], ref[1:], (top, top, top * top)):
+            assert abs(a - b) < 2.0 * 2e-13 * s
+    m.close()
+
+
+# the fast diagonalization's systems of two and four warps per row and its
+# products' ragged tiles; the stopping rule with a factor 2 for the residual's
+# rounding (at 1e-10: rows of 1000 cells round at about 1e-12)
+@pytest.mark.parametrize("combo", ["cavity", "per_x_walls", "per_y_open"])
+@pytest.mark.parametrize("shape", [(257, 20), (20, 512), (513, 20), (24, 1024), (1024, 33), (130, 129)])
+def test_long_rows(shape, combo):
+    bc = BC_COMBOS[combo]
+    x, y = grid_stretched(shape[0], 0.0, 1.7), grid_stretched(shape[1], -0.5, 0.5, beta=1.2)
+    m = api.Options(x, y, bc, poisson=4, CG_acc=1e-10, CG_maxit=50, precond="fdm")
+    o = R.make_options(x, y, bc, poisson=1)
+    f = o.discretization.M @ np.random.default_rng(5).standard_normal(o.grid.NV)
+    dp, st = m.pressure_poisson(f, return_stats=True)
+    assert np.linalg.norm(o.discretization.A @ dp - f) <= 2e-10 * np.linalg.norm(f) and st["iters"] <= 4
+    assert np.all(m.pressure_poisson(np.zeros(m.Np)) == 0.0)
+    m.close()
+
+
+# ensembles of members below a tile, of a ring of boundary points only, and of
+# several tiles, against their own runs (solver tolerance 1e-12 per solve)
+def test_ensemble_edges():
+    import ins2d_b200
+    from ins2d_b200 import cases
+    members = []
+    for k, (nx, ny) in enumerate([(4, 3), (5, 40), (33, 31), (65, 200), (32, 32), (140, 6)]):
+        kw = dict(Re=200.0, poisson=4, CG_acc=1e-12, CG_maxit=200, RK="RK44")
+        if k % 2 == 0:
+            kw.update(x=cases.tanh_grid(nx, 0.0, 1.0, 1.05), y=cases.tanh_grid(ny, 0.0, 1.0, 1.05),
+                      BC=cases.BC_CAVITY, uBC=cases.lid_uBC(1.0, 1.0))
+        else:
+            kw.update(x=cases.tanh_grid(nx, 0.0, 4.0, 1.05), y=cases.tanh_grid(ny, -0.5, 0.5, 1.05),
+                      BC=cases.BC_CHANNEL, uBC=cases.channel_uBC(lambda yy: 1 - 4 * np.asarray(yy) ** 2))
+        members.append(kw)
+    ens = ins2d_b200.Ensemble(members)
+    ens.set_solver(0)
+    singles, V0 = [], []
+    for k, kw in enumerate(members):
+        m = ins2d_b200.Options(**kw)
+        V = np.zeros(m.NV)
+        p = m.pressure_additional_solve(V, np.zeros(m.Np), 0.0)
+        ens.set_state(k, V, p)
+        singles.append(m)
+        V0.append((V, p))
+    ens.time_ERK(0.0, 1e-4, 4)
+    for k, m in enumerate(singles):
+        V, p = ens.get_state(k)
+        Vs, ps = m.time_ERK(V0[k][0], V0[k][1], 0.0, 1e-4, nsteps=4)
+        assert _rel(V, Vs) < 1e-9 and _rel(p, ps) < 1e-7, (k, _rel(V, Vs), _rel(p, ps))
