@@ -2044,6 +2044,7 @@ void ens_build_batch(ins2d_ens *e, const std::vector<int> &order) {
     cg[m] = EnsCg{};
     cg[m].tol2 = e->tol2;
     cg[m].maxit = e->maxit;
+    cg[m].zero = 1;
     if (e->use_fdm) {
       const DevOps &P = e->mem[m]->P;
       cg[m].part = ens_alloc<double>(e, ens_fdm_scratch(P.Npx, P.Npy));

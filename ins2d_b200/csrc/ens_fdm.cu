@@ -105,6 +105,8 @@ __global__ void __launch_bounds__(kThreads) k_ef_init(const EnsFdmRun R, int mod
     }
     if (done) add_stats(C, R.stats[t.x]);
     C.done = done;
+    C.stage = mode == 0;
+    if (done && C.stage && C.status == 0) C.zero = 1;
     end_member(R, cond, !done, true);
   }
 }
@@ -163,7 +165,8 @@ __global__ void __launch_bounds__(kThreads) k_ef_step(const EnsFdmRun R) {
 }
 
 // x += alpha p, r -= alpha q (x = 0, r = f before the first pass), the stopping
-// rule, statistics and loop condition
+// rule, statistics and loop condition; a stage's solution becomes the member's
+// when it has converged (a failed solve leaves the one before)
 __global__ void __launch_bounds__(kThreads) k_ef_update(const EnsFdmRun R, const LoopCond cond) {
   const int4 t = R.tiles[blockIdx.x];
   EnsCg &C = R.cg[t.x];
@@ -171,7 +174,9 @@ __global__ void __launch_bounds__(kThreads) k_ef_update(const EnsFdmRun R, const
   const int stop = *(volatile int *)&C.done;  // with the other scalars: one latency
   const long long it = C.it;
   const double alpha = C.alpha;
+  const int sol = C.sol;
   const PcgWork W = M.W;
+  double *xw = sol == 0 ? M.dp : M.W.x;
   const double *__restrict__ f = M.f;
   const int Np = (int)M.P.Np;
   if (stop) {
@@ -189,7 +194,7 @@ __global__ void __launch_bounds__(kThreads) k_ef_update(const EnsFdmRun R, const
     const int k = t.y + u * kThreads + threadIdx.x;
     x[u] = r[u] = 0.0;
     if (k < Np) {
-      x[u] = (first ? 0.0 : W.x[k]) + alpha * __ldg(p + k);
+      x[u] = (first ? 0.0 : xw[k]) + alpha * __ldg(p + k);
       r[u] = ro[k] - alpha * __ldg(W.q + k);
     }
   }
@@ -197,7 +202,7 @@ __global__ void __launch_bounds__(kThreads) k_ef_update(const EnsFdmRun R, const
   for (int u = 0; u < kPer; ++u) {
     const int k = t.y + u * kThreads + threadIdx.x;
     if (k < Np) {
-      W.x[k] = x[u];
+      xw[k] = x[u];
       W.r[k] = r[u];
       q[0] += r[u] * r[u];
     }
@@ -222,6 +227,10 @@ __global__ void __launch_bounds__(kThreads) k_ef_update(const EnsFdmRun R, const
     }
     if (done) add_stats(C, R.stats[t.x]);
     C.done = done;
+    if (done && C.stage && C.status == 0) {
+      C.sol = sol ^ 1;
+      C.zero = 0;
+    }
     end_member(R, cond, !done, false);
   }
 }
@@ -231,10 +240,11 @@ __global__ void __launch_bounds__(kThreads) k_ef_finish(const EnsFdmRun R) {
   const EnsCg &C = R.cg[t.x];
   if (C.it == 0 || C.status != 0) return;
   const EnsMemberD &M = R.mem[t.x];
+  const double *__restrict__ x = C.sol == 0 ? M.dp : M.W.x;
 #pragma unroll
   for (int u = 0; u < kPer; ++u) {
     const int k = t.y + u * kThreads + threadIdx.x;
-    if (k < M.P.Np) M.p[k] += M.W.x[k];
+    if (k < M.P.Np) M.p[k] += x[k];
   }
 }
 

@@ -330,9 +330,17 @@ __global__ void __launch_bounds__(256) k_project_ens(const EnsMemberD *__restric
   const EnsMemberD &M = mem[t.x];
   copy_ops(&sP, &M.P);
   __syncthreads();
-  const bool zero = cg && cg[t.x].it == 0;  // solved without a pass: dp = 0 (any finite field will do)
-  project_cell(sP, M.Wt, from_p ? M.p : (cg ? (zero ? M.f : M.W.x) : M.dp), M.dt, zero ? 0.0 : c, last ? M.V : M.Vs,
-               t.y * BX + threadIdx.x, t.z * BY + threadIdx.y);
+  const int i = t.y * BX + threadIdx.x, j = t.z * BY + threadIdx.y;
+  double *__restrict__ Vo = last ? M.V : M.Vs;
+  if (cg && cg[t.x].zero) {  // dp = 0
+    if (i < sP.Nux && j < sP.Nuy) Vo[(long long)j * sP.Nux + i] = M.dt * M.Wt[(long long)j * sP.Nux + i];
+    if (i < sP.Nvx && j < sP.Nvy) {
+      const long long k = sP.Nu + (long long)j * sP.Nvx + i;
+      Vo[k] = M.dt * M.Wt[k];
+    }
+    return;
+  }
+  project_cell(sP, M.Wt, from_p ? M.p : (cg && cg[t.x].sol == 0 ? M.W.x : M.dp), M.dt, c, Vo, i, j);
 }
 
 __global__ void __launch_bounds__(256) k_stage_cached_ens(const EnsMemberD *__restrict__ mem,

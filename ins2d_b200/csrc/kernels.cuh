@@ -174,9 +174,9 @@ void launch_walk_ens(const EnsMemberD *mem, const int4 *work, int n, int rows, c
 void cell_tiles(const DevOps &P, int member, std::vector<int4> &out);
 // f = (M Wt + yM/dt) gamma (mode 0, stage) or f = M wres (mode 1, residual)
 void launch_div_ens(const EnsMemberD *mem, const int4 *tiles, int n, int mode, double gamma, cudaStream_t s);
-// V_out = dt (Wt - c Om^-1 G dp_src); dp_src = p (from_p) or dp, or the CG
-// iterate where cg is given (zero before its first pass); V_out = V (last
-// stage) or Vs
+// V_out = dt (Wt - c Om^-1 G dp_src); dp_src = p (from_p) or dp, or where cg is
+// given the last converged stage solution (EnsCg::sol); V_out = V (last stage)
+// or Vs
 struct EnsCg;
 void launch_project_ens(const EnsMemberD *mem, const int4 *tiles, int n, double c, int from_p, int last,
                         const EnsCg *cg, cudaStream_t s);
@@ -398,6 +398,10 @@ struct EnsCg {
   double *part;
   unsigned int ticket;
   int ntiles;
+  // the last converged stage solution, which the projection reads: in the
+  // iterate (sol 0) or in dp (1), the running solve taking the other one; none
+  // yet, or solved without a pass: zero.  stage: the running solve is a stage's
+  int sol, zero, stage;
 };
 // --- ensembles with fast diagonalization (ens_fdm.cu) -----------------------
 // cell tiles {member, first cell, number within the member, 0} of kEnsCells
@@ -420,7 +424,7 @@ size_t ens_fdm_scratch(int nx, int ny);
 void ens_fdm_init(const EnsFdmRun &R, int mode, double gamma, cudaGraphConditionalHandle h, int limit, cudaStream_t s);
 // one pass: application, direction and product, update (cf. pcg_pass_fdm)
 void ens_fdm_pass(const EnsFdmRun &R, const EnsFdmPlan &pl, cudaGraphConditionalHandle h, int limit, cudaStream_t s);
-// p += x (the additional solve; a stage's projection reads x itself)
+// p += solution (the additional solve; a stage's projection reads it itself)
 void ens_fdm_finish(const EnsFdmRun &R, cudaStream_t s);
 // members' multigrid levels: lev[m * kMgMaxLevels + l]
 struct EnsMgD {
