@@ -359,7 +359,8 @@ int ins2d_ens_set_solver(ins2d_ens *e, int32_t threads);
 /* form of the member solves chosen by the tuner on the first run: threads
  * per member of the persistent solve (512 or 256; 0 = solves batched across
  * members, one launch per phase), its resident blocks, and the tuner's
- * timings (ms of one solve phase for 512, 256 threads and batched) */
+ * timings (ms of one solve phase for 512, 256 threads and batched; zero for a
+ * fast-diagonalization ensemble, which has the batched form only) */
 int ins2d_ens_solve_shape(const ins2d_ens *e, int32_t *threads, int32_t *blocks, double tuned_ms[3]);
 
 /* --- learned initial guess of the PCG ---------------------------------------

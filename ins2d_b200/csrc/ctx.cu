@@ -2060,33 +2060,21 @@ void ens_build_batch(ins2d_ens *e, const std::vector<int> &order) {
     R.mem = e->d_mem;
     R.cg = e->d_cg;
     R.stats = e->d_stats;
-    R.active = e->d_active;
     R.loops = e->d_loops;
   }
 }
 
 // The same with fast diagonalization (ens_fdm.cu), from the velocities: mode 0
 // solves the stage's equation (the projection reads the solution), 1 adds the
-// additional solve's to p.
+// additional solve's to p.  Always inside a step graph: the passes are a WHILE
+// node.
 void ens_solve_fdm(ins2d_ens *e, int mode, double gamma) {
   const EnsFdmRun &R = e->fdm_run;
   cudaStream_t s = e->stream;
-  if (e->dev_loop) {
-    const int limit = (int)std::min<long long>(e->maxit + 4, 1 << 30);
-    capture_while(
-        s, e->body_stream, [&](cudaGraphConditionalHandle h) { ens_fdm_init(R, mode, gamma, h, limit, s); },
-        [&](cudaStream_t bs, cudaGraphConditionalHandle h) { ens_fdm_pass(R, e->fdm_plan, h, limit, bs); });
-  } else {
-    ens_fdm_init(R, mode, gamma, 0, -1, s);
-    for (long long done_it = 0;; ++done_it) {
-      ens_fdm_pass(R, e->fdm_plan, 0, -1, s);
-      CK(cudaGetLastError());
-      CK(cudaMemcpyAsync(e->h_active, e->d_active, sizeof(int), cudaMemcpyDeviceToHost, s));
-      CK(cudaStreamSynchronize(s));
-      if (*e->h_active == 0) break;
-      if (done_it > e->maxit + 2) throw CudaError("ensemble PCG: members still active after CG_maxit");
-    }
-  }
+  const int limit = (int)std::min<long long>(e->maxit + 4, 1 << 30);
+  capture_while(
+      s, e->body_stream, [&](cudaGraphConditionalHandle h) { ens_fdm_init(R, mode, gamma, h, limit, s); },
+      [&](cudaStream_t bs, cudaGraphConditionalHandle h) { ens_fdm_pass(R, e->fdm_plan, h, limit, bs); });
   if (mode == 1) ens_fdm_finish(R, s);
 }
 
@@ -2267,9 +2255,8 @@ void ens_step(ins2d_ens *e, bool k0_cached) {
 // reductions) and keeps the fastest.
 void ens_autotune(ins2d_ens *e) {
   const int sms = sm_count(e->device), n = (int)e->mem.size();
-  // 0: batched across members; fast-diagonalization ensembles solve batched
-  const int cand[3] = {e->use_fdm ? 0 : 512, 256, 0};
-  const int ncand = e->use_fdm ? 1 : (e->can_batch ? 3 : 2);
+  const int cand[3] = {512, 256, 0};  // 0: batched across members
+  const int ncand = e->can_batch ? 3 : 2;
   cudaEvent_t a, b;
   CK(cudaEventCreate(&a));
   CK(cudaEventCreate(&b));
@@ -2278,15 +2265,9 @@ void ens_autotune(ins2d_ens *e) {
   for (int k = 0; k < ncand; ++k) {
     e->solve_threads = cand[k];
     e->solve_blocks = cand[k] ? std::min(n, sms * (512 / cand[k])) : 0;
-    auto solve = [&] {
-      if (e->use_fdm)
-        ens_solve_fdm(e, 0, 1.0);
-      else
-        ens_solve(e, 0);
-    };
-    solve();  // warm-up
+    ens_solve(e, 0);  // warm-up
     CK(cudaEventRecord(a, e->stream));
-    solve();
+    ens_solve(e, 0);
     CK(cudaEventRecord(b, e->stream));
     CK(cudaEventSynchronize(b));
     float ms = 0.f;
@@ -2528,13 +2509,14 @@ int ins2d_ens_erk_run(ins2d_ens *e, double t, double dt, int32_t nsteps, ins2d_s
   CK(cudaMemsetAsync(e->d_stats, 0, n * sizeof(EnsStats), e->stream));
   for (int k = 0; k < nsteps; ++k) {
     const int g = k > 0 ? 1 : 0;  // graph 1: first stage from the cached residual
-    if (e->forced < 0 && !e->tuned) {
+    if (e->forced < 0 && !e->tuned && !e->use_fdm) {
       // first use: one direct step, then tune the solve launch on the
       // right-hand side it left behind (re-solving it changes no state: the
       // tuner writes dp, which every stage overwrites); the step's
-      // statistics are kept
-      e->solve_threads = e->use_fdm ? 0 : 512;
-      e->solve_blocks = e->use_fdm ? 0 : std::min(n, sm_count(e->device));
+      // statistics are kept.  Fast diagonalization has one form only, and its
+      // solves leave a field that a later failed one falls back to.
+      e->solve_threads = 512;
+      e->solve_blocks = std::min(n, sm_count(e->device));
       ens_step(e, g == 1);
       std::vector<EnsStats> keep(n);
       CK(cudaMemcpyAsync(keep.data(), e->d_stats, n * sizeof(EnsStats), cudaMemcpyDeviceToHost, e->stream));

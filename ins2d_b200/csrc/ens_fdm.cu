@@ -51,7 +51,6 @@ __device__ __forceinline__ void end_member(const EnsFdmRun &R, const LoopCond &c
   if ((unsigned)t != (unsigned)R.n) return;
   const int act = (int)(t >> 32), loops = first ? 0 : *R.loops + 1;
   *R.ticket = 0ull;
-  *R.active = act;
   *R.loops = loops;
   set_cond(cond, act > 0 && loops < cond.limit);
 }

@@ -414,7 +414,6 @@ struct EnsFdmRun {
   const int4 *tiles;
   int ntiles, n;      // cell tiles, members
   unsigned long long *ticket;  // members finished (low half) and still iterating (high half) in a launch; else zero
-  int *active;        // members still iterating
   int *loops;         // passes of the current solve
 };
 // doubles of a member's reduction scratch

@@ -45,3 +45,26 @@ def test_unconverged_member_projection(solver, nsteps):
         Ve, pe = ens.get_state(m)
         assert np.max(np.abs(Ve - V)) <= 1e-12 * np.max(np.abs(V)), m
         assert np.all(pe == 0.0)
+
+
+# A fast-diagonalization ensemble has one form of solve and times none: a first
+# run in the tuned setting takes the steps of a second ensemble's with the form
+# given, and its statistics count those solves only
+def test_ensemble_without_tuning():
+    import ins2d_b200
+    from ins2d_b200 import ensembles
+    states, ens = [], None
+    for solver in (-1, 0):
+        members = ensembles.random_members(3, seed=3, sizes=(24, 40), CG_acc=1e-12)
+        ens = ins2d_b200.Ensemble(members)
+        ens.set_solver(solver)
+        for m in range(3):
+            o = ens.member(m)
+            ens.set_state(m, np.zeros(o.NV), np.zeros(o.Np))
+        st = ens.time_ERK(0.0, 1e-4, 3)
+        assert all(s["n_solves"] == 12 for s in st)
+        shape = ens.solve_shape()
+        assert shape["batched"] and all(v == 0.0 for v in shape["tuned_ms"].values())
+        states.append([ens.get_state(m) for m in range(3)])
+    for a, b in zip(*states):
+        assert all(np.array_equal(p, q) for p, q in zip(a, b))
