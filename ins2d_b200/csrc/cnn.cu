@@ -915,6 +915,9 @@ __global__ void __launch_bounds__(kRThreads, kTcBlocksPerSm)
 // Rows come by TMA as in k_conv_row_tc; 126 outputs of 128 columns.  Bound by
 // the epilogue's adds and barriers, near its 67 MB of reads (10 us) for 4 fields
 // of 512^2: 15.5 us on B200, against 40 us on the FP32 cores (k_conv_out).
+// Parts of an infinite activation cancel (or meet a zero part), and a weight
+// beyond BF16's range has infinite parts: a result that is not finite is formed
+// again from the FP32 weights (conv_out_pixel).
 constexpr int kOStages = 4;                     // staged rows and accumulators
 constexpr int kORow = kRM * 2 * kC;             // 8192
 constexpr int kOBBytes = kC * kC * 2;
@@ -922,9 +925,22 @@ constexpr int kOW = kRM - 2;                    // output columns of a strip
 constexpr int kOBars = 4 * kOStages + 1;
 constexpr int kOSmem = kOStages * kORow + kOBBytes + 2 * 3 * kRM * 4 + 8 * kOBars + 16;
 constexpr int kOThreads = 192, kOBlocksPerSm = 4;
+
+// layer 6 at pixel (x, y) of the field at a: FP32 sums over the taps inside it
+__device__ __noinline__ float conv_out_pixel(const bf16 *__restrict__ a, const float *__restrict__ w6, float scale,
+                                             int x, int y, int H, int W) {
+  float s = 0.0f;
+  for (int t = 0; t < kTaps; ++t) {
+    const int xx = x + t % 3 - 1, yy = y + t / 3 - 1;
+    if (xx < 0 || xx >= W || yy < 0 || yy >= H) continue;
+    for (int c = 0; c < kC; ++c) s = fmaf(__ldg(w6 + t * kC + c), __bfloat162float(a[((long long)yy * W + xx) * kC + c]), s);
+  }
+  return scale * s;
+}
+
 __global__ void __launch_bounds__(kOThreads, kOBlocksPerSm)
-    k_conv_out_tc(const __grid_constant__ CUtensorMap a5, const float *__restrict__ w6, float scale,
-                  float *__restrict__ y, int H, int W, int strips, int chunks, int R, int nitems,
+    k_conv_out_tc(const __grid_constant__ CUtensorMap a5, const bf16 *__restrict__ act, const float *__restrict__ w6,
+                  float scale, float *__restrict__ y, int H, int W, int strips, int chunks, int R, int nitems,
                   unsigned *__restrict__ err) {
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t *sB = smem + kOStages * kORow;
@@ -1006,8 +1022,12 @@ __global__ void __launch_bounds__(kOThreads, kOBlocksPerSm)
 #pragma unroll
         for (int k = 0; k < 3; ++k) sv[it & 1][k][tid] = o[k];
         asm volatile("bar.sync 1, 128;\n" ::: "memory");
-        if (store)
-          dst[(long long)(q - 2) * W] = scale * (sv[it & 1][0][tid] + sv[it & 1][1][tid + 1] + sv[it & 1][2][tid + 2]);
+        if (store) {
+          float s = scale * (sv[it & 1][0][tid] + sv[it & 1][1][tid + 1] + sv[it & 1][2][tid + 2]);
+          if (!isfinite(s))
+            s = conv_out_pixel(act + (long long)t.b * H * W * kC, w6, scale, t.x0 + tid, t.y0 + q - 2, H, W);
+          dst[(long long)(q - 2) * W] = s;
+        }
       }
     }
   } else if (warp == 4) {
@@ -1720,7 +1740,7 @@ void forward(ins2d_cnn *net, const float *in, int B, int H, int W, cudaStream_t 
     const long long per = (long long)strips * B;
     const int R = item_rows(per, H, cap), chunks = (H + R - 1) / R, nitems = (int)(per * chunks);
     launch_kp(true, k_conv_out_tc, std::min(nitems, cap), kOThreads, kOSmem, s, act_map(net->act[4], B, H, W, kRM, 1),
-              net->w + kOffW6, net->out_scale, net->y, H, W, strips, chunks, R, nitems, net->flag);
+              net->act[4], net->w + kOffW6, net->out_scale, net->y, H, W, strips, chunks, R, nitems, net->flag);
   } else {
     const EdgeGrid eo = edge_grid(net, B, H, W, kEC - 2);
     launch_kp(true, k_conv_out, eo.blocks, kEThreads, 0, s, net->act[4], net->w + kOffW6, net->out_scale, net->y, B, H,

@@ -1,4 +1,6 @@
 """Behaviour at the edges of what the kernels accept."""
+import functools
+
 import numpy as np
 import pytest
 
@@ -68,3 +70,87 @@ def test_ensemble_without_tuning():
         states.append([ens.get_state(m) for m in range(3)])
     for a, b in zip(*states):
         assert all(np.array_equal(p, q) for p, q in zip(a, b))
+
+
+# Weights of two nonzero taps per output and per input channel: activations
+# are whole numbers up to 64, gradients up to 16 times a power of two, so every
+# value is exact in BF16 and every sum in FP32, and the device's result must
+# equal the oracle's to the last bit.  Tiles of 62 to 128 columns, rows left
+# over, several tiles per block, many small fields.
+@functools.lru_cache(maxsize=1)
+def _exact_case(shape):
+    from oracle import cnn_ref as N
+    rng = np.random.default_rng(shape[1])
+
+    def signs(n):
+        return rng.choice([-1.0, 1.0], n, p=[0.25, 0.75])
+
+    W1, W6, Wm = np.zeros((N.C, N.TAPS)), np.zeros((N.TAPS, N.C)), []
+    for c in range(N.C):
+        W1[c, rng.choice(N.TAPS, 2, replace=False)] = signs(2)
+    for _ in range(N.NMID):
+        W = np.zeros((N.C, N.TAPS, N.C))
+        for _ in range(2):
+            W[np.arange(N.C), rng.integers(N.TAPS, size=N.C), rng.permutation(N.C)] += signs(N.C)
+        Wm.append(W)
+    W6[rng.integers(N.TAPS, size=N.C), np.arange(N.C)] = signs(N.C)
+    w = N.join(W1, Wm, W6)
+    inp = rng.integers(-1, 3, shape).astype(np.float32)
+    y, acts = N.forward(w, 1.0, inp)
+    tgt = (y - rng.integers(-1, 2, shape)).astype(np.float32)
+    loss, g = N.loss_grad(w, 1.0, inp, tgt, acts=acts[1:])
+    assert all(np.mean(q != 0.0) > 0.3 for q in [*N.split(g)[1], *N.split(g)[::2]])  # every layer takes part
+    return w.astype(np.float32), inp, tgt, y, acts, loss, g
+
+
+@pytest.mark.parametrize("shape", [(1, 8, 64), (2, 16, 32), (4, 64, 128), (2, 512, 256), (256, 8, 64)])
+@pytest.mark.parametrize("path", ["tcgen05", "mma_sync"])
+def test_network_exact_arithmetic(path, shape):
+    import torch
+    from ins2d_b200.learned import ConvNet
+    w, inp, tgt, y, acts, loss, g = _exact_case(shape)
+    net = ConvNet(device=0, seed=1)
+    net.set_path(path)
+    net.set_params(w, 1.0)
+    ti, tt = torch.from_numpy(inp).cuda(), torch.from_numpy(tgt).cuda()
+    assert np.array_equal(net.forward(ti).cpu().numpy(), y)
+    for l in range(1, 6):
+        assert np.array_equal(net.activations(l, y.size).reshape(shape + (32,)), acts[l]), l
+    loss_d, g_d = net.loss_grad(ti, tt)
+    assert loss_d == loss and np.array_equal(np.asarray(g_d, dtype=np.float64), g)
+
+
+# The output layer's sums with activations that overflowed to infinity, and
+# with weights beyond BF16's largest value: infinite where one sign of infinity
+# reaches a pixel, NaN where both do, else FP32 sums (the learned tests' bound)
+@pytest.mark.parametrize("path", ["tcgen05", "mma_sync"])
+@pytest.mark.parametrize("what", ["positive", "mixed", "weight"])
+@pytest.mark.parametrize("shape", [(2, 16, 32), (1, 9, 140), (1, 64, 16)])
+def test_output_layer_overflow(shape, what, path):
+    import torch
+    from ins2d_b200.learned import ConvNet
+    from oracle import cnn_ref as N
+    w = _exact_case((2, 16, 32))[0].copy()
+    rng = np.random.default_rng(shape[2])
+    W6 = np.exp2(-100.0) * rng.uniform(0.5, 1.5, N.K)
+    if what == "mixed":
+        W6 *= rng.choice([-1.0, 1.0], N.K)
+    # layer 5's whole numbers by 2^124: 16 and more are infinite
+    w[N.OFF_W6 - N.SZ_WM:N.OFF_W6] *= np.float32(2.0 ** (-30 if what == "weight" else 124))
+    if what == "weight":
+        W6[rng.integers(N.K, size=4)] = 3.4e38
+    w[N.OFF_W6:] = W6
+    net = ConvNet(device=0, seed=1)
+    net.set_path(path)
+    net.set_params(w, 1.0)
+    inp = rng.integers(-1, 3, shape).astype(np.float32)
+    y = net.forward(torch.from_numpy(inp).cuda()).cpu().numpy().astype(np.float64)
+    a5 = net.activations(5, y.size).reshape(shape + (N.C,)).astype(np.float64)
+    with np.errstate(invalid="ignore"):
+        ref = N.layer(w.astype(np.float64), 6, a5)
+    inf = np.isinf(ref)
+    assert np.array_equal(np.isnan(y), np.isnan(ref)) and np.array_equal(y[inf], ref[inf])
+    assert what == "weight" or np.isinf(a5).any() and np.isfinite(ref).any()
+    assert {"positive": inf.any(), "mixed": np.isnan(ref).any() and inf.any(), "weight": np.isfinite(ref).all()}[what]
+    fin = np.isfinite(ref)
+    assert np.max(np.abs(y[fin] - ref[fin])) <= 1e-5 * np.max(np.abs(ref[fin]))
