@@ -243,9 +243,28 @@ __global__ void __launch_bounds__(kEThreads, kEBlocksPerSm)
   }
 }
 
+// the part of g[c][t] below of the calling block's tiles, tap by tap
+__device__ __noinline__ float wgrad_edge_sum(const bf16 *__restrict__ xv, const float *__restrict__ s, int c, int t,
+                                             int B, int H, int W, int tiles_x, int tiles_y) {
+  const int dx = t % 3 - 1, dy = t / 3 - 1;
+  const long long ntiles = (long long)B * tiles_x * tiles_y;
+  float v = 0.0f;
+  for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    const EdgeTile e = edge_tile(tile, tiles_x, tiles_y, kEC, H, W);
+    for (int y = max(e.y0, -dy); y < min(e.y0 + kER, H - max(dy, 0)); ++y)
+      for (int x = max(e.x0, -dx); x < min(e.x0 + kEC, W - max(dx, 0)); ++x) {
+        const long long p = e.f + (long long)y * W + x;
+        v = fmaf(__bfloat162float(xv[p * kC + c]), __ldg(s + p + (long long)dy * W + dx), v);
+      }
+  }
+  return v;
+}
+
 // Weight gradients of the edge layers: g[c][t] = sum_p x[p][c] s[p + t], one
 // partial sum per block at part[t' * 32 + c]; LAYER 1: x = dZ1, s = in, t' = t;
-// LAYER 6: x = A5, s = dy, t' = 8 - t (dW6[t][c] = sum_p dy[p] A5[p + t][c])
+// LAYER 6: x = A5, s = dy, t' = 8 - t (dW6[t][c] = sum_p dy[p] A5[p + t][c]).
+// Taps outside the field are staged zeros, which make NaN of an infinite x: a
+// sum that is NaN is formed again without them.
 template <int LAYER>
 __global__ void __launch_bounds__(kEThreads, kEBlocksPerSm)
     k_wgrad_edge(const bf16 *__restrict__ xv, const float *__restrict__ s, float *__restrict__ part, int B, int H,
@@ -298,6 +317,7 @@ __global__ void __launch_bounds__(kEThreads, kEBlocksPerSm)
     float v = 0.0f;
 #pragma unroll
     for (int q = 0; q < kEThreads / 32; ++q) v += red[q][i];
+    if (isnan(v)) v = wgrad_edge_sum(xv, s, i % kC, LAYER == 1 ? i / kC : kTaps - 1 - i / kC, B, H, W, tiles_x, tiles_y);
     part[(long long)blockIdx.x * kK + i] = v;
   }
 }

@@ -154,3 +154,31 @@ def test_output_layer_overflow(shape, what, path):
     assert {"positive": inf.any(), "mixed": np.isnan(ref).any() and inf.any(), "weight": np.isfinite(ref).all()}[what]
     fin = np.isfinite(ref)
     assert np.max(np.abs(y[fin] - ref[fin])) <= 1e-5 * np.max(np.abs(ref[fin]))
+
+
+# Layer 1's weight gradient where the data gradient overflowed at a corner, an
+# edge or inside (identity layers: one pixel's gradient stays that pixel's): a
+# tap outside the field takes no part, the others are infinite
+@pytest.mark.parametrize("pixel", [(0, 0), (0, 69), (16, 33), (8, 0), (8, 68)])
+def test_first_layer_gradient_overflow(pixel):
+    import torch
+    from ins2d_b200.learned import ConvNet
+    from oracle import cnn_ref as N
+    H, W = 17, 70
+    W1, W6, eye = np.zeros((N.C, N.TAPS)), np.zeros((N.TAPS, N.C)), np.zeros((N.C, N.TAPS, N.C))
+    W1[:, 4], W6[4] = 2.0 ** -60, 1.0
+    eye[np.arange(N.C), 4, np.arange(N.C)] = 1.0
+    w = N.join(W1, [eye * 2.0 ** 60, eye, eye, eye], W6)
+    net = ConvNet(device=0, seed=1)
+    net.set_params(w.astype(np.float32), 1.0)
+    inp = torch.ones((1, H, W), device="cuda")
+    tgt = net.forward(inp).clone()
+    tgt[0, pixel[0], pixel[1]] = -2.0 ** 100
+    g = np.asarray(net.loss_grad(inp, tgt)[1])
+    ref = np.zeros((N.C, N.TAPS))
+    for t in range(N.TAPS):
+        y, x = pixel[0] + t // 3 - 1, pixel[1] + t % 3 - 1
+        if 0 <= y < H and 0 <= x < W:
+            ref[:, t] = np.inf
+    assert np.array_equal(g[:N.OFF_WM].reshape(N.C, N.TAPS), ref)
+    assert np.all(np.isfinite(g[N.OFF_WM:]))
