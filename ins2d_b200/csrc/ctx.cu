@@ -726,7 +726,7 @@ int additional_solve(ins2d_ctx *c, const double *V, double *p, double t, ins2d_s
   int rc = sample_bc(c, t);
   if (rc) return rc;
   {
-    Prof pr(c, INS2D_PROF_RESIDUAL, 1);
+    Prof pr(c, INS2D_PROF_RESIDUAL, walk_launches(c->P));
     double *kn = (cache && !c->store32) ? c->kV[0] : nullptr;
     float *kn32 = (cache && c->store32) ? c->kV32[0] : nullptr;
     launch_residual(c->P, V, p, c->wres, kn, kn32, c->fp32, c->stream);
@@ -790,7 +790,7 @@ int erk_step32(ins2d_ctx *c, double *V, double *p, double t, double dt, ins2d_st
       a.inv_dt = 1.0 / dt;
       a.kV32 = (c->need_store[i] || a.nprev == 0) ? c->kV32[i] : nullptr;
       a.Vt32 = a.nprev > 0 ? c->Vt32 : nullptr;
-      Prof pr(c, INS2D_PROF_STAGE, 1);
+      Prof pr(c, INS2D_PROF_STAGE, walk_launches(P));
       launch_stage(P, a, true, c->stream);
       if (a.nprev > 0) {
         Ti = c->Vt32;
@@ -876,7 +876,7 @@ int erk_step(ins2d_ctx *c, double *V, double *p, double t, double dt, ins2d_step
       a.aii = c->A[i][i];
       a.inv_dt = 1.0 / dt;
       a.Wt = c->Wt;
-      Prof pr(c, INS2D_PROF_STAGE, 1);
+      Prof pr(c, INS2D_PROF_STAGE, walk_launches(P));
       launch_stage(P, a, c->fp32, c->stream);
     }
     const double ti = t + c->c[i] * dt;
@@ -1367,7 +1367,7 @@ int ins2d_F(ins2d_ctx *ctx, const double *V, const double *C, const double *p, d
   double *dO = mem == INS2D_MEM_DEVICE ? F_out : ctx->stO;
   if (dP && dC == dV && !ctx->fp32) {
     // the stencil walkers (the stage kernels' F), which also take max|F|
-    Prof pr(ctx, INS2D_PROF_OTHER, 1);
+    Prof pr(ctx, INS2D_PROF_OTHER, walk_launches(ctx->P));
     launch_F_walk(ctx->P, dV, dP, dO, ctx->fmax, ctx->fcount, ctx->h_red, ctx->stream);
   } else {
     // C != V (F.m's linearisation point), nopressure, or FP32-stencil

@@ -101,6 +101,8 @@ struct StageArgs {
 // One RK stage right-hand side: kV = Om^-1 (-conv + Diff V + yDiff - y_p),
 // Vtemp = sum_m A(i,m) kV_m, Wt = Vn/dt + Vtemp   (time_ERK.m:90-101,117)
 void launch_stage(const DevOps &P, const StageArgs &a, bool fp32, cudaStream_t s);
+// launches of a walk over the grid: the interior tiles, the others
+inline int walk_launches(const DevOps &P) { return (P.fbx1 > P.fbx0 && P.fby1 > P.fby0) + !P.all_fast; }
 // computes P.fbx0.., P.ru, P.rv (the regular tiles and points of the walkers)
 void walker_rectangle(DevOps &P);
 // opts the tiled walkers in to their dynamic shared memory on the current

@@ -182,3 +182,23 @@ def test_first_layer_gradient_overflow(pixel):
             ref[:, t] = np.inf
     assert np.array_equal(g[:N.OFF_WM].reshape(N.C, N.TAPS), ref)
     assert np.all(np.isfinite(g[N.OFF_WM:]))
+
+
+# F's launches as counted by the profile: the tiled walkers, the table walkers
+# around them, or both
+@pytest.mark.parametrize("shape,bc,n", [((128, 64), "periodic", 1), ((300, 260), "cavity", 2), ((40, 30), "cavity", 1)])
+def test_launch_count(shape, bc, n):
+    import ins2d_b200
+    from ins2d_b200 import cases
+    from tests.cases_common import BC_COMBOS
+    m = ins2d_b200.Options(cases.uniform_grid(shape[0], 0.0, 1.0), cases.uniform_grid(shape[1], 0.0, 1.0), BC_COMBOS[bc],
+                           Re=100.0, poisson=6 if bc == "periodic" else 4, precond="jacobi")
+    V, p = np.random.default_rng(1).standard_normal(m.NV), np.zeros(m.Np)
+    m.profile()
+    m.F(V, None, p)
+    assert m.profile_read()["other"][1] == n
+    # a step from its own first stage: four stages and the residual, then as
+    # many without the first stage
+    m.time_ERK(V, p, 0.0, 1e-6)
+    fam = m.profile_read()
+    assert fam["stage"][1] + fam["residual"][1] == 5 * n, fam
