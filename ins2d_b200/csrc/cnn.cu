@@ -255,6 +255,7 @@ __device__ __noinline__ float wgrad_edge_sum(const bf16 *__restrict__ xv, const 
       for (int x = max(e.x0, -dx); x < min(e.x0 + kEC, W - max(dx, 0)); ++x) {
         const long long p = e.f + (long long)y * W + x;
         v = fmaf(__bfloat162float(xv[p * kC + c]), __ldg(s + p + (long long)dy * W + dx), v);
+        if (isnan(v)) return v;  // whatever follows
       }
   }
   return v;
@@ -953,7 +954,15 @@ __device__ __noinline__ float conv_out_pixel(const bf16 *__restrict__ a, const f
   for (int t = 0; t < kTaps; ++t) {
     const int xx = x + t % 3 - 1, yy = y + t / 3 - 1;
     if (xx < 0 || xx >= W || yy < 0 || yy >= H) continue;
-    for (int c = 0; c < kC; ++c) s = fmaf(__ldg(w6 + t * kC + c), __bfloat162float(a[((long long)yy * W + xx) * kC + c]), s);
+    const uint4 *p = reinterpret_cast<const uint4 *>(a + ((long long)yy * W + xx) * kC);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      float v[8];
+      unpack8(__ldg(p + q), v);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) s = fmaf(__ldg(w6 + t * kC + 8 * q + e), v[e], s);
+    }
+    if (isnan(s)) break;  // whatever follows
   }
   return scale * s;
 }
