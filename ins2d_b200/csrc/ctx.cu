@@ -159,7 +159,8 @@ const double *upload_vec(ins2d_ctx *c, const std::vector<double> &v) {
   return d;
 }
 
-// the separable inverse of c's pressure matrix (fdm_host.hpp) into D
+// the separable inverse of c's pressure matrix (fdm_host.hpp) into D, without
+// the work arrays (fdm_work)
 void upload_fdm(ins2d_ctx *c, FdmD &D) {
   const FdmTri T = fdm_tri(c->H.TX, c->H.hx, c->H.TY, c->H.hy);
   D.nx = c->H.Npx;
@@ -179,7 +180,14 @@ void upload_fdm(ins2d_ctx *c, FdmD &D) {
     D.ng = upload_vec(c, T.ng);
     D.nmu = upload_vec(c, T.nmu);
   }
-  D.t = dalloc<double>(c, (size_t)c->P.Np);
+}
+
+// work arrays of the solves in several launches: application and second direction
+void fdm_work(ins2d_ctx *c, FdmD &D) {
+  const size_t Np = (size_t)c->P.Np;
+  if (!D.spectral) D.t = dalloc<double>(c, Np);
+  D.z = dalloc<double>(c, Np);
+  c->pcg.p2 = dalloc<double>(c, Np);
 }
 
 // Layout of the boundary-value blob: {name, length}.
@@ -1108,7 +1116,6 @@ int ins2d_ctx_create(const ins2d_grid_desc *grid, const ins2d_bc_desc *bc, const
       W.r = dalloc<double>(c, Np);
       W.p = dalloc<double>(c, Np);
       W.q = dalloc<double>(c, Np);
-      W.p2 = dalloc<double>(c, Np);
       W.sc = dalloc<PcgScalars>(c, 1);
       W.blocks = pcg_blocks(P);
       W.partials = dalloc<double>(c, (size_t)W.blocks * 8 + 16);
@@ -1121,7 +1128,6 @@ int ins2d_ctx_create(const ins2d_grid_desc *grid, const ins2d_bc_desc *bc, const
         FdmD &D = c->fdm;
         D.nx = H.Npx;
         D.ny = H.Npy;
-        D.z = dalloc<double>(c, Np);
         if (H.fft_ok && fft_supported(H.Nx, H.Ny)) {
           // periodic uniform grid: the Fourier basis, i.e. the FFT solve
           CK(fft_prepare());
@@ -1153,6 +1159,7 @@ int ins2d_ctx_create(const ins2d_grid_desc *grid, const ins2d_bc_desc *bc, const
             P.pdl = 1;
           }
         }
+        if (!pcg_use_cluster(D)) fdm_work(c, D);  // a cluster keeps them in shared memory
         c->use_fdm = true;
       } else if (opts->precond != INS2D_PRECOND_JACOBI) {
         std::vector<MgHostLevel> lv;
@@ -2388,7 +2395,7 @@ int ins2d_ens_create(int32_t n, const ins2d_grid_desc *grids, const ins2d_bc_des
           upload_fdm(c, D);
           D.f = c->f;
           D.r = c->pcg.r;
-          D.z = dalloc<double>(c, (size_t)c->P.Np);
+          fdm_work(c, D);
           e->fdm_z.push_back(D.z);
         }
         FdmD *df = ens_alloc<FdmD>(e, n);

@@ -202,3 +202,25 @@ def test_launch_count(shape, bc, n):
     m.time_ERK(V, p, 0.0, 1e-6)
     fam = m.profile_read()
     assert fam["stage"][1] + fam["residual"][1] == 5 * n, fam
+
+
+# Work arrays that only one solver reads are not allocated for the others: of
+# the pressure-sized ones fast diagonalization holds five more than Jacobi
+# (second direction, application's input and output, pivots, basis / 2)
+def test_work_arrays():
+    import ins2d_b200
+    import torch
+    from ins2d_b200 import cases
+    from tests.cases_common import BC_COMBOS
+    x, y = cases.uniform_grid(512, 0.0, 1.0), cases.uniform_grid(1024, 0.0, 2.0)
+
+    def used(precond):
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        m = ins2d_b200.Options(x, y, BC_COMBOS["cavity"], Re=100.0, poisson=4, precond=precond)
+        n = free - torch.cuda.mem_get_info()[0]
+        m.close()
+        return n
+
+    used("jacobi"), used("fdm")  # kernels and pools loaded
+    assert used("fdm") - used("jacobi") >= 4 * 512 * 1024 * 8
