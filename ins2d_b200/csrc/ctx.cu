@@ -159,6 +159,20 @@ const double *upload_vec(ins2d_ctx *c, const std::vector<double> &v) {
   return d;
 }
 
+// the transform solve of c's grid: plan, tables and scratch
+void make_fft(ins2d_ctx *c, FftPlan &F) {
+  CK(fft_prepare());
+  const int Nx = c->H.Nx, Ny = c->H.Ny;
+  F = fft_plan(Nx, Ny);
+  const std::vector<double> tx = fft_twiddle_table(Nx), ty = fft_twiddle_table(Ny);
+  F.twx = dalloc<double2>(c, tx.size() / 2);
+  F.twy = dalloc<double2>(c, ty.size() / 2);
+  CK(cudaMemcpy(F.twx, tx.data(), tx.size() * sizeof(double), cudaMemcpyHostToDevice));
+  CK(cudaMemcpy(F.twy, ty.data(), ty.size() * sizeof(double), cudaMemcpyHostToDevice));
+  F.spec = dalloc<double2>(c, (size_t)(Nx / 2 + 1) * Ny);
+  F.maxabs = dalloc<double>(c, 1);
+}
+
 // the separable inverse of c's pressure matrix (fdm_host.hpp) into D, without
 // the work arrays (fdm_work)
 void upload_fdm(ins2d_ctx *c, FdmD &D) {
@@ -244,8 +258,6 @@ int fail(ins2d_ctx *c, int code, const std::string &msg) {
   if (c) c->err = msg;
   return code;
 }
-
-bool is_pow2(int n) { return n > 0 && (n & (n - 1)) == 0; }
 
 void setup_rk(ins2d_ctx *c) {
   // default: classical RK44 (getRKmethod.m:313-316)
@@ -1097,19 +1109,7 @@ int ins2d_ctx_create(const ins2d_grid_desc *grid, const ins2d_bc_desc *bc, const
     c->red.max_blocks = maxb;
     CK(cudaMemset(c->red.counter, 0, sizeof(unsigned int)));
     if (c->poisson == INS2D_POISSON_FFT) {
-      CK(fft_prepare());
-      FftPlan &F = c->fft;
-      F.Nx = H.Nx;
-      F.Ny = H.Ny;
-      F.logx = is_pow2(H.Nx) ? (int)std::lround(std::log2((double)H.Nx)) : -1;
-      F.logy = is_pow2(H.Ny) ? (int)std::lround(std::log2((double)H.Ny)) : -1;
-      const std::vector<double> tx = fft_twiddle_table(H.Nx), ty = fft_twiddle_table(H.Ny);
-      F.twx = dalloc<double2>(c, tx.size() / 2);
-      F.twy = dalloc<double2>(c, ty.size() / 2);
-      CK(cudaMemcpy(F.twx, tx.data(), tx.size() * sizeof(double), cudaMemcpyHostToDevice));
-      CK(cudaMemcpy(F.twy, ty.data(), ty.size() * sizeof(double), cudaMemcpyHostToDevice));
-      F.spec = dalloc<double2>(c, (size_t)(H.Nx / 2 + 1) * H.Ny);
-      F.maxabs = dalloc<double>(c, 1);
+      make_fft(c, c->fft);
     } else {
       PcgWork &W = c->pcg;
       W.x = dalloc<double>(c, Np);
@@ -1130,19 +1130,7 @@ int ins2d_ctx_create(const ins2d_grid_desc *grid, const ins2d_bc_desc *bc, const
         D.ny = H.Npy;
         if (H.fft_ok && fft_supported(H.Nx, H.Ny)) {
           // periodic uniform grid: the Fourier basis, i.e. the FFT solve
-          CK(fft_prepare());
-          FftPlan &F = c->fdm_fft;
-          F.Nx = H.Nx;
-          F.Ny = H.Ny;
-          F.logx = is_pow2(H.Nx) ? (int)std::lround(std::log2((double)H.Nx)) : -1;
-          F.logy = is_pow2(H.Ny) ? (int)std::lround(std::log2((double)H.Ny)) : -1;
-          const std::vector<double> tx = fft_twiddle_table(H.Nx), ty = fft_twiddle_table(H.Ny);
-          F.twx = dalloc<double2>(c, tx.size() / 2);
-          F.twy = dalloc<double2>(c, ty.size() / 2);
-          CK(cudaMemcpy(F.twx, tx.data(), tx.size() * sizeof(double), cudaMemcpyHostToDevice));
-          CK(cudaMemcpy(F.twy, ty.data(), ty.size() * sizeof(double), cudaMemcpyHostToDevice));
-          F.spec = dalloc<double2>(c, (size_t)(H.Nx / 2 + 1) * H.Ny);
-          F.maxabs = dalloc<double>(c, 1);  // the symbol factors P.fft_ax, fft_ay are set above
+          make_fft(c, c->fdm_fft);  // the symbol factors P.fft_ax, fft_ay are set above
           double *gate = dalloc<double>(c, 1);
           const double one = 1.0;
           CK(cudaMemcpy(gate, &one, sizeof one, cudaMemcpyHostToDevice));

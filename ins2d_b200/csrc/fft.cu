@@ -924,12 +924,6 @@ int cols_group(const FftLine &L) {
 int fft_small_cap(const FftLine &Lx, const FftLine &Ly) {  // complex values per buffer
   return std::max((Ly.n + 1) / 2 * line_ld(Lx.n), (Lx.n / 2 + 1) * line_ld(Ly.n));
 }
-bool fft_small(const FftPlan &plan) {
-  if (plan.logx >= kFusedMinLog || plan.logy >= kFusedMinLog || plan.Nx * (long long)plan.Ny > INS2D_FFT_SMALL_MAX)
-    return false;
-  const FftLine Lx = fft_line(plan.Nx), Ly = fft_line(plan.Ny);
-  return Lx.m == Lx.n && Ly.m == Ly.n && 32 * (size_t)fft_small_cap(Lx, Ly) <= 200 * 1024;
-}
 // threads per block for `lines` lines: about one butterfly of radix 4 each
 int line_threads(const FftLine &L, int lines) {
   int t = 32;
@@ -962,8 +956,6 @@ void host_fft(std::vector<long double> &re, std::vector<long double> &im) {
       }
     }
 }
-
-}  // namespace
 
 FftLine fft_line(int n) {
   FftLine L;
@@ -1004,6 +996,24 @@ FftLine fft_line(int n) {
     s *= r;
   }
   return L;
+}
+
+}  // namespace
+
+FftPlan fft_plan(int Nx, int Ny) {
+  FftPlan p;
+  p.Nx = Nx;
+  p.Ny = Ny;
+  p.logx = ilog2_exact(Nx);
+  p.logy = ilog2_exact(Ny);
+  const bool fx = p.logx >= kFusedMinLog, fy = p.logy >= kFusedMinLog;
+  if (!fx) p.lx = fft_line(Nx);
+  if (!fy) p.ly = fft_line(Ny);
+  if (!fx && !fy && (long long)Nx * Ny <= INS2D_FFT_SMALL_MAX && p.lx.m == Nx && p.ly.m == Ny) {
+    const int cap = fft_small_cap(p.lx, p.ly);
+    if (32 * (size_t)cap <= 200 * 1024) p.small = cap;
+  }
+  return p;
 }
 
 std::vector<double> fft_twiddle_table(int n) {
@@ -1101,9 +1111,9 @@ cudaError_t fft_passes(const DevOps &P, const FftPlan &plan, const double *src, 
   const int pairs = (Ny + 1) / 2;
   const int H = Nx / 2 + 1;
   unsigned long long *maxbits = (unsigned long long *)plan.maxabs;
-  if (fft_small(plan)) {
-    const FftLine Lx = fft_line(Nx), Ly = fft_line(Ny);
-    const int cap = fft_small_cap(Lx, Ly), acc = accumulate ? 1 : 0;
+  const FftLine &Lx = plan.lx, &Ly = plan.ly;
+  if (plan.small) {
+    const int cap = plan.small, acc = accumulate ? 1 : 0;
     const size_t sm = 2 * (size_t)cap * sizeof(double2);
     if (ws)
       k_fft_small<2><<<1, kSmallThreads, sm, s>>>(Lx, Ly, cap, plan.twx, plan.twy, nullptr, *ws, P, alpha, beta, gamma,
@@ -1134,7 +1144,6 @@ cudaError_t fft_passes(const DevOps &P, const FftPlan &plan, const double *src, 
       launch_k(k_rows_r2c_t<L, 0>, dim3(pairs), dim3(kThreads), sm, s, Ny, plan.twx, src, w0, plan.spec, P, 0.0,
                0.0, 0.0, 0, skip, maxbits);
   });
-  const FftLine Lx = fx ? FftLine{} : fft_line(Nx);
   const size_t smx = fx ? 0 : 2 * (size_t)line_ld(Lx.m) * sizeof(double2);
   if (!fx) {
     const int t = line_threads(Lx, 1);
@@ -1157,7 +1166,6 @@ cudaError_t fft_passes(const DevOps &P, const FftPlan &plan, const double *src, 
     });
   });
   if (!fy) {
-    const FftLine Ly = fft_line(Ny);
     const int G = cols_group(Ly);
     const size_t smy = 2 * (size_t)G * line_ld(Ly.m) * sizeof(double2);
     k_cols<<<(H + G - 1) / G, line_threads(Ly, G), smy, s>>>(Ly, H, G, plan.twy, P.fft_ax, P.fft_ay, P.fft_dxdy,
@@ -1183,7 +1191,7 @@ cudaError_t launch_fft_poisson(const DevOps &P, const FftPlan &plan, const doubl
   return fft_passes(P, plan, f, nullptr, false, 0.0, 0.0, 0.0, dp, accumulate, s);
 }
 
-int fft_kernels(const FftPlan &plan) { return fft_small(plan) ? 1 : 3; }
+int fft_kernels(const FftPlan &plan) { return plan.small ? 1 : 3; }
 
 cudaError_t launch_fft_poisson_div(const DevOps &P, const FftPlan &plan, const double *W, double alpha,
                                    double beta, double gamma, double *dp, bool accumulate, cudaStream_t s) {

@@ -13,21 +13,11 @@
 // 8.6 and 8.5 us, columns 18.6 us), 40 x 40 step on host arrays 225 -> 203 us.
 #pragma once
 
-#include <cuda_runtime.h>
+#include "kernels.cuh"
 
 namespace ins2d {
 
 constexpr int kMaxFactor = 31;
-constexpr int kMaxPasses = 12;
-
-struct FftLine {
-  int n = 0, m = 0;  // length, length of the Stockham passes (m > n: Bluestein)
-  int np = 0;        // passes
-  int r[kMaxPasses] = {}, s[kMaxPasses] = {};  // radix and stride of each pass
-  unsigned inv_s[kMaxPasses] = {};             // ceil(2^32 / s): b / s = umulhi(b, inv_s) for b s < 2^32
-  unsigned inv_b[kMaxPasses] = {};             // the same for the butterflies per line m / r
-};
-FftLine fft_line(int n);
 
 // shared-memory slot of value i: eight lanes of 16-byte accesses a power of
 // two apart fall on distinct banks

@@ -186,13 +186,27 @@ void launch_project_ens(const EnsMemberD *mem, const int4 *tiles, int n, double 
 void launch_stage_cached_ens(const EnsMemberD *mem, const int4 *tiles, int n, double aii, cudaStream_t s);
 
 // --- FFT Poisson (fft.cu) -------------------------------------------------------
+// Passes of a line without a compile-time shape (fft_line.cuh)
+constexpr int kMaxPasses = 12;
+struct FftLine {
+  int n = 0, m = 0;  // length, length of the Stockham passes (m > n: Bluestein)
+  int np = 0;        // passes
+  int r[kMaxPasses] = {}, s[kMaxPasses] = {};  // radix and stride of each pass
+  unsigned inv_s[kMaxPasses] = {};             // ceil(2^32 / s): b / s = umulhi(b, inv_s) for b s < 2^32
+  unsigned inv_b[kMaxPasses] = {};             // the same for the butterflies per line m / r
+};
 struct FftPlan {
   int Nx = 0, Ny = 0, logx = -1, logy = -1;  // log2 when a power of two, else -1
+  FftLine lx, ly;                            // of sides without a compile-time shape
+  int small = 0;                             // one block solves: complex values per buffer; else 0
   double2 *twx = nullptr, *twy = nullptr;    // fft_twiddle_table of Nx and Ny
   double2 *spec = nullptr;                   // (Nx/2+1) x Ny complex spectrum
   double *maxabs = nullptr;                  // max |fhat| of the last solve
 };
 bool fft_supported(int Nx, int Ny);
+// the host part of the plan (everything but the device arrays); made once, so
+// that a solve factorizes no lengths and allocates nothing
+FftPlan fft_plan(int Nx, int Ny);
 // Tables of a length-n transform as complex values (pairs of doubles).
 // Powers of two from 64: 2n values, e^{-2 pi i k/n} at k and e^{-2 pi i k/Lt}
 // at n + Lt/2 + k for every power of two 2 <= Lt <= n, k < Lt/2.  Other
@@ -207,7 +221,7 @@ cudaError_t launch_fft_poisson(const DevOps &P, const FftPlan &plan, const doubl
                                cudaStream_t s);
 // Same with the right-hand side f = (M W + alpha yM + beta ydM) gamma computed
 // inside the first pass.
-// kernel launches of one solve (the column transform takes one or three)
+// kernel launches of one solve (one block's, or three passes)
 int fft_kernels(const FftPlan &plan);
 cudaError_t launch_fft_poisson_div(const DevOps &P, const FftPlan &plan, const double *W, double alpha,
                                    double beta, double gamma, double *dp, bool accumulate, cudaStream_t s);

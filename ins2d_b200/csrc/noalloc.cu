@@ -11,6 +11,7 @@
 
 #include <cmath>
 #include <mutex>
+#include <new>
 #include <vector>
 
 #include "ins2d.h"
@@ -41,13 +42,8 @@ struct TableKey {
   double dx = 0.0, dy = 0.0;
 };
 TableKey g_tables[kMaxDevices];
+FftPlan g_plans[kMaxDevices];  // of the same size, without the device arrays
 std::mutex g_setup_mu;
-
-int log2_exact(int n) {
-  int l = 0;
-  while ((1 << l) < n) ++l;
-  return ((1 << l) == n) ? l : -1;
-}
 
 }  // namespace
 
@@ -64,6 +60,7 @@ extern "C" int ins2d_fft_poisson_noalloc(const double *f, double *dp, int32_t Nx
   // shared-memory limits
   double2 *base = nullptr;
   bool upload = true;
+  FftPlan plan;
   {
     std::lock_guard<std::mutex> lk(g_setup_mu);
     if (!g_scratch_addr[dev]) {
@@ -77,7 +74,10 @@ extern "C" int ins2d_fft_poisson_noalloc(const double *f, double *dp, int32_t Nx
     upload = !(k.Nx == Nx && k.Ny == Ny && k.dx == dx && k.dy == dy);
     // forget the key until the new tables are uploaded: a failed upload must
     // not leave a key that claims them
-    if (upload) g_tables[dev] = TableKey{};
+    if (upload)
+      g_tables[dev] = TableKey{};
+    else
+      plan = g_plans[dev];
   }
   cudaStream_t s = (cudaStream_t)stream;
   double2 *spec = base;
@@ -86,7 +86,8 @@ extern "C" int ins2d_fft_poisson_noalloc(const double *f, double *dp, int32_t Nx
   double *axd = (double *)(twy + 2 * (size_t)kMaxN);  // kMaxN doubles
   double *ayd = axd + kMaxN;                           // kMaxN doubles
   double *maxabs = (double *)(base + kSpec + 5 * (size_t)kMaxN);
-  if (upload) {
+  if (upload) try {
+    plan = fft_plan(Nx, Ny);
     // twiddle tables and the symbol factors (1/dx^2) sin^2(I pi/Nx),
     // (1/dy^2) sin^2(J pi/Ny) of operator_divergence.m:283, as in the context path
     const std::vector<double> tx = fft_twiddle_table(Nx), ty = fft_twiddle_table(Ny);
@@ -109,16 +110,14 @@ extern "C" int ins2d_fft_poisson_noalloc(const double *f, double *dp, int32_t Nx
     if (cudaStreamSynchronize(s) != cudaSuccess) return INS2D_ECUDA;
     std::lock_guard<std::mutex> lk(g_setup_mu);
     g_tables[dev] = TableKey{Nx, Ny, dx, dy};
+    g_plans[dev] = plan;
+  } catch (const std::bad_alloc &) {  // the host tables
+    return INS2D_ENOMEM;
   }
   DevOps P{};
   P.fft_ax = axd;
   P.fft_ay = ayd;
   P.fft_dxdy = dx * dy;
-  FftPlan plan;
-  plan.Nx = Nx;
-  plan.Ny = Ny;
-  plan.logx = log2_exact(Nx);
-  plan.logy = log2_exact(Ny);
   plan.twx = twx;
   plan.twy = twy;
   plan.spec = spec;
