@@ -161,9 +161,9 @@ const double *upload_vec(ins2d_ctx *c, const std::vector<double> &v) {
 
 // the transform solve of c's grid: plan, tables and scratch
 void make_fft(ins2d_ctx *c, FftPlan &F) {
-  CK(fft_prepare());
   const int Nx = c->H.Nx, Ny = c->H.Ny;
   F = fft_plan(Nx, Ny);
+  CK(fft_prepare(F, c->P.nsm));
   const std::vector<double> tx = fft_twiddle_table(Nx), ty = fft_twiddle_table(Ny);
   F.twx = dalloc<double2>(c, tx.size() / 2);
   F.twy = dalloc<double2>(c, ty.size() / 2);

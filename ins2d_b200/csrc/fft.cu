@@ -1066,39 +1066,44 @@ bool fft_supported(int Nx, int Ny) {
   return ok(Nx) && ok(Ny);
 }
 
-// Opt the transform kernels in to large dynamic shared memory on the current
-// device (called once per context); returns the first failure.
-cudaError_t fft_prepare() {
+namespace {
+// Dynamic shared memory of `bytes` (of at most 200 KB) for kernels on the
+// current device.  Below every kernel's default nothing is done: the call
+// would load the kernel, as it does for each one it opts in (0.1 to 0.3 ms).
+template <typename... K>
+cudaError_t opt_in(size_t bytes, K... k) {
   cudaError_t first = cudaSuccess;
-  auto opt_in = [&](const void *k, size_t bytes = 200 * 1024) {
-    if (bytes <= 47 * 1024) return;  // within every kernel's default; the call would load the kernel (about 0.1 ms)
-    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+  if (bytes <= 47 * 1024) return first;
+  for (const void *f : {(const void *)k...}) {
+    const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     if (first == cudaSuccess) first = e;
-  };
-  for (int l = kFusedMinLog; l <= 13; ++l)
-    with_log2<kFusedMinLog>(l, [&](auto c) {
-      constexpr int L = decltype(c)::value;
-      constexpr size_t rows = (size_t)paddedl<L>() * sizeof(double2);
-      opt_in((const void *)k_rows_r2c_t<L, 0>, rows);
-      opt_in((const void *)k_rows_r2c_t<L, 1>, rows);
-      opt_in((const void *)k_rows_r2c_t<L, 2>, rows);
-      constexpr int G = cols_per_block<L>();
-      opt_in((const void *)k_cols_t<L, G, cols_radix<L>()>, cols_smem<L, G>());
-      if constexpr (G >= 4) {
-        opt_in((const void *)k_cols_t<L, G / 2, cols_radix<L>()>, cols_smem<L, G / 2>());
-        opt_in((const void *)k_cols_t<L, G / 4, cols_radix<L>()>, cols_smem<L, G / 4>());
-      }
-      opt_in((const void *)k_rows_c2r_t<L>, rows);
-    });
-  opt_in((const void *)k_rows_r2c<0>);
-  opt_in((const void *)k_rows_r2c<1>);
-  opt_in((const void *)k_rows_r2c<2>);
-  opt_in((const void *)k_cols);
-  opt_in((const void *)k_fft_small<0>);
-  opt_in((const void *)k_fft_small<1>);
-  opt_in((const void *)k_fft_small<2>);
-  opt_in((const void *)k_rows_c2r);
+  }
   return first;
+}
+template <int L>
+cudaError_t opt_in_rows() {
+  return opt_in((size_t)paddedl<L>() * sizeof(double2), k_rows_r2c_t<L, 0>, k_rows_r2c_t<L, 1>, k_rows_r2c_t<L, 2>,
+                k_rows_c2r_t<L>);
+}
+template <int L, int G>
+cudaError_t opt_in_cols() {
+  return opt_in(cols_smem<L, G>(), k_cols_t<L, G, cols_radix<L>()>);
+}
+}  // namespace
+
+// Only the kernels that fft_passes launches for this plan: opting in all of
+// every length cost a process's first context of 512^2 3 ms.
+cudaError_t fft_prepare(const FftPlan &plan, int nsm) {
+  if (plan.small) return opt_in(2 * (size_t)plan.small * sizeof(double2), k_fft_small<0>, k_fft_small<1>, k_fft_small<2>);
+  cudaError_t ex = cudaSuccess, ey = cudaSuccess;
+  if (!with_log2<kFusedMinLog>(plan.logx, [&](auto c) { ex = opt_in_rows<decltype(c)::value>(); }))
+    ex = opt_in(2 * (size_t)line_ld(plan.lx.m) * sizeof(double2), k_rows_r2c<0>, k_rows_r2c<1>, k_rows_r2c<2>, k_rows_c2r);
+  if (!with_log2<kFusedMinLog>(plan.logy, [&](auto c) {
+        constexpr int L = decltype(c)::value;
+        with_cols_g<L>(plan.Nx / 2 + 1, nsm, [&](auto cg) { ey = opt_in_cols<L, decltype(cg)::value>(); });
+      }))
+    ey = opt_in(2 * (size_t)cols_group(plan.ly) * line_ld(plan.ly.m) * sizeof(double2), k_cols);
+  return ex != cudaSuccess ? ex : ey;
 }
 
 namespace {
@@ -1214,6 +1219,16 @@ cudaError_t launch_fft_poisson_div_split(const DevOps &P, const FftPlan &plan, c
 bool slab_fft_supported(int Nx, int Ny) {
   const int lx = ilog2_exact(Nx), ly = ilog2_exact(Ny);
   return lx >= kFusedMinLog && lx <= 13 && ly >= kFusedMinLog && ly <= 13;
+}
+
+cudaError_t slab_prepare(int Nx, int Ny) {
+  cudaError_t ex = cudaSuccess, ey = cudaSuccess;
+  with_log2<kFusedMinLog>(ilog2_exact(Nx), [&](auto c) { ex = opt_in_rows<decltype(c)::value>(); });
+  with_log2<kFusedMinLog>(ilog2_exact(Ny), [&](auto c) {
+    constexpr int L = decltype(c)::value;
+    ey = opt_in_cols<L, cols_per_block<L>()>();
+  });
+  return ex != cudaSuccess ? ex : ey;
 }
 
 cudaError_t slab_rows_forward(int Nx, const double2 *twx, const double *f, int nrows, double2 *spec, cudaStream_t s) {

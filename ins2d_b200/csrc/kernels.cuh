@@ -235,9 +235,9 @@ cudaError_t launch_fft_precond(const DevOps &P, const FftPlan &plan, const doubl
 cudaError_t launch_fft_poisson_div_split(const DevOps &P, const FftPlan &plan, const double *Vn, const float *T,
                                          double sv, double sa, double alpha, double beta, double gamma, double *dp,
                                          bool accumulate, cudaStream_t s);
-// Opts the transform kernels in to large dynamic shared memory on the current
-// device; returns the first failure.
-cudaError_t fft_prepare();
+// Opts the plan's kernels in to their dynamic shared memory on the current
+// device (nsm: DevOps::nsm of its solves); returns the first failure.
+cudaError_t fft_prepare(const FftPlan &plan, int nsm);
 
 // --- fast-diagonalization preconditioner (fdm.cu, fdm_tri.cuh) ----------------------
 // The separable inverse with one diagonalized direction (fdm_host.hpp,

@@ -56,8 +56,7 @@ extern "C" int ins2d_fft_poisson_noalloc(const double *f, double *dp, int32_t Nx
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return INS2D_ECUDA;
   // once per device, with that device current: the device address of the
-  // static array (its host-side name is only a stand-in) and the kernels'
-  // shared-memory limits
+  // static array (its host-side name is only a stand-in)
   double2 *base = nullptr;
   bool upload = true;
   FftPlan plan;
@@ -66,7 +65,6 @@ extern "C" int ins2d_fft_poisson_noalloc(const double *f, double *dp, int32_t Nx
     if (!g_scratch_addr[dev]) {
       void *ptr = nullptr;
       if (cudaGetSymbolAddress(&ptr, g_scratch) != cudaSuccess || !ptr) return INS2D_ECUDA;
-      if (fft_prepare() != cudaSuccess) return INS2D_ECUDA;
       g_scratch_addr[dev] = (double2 *)ptr;
     }
     base = g_scratch_addr[dev];
@@ -88,6 +86,7 @@ extern "C" int ins2d_fft_poisson_noalloc(const double *f, double *dp, int32_t Nx
   double *maxabs = (double *)(base + kSpec + 5 * (size_t)kMaxN);
   if (upload) try {
     plan = fft_plan(Nx, Ny);
+    if (fft_prepare(plan, 0) != cudaSuccess) return INS2D_ECUDA;  // the kernels' shared-memory limits
     // twiddle tables and the symbol factors (1/dx^2) sin^2(I pi/Nx),
     // (1/dy^2) sin^2(J pi/Ny) of operator_divergence.m:283, as in the context path
     const std::vector<double> tx = fft_twiddle_table(Nx), ty = fft_twiddle_table(Ny);

@@ -19,6 +19,7 @@
 
 namespace ins2d {
 bool slab_fft_supported(int Nx, int Ny);
+cudaError_t slab_prepare(int Nx, int Ny);  // opts the kernels of these lengths in to their shared memory
 cudaError_t slab_rows_forward(int Nx, const double2 *twx, const double *f, int nrows, double2 *spec, cudaStream_t s);
 cudaError_t slab_columns(int Ny, const double2 *twy, const double *ax, const double *ay, double dxdy, double2 *cols,
                          int width, int ncols, int I0, unsigned long long *maxbits, cudaStream_t s);
@@ -97,7 +98,7 @@ int ins2d_slab_fft_create(int32_t Nx, int32_t Ny, double dx, double dy, int32_t 
       !sok(s, cudaMemcpy(s->twy, ty.data(), ty.size() * sizeof(double), cudaMemcpyHostToDevice), "copy") ||
       !sok(s, cudaMemcpy(s->ax, ax.data(), ax.size() * sizeof(double), cudaMemcpyHostToDevice), "copy") ||
       !sok(s, cudaMemcpy(s->ay, ay.data(), ay.size() * sizeof(double), cudaMemcpyHostToDevice), "copy") ||
-      !sok(s, fft_prepare(), "fft_prepare"))
+      !sok(s, slab_prepare(Nx, Ny), "slab_prepare"))
     return INS2D_ECUDA;
   return INS2D_OK;
 }
