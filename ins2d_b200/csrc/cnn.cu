@@ -1637,6 +1637,17 @@ int item_rows(long long per, int H, int cap) {
   return R;
 }
 
+// Opts a kernel in to its dynamic shared memory on the network's device at its
+// first launch there: the call loads the kernel, and a network launches three
+// of the seven (all of them at set-up: 3.0 instead of 1.8 ms for a process's
+// first network).
+template <typename K>
+void opt_in(ins2d_cnn *net, unsigned bit, K k, int bytes) {
+  if (net->opted & bit) return;
+  CK(cudaFuncSetAttribute((const void *)k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  net->opted |= bit;
+}
+
 template <int MODE>
 void launch_mid(ins2d_cnn *net, const bf16 *in, const bf16 *wt, const bf16 *mask, bf16 *out, int B, int H, int W,
                 cudaStream_t s) {
@@ -1646,12 +1657,14 @@ void launch_mid(ins2d_cnn *net, const bf16 *in, const bf16 *wt, const bf16 *mask
     const int R = item_rows(per, H, cap);
     const int chunks = (H + R - 1) / R;
     const int nitems = (int)(per * chunks), grid = std::min(nitems, cap);
+    opt_in(net, 1u << MODE, k_conv_row_tc<MODE>, kRSmem);
     launch_kp(true, k_conv_row_tc<MODE>, grid, kRThreads, kRSmem, s, act_map(in, B, H, W, kRM + 2, 1), wt, mask, out, H,
               W, strips, chunks, R, nitems, net->flag);
   } else if (net->path == INS2D_CNN_PATH_TCGEN05) {
     const int tx = (W + kTcT - 1) / kTcT, ty = (H + kTcT - 1) / kTcT;
     const long long nt = (long long)tx * ty * B;
     const int grid = (int)std::min<long long>(nt, (long long)kTcBlocksPerSm * net->sms);
+    opt_in(net, 4u << MODE, k_conv_mid_tc<MODE>, kTcSmem);
     launch_kp(true, k_conv_mid_tc<MODE>, grid, kTcThreads, kTcSmem, s, in, wt, mask, out, B, H, W, tx, ty, net->flag);
   } else {
     const int tiles_x = (W + TW - 1) / TW, tiles_y = (H + TH - 1) / TH;
@@ -1768,6 +1781,7 @@ void forward(ins2d_cnn *net, const float *in, int B, int H, int W, cudaStream_t 
     const int strips = (W + kOW - 1) / kOW, cap = kOBlocksPerSm * net->sms;
     const long long per = (long long)strips * B;
     const int R = item_rows(per, H, cap), chunks = (H + R - 1) / R, nitems = (int)(per * chunks);
+    opt_in(net, 16u, k_conv_out_tc, kOSmem);
     launch_kp(true, k_conv_out_tc, std::min(nitems, cap), kOThreads, kOSmem, s, act_map(net->act[4], B, H, W, kRM, 1),
               net->act[4], net->w + kOffW6, net->out_scale, net->y, H, W, strips, chunks, R, nitems, net->flag);
   } else {
@@ -1806,6 +1820,10 @@ double loss_grad(ins2d_cnn *net, const float *in, const float *tgt, int B, int H
   const long long ntiles = (long long)tiles_x * tiles_y * B;
   const int wb = (int)std::min({(long long)kWgBlocks, (long long)net->sms, ntiles});
   int cur = 0;
+  if (tc)
+    opt_in(net, 32u, k_wgrad_tc, kGSmem);
+  else
+    opt_in(net, 64u, k_wgrad_mid, kWgSmem);
   for (int l = kMid - 1; l >= 0; --l) {
     // layer index l: input act[l], output act[l + 1], gradient dZ in dz[cur]
     if (tc)
@@ -1968,23 +1986,6 @@ void residual(long long n, const double *f, const double *q, double a, double *x
   CK(cudaStreamSynchronize(s));
 }
 
-// opts the kernels in to their dynamic shared memory on the current device
-cudaError_t prepare_kernels() {
-  cudaError_t e = cudaSuccess;
-  auto opt_in = [&](const void *k, int bytes) {
-    const cudaError_t r = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e == cudaSuccess) e = r;
-  };
-  opt_in((const void *)k_wgrad_mid, kWgSmem);
-  opt_in((const void *)k_wgrad_tc, kGSmem);
-  opt_in((const void *)k_conv_mid_tc<0>, kTcSmem);
-  opt_in((const void *)k_conv_mid_tc<1>, kTcSmem);
-  opt_in((const void *)k_conv_row_tc<0>, kRSmem);
-  opt_in((const void *)k_conv_out_tc, kOSmem);
-  opt_in((const void *)k_conv_row_tc<1>, kRSmem);
-  return e;
-}
-
 size_t red_doubles() { return 4 * (size_t)kRedBlocks + 8; }
 
 }  // namespace cnn
@@ -2064,7 +2065,6 @@ int ins2d_cnn_create(int32_t device, uint64_t seed, ins2d_cnn **out) {
     if (cudaMalloc(&n->red, cnn::red_doubles() * sizeof(double)) != cudaSuccess) throw std::bad_alloc();
     if (cudaMalloc(&n->flag, sizeof(unsigned)) != cudaSuccess) throw std::bad_alloc();
     CK(cudaMemset(n->flag, 0, sizeof(unsigned)));
-    CK(cnn::prepare_kernels());
     CK(cudaDeviceGetAttribute(&n->sms, cudaDevAttrMultiProcessorCount, device));
     std::vector<float> w;
     init_weights(w, seed);

@@ -57,6 +57,7 @@ struct ins2d_cnn {
   unsigned *flag = nullptr;              // set by a tensor-core kernel whose wait gave up
   int sms = 148;
   int path = INS2D_CNN_PATH_TCGEN05;     // tensor-core instructions of the 32 -> 32 layers
+  unsigned opted = 0;                    // kernels opted in to their shared memory
 };
 
 namespace ins2d {
@@ -67,7 +68,6 @@ struct CudaError : std::runtime_error {
   using std::runtime_error::runtime_error;
 };
 // doubles of reduction scratch the helpers below need
-cudaError_t prepare_kernels();
 size_t red_doubles();
 
 // network inputs (and targets) from a Poisson right-hand side f (and its
