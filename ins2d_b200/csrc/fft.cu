@@ -908,26 +908,37 @@ int ilog2_exact(int n) {
 }
 
 // columns per block of k_cols: up to 64-byte row segments within the
-// shared-memory budget (two buffers per line)
-int cols_group(const FftLine &L) {
+// shared-memory budget (two buffers per line), fewer while that leaves SMs idle
+int cols_group(const FftLine &L, int ncols, int nsm) {
   const size_t per = 2 * (size_t)line_ld(L.m) * sizeof(double2);
-  return (int)std::max<size_t>(1, std::min<size_t>(4, (INS2D_FFT_COLS_BUDGET * 1024) / per));
+  int G = (int)std::max<size_t>(1, std::min<size_t>(4, (INS2D_FFT_COLS_BUDGET * 1024) / per));
+  while (G > 1 && (ncols + G - 1) / G < nsm) G /= 2;
+  return G;
 }
 // One block for the whole solve: both sides of general length without
-// Bluestein's algorithm, at most INS2D_FFT_SMALL_MAX cells.  Four solves of a
-// step against three kernels each, B200, us per step: 24 x 24 80.6 and 88.8,
-// 40 x 40 92.9 and 96.9 (called from the host a step at a time 181 and 204),
-// 48 x 60 110 and 99: one SM's throughput takes over from the launches' latency.
+// Bluestein's algorithm, at most INS2D_FFT_SMALL_MAX cells, and direct sums of
+// at most kSmallSums products (cells by radices).  Four solves of a step against
+// three kernels each, B200, us per step: 24 x 24 80.6 and 88.8, 40 x 40 92.9 and
+// 96.9 (called from the host a step at a time 181 and 204), 48 x 60 110 and 99:
+// one SM's throughput takes over from the launches' latency.  With direct sums, one
+// solve called from the host: 31 x 31 29.9 and 35.3 us (60 thousand products), 37 x
+// 37 34.0 and 35.9 (101), 41 x 41 37.3 and 36.4 (138), 61 x 29 40.2 and 37.0 (159).
 #ifndef INS2D_FFT_SMALL_MAX
 #define INS2D_FFT_SMALL_MAX 1800
 #endif
+constexpr long long kSmallSums = 120000;
 int fft_small_cap(const FftLine &Lx, const FftLine &Ly) {  // complex values per buffer
   return std::max((Ly.n + 1) / 2 * line_ld(Lx.n), (Lx.n / 2 + 1) * line_ld(Ly.n));
 }
-// threads per block for `lines` lines: about one butterfly of radix 4 each
-int line_threads(const FftLine &L, int lines) {
-  int t = 32;
-  while (t < kThreads && t * 4 < lines * L.m) t *= 2;
+// Threads per block for `lines` lines: one per value while the launch has less
+// than one block per SM, else about one butterfly of radix 4 each (375 x 2000:
+// 64.4 us, with one per value 69.2), or one pair of a direct sum's outputs (a
+// quarter of the values made chains of them: 64 x 31 solve 41.3 instead of 31.8)
+int line_threads(const FftLine &L, int lines, int blocks, int nsm) {
+  int need = lines * L.m / (blocks < nsm ? 1 : 4), t = 32;
+  for (int i = 0; i < L.np; ++i)
+    if (L.r[i] > 8) need = std::max(need, lines * (L.m / L.r[i]) * (L.r[i] / 2 + 1));
+  while (t < kThreads && t < need) t *= 2;
   return t;
 }
 // in-place transform of length 2^l values in extended precision (tables only)
@@ -1011,7 +1022,11 @@ FftPlan fft_plan(int Nx, int Ny) {
   if (!fy) p.ly = fft_line(Ny);
   if (!fx && !fy && (long long)Nx * Ny <= INS2D_FFT_SMALL_MAX && p.lx.m == Nx && p.ly.m == Ny) {
     const int cap = fft_small_cap(p.lx, p.ly);
-    if (32 * (size_t)cap <= 200 * 1024) p.small = cap;
+    long long sums = 0;  // radices done by direct sums
+    for (const FftLine *l : {&p.lx, &p.ly})
+      for (int i = 0; i < l->np; ++i)
+        if (l->r[i] > 8) sums += l->r[i];
+    if (32 * (size_t)cap <= 200 * 1024 && sums * Nx * Ny <= kSmallSums) p.small = cap;
   }
   return p;
 }
@@ -1102,7 +1117,7 @@ cudaError_t fft_prepare(const FftPlan &plan, int nsm) {
         constexpr int L = decltype(c)::value;
         with_cols_g<L>(plan.Nx / 2 + 1, nsm, [&](auto cg) { ey = opt_in_cols<L, decltype(cg)::value>(); });
       }))
-    ey = opt_in(2 * (size_t)cols_group(plan.ly) * line_ld(plan.ly.m) * sizeof(double2), k_cols);
+    ey = opt_in(2 * (size_t)cols_group(plan.ly, plan.Nx / 2 + 1, nsm) * line_ld(plan.ly.m) * sizeof(double2), k_cols);
   return ex != cudaSuccess ? ex : ey;
 }
 
@@ -1151,7 +1166,7 @@ cudaError_t fft_passes(const DevOps &P, const FftPlan &plan, const double *src, 
   });
   const size_t smx = fx ? 0 : 2 * (size_t)line_ld(Lx.m) * sizeof(double2);
   if (!fx) {
-    const int t = line_threads(Lx, 1);
+    const int t = line_threads(Lx, 1, pairs, P.nsm);
     if (ws)
       k_rows_r2c<2><<<pairs, t, smx, s>>>(Lx, Ny, plan.twx, nullptr, *ws, plan.spec, P, alpha, beta, gamma, skip,
                                          maxbits);
@@ -1171,9 +1186,9 @@ cudaError_t fft_passes(const DevOps &P, const FftPlan &plan, const double *src, 
     });
   });
   if (!fy) {
-    const int G = cols_group(Ly);
+    const int G = cols_group(Ly, H, P.nsm);
     const size_t smy = 2 * (size_t)G * line_ld(Ly.m) * sizeof(double2);
-    k_cols<<<(H + G - 1) / G, line_threads(Ly, G), smy, s>>>(Ly, H, G, plan.twy, P.fft_ax, P.fft_ay, P.fft_dxdy,
+    k_cols<<<(H + G - 1) / G, line_threads(Ly, G, (H + G - 1) / G, P.nsm), smy, s>>>(Ly, H, G, plan.twy, P.fft_ax, P.fft_ay, P.fft_dxdy,
                                                             plan.spec, maxbits, skip);
   }
   // rows, half spectrum -> real
@@ -1185,7 +1200,7 @@ cudaError_t fft_passes(const DevOps &P, const FftPlan &plan, const double *src, 
              skip);
   });
   if (!fx2)
-    k_rows_c2r<<<pairs, line_threads(Lx, 1), smx, s>>>(Lx, Ny, plan.twx, plan.spec, dp, accumulate ? 1 : 0,
+    k_rows_c2r<<<pairs, line_threads(Lx, 1, pairs, P.nsm), smx, s>>>(Lx, Ny, plan.twx, plan.spec, dp, accumulate ? 1 : 0,
                                                        gate ? gate : maxbits, skip);
   return cudaSuccess;
 }

@@ -9,6 +9,10 @@
 // of power-of-two length m >= 2n - 1.  Either way O(n log n) operations per
 // line, where direct sums take n^2.  A pass is bound by its shared-memory
 // round trip and barrier, so the passes are few and their reads contiguous.
+// A prime of up to 127 is a pass of direct sums: one pass where Bluestein's
+// algorithm takes two transforms of twice the length and three products (67 x 67
+// solve 38.9 and 48.7 us, 113 x 113 46.3 and 49.1, 127 x 127 the same; with 31 for
+// the limit 37 x 37 took 48.6 us instead of 34.4, plain sums over the line 39.1).
 // Measured on B200 against direct sums: 1000 x 600 solve 2271 -> 54 us (rows
 // 8.6 and 8.5 us, columns 18.6 us), 40 x 40 step on host arrays 225 -> 203 us.
 #pragma once
@@ -17,7 +21,7 @@
 
 namespace ins2d {
 
-constexpr int kMaxFactor = 31;
+constexpr int kMaxFactor = 127;
 
 // shared-memory slot of value i: eight lanes of 16-byte accesses a power of
 // two apart fall on distinct banks
@@ -133,23 +137,40 @@ __device__ __forceinline__ void line_pass(const FftLine &L, int i, const double2
     for (int k = 1; k < R; ++k) B[line_slot(o + s * k)] = c_mul(x[k], w[k]);
   }
 }
-// the same for any radix, one output value per thread
+// the same for any odd radix by direct sums.  A thread forms outputs k and R - k
+// of a butterfly together (their sums over the pairs j, R - j differ in a sign
+// only): a quarter of the loads of one output per thread.
 __device__ __forceinline__ void line_pass_any(const FftLine &L, int i, const double2 *a, double2 *b, int lines,
                                               int ld, const double2 *__restrict__ tw) {
-  const unsigned R = L.r[i], nb = L.m / R, s = L.s[i], m = L.m;
-  for (unsigned idx = threadIdx.x; idx < lines * m; idx += blockDim.x) {
-    const unsigned line = lines > 1 ? idx / m : 0u, v = idx - line * m;
-    const unsigned k = v / nb, u = v - k * nb;  // output k of butterfly u
+  const unsigned R = L.r[i], nb = L.m / R, s = L.s[i], h = R / 2, per = nb * (h + 1);
+  for (unsigned idx = threadIdx.x; idx < lines * per; idx += blockDim.x) {
+    const unsigned line = lines > 1 ? idx / per : 0u, v = idx - line * per;
+    const unsigned k = v / nb, u = v - k * nb;  // outputs k, R - k of butterfly u
     const unsigned p = fast_div(u, s, L.inv_s[i]), q = u - p * s;
     const double2 *A = a + line * ld;
-    double2 acc = A[line_slot(u)];
+    double2 *B = b + line * ld;
+    const unsigned o = q + s * R * p;
+    double2 x = A[line_slot(u)], y = make_double2(0.0, 0.0);
     unsigned jk = 0;
-    for (unsigned j = 1; j < R; ++j) {
+#pragma unroll 2
+    for (unsigned j = 1; j <= h; ++j) {
+      const double2 f = A[line_slot(u + j * nb)], g = A[line_slot(u + (R - j) * nb)];
       jk += k;
       if (jk >= R) jk -= R;
-      acc = c_add(acc, c_mul(A[line_slot(u + j * nb)], __ldg(tw + jk * nb)));
+      const double2 w = __ldg(tw + jk * nb);  // cos, -sin
+      x.x += w.x * (f.x + g.x);
+      x.y += w.x * (f.y + g.y);
+      y.x += w.y * (f.x - g.x);
+      y.y += w.y * (f.y - g.y);
     }
-    b[line * ld + line_slot(q + s * (R * p + k))] = c_mul(acc, __ldg(tw + p * s * k));
+    // x + i y and x - i y
+    if (k == 0) {
+      B[line_slot(o)] = x;
+    } else {
+      const unsigned e = p * s * k, m = R - k;
+      B[line_slot(o + s * k)] = c_mul(make_double2(x.x - y.y, x.y + y.x), __ldg(tw + e));
+      B[line_slot(o + s * m)] = c_mul(make_double2(x.x + y.y, x.y - y.x), __ldg(tw + p * s * m));
+    }
   }
 }
 

@@ -35,6 +35,7 @@ static __device__ __align__(256) double2 g_scratch[kTotal];
 
 constexpr int kMaxDevices = 64;
 double2 *g_scratch_addr[kMaxDevices] = {nullptr};
+int g_nsm[kMaxDevices];
 // the (Nx, Ny, dx, dy) whose twiddle and symbol tables the device's scratch
 // holds, so repeated calls of one size upload nothing
 struct TableKey {
@@ -56,18 +57,22 @@ extern "C" int ins2d_fft_poisson_noalloc(const double *f, double *dp, int32_t Nx
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return INS2D_ECUDA;
   // once per device, with that device current: the device address of the
-  // static array (its host-side name is only a stand-in)
+  // static array (its host-side name is only a stand-in) and its SM count,
+  // which the launch rules read
   double2 *base = nullptr;
   bool upload = true;
+  int nsm = 0;
   FftPlan plan;
   {
     std::lock_guard<std::mutex> lk(g_setup_mu);
     if (!g_scratch_addr[dev]) {
       void *ptr = nullptr;
       if (cudaGetSymbolAddress(&ptr, g_scratch) != cudaSuccess || !ptr) return INS2D_ECUDA;
+      if (cudaDeviceGetAttribute(&g_nsm[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return INS2D_ECUDA;
       g_scratch_addr[dev] = (double2 *)ptr;
     }
     base = g_scratch_addr[dev];
+    nsm = g_nsm[dev];
     const TableKey &k = g_tables[dev];
     upload = !(k.Nx == Nx && k.Ny == Ny && k.dx == dx && k.dy == dy);
     // forget the key until the new tables are uploaded: a failed upload must
@@ -86,7 +91,7 @@ extern "C" int ins2d_fft_poisson_noalloc(const double *f, double *dp, int32_t Nx
   double *maxabs = (double *)(base + kSpec + 5 * (size_t)kMaxN);
   if (upload) try {
     plan = fft_plan(Nx, Ny);
-    if (fft_prepare(plan, 0) != cudaSuccess) return INS2D_ECUDA;  // the kernels' shared-memory limits
+    if (fft_prepare(plan, nsm) != cudaSuccess) return INS2D_ECUDA;  // the kernels' shared-memory limits
     // twiddle tables and the symbol factors (1/dx^2) sin^2(I pi/Nx),
     // (1/dy^2) sin^2(J pi/Ny) of operator_divergence.m:283, as in the context path
     const std::vector<double> tx = fft_twiddle_table(Nx), ty = fft_twiddle_table(Ny);
@@ -114,6 +119,7 @@ extern "C" int ins2d_fft_poisson_noalloc(const double *f, double *dp, int32_t Nx
     return INS2D_ENOMEM;
   }
   DevOps P{};
+  P.nsm = nsm;
   P.fft_ax = axd;
   P.fft_ay = ayd;
   P.fft_dxdy = dx * dy;

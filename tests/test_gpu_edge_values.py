@@ -224,3 +224,33 @@ def test_work_arrays():
 
     used("jacobi"), used("fdm")  # kernels and pools loaded
     assert used("fdm") - used("jacobi") >= 4 * 512 * 1024 * 8
+
+
+# Transform solves on sides with primes above 31: direct sums up to 127 (alone,
+# beside other radices, in one block and in three kernels), Bluestein's algorithm
+# from 131 on; right-hand sides formed from a velocity as well.  The parity
+# tests' bounds for one evaluation and for a step.
+@pytest.mark.parametrize("shape", [(37, 37), (41, 41), (61, 29), (127, 8), (8, 127), (64, 113), (127, 64), (254, 67),
+                                   (8, 381), (536, 201), (131, 64), (64, 137), (12, 131)])
+def test_direct_sums(shape):
+    import ins2d_b200
+    from oracle import ins2d_ref as R
+    from tests.cases_common import BC_COMBOS
+    nx, ny = shape
+    x, y = np.arange(nx + 1) / nx * 1.5, np.arange(ny + 1) / ny
+    m = ins2d_b200.Options(x, y, BC_COMBOS["periodic"], poisson=6, Re=100.0)
+    rng = np.random.default_rng(nx)
+    f = rng.standard_normal((ny, nx))
+    f -= f.mean()
+    J, I = np.arange(ny)[:, None], np.arange(nx)[None, :]
+    a = 4 * x[1] * y[1] * (np.sin(np.pi * I / nx) ** 2 / x[1] ** 2 + np.sin(np.pi * J / ny) ** 2 / y[1] ** 2)
+    a[0, 0] = 1.0
+    ref = np.real(np.fft.ifft2(-np.fft.fft2(f) / a)).ravel()
+    assert np.max(np.abs(m.pressure_poisson(f.ravel()) - ref)) < 1e-12 * np.max(np.abs(ref))
+    assert np.all(m.pressure_poisson(np.zeros(nx * ny)) == 0.0)
+    o = R.make_options(x, y, BC_COMBOS["periodic"], poisson=6, Re=100.0)
+    V = R.initial_projection(rng.standard_normal(o.grid.NV), 0.0, o)
+    ref, _ = R.time_ERK(V, np.zeros(m.Np), 0.0, 1e-4, o)
+    for precision, tol in (("fp64", 1e-11), ("fp32", 1e-5)):
+        m = ins2d_b200.Options(x, y, BC_COMBOS["periodic"], poisson=6, Re=100.0, precision=precision)
+        assert np.max(np.abs(m.time_ERK(V, np.zeros(m.Np), 0.0, 1e-4)[0] - ref)) < tol * np.max(np.abs(ref))
