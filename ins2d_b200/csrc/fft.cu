@@ -589,23 +589,23 @@ __device__ __forceinline__ void dit16_passes(double2 *a, int ld, int lines, cons
   }
 }
 
-// A row line's points v(i) into shared memory: with the first three DIF stages
-// on the way where every thread then has eight points to load; below that
-// (L <= 10) the points are spread over all threads and the passes start from
-// shared memory (line_top), since a quarter of the threads with eight points of
-// five loads each is bound by the latency of its loads (a 512^2 step, ten per
-// call: 1.224 -> 1.052 ms; at 2048 points staging is 1% slower).
+// A row line's points v(i) into shared memory, with the first three DIF stages
+// on the way: the passes go on from stage line_top.  Where that leaves threads
+// idle (L <= 10) and a point is the divergence's five loads (DIV), the points are
+// spread over all threads instead and the passes start from shared memory: a
+// quarter of the threads is bound by the latency of those loads (a 512^2 step, ten
+// per call: 1.224 -> 1.052 ms; at 2048 points staging is 1% slower).
 #ifndef INS2D_FFT_STAGE_L
 #define INS2D_FFT_STAGE_L 10
 #endif
-template <int L>
+template <int L, bool DIV>
 __host__ __device__ constexpr int line_top() {
-  return L <= INS2D_FFT_STAGE_L ? L : L - 3;
+  return DIV && L <= INS2D_FFT_STAGE_L ? L : L - 3;
 }
-template <int L, typename Fn>
+template <int L, bool DIV, typename Fn>
 __device__ __forceinline__ void load_line(double2 *sm, const double2 *pyr, bool inv, Fn &&v) {
   constexpr int N = 1 << L, PER = N >> 3;
-  if constexpr (line_top<L>() == L) {
+  if constexpr (line_top<L, DIV>() == L) {
     constexpr int U = N >= 4 * kThreads ? 4 : N >= 2 * kThreads ? 2 : 1;
 #pragma unroll U
     for (int i = threadIdx.x; i < N; i += kThreads) sm[pdl<L>(i)] = v(i);
@@ -668,10 +668,10 @@ __global__ void __launch_bounds__(kThreads, INS2D_FFT_ROWS_MINB)
       const double d1 = hy1 * (w0 * W(ub + c0) + w1 * W(ub + c1)) + hx * (m10 * vb_i + m11 * W(vc + i));
       return make_double2(d0 * gamma, has1 ? d1 * gamma : 0.0);
     };
-    load_line<L>(sm, pyr, false, cell);
+    load_line<L, DIV>(sm, pyr, false, cell);
   } else {
     const double *r0 = f + (size_t)j0 * N, *r1 = f + (size_t)j1 * N;
-    load_line<L>(sm, pyr, false, [&](int i) -> double2 {
+    load_line<L, DIV>(sm, pyr, false, [&](int i) -> double2 {
       if constexpr (SRC == 2)
         return make_double2(div_cell_f(P, ws, alpha, beta, gamma, i, j0),
                             has1 ? div_cell_f(P, ws, alpha, beta, gamma, i, j1) : 0.0);
@@ -683,7 +683,7 @@ __global__ void __launch_bounds__(kThreads, INS2D_FFT_ROWS_MINB)
     });
   }
   __syncthreads();
-  dif_passes<L, line_top<L>(), 1, 1>(sm, 0, 1, pyr, false);
+  dif_passes<L, line_top<L, DIV>(), 1, 1>(sm, 0, 1, pyr, false);
   for (int I = threadIdx.x; I < H; I += kThreads) {
     const double2 z = sm[pdl<L>(brev(I, L))], m = sm[pdl<L>(brev((N - I) & (N - 1), L))];
     spec[(size_t)j0 * H + I] = make_double2(0.5 * (z.x + m.x), 0.5 * (z.y - m.y));
@@ -837,7 +837,7 @@ __global__ void __launch_bounds__(kThreads, INS2D_FFT_ROWS_MINB)
   }
   const double2 *pyr = tw + N;
   const double2 *s0 = spec + (size_t)j0 * H, *s1 = spec + (size_t)j1 * H;
-  load_line<L>(sm, pyr, true, [&](int q) -> double2 {
+  load_line<L, false>(sm, pyr, true, [&](int q) -> double2 {
     double2 g0, g1;
     if (q < H) {
       g0 = s0[q];
@@ -851,7 +851,7 @@ __global__ void __launch_bounds__(kThreads, INS2D_FFT_ROWS_MINB)
     return make_double2(g0.x - g1.y, g0.y + g1.x);
   });
   __syncthreads();
-  dif_passes<L, line_top<L>(), 1, 1>(sm, 0, 1, pyr, true);
+  dif_passes<L, line_top<L, false>(), 1, 1>(sm, 0, 1, pyr, true);
   const double sc = 1.0 / N;
   for (int k = threadIdx.x; k < N; k += kThreads) {
     const double2 w = sm[pdl<L>(brev(k, L))];
