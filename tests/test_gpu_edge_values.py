@@ -254,3 +254,41 @@ def test_direct_sums(shape):
     for precision, tol in (("fp64", 1e-11), ("fp32", 1e-5)):
         m = ins2d_b200.Options(x, y, BC_COMBOS["periodic"], poisson=6, Re=100.0, precision=precision)
         assert np.max(np.abs(m.time_ERK(V, np.zeros(m.Np), 0.0, 1e-4)[0] - ref)) < tol * np.max(np.abs(ref))
+
+
+# The spectral preconditioner on sides that are no powers of two (one block,
+# mixed radix, direct sums, one compile-time side): its solves against the
+# transform solver's; a right-hand side near the zero threshold, where the
+# preconditioner must not take the early return of a direct solve (a tolerance
+# of 1e-18 takes it to residuals below 1e-26 in a second pass, met or not; a
+# zero application would end as a breakdown); steps in a captured run
+@pytest.mark.parametrize("shape", [(40, 40), (74, 60), (100, 60), (64, 45), (37, 61), (256, 134)])
+def test_spectral_preconditioner_sides(shape):
+    import ins2d_b200
+    from ins2d_b200 import cases
+    nx, ny = shape
+    x, y = cases.uniform_grid(nx, 0.0, 1.0), cases.uniform_grid(ny, 0.0, ny / nx)
+    kw = dict(Re=100.0, precond="fdm")
+    m = ins2d_b200.Options(x, y, cases.BC_PERIODIC, poisson=4, CG_acc=1e-12, **kw)
+    mf = ins2d_b200.Options(x, y, cases.BC_PERIODIC, poisson=6, Re=100.0)
+    rng = np.random.default_rng(nx)
+    f = rng.standard_normal(nx * ny)
+    f -= f.mean()
+    ref = mf.pressure_poisson(f)
+    ref -= ref.mean()
+    for scale in (1.0, 2.0 ** -43):
+        dp, st = m.pressure_poisson(scale * f, return_stats=True)
+        assert 1 <= st["iters"] <= 2
+        assert np.max(np.abs(dp - dp.mean() - scale * ref)) < 1e-11 * scale * np.max(np.abs(ref))
+    assert np.all(m.pressure_poisson(np.zeros(nx * ny)) == 0.0)
+    never = ins2d_b200.Options(x, y, cases.BC_PERIODIC, poisson=4, CG_acc=1e-18, CG_maxit=3, **kw)
+    try:
+        assert never.pressure_poisson(2.0 ** -43 * f, return_stats=True)[1]["iters"] >= 2
+    except ins2d_b200.Ins2dError as e:
+        assert e.status == 2
+    V, p = 0.1 * rng.standard_normal(m.NV), np.zeros(m.Np)
+    V = mf.time_ERK(V, p, 0.0, 1e-4)[0]
+    Va, pa = m.time_ERK(V, p, 0.0, 1e-4, nsteps=3)
+    Vb, pb = mf.time_ERK(V, p, 0.0, 1e-4, nsteps=3)
+    assert np.max(np.abs(Va - Vb)) < 1e-10 * np.max(np.abs(Vb))
+    assert np.max(np.abs((pa - pa.mean()) - (pb - pb.mean()))) < 1e-8 * np.max(np.abs(pb))
