@@ -45,12 +45,18 @@ struct RegD {
 };
 __device__ __forceinline__ int wrapn(int c, int n) { return c < 0 ? c + n : (c >= n ? c - n : c); }
 
-// Programmatic dependent launch (kernels started by launch_k with the
+// Programmatic dependent launch (kernels started by launch_kp with the
 // attribute set): pdl_wait returns once the previous kernel in the stream has
-// completed and its writes are visible; it is a no-op for a plain launch.  A
-// kernel that calls it touches no global memory before it.  pdl_trigger,
-// after the wait, lets the next kernel's blocks be scheduled while this
-// kernel's last blocks run (they wait in their own pdl_wait).
+// completed and its writes are visible; it is a no-op for a plain launch.
+// pdl_trigger, after the wait, lets the next kernel's blocks be scheduled while
+// this kernel's last blocks run (they wait in their own pdl_wait).  Before the
+// wait a kernel writes nothing to global memory, and reads only what was complete
+// before the previous kernel could start: every kernel triggers after its own
+// wait, so that is what the kernel before the previous one, or a copy, had
+// finished.  Three kinds of data are read so: tables of the context; boundary
+// values (copied in and waited for, ins2d_set_bc_values); the network's weights
+// (packed before layer 1, which waits, and read from layer 2 on).  A kernel that
+// writes one of them directly before such a launch would race.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 

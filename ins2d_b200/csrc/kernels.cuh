@@ -306,7 +306,7 @@ struct PcgWork {
   double *x, *r, *p, *q;
   double *p2;          // fast diagonalization: directions alternate between p and p2
   PcgScalars *sc;      // device
-  double *partials;    // >= blocks * 4
+  double *partials;    // blocks * 8, then a reduction's results
   int blocks;
   PcgScalars *hsc;     // fast diagonalization: also the solve's scalars as they end a kernel (host memory; may be null)
 };

@@ -13,8 +13,8 @@
 // the modes b, a warp per system).  A pass takes five cluster barriers.
 // Beside the barriers (about 1000 cycles each) a launch pays for the first
 // touch of its parameters, tables and instructions; what depends on the
-// context alone is loaded before the wait for the previous kernel
-// (programmatic dependent launch, DevOps::pdl).  Measured on B200, RK44 step
+// context and the boundary values alone is loaded before the wait for the previous
+// kernel (programmatic dependent launch, DevOps::pdl).  Measured on B200, RK44 step
 // of the 64^2 cavity (four solves): one thread block working from L1/L2 and a
 // separate divergence launch 0.228 ms; eight blocks of 256 threads with
 // scattered 8-byte exchanges 0.117 ms; 512 threads, 16-byte exchanges and
@@ -263,8 +263,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   const int b0 = c * g.nb, b1 = min(b0 + g.nb, nm);
   TriTab<kTriC> tab;
   tri_tables<kTriC>(F, b0 + warp < b1 ? b0 + warp : nm, lane * kTriC, tab);
-  // everything above depends on the context alone; the right-hand side on the
-  // kernels before this one
+  // everything above reads tables of the context and boundary values, complete
+  // before the previous kernel started (pdl_wait); the right-hand side is its work
   pdl_wait();
   pdl_trigger();
   // right-hand side (cg.F:207-229 with x_in = 0)
