@@ -46,6 +46,8 @@ extern "C" {
 #define INS2D_OK 0
 #define INS2D_EINVAL 1      /* invalid argument / unsupported BC combination */
 #define INS2D_ENOTCONV 2    /* PCG did not reach CG_acc within CG_maxit */
+                               /* (or cannot: a right-hand side whose sum is not zero on a closed
+                                  or periodic domain, with fast diagonalization found at once) */
 #define INS2D_EBREAKDOWN 3  /* PCG breakdown (p'Ap = 0) */
 #define INS2D_ENONFINITE 4  /* NaN/Inf met in a solve or step */
 #define INS2D_ETIMEOUT 5    /* a bounded device wait gave up */

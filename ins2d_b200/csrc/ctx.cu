@@ -2042,6 +2042,7 @@ void ens_build_batch(ins2d_ens *e, const std::vector<int> &order) {
     cg[m].zero = 1;
     if (e->use_fdm) {
       const DevOps &P = e->mem[m]->P;
+      cg[m].singular = e->h_fdm[m].null_mode >= 0;
       cg[m].part = ens_alloc<double>(e, ens_fdm_scratch(P.Npx, P.Npy));
       cg[m].ntiles = (int)((P.Np + kEnsCells - 1) / kEnsCells);
     }

@@ -60,7 +60,7 @@ __device__ __forceinline__ void copy_ops(DevOps *dst, const DevOps *src) {
     ((long long *)dst)[k] = ((const long long *)src)[k];
 }
 
-// f = (M Wt + yM/dt) gamma (mode 0) or M wres (mode 1); f'f, max|f|
+// f = (M Wt + yM/dt) gamma (mode 0) or M wres (mode 1); f'f, max|f|, sum
 __global__ void __launch_bounds__(kThreads) k_ef_init(const EnsFdmRun R, int mode, double gamma, const LoopCond cond) {
   __shared__ __align__(16) DevOps sP;
   const int4 t = R.tiles[blockIdx.x];
@@ -70,8 +70,8 @@ __global__ void __launch_bounds__(kThreads) k_ef_init(const EnsFdmRun R, int mod
   __syncthreads();
   const double *W = mode == 0 ? M.Wt : M.wres;
   const double alpha = mode == 0 ? 1.0 / M.dt : 0.0, g = mode == 0 ? gamma : 1.0;
-  double q[2] = {0.0, 0.0};
-  const int ops[2] = {R_SUM, R_MAX};
+  double q[3] = {0.0, 0.0, 0.0};
+  const int ops[3] = {R_SUM, R_MAX, R_SUM};
   // loads of all the thread's cells before the first store, here and below: a
   // store in between orders the next cell's loads behind it
   const int Np = (int)sP.Np, Npx = sP.Npx;
@@ -88,9 +88,13 @@ __global__ void __launch_bounds__(kThreads) k_ef_init(const EnsFdmRun R, int mod
     if (k < Np) f[k] = fv[u];
     q[0] += fv[u] * fv[u];
     q[1] = fmax(q[1], fabs(fv[u]));
+    q[2] += fv[u];
   }
-  double out[2];
-  if (grid_reduce_at<2>(q, ops, member_red(C, 2), out, t.z, C.ntiles)) {
+  double out[3];
+  if (grid_reduce_at<3>(q, ops, member_red(C, 3), out, t.z, C.ntiles)) {
+    const RhsRange range = C.singular ? RhsRange::of(out[2], (double)Np, out[0], C.tol2) : RhsRange::none();
+    C.mean = range.mean;
+    C.irr = range.irr;
     C.rr0 = out[0];
     C.rr = 0.0;
     C.rz = 0.0;
@@ -100,6 +104,11 @@ __global__ void __launch_bounds__(kThreads) k_ef_init(const EnsFdmRun R, int mod
     int done = (out[1] < 1e-14 || C.rr0 <= C.tol2) ? 1 : 0;
     if (!isfinite(C.rr0)) {
       C.status = INS2D_ENONFINITE;
+      done = 1;
+    }
+    if (!done && C.singular && RhsRange::refused(out[2], (double)Np, out[0], C.tol2)) {
+      C.status = INS2D_ENOTCONV;
+      C.rr = range.q;
       done = 1;
     }
     if (done) add_stats(C, R.stats[t.x]);
@@ -172,7 +181,7 @@ __global__ void __launch_bounds__(kThreads) k_ef_update(const EnsFdmRun R, const
   const EnsMemberD &M = R.mem[t.x];
   const int stop = *(volatile int *)&C.done;  // with the other scalars: one latency
   const long long it = C.it;
-  const double alpha = C.alpha;
+  const double alpha = C.alpha, sub = it == 0 ? C.mean : 0.0;
   const int sol = C.sol;
   const PcgWork W = M.W;
   double *xw = sol == 0 ? M.dp : M.W.x;
@@ -194,7 +203,7 @@ __global__ void __launch_bounds__(kThreads) k_ef_update(const EnsFdmRun R, const
     x[u] = r[u] = 0.0;
     if (k < Np) {
       x[u] = (first ? 0.0 : xw[k]) + alpha * __ldg(p + k);
-      r[u] = ro[k] - alpha * __ldg(W.q + k);
+      r[u] = (ro[k] - sub) - alpha * __ldg(W.q + k);
     }
   }
 #pragma unroll
@@ -213,7 +222,7 @@ __global__ void __launch_bounds__(kThreads) k_ef_update(const EnsFdmRun R, const
       done = 1;
     } else {
       C.it += 1;
-      C.rr = out[0] / C.rr0;
+      C.rr = out[0] / C.rr0 + C.irr;
       if (!isfinite(C.rr)) {
         C.status = INS2D_ENONFINITE;
         done = 1;
@@ -252,7 +261,7 @@ __global__ void __launch_bounds__(kThreads) k_ef_finish(const EnsFdmRun R) {
 size_t ens_fdm_scratch(int nx, int ny) {
   const size_t cells = ((size_t)nx * ny + kEnsCells - 1) / kEnsCells;
   const size_t tiles = (size_t)((nx + 31) / 32) * ((ny + 31) / 32);  // fdm.cu's output tiles
-  return 2 * cells + tiles + 8;
+  return 3 * cells + tiles + 8;
 }
 
 void ens_fdm_init(const EnsFdmRun &R, int mode, double gamma, cudaGraphConditionalHandle h, int limit, cudaStream_t s) {

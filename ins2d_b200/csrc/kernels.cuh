@@ -285,6 +285,7 @@ struct PcgScalars {
   int done, status;
   unsigned int counter;
   int loops;  // passes of a device-side iteration loop (graph form)
+  double mean, irr;  // fast diagonalization: RhsRange of the solve
 };
 // Solve statistics accumulated on the device by the solves of a captured
 // step graph (the host reads them after the graph launches).
@@ -339,6 +340,29 @@ struct LoopCond {
 __device__ __forceinline__ void set_cond(const LoopCond &c, bool go) {
   if (c.limit >= 0) cudaGraphSetConditional(c.h, go ? 1u : 0u);
 }
+// What of a right-hand side a singular A cannot produce.  Its range is the fields
+// whose sum is zero, so the mean of f stays in the residual for good: q = n mean^2
+// / f'f is the least ||r||^2 / ||f||^2.  The first update takes the mean off and it
+// counts in the stopping rule as long as that can hold at all.  (Left in, it is
+// most of the residual after one pass, the application's rounding of it has a mean
+// of its own, and the iteration "converged" to solutions with constants of 1e16
+// times the mean.)  Beyond the rule, up to kInconsistent is taken for what the
+// cancellation in a divergence leaves (1e-12 and more on small grids near rest);
+// above that the solve is refused at once as not converging.
+constexpr double kInconsistent = 1e-10;
+struct RhsRange {
+  double mean, irr, q;  // irr: added to ||r||^2 / ||f||^2
+  __device__ static RhsRange none() { return {0.0, 0.0, 0.0}; }
+  __device__ static RhsRange of(double sum, double n, double rr0, double tol2) {
+    const double mean = sum / n, q = sum * mean / rr0;
+    return {mean, q <= tol2 ? q : 0.0, q};
+  }
+  // whether the solve is refused (no divisions: every thread of a cluster asks)
+  __device__ static bool refused(double sum, double n, double rr0, double tol2) {
+    const double s2 = sum * sum, m = n * rr0;
+    return s2 > tol2 * m && s2 > kInconsistent * kInconsistent * m;
+  }
+};
 // r'z of a new application (one thread): the first one's, or beta
 __device__ __forceinline__ void pcg_new_rz(PcgScalars *s, double rz) {
   if (!isfinite(rz)) {
@@ -418,6 +442,8 @@ struct EnsCg {
   // iterate (sol 0) or in dp (1), the running solve taking the other one; none
   // yet, or solved without a pass: zero.  stage: the running solve is a stage's
   int sol, zero, stage;
+  int singular;      // the member's A is
+  double mean, irr;  // RhsRange of the solve
 };
 // --- ensembles with fast diagonalization (ens_fdm.cu) -----------------------
 // cell tiles {member, first cell, number within the member, 0} of kEnsCells

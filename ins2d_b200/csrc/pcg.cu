@@ -503,13 +503,13 @@ __global__ void __launch_bounds__(kVecThreads) k_pupdate_g(const PcgWork W, cons
 // kernels, measured on B200: stretched 512^2 channel step 0.890 -> 0.773 ms,
 // 301 x 257 channel solve 198 -> 163 us.
 
-// sums over f: f'f and max|f|; the solve's scalars (copy: also r = f, the
+// f'f, max|f| and the sum of f; the solve's scalars (copy: also r = f, the
 // spectral application's input)
 __global__ void __launch_bounds__(kVecThreads) k_init_f(const PcgWork W, const double *__restrict__ f, long long n,
-                                                        double tol2, long long maxit, int copy,
+                                                        double tol2, long long maxit, int copy, int singular,
                                                         const LoopCond cond) {
-  double q[2] = {0.0, 0.0};
-  const int ops[2] = {R_SUM, R_MAX};
+  double q[3] = {0.0, 0.0, 0.0};
+  const int ops[3] = {R_SUM, R_MAX, R_SUM};
   const long long stride = (long long)gridDim.x * blockDim.x;
 #pragma unroll 4
   for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += stride) {
@@ -517,10 +517,14 @@ __global__ void __launch_bounds__(kVecThreads) k_init_f(const PcgWork W, const d
     if (copy) W.r[k] = fv;
     q[0] += fv * fv;
     q[1] = fmax(q[1], fabs(fv));
+    q[2] += fv;
   }
-  double out[2];
-  if (grid_reduce<2>(q, ops, red_of(W), out)) {
+  double out[3];
+  if (grid_reduce<3>(q, ops, red_of(W), out)) {
     PcgScalars *s = W.sc;
+    const RhsRange R = singular ? RhsRange::of(out[2], (double)n, out[0], tol2) : RhsRange::none();
+    s->mean = R.mean;
+    s->irr = R.irr;
     s->tol2 = tol2;
     s->maxit = maxit;
     s->rr0 = out[0];
@@ -534,6 +538,11 @@ __global__ void __launch_bounds__(kVecThreads) k_init_f(const PcgWork W, const d
     s->done = (out[1] < 1e-14 || out[0] <= tol2) ? 1 : 0;
     if (!isfinite(out[0])) {
       s->status = INS2D_ENONFINITE;
+      s->done = 1;
+    }
+    if (!s->done && singular && RhsRange::refused(out[2], (double)n, out[0], tol2)) {
+      s->status = INS2D_ENOTCONV;
+      s->rr = R.q;
       s->done = 1;
     }
     set_cond(cond, !s->done && 0 < cond.limit);
@@ -623,6 +632,7 @@ __global__ void __launch_bounds__(kVecThreads) k_update_f(const PcgWork W, const
                                                           const LoopCond cond) {
   const int done = *(volatile int *)&W.sc->done;
   const double alpha = W.sc->alpha;  // read together with done: one latency
+  const double mean = W.sc->mean;
   const long long it = W.sc->it;
   if (done) {  // an earlier kernel of this pass found an error
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -637,6 +647,7 @@ __global__ void __launch_bounds__(kVecThreads) k_update_f(const PcgWork W, const
   const int ops[4] = {R_SUM, R_MAX, R_MIN, R_MAX};
   const long long stride = (long long)gridDim.x * blockDim.x;
   const double *ro = first ? f : W.r;
+  const double sub = first ? mean : 0.0;
   // four points' loads before the first store, which would order the next
   // points' loads behind it
   for (long long k0 = blockIdx.x * (long long)blockDim.x + threadIdx.x; k0 < n; k0 += 4 * stride) {
@@ -646,7 +657,7 @@ __global__ void __launch_bounds__(kVecThreads) k_update_f(const PcgWork W, const
       const long long k = k0 + u * stride;
       if (k < n) {
         x[u] = (first ? 0.0 : W.x[k]) + alpha * __ldg(p + k);
-        r[u] = ro[k] - alpha * __ldg(W.q + k);
+        r[u] = (ro[k] - sub) - alpha * __ldg(W.q + k);
       }
     }
 #pragma unroll
@@ -666,7 +677,7 @@ __global__ void __launch_bounds__(kVecThreads) k_update_f(const PcgWork W, const
   if (grid_reduce<4>(q, ops, red_of(W), out)) {
     PcgScalars *s = W.sc;
     s->it += 1;
-    s->rr = out[0] / s->rr0;
+    s->rr = out[0] / s->rr0 + s->irr;
     s->maxx = out[1];
     s->minx = out[2];
     s->maxres = out[3];
@@ -843,7 +854,7 @@ unsigned vec_blocks_f(const DevOps &P, const PcgWork &W) {
 void pcg_init_fdm(const DevOps &P, const FdmD &F, const PcgWork &W, const double *f, double tol, long long maxit,
                   cudaGraphConditionalHandle h, int limit, cudaStream_t s) {
   k_init_f<<<vec_blocks_f(P, W), kVecThreads, 0, s>>>(W, f, P.Np, tol * tol, maxit, F.spectral ? 1 : 0,
-                                                     LoopCond{h, limit});
+                                                     !F.spectral && F.null_mode >= 0, LoopCond{h, limit});
 }
 
 cudaError_t pcg_pass_fdm(const DevOps &P, const FdmD &F, const PcgWork &W, const double *f,

@@ -192,6 +192,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   extern __shared__ __align__(16) double sm[];
   __shared__ double warp_part[4][kWarps];
   __shared__ __align__(16) double part2[2][kC][4], part4[2][kC][4];
+  __shared__ RhsRange range;
   __shared__ DirRows dm, ds;  // along the modes' and the systems' direction
   cg::cluster_group cl = cg::this_cluster();
   cl.barrier_arrive();  // every block runs before any other writes to its shared memory (waited for below)
@@ -302,7 +303,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     status = INS2D_ENONFINITE;
     done = true;
   }
-  const int op1[1] = {R_SUM};
+  const int op1[1] = {R_SUM}, opz[2] = {R_SUM, R_SUM};
   if (QS) {
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     __syncthreads();
@@ -348,33 +349,43 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
     }
     cl.sync();
-    double a1[1] = {0.0};
+    double az[2] = {0.0, 0.0};  // r'z and the sum of r (a packet holds two values)
     product<false>(g, basis, zh, [&](int m, int sl, double v0, double v1) {
       if (m >= nm || sl >= nl) return;
       const int k = m * ld + sl;
       z[k] = v0;
-      a1[0] += r[k] * v0;
+      az[0] += r[k] * v0;
+      az[1] += r[k];
       if (sl == 0) cl.map_shared_rank(zhalo, br)[g.mp + m] = v0;
       if (sl + 1 < nl) {
         z[k + 1] = v1;
-        a1[0] += r[k + 1] * v1;
+        az[0] += r[k + 1] * v1;
+        az[1] += r[k + 1];
       }
       if (sl + 2 >= nl) cl.map_shared_rank(zhalo, bl)[m] = sl + 1 < nl ? v1 : v0;
     });
-    cluster_reduce<1>(cl, a1, op1, warp_part, part2, slot2);
-    if (!isfinite(a1[0])) {
+    cluster_reduce<2>(cl, az, opz, warp_part, part2, slot2);
+    if (!isfinite(az[0])) {
       status = INS2D_ENONFINITE;
       break;
     }
     const bool first = it == 0;
-    const double beta = first ? 0.0 : a1[0] / rz;
-    rz = a1[0];
+    if (first) {  // read after the next barriers
+      const bool singular = F.null_mode >= 0;
+      if (tid == 0) range = singular ? RhsRange::of(az[1], (double)nm * n, rr0, tol2) : RhsRange::none();
+      if (singular && RhsRange::refused(az[1], (double)nm * n, rr0, tol2)) {
+        status = INS2D_ENOTCONV;
+        break;
+      }
+    }
+    const double beta = first ? 0.0 : az[0] / rz;
+    rz = az[0];
     // p = z + beta p, with the neighbouring columns'
     for (int k = tid; k < (int)nc; k += kThreads) p[k] = first ? z[k] : z[k] + beta * p[k];
     for (int k = tid; k < 2 * g.mp; k += kThreads) ph[k] = first ? zhalo[k] : zhalo[k] + beta * ph[k];
     __syncthreads();
     // q = A p, p'q
-    a1[0] = 0.0;
+    double a1[1] = {0.0};
 #pragma unroll 2
     for (int l = tid; l < nslots; l += kThreads) {
       int m, sl;
@@ -410,7 +421,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       if (!cell(l, m, sl)) continue;
       const int k = m * ld + sl;
       const double xv = (first ? 0.0 : x[k]) + alpha * p[k];
-      const double rv = r[k] - alpha * q[k];
+      const double rv = (r[k] - (first ? range.mean : 0.0)) - alpha * q[k];
       x[k] = xv;
       r[k] = rv;
       a4[0] += rv * rv;
@@ -420,7 +431,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
     cluster_reduce<4>(cl, a4, op4, warp_part, part4, slot4);
     ++it;
-    rr = a4[0] / rr0;
+    rr = a4[0] / rr0 + range.irr;
     maxx = a4[1];
     minx = a4[2];
     maxres = a4[3];
@@ -448,7 +459,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   if (c == 0 && tid == 0) {
     PcgScalars *out = W.sc;
     out->rr0 = rr0;
-    out->rr = rr;
+    out->rr = it == 0 && status == INS2D_ENOTCONV ? range.q : rr;
     out->it = it;
     out->maxx = maxx;
     out->minx = minx;

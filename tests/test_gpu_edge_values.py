@@ -292,3 +292,51 @@ def test_spectral_preconditioner_sides(shape):
     Vb, pb = mf.time_ERK(V, p, 0.0, 1e-4, nsteps=3)
     assert np.max(np.abs(Va - Vb)) < 1e-10 * np.max(np.abs(Vb))
     assert np.max(np.abs((pa - pa.mean()) - (pb - pb.mean()))) < 1e-8 * np.max(np.abs(pb))
+
+
+# Right-hand sides outside the range of A (closed and periodic domains; their sum
+# is what A cannot produce): a solve with fast diagonalization ends with an error,
+# whichever form it takes (cluster, one to four warps per system, cyclic
+# systems); steps from rest on small grids, whose pressure update's right-hand
+# side is inconsistent by the rounding of its divergence, still end well
+@pytest.mark.parametrize("combo", ["cavity", "per_x_walls", "periodic"])
+@pytest.mark.parametrize("shape", [(12, 10), (7, 16), (64, 64), (128, 100), (200, 150), (20, 300), (600, 40)])
+def test_inconsistent_right_hand_side(shape, combo):
+    import ins2d_b200
+    from tests.cases_common import BC_COMBOS, grid_stretched
+    x, y = grid_stretched(shape[0], 0.0, 1.7), grid_stretched(shape[1], -0.5, 0.5, beta=1.2)
+    m = ins2d_b200.Options(x, y, BC_COMBOS[combo], Re=100.0, poisson=4, CG_acc=1e-10, CG_maxit=300)
+    rng = np.random.default_rng(shape[0])
+    f = rng.standard_normal(m.Np)
+    f -= f.mean()
+    vol = np.kron(np.diff(y), np.diff(x))
+    for g in (np.ones(m.Np), vol / vol.mean(), f + 1.0, f + 1e-3):
+        with pytest.raises(ins2d_b200.Ins2dError) as ei:
+            m.pressure_poisson(g)
+        assert ei.value.status in (2, 4)
+    dp = m.pressure_poisson(f)
+    assert abs(vol @ dp) <= 1e-12 * vol.sum() * np.max(np.abs(dp))
+
+
+@pytest.mark.parametrize("shape", [(3, 3), (4, 3), (8, 8), (140, 6), (33, 200)])
+@pytest.mark.parametrize("form", ["single", "ensemble"])
+def test_steps_from_rest(form, shape):
+    import ins2d_b200
+    from ins2d_b200 import cases
+    kw = dict(x=cases.tanh_grid(shape[0], 0.0, 1.0, 1.05), y=cases.tanh_grid(shape[1], 0.0, 1.0, 1.05), BC=cases.BC_CAVITY,
+              uBC=cases.lid_uBC(1.0, 1.0), Re=200.0, poisson=4, CG_acc=1e-12, CG_maxit=200, RK="RK44")
+    m = ins2d_b200.Options(**kw)
+    V, p = np.zeros(m.NV), np.zeros(m.Np)
+    p = m.pressure_additional_solve(V, p, 0.0)
+    scale = np.max(np.abs(p))
+    for nsteps in (1, 4):
+        if form == "single":
+            V1, p1 = m.time_ERK(V, p, 0.0, 1e-4, nsteps=nsteps)
+        else:
+            e = ins2d_b200.Ensemble([kw])
+            e.set_solver(0)
+            e.set_state(0, V, p)
+            e.time_ERK(0.0, 1e-4, nsteps)
+            V1, p1 = e.get_state(0)
+        assert np.max(np.abs(V1)) <= 1.0 and np.max(np.abs(p1)) <= 4.0 * scale  # no constant of the null space
+        assert m.check_conservation(V1, 0.0)[0] < 1e-10
