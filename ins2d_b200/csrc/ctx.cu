@@ -193,6 +193,7 @@ void upload_fdm(ins2d_ctx *c, FdmD &D) {
   if (T.null_mode >= 0) {
     D.ng = upload_vec(c, T.ng);
     D.nmu = upload_vec(c, T.nmu);
+    D.mean_w = 1.0 / (T.Q[T.null_mode] * T.nm * T.n);
   }
 }
 

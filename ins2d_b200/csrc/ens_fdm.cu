@@ -92,9 +92,9 @@ __global__ void __launch_bounds__(kThreads) k_ef_init(const EnsFdmRun R, int mod
   }
   double out[3];
   if (grid_reduce_at<3>(q, ops, member_red(C, 3), out, t.z, C.ntiles)) {
-    const RhsRange range = C.singular ? RhsRange::of(out[2], (double)Np, out[0], C.tol2) : RhsRange::none();
+    const RhsRange range = C.singular ? RhsRange::of(out[2] / Np, Np, out[0], C.tol2) : RhsRange::none();
     C.mean = range.mean;
-    C.irr = range.irr;
+    C.add = range.add(out[0], C.tol2);
     C.rr0 = out[0];
     C.rr = 0.0;
     C.rz = 0.0;
@@ -106,9 +106,9 @@ __global__ void __launch_bounds__(kThreads) k_ef_init(const EnsFdmRun R, int mod
       C.status = INS2D_ENONFINITE;
       done = 1;
     }
-    if (!done && C.singular && RhsRange::refused(out[2], (double)Np, out[0], C.tol2)) {
+    if (!done && range.refused(out[0], C.tol2)) {
       C.status = INS2D_ENOTCONV;
-      C.rr = range.q;
+      C.rr = range.miss / C.rr0;
       done = 1;
     }
     if (done) add_stats(C, R.stats[t.x]);
@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(kThreads) k_ef_update(const EnsFdmRun R, const
       done = 1;
     } else {
       C.it += 1;
-      C.rr = out[0] / C.rr0 + C.irr;
+      C.rr = (out[0] + C.add) / C.rr0;
       if (!isfinite(C.rr)) {
         C.status = INS2D_ENONFINITE;
         done = 1;

@@ -215,14 +215,13 @@ FftPlan fft_plan(int Nx, int Ny);
 std::vector<double> fft_twiddle_table(int n);
 // dp = real(ifft2(-fft2(f)./Ahat)) (pressure_poisson.m:92-104); dp += result when
 // accumulate.  Returns 0 (dp untouched / zero) when max|fhat| < 1e-14 (:21-32).
-// The return value is the error of the enqueued memset (kernel launch errors
-// are left to cudaGetLastError as for every launch).
+// Launch errors of this and the others below are left to cudaGetLastError.
 cudaError_t launch_fft_poisson(const DevOps &P, const FftPlan &plan, const double *f, double *dp, bool accumulate,
                                cudaStream_t s);
-// Same with the right-hand side f = (M W + alpha yM + beta ydM) gamma computed
-// inside the first pass.
 // kernel launches of one solve (one block's, or three passes)
 int fft_kernels(const FftPlan &plan);
+// Same with the right-hand side f = (M W + alpha yM + beta ydM) gamma computed
+// inside the first pass.
 cudaError_t launch_fft_poisson_div(const DevOps &P, const FftPlan &plan, const double *W, double alpha,
                                    double beta, double gamma, double *dp, bool accumulate, cudaStream_t s);
 // z = A^+ r by the same transform (the exact inverse of a periodic uniform
@@ -250,6 +249,7 @@ struct FdmD {
   const double *g = nullptr, *cr = nullptr;                 // cyclic systems: nm x n, nm
   int null_mode = -1;
   const double *ng = nullptr, *nmu = nullptr;               // its corrections: n
+  double mean_w = 0.0;  // the mean of r by the sum over its row of w = Q' r (a constant basis vector)
   const double *f = nullptr, *r = nullptr;  // ensembles: the member's right-hand side and CG residual
   double *t = nullptr;        // nm x n: transformed residual, then the systems' solutions
   double *z = nullptr;        // the preconditioned residual
@@ -285,7 +285,7 @@ struct PcgScalars {
   int done, status;
   unsigned int counter;
   int loops;  // passes of a device-side iteration loop (graph form)
-  double mean, irr;  // fast diagonalization: RhsRange of the solve
+  double mean, add;  // fast diagonalization: RhsRange of the solve
 };
 // Solve statistics accumulated on the device by the solves of a captured
 // step graph (the host reads them after the graph launches).
@@ -341,27 +341,28 @@ __device__ __forceinline__ void set_cond(const LoopCond &c, bool go) {
   if (c.limit >= 0) cudaGraphSetConditional(c.h, go ? 1u : 0u);
 }
 // What of a right-hand side a singular A cannot produce.  Its range is the fields
-// whose sum is zero, so the mean of f stays in the residual for good: q = n mean^2
-// / f'f is the least ||r||^2 / ||f||^2.  The first update takes the mean off and it
-// counts in the stopping rule as long as that can hold at all.  (Left in, it is
-// most of the residual after one pass, the application's rounding of it has a mean
-// of its own, and the iteration "converged" to solutions with constants of 1e16
-// times the mean.)  Beyond the rule, up to kInconsistent is taken for what the
-// cancellation in a divergence leaves (1e-12 and more on small grids near rest);
-// above that the solve is refused at once as not converging.
+// whose sum is zero, so the mean of f stays in the residual for good: miss = n mean^2
+// is the least ||r||^2.  Where that counts (a hundredth of the stopping rule) the
+// first update takes the mean off and miss is added in the rule, as long as that
+// can hold at all.  (Left in, it is most of the residual after one pass, the
+// application's rounding of it has a mean of its own, and the iteration "converged"
+// to solutions with constants of 1e16 times the mean.)  Beyond the rule, up to
+// kInconsistent of ||f|| is taken for what the cancellation in a divergence leaves
+// (1e-12 and more on small grids near rest); above that the solve is refused at
+// once as not converging.
 constexpr double kInconsistent = 1e-10;
-struct RhsRange {
-  double mean, irr, q;  // irr: added to ||r||^2 / ||f||^2
-  __device__ static RhsRange none() { return {0.0, 0.0, 0.0}; }
-  __device__ static RhsRange of(double sum, double n, double rr0, double tol2) {
-    const double mean = sum / n, q = sum * mean / rr0;
-    return {mean, q <= tol2 ? q : 0.0, q};
+struct __align__(16) RhsRange {
+  double mean, miss;
+  __device__ static RhsRange none() { return {0.0, 0.0}; }
+  __device__ static RhsRange of(double mean, double n, double rr0, double tol2) {
+    const double miss = mean * mean * n;
+    return miss > 0.01 * tol2 * rr0 ? RhsRange{mean, miss} : none();
   }
-  // whether the solve is refused (no divisions: every thread of a cluster asks)
-  __device__ static bool refused(double sum, double n, double rr0, double tol2) {
-    const double s2 = sum * sum, m = n * rr0;
-    return s2 > tol2 * m && s2 > kInconsistent * kInconsistent * m;
+  __device__ bool refused(double rr0, double tol2) const {
+    return miss > tol2 * rr0 && miss > kInconsistent * kInconsistent * rr0;
   }
+  // to ||r||^2 in the stopping rule
+  __device__ double add(double rr0, double tol2) const { return miss <= tol2 * rr0 ? miss : 0.0; }
 };
 // r'z of a new application (one thread): the first one's, or beta
 __device__ __forceinline__ void pcg_new_rz(PcgScalars *s, double rz) {
@@ -443,7 +444,7 @@ struct EnsCg {
   // yet, or solved without a pass: zero.  stage: the running solve is a stage's
   int sol, zero, stage;
   int singular;      // the member's A is
-  double mean, irr;  // RhsRange of the solve
+  double mean, add;  // RhsRange of the solve
 };
 // --- ensembles with fast diagonalization (ens_fdm.cu) -----------------------
 // cell tiles {member, first cell, number within the member, 0} of kEnsCells

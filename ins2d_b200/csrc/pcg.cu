@@ -522,9 +522,9 @@ __global__ void __launch_bounds__(kVecThreads) k_init_f(const PcgWork W, const d
   double out[3];
   if (grid_reduce<3>(q, ops, red_of(W), out)) {
     PcgScalars *s = W.sc;
-    const RhsRange R = singular ? RhsRange::of(out[2], (double)n, out[0], tol2) : RhsRange::none();
+    const RhsRange R = singular ? RhsRange::of(out[2] / n, n, out[0], tol2) : RhsRange::none();
     s->mean = R.mean;
-    s->irr = R.irr;
+    s->add = R.add(out[0], tol2);
     s->tol2 = tol2;
     s->maxit = maxit;
     s->rr0 = out[0];
@@ -540,9 +540,9 @@ __global__ void __launch_bounds__(kVecThreads) k_init_f(const PcgWork W, const d
       s->status = INS2D_ENONFINITE;
       s->done = 1;
     }
-    if (!s->done && singular && RhsRange::refused(out[2], (double)n, out[0], tol2)) {
+    if (!s->done && R.refused(out[0], tol2)) {
       s->status = INS2D_ENOTCONV;
-      s->rr = R.q;
+      s->rr = R.miss / s->rr0;
       s->done = 1;
     }
     set_cond(cond, !s->done && 0 < cond.limit);
@@ -677,7 +677,7 @@ __global__ void __launch_bounds__(kVecThreads) k_update_f(const PcgWork W, const
   if (grid_reduce<4>(q, ops, red_of(W), out)) {
     PcgScalars *s = W.sc;
     s->it += 1;
-    s->rr = out[0] / s->rr0 + s->irr;
+    s->rr = (out[0] + s->add) / s->rr0;
     s->maxx = out[1];
     s->minx = out[2];
     s->maxres = out[3];

@@ -192,6 +192,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   extern __shared__ __align__(16) double sm[];
   __shared__ double warp_part[4][kWarps];
   __shared__ __align__(16) double part2[2][kC][4], part4[2][kC][4];
+  // of the first pass: the sum over the null mode's w (in its block) and what follows
+  __shared__ double wsum;
   __shared__ RhsRange range;
   __shared__ DirRows dm, ds;  // along the modes' and the systems' direction
   cg::cluster_group cl = cg::this_cluster();
@@ -230,6 +232,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   else if (tid >= kThreads / 2 && tid - kThreads / 2 < nl)
     load_dir(ds, tid - kThreads / 2, xm ? P.TY : P.TX, xm ? P.MY : P.MX, xm ? P.hy : P.hx, s0 + tid - kThreads / 2,
              div, xm ? P.bc.uLe_i : P.bc.vLo_i, xm ? P.bc.uRi_i : P.bc.vUp_i);
+  if (tid == 0) range = RhsRange::none();
   // zero padding of the products' right operands
   for (int k = tid; k < (int)nc; k += kThreads) {
     r[k] = 0.0;
@@ -303,7 +306,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     status = INS2D_ENONFINITE;
     done = true;
   }
-  const int op1[1] = {R_SUM}, opz[2] = {R_SUM, R_SUM};
+  const int op1[1] = {R_SUM};
   if (QS) {
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     __syncthreads();
@@ -325,6 +328,13 @@ __global__ void __launch_bounds__(kThreads, 1)
       double y[kTriC];
 #pragma unroll
       for (int k = 0; k < kTriC; ++k) y[k] = lane * kTriC + k < n ? w[lane * kTriC + k] : 0.0;
+      if (it == 0 && b == F.null_mode) {
+        double ws = 0.0;
+#pragma unroll
+        for (int k = 0; k < kTriC; ++k) ws += y[k];
+        ws = tri_warp_sum(ws);
+        if (lane == 0) wsum = ws;
+      }
       if (b != b0 + warp) {
         TriTab<kTriC> t2;
         tri_tables<kTriC>(F, b, lane * kTriC, t2);
@@ -349,43 +359,40 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
     }
     cl.sync();
-    double az[2] = {0.0, 0.0};  // r'z and the sum of r (a packet holds two values)
+    // by a warp that has no fragment of the product on small grids
+    if (it == 0 && F.null_mode >= 0 && tid == kThreads - 1)
+      range = RhsRange::of(*cl.map_shared_rank(&wsum, F.null_mode / g.nb) * F.mean_w, (double)nm * n, rr0, tol2);
+    double a1[1] = {0.0};
     product<false>(g, basis, zh, [&](int m, int sl, double v0, double v1) {
       if (m >= nm || sl >= nl) return;
       const int k = m * ld + sl;
       z[k] = v0;
-      az[0] += r[k] * v0;
-      az[1] += r[k];
+      a1[0] += r[k] * v0;
       if (sl == 0) cl.map_shared_rank(zhalo, br)[g.mp + m] = v0;
       if (sl + 1 < nl) {
         z[k + 1] = v1;
-        az[0] += r[k + 1] * v1;
-        az[1] += r[k + 1];
+        a1[0] += r[k + 1] * v1;
       }
       if (sl + 2 >= nl) cl.map_shared_rank(zhalo, bl)[m] = sl + 1 < nl ? v1 : v0;
     });
-    cluster_reduce<2>(cl, az, opz, warp_part, part2, slot2);
-    if (!isfinite(az[0])) {
+    cluster_reduce<1>(cl, a1, op1, warp_part, part2, slot2);
+    if (!isfinite(a1[0])) {
       status = INS2D_ENONFINITE;
       break;
     }
     const bool first = it == 0;
-    if (first) {  // read after the next barriers
-      const bool singular = F.null_mode >= 0;
-      if (tid == 0) range = singular ? RhsRange::of(az[1], (double)nm * n, rr0, tol2) : RhsRange::none();
-      if (singular && RhsRange::refused(az[1], (double)nm * n, rr0, tol2)) {
-        status = INS2D_ENOTCONV;
-        break;
-      }
+    if (first && range.refused(rr0, tol2)) {
+      status = INS2D_ENOTCONV;
+      break;
     }
-    const double beta = first ? 0.0 : az[0] / rz;
-    rz = az[0];
+    const double beta = first ? 0.0 : a1[0] / rz;
+    rz = a1[0];
     // p = z + beta p, with the neighbouring columns'
     for (int k = tid; k < (int)nc; k += kThreads) p[k] = first ? z[k] : z[k] + beta * p[k];
     for (int k = tid; k < 2 * g.mp; k += kThreads) ph[k] = first ? zhalo[k] : zhalo[k] + beta * ph[k];
     __syncthreads();
     // q = A p, p'q
-    double a1[1] = {0.0};
+    a1[0] = 0.0;
 #pragma unroll 2
     for (int l = tid; l < nslots; l += kThreads) {
       int m, sl;
@@ -431,7 +438,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
     cluster_reduce<4>(cl, a4, op4, warp_part, part4, slot4);
     ++it;
-    rr = a4[0] / rr0 + range.irr;
+    rr = (a4[0] + range.add(rr0, tol2)) / rr0;
     maxx = a4[1];
     minx = a4[2];
     maxres = a4[3];
@@ -459,7 +466,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   if (c == 0 && tid == 0) {
     PcgScalars *out = W.sc;
     out->rr0 = rr0;
-    out->rr = it == 0 && status == INS2D_ENOTCONV ? range.q : rr;
+    out->rr = it == 0 && status == INS2D_ENOTCONV ? range.miss / rr0 : rr;
     out->it = it;
     out->maxx = maxx;
     out->minx = minx;
