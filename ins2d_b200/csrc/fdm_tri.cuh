@@ -44,10 +44,14 @@ __device__ __forceinline__ void tri_tables(const FdmD &F, int b, int s0, TriTab<
 // barriers) by W warps; wr: this warp's place among them.  y: the lane's C
 // values of w_b from unknown s0 = (32 wr + lane) C (zero outside), replaced by
 // those of zh_b.  sh: 4 doubles per warp of the block, unused (may be null)
-// for W == 1, which has no block-level synchronisation.
-template <int W, int C>
+// for W == 1, which has no block-level synchronisation.  on_sum(the warp's sum
+// over w_b) is called for the null mode.
+struct TriNoSum {
+  __device__ void operator()(double) const {}
+};
+template <int W, int C, class OnSum = TriNoSum>
 __device__ __forceinline__ void tri_solve(const FdmD &F, int b, int wr, const TriTab<C> &T, double (&y)[C],
-                                          double (*sh)[4]) {
+                                          double (*sh)[4], OnSum on_sum = OnSum()) {
   constexpr unsigned ALL = 0xffffffffu;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, w0 = warp - wr;  // w0: the row's first warp
   const int n = F.n, s0 = (wr * 32 + lane) * C;
@@ -67,6 +71,7 @@ __device__ __forceinline__ void tri_solve(const FdmD &F, int b, int wr, const Tr
     }
     sum = tri_warp_sum(sum);
     part = tri_warp_sum(part);
+    on_sum(sum);
   }
   if constexpr (W > 1) {
     if (lane == 0) {

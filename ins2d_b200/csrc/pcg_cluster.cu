@@ -192,7 +192,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   extern __shared__ __align__(16) double sm[];
   __shared__ double warp_part[4][kWarps];
   __shared__ __align__(16) double part2[2][kC][4], part4[2][kC][4];
-  // of the first pass: the sum over the null mode's w (in its block) and what follows
+  // the sum over the null mode's w, as its block sends it, and what follows from the
+  // first pass's (kept here: 20 bytes of spills made ten steps 28 us longer)
   __shared__ double wsum;
   __shared__ RhsRange range;
   __shared__ DirRows dm, ds;  // along the modes' and the systems' direction
@@ -328,19 +329,14 @@ __global__ void __launch_bounds__(kThreads, 1)
       double y[kTriC];
 #pragma unroll
       for (int k = 0; k < kTriC; ++k) y[k] = lane * kTriC + k < n ? w[lane * kTriC + k] : 0.0;
-      if (it == 0 && b == F.null_mode) {
-        double ws = 0.0;
-#pragma unroll
-        for (int k = 0; k < kTriC; ++k) ws += y[k];
-        ws = tri_warp_sum(ws);
-        if (lane == 0) wsum = ws;
-      }
       if (b != b0 + warp) {
         TriTab<kTriC> t2;
         tri_tables<kTriC>(F, b, lane * kTriC, t2);
         tri_solve<1, kTriC>(F, b, 0, t2, y, nullptr);
       } else {
-        tri_solve<1, kTriC>(F, b, 0, tab, y, nullptr);
+        tri_solve<1, kTriC>(F, b, 0, tab, y, nullptr, [&](double s) {
+          if (lane < kC) *cl.map_shared_rank(&wsum, lane) = s;  // the first pass's is read
+        });
       }
       // back through the row, so that consecutive lanes send consecutive values
 #pragma unroll
@@ -361,7 +357,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     cl.sync();
     // by a warp that has no fragment of the product on small grids
     if (it == 0 && F.null_mode >= 0 && tid == kThreads - 1)
-      range = RhsRange::of(*cl.map_shared_rank(&wsum, F.null_mode / g.nb) * F.mean_w, (double)nm * n, rr0, tol2);
+      range = RhsRange::of(wsum * F.mean_w, (double)nm * n, rr0, tol2);
     double a1[1] = {0.0};
     product<false>(g, basis, zh, [&](int m, int sl, double v0, double v1) {
       if (m >= nm || sl >= nl) return;
