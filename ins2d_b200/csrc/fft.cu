@@ -1188,8 +1188,9 @@ cudaError_t fft_passes(const DevOps &P, const FftPlan &plan, const double *src, 
   if (!fy) {
     const int G = cols_group(Ly, H, P.nsm);
     const size_t smy = 2 * (size_t)G * line_ld(Ly.m) * sizeof(double2);
-    k_cols<<<(H + G - 1) / G, line_threads(Ly, G, (H + G - 1) / G, P.nsm), smy, s>>>(Ly, H, G, plan.twy, P.fft_ax, P.fft_ay, P.fft_dxdy,
-                                                            plan.spec, maxbits, skip);
+    const int blocks = (H + G - 1) / G;
+    k_cols<<<blocks, line_threads(Ly, G, blocks, P.nsm), smy, s>>>(Ly, H, G, plan.twy, P.fft_ax, P.fft_ay, P.fft_dxdy,
+                                                                   plan.spec, maxbits, skip);
   }
   // rows, half spectrum -> real
   const bool fx2 = with_log2<kFusedMinLog>(plan.logx, [&](auto c) {
@@ -1201,7 +1202,7 @@ cudaError_t fft_passes(const DevOps &P, const FftPlan &plan, const double *src, 
   });
   if (!fx2)
     k_rows_c2r<<<pairs, line_threads(Lx, 1, pairs, P.nsm), smx, s>>>(Lx, Ny, plan.twx, plan.spec, dp, accumulate ? 1 : 0,
-                                                       gate ? gate : maxbits, skip);
+                                                                     gate ? gate : maxbits, skip);
   return cudaSuccess;
 }
 }  // namespace

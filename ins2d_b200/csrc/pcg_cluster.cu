@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   __shared__ double warp_part[4][kWarps];
   __shared__ __align__(16) double part2[2][kC][4], part4[2][kC][4];
   // the sum over the null mode's w, as its block sends it, and what follows from the
-  // first pass's (kept here: 20 bytes of spills made ten steps 28 us longer)
+  // first pass's (tests of it made here once spilled 24 bytes: ten steps 28 us longer)
   __shared__ double wsum;
   __shared__ RhsRange range;
   __shared__ DirRows dm, ds;  // along the modes' and the systems' direction
